@@ -5,15 +5,14 @@
 // 2-byte symbols to build_small_texts, grouped by alphabet size.  Built one
 // by one, such texts cost a few hundred CUDA calls each (launches, pool
 // allocations, small copies, synchronisations) for very little GPU work.
-// Here a group of G texts is built as one tree whose top a0 = ceil(log2 G)
-// levels are the text number: the concatenated texts are that tree's
-// level-a0 order, its level a0 + j holds every text's level j side by side,
-// and one run of the pass pipeline (passes.cuh) writes all of them.  One
-// launch then cuts each of those levels into the texts' own arrays, laid out
-// back to back in one shared RankSelect store; one launch of each RankSelect
-// kernel (counts, select samples, rank blocks) covers every array of every
-// text, one launch counts every text's symbols and one computes every
-// node-start rank.
+// Here the G texts of a group are concatenated and run through the bit-plane
+// passes (planes.cuh) once, every text a node of its own, so each of the
+// passes' levels holds every text's level side by side.  One launch then
+// cuts each of those levels into the texts' own arrays, laid out back to
+// back in one shared RankSelect store; one launch of each RankSelect kernel
+// (counts, select samples, rank blocks) covers every array of every text,
+// the passes' class starts are every text's symbol counts, and one launch
+// computes every node-start rank.
 //
 // Every text still gets its own tree with the exports and answers of a
 // single build (same level bits, counts, samples and node ranks): its
@@ -28,7 +27,7 @@
 #include <vector>
 
 #include "internal.cuh"
-#include "passes.cuh"
+#include "planes.cuh"
 
 namespace ewt {
 namespace {
@@ -55,53 +54,6 @@ struct SharedStore {
     }
   }
 };
-
-// Level a0 of the group tree (every text's level 0): the top bit of each
-// of the n concatenated symbols, 32 per word; symbols at or above 2^L set
-// bit 0 of err.
-template <class T>
-__global__ void __launch_bounds__(256)
-concat_level0_kernel(T const* __restrict__ x, uint64_t n, uint32_t L,
-                     uint32_t* __restrict__ words, uint32_t* __restrict__ err) {
-  uint64_t const nw = (n + 31) / 32;
-  uint64_t const stride = uint64_t(gridDim.x) * blockDim.x;
-  uint32_t bad = 0;
-  for (uint64_t w = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; w < nw;
-       w += stride) {
-    uint64_t const p0 = w * 32;
-    uint32_t const cnt = static_cast<uint32_t>(min(uint64_t(32), n - p0));
-    uint32_t bits = 0;
-    if (cnt == 32) {
-      // 32 symbols: 32 * sizeof(T) bytes at a 32-byte aligned offset
-      constexpr uint32_t kU = 32 * sizeof(T) / 16;
-      uint4 const* v = reinterpret_cast<uint4 const*>(x + p0);
-#pragma unroll
-      for (uint32_t u = 0; u < kU; ++u) {
-        uint4 const q = v[u];
-        uint32_t const wd[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-        for (uint32_t j = 0; j < 4; ++j) {
-#pragma unroll
-          for (uint32_t h = 0; h < 4 / sizeof(T); ++h) {
-            uint32_t const s = (wd[j] >> (8 * sizeof(T) * h)) &
-                               (sizeof(T) == 1 ? 0xFFu : 0xFFFFu);
-            uint32_t const i = (u * 4 + j) * (4 / sizeof(T)) + h;
-            bad |= s >> L;
-            bits |= ((s >> (L - 1)) & 1u) << i;
-          }
-        }
-      }
-    } else {
-      for (uint32_t i = 0; i < cnt; ++i) {
-        uint32_t const s = x[p0 + i];
-        bad |= s >> L;
-        bits |= ((s >> (L - 1)) & 1u) << i;
-      }
-    }
-    words[w] = bits;
-  }
-  if (bad) atomicOr(err, 1u);
-}
 
 // One text's level: `bits` bits from bit src_shift of word src_word of the
 // group level go to word dst_word onwards of the shared store.  `first`:
@@ -133,35 +85,6 @@ split_levels_kernel(uint32_t const* __restrict__ src, uint32_t* __restrict__ dst
   }
 }
 
-// Symbol counts of every text: a job is a stretch of at most 65536 symbols
-// of one text, counted in shared memory (sigma bins) and added to
-// occ[text * sigma + symbol].
-struct HistJob {
-  uint64_t start;
-  uint32_t len, text;
-};
-
-template <class T>
-__global__ void __launch_bounds__(256)
-group_hist_kernel(T const* __restrict__ x, HistJob const* __restrict__ jobs,
-                  uint32_t njobs, uint32_t sigma,
-                  unsigned long long* __restrict__ occ) {
-  extern __shared__ uint32_t h[];
-  for (uint32_t jb = blockIdx.x; jb < njobs; jb += gridDim.x) {
-    HistJob const j = jobs[jb];
-    for (uint32_t s = threadIdx.x; s < sigma; s += blockDim.x) h[s] = 0;
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < j.len; i += blockDim.x) {
-      uint32_t const s = x[j.start + i];
-      if (s < sigma) atomicAdd(&h[s], 1u);  // larger ones were reported
-    }
-    __syncthreads();
-    for (uint32_t s = threadIdx.x; s < sigma; s += blockDim.x)
-      if (h[s]) atomicAdd(&occ[uint64_t(j.text) * sigma + s], h[s]);
-    __syncthreads();
-  }
-}
-
 // rank0 at a node start (precomputeRanksKernel, wavelet_tree.cuh:332-352):
 // out[i] = zeros of array `array` before position `pos`.
 struct RankJob {
@@ -179,26 +102,6 @@ node_rank_jobs_kernel(RSView v, RankJob const* __restrict__ jobs, uint64_t njobs
     ArrayMeta const m = v.meta[j.array];
     out[j.out] = j.pos - ecl::detail::rs_rank1<false>(v, m, j.pos, nullptr);
   }
-}
-
-uint32_t log2_ceil(uint64_t g) {
-  uint32_t a = 0;
-  while ((uint64_t(1) << a) < g) ++a;
-  return a;
-}
-
-// The start level of the pass pipeline's last pass for a group tree of
-// levels a0 .. a0 + L - 1 (as run_pass_pipeline plans it).
-uint32_t last_pass_start(uint32_t a0, uint32_t L) {
-  uint32_t const levels = L - 1;
-  if (levels == 0) return a0;
-  uint32_t const np = (levels + kPMaxK - 1) / kPMaxK;
-  uint32_t a = a0, last = a0;
-  for (uint32_t i = 0; i < np; ++i) {
-    last = a;
-    a += levels / np + (i < levels % np ? 1u : 0u);
-  }
-  return last;
 }
 
 size_t round_up(size_t x) { return (x + 255) / 256 * 256; }
@@ -223,15 +126,9 @@ void build_group(void const* const* texts, uint64_t const* lengths,
   for (uint32_t g = 0; g < G; ++g)
     EWT_CUDA(cudaMemcpyAsync(x.as<T>() + off[g], texts[ids[g]],
                              lengths[ids[g]] * sizeof(T), cudaMemcpyDefault, st));
-  // ---- the group tree: text number above the symbol, a0 + L levels
-  uint32_t const a0 = log2_ceil(G);
-  uint32_t const Lg = a0 + L;
-  std::vector<uint64_t> c_host((uint64_t(1) << Lg) + 1, 0);
-  for (uint64_t t = 0; t < (uint64_t(1) << a0); ++t)
-    c_host[t << L] = t < G ? off[t] : N;
-  c_host.back() = N;
-  DevBuf c_d(c_host.size() * 8);
-  EWT_CUDA(cudaMemcpyAsync(c_d.get(), c_host.data(), c_host.size() * 8,
+  // ---- one run of the plane passes, a node per text
+  DevBuf starts(off.size() * 8), c_d((uint64_t(G) * sigma + 1) * 8);
+  EWT_CUDA(cudaMemcpyAsync(starts.get(), off.data(), off.size() * 8,
                            cudaMemcpyHostToDevice, st));
   uint64_t const stride_w = ceil_div(N, 32) + 64;  // words per group level
   DevBuf lw(L * stride_w * 4);
@@ -239,19 +136,16 @@ void build_group(void const* const* texts, uint64_t const* lengths,
   DevBuf err(16);
   EWT_CUDA(cudaMemsetAsync(err.get(), 0, 16, st));
   uint32_t* const words = lw.as<uint32_t>();
-  concat_level0_kernel<T><<<static_cast<uint32_t>(std::max<uint64_t>(
-                                1, std::min<uint64_t>(ceil_div(ceil_div(N, 32), 256),
-                                                      uint64_t(sms) * 8))),
-                            256, 0, st>>>(x.as<T>(), N, L, words,
-                                          err.as<uint32_t>());
-  EWT_LAUNCHED();
-  std::vector<uint64_t> woff(Lg, 0), wbits(Lg, 0);
-  for (uint32_t j = 0; j < L; ++j) {
-    woff[a0 + j] = j * stride_w;
-    wbits[a0 + j] = N;
-  }
-  run_pass_pipeline<T>(x.as<T>(), N, Lg, a0, words, woff.data(), wbits.data(),
-                       c_d.as<uint64_t>(), err.as<uint32_t>() + 1, st);
+  std::vector<uint32_t*> wp(L);
+  std::vector<uint64_t> wc(L, ceil_div(N, 32));
+  for (uint32_t j = 0; j < L; ++j) wp[j] = words + j * stride_w;
+  PlaneText<T> pt;
+  pt.sym = x.as<T>();
+  pt.n = N;
+  pt.L = L;
+  pt.nodes = G;
+  pt.starts = starts.as<uint64_t>();
+  run_plane_passes<T>(pt, wp.data(), wc.data(), c_d.as<uint64_t>(), {}, err.as<uint32_t>(), st);
   // ---- every text's arrays in one store; cut the group levels into them
   std::vector<uint64_t> bits;
   bits.reserve(uint64_t(G) * L);
@@ -289,36 +183,15 @@ void build_group(void const* const* texts, uint64_t const* lengths,
   build_rs_samples(rs, st);
   rs.skip_blocks.assign(arrays, 0);
   build_rank_blocks(rs, st);
-  // ---- symbol counts of every text
-  std::vector<HistJob> hj;
-  for (uint32_t g = 0; g < G; ++g)
-    for (uint64_t s0 = 0; s0 < lengths[ids[g]]; s0 += 65536)
-      hj.push_back({off[g] + s0,
-                    static_cast<uint32_t>(std::min<uint64_t>(65536, lengths[ids[g]] - s0)),
-                    g});
-  DevBuf hj_d(hj.size() * sizeof(HistJob));
-  EWT_CUDA(cudaMemcpyAsync(hj_d.get(), hj.data(), hj.size() * sizeof(HistJob),
-                           cudaMemcpyHostToDevice, st));
-  DevBuf occ_d(uint64_t(G) * sigma * 8);
-  EWT_CUDA(cudaMemsetAsync(occ_d.get(), 0, uint64_t(G) * sigma * 8, st));
-  group_hist_kernel<T><<<static_cast<uint32_t>(std::min<uint64_t>(
-                             hj.size(), uint64_t(sms) * 8)),
-                         256, sigma * 4, st>>>(x.as<T>(), hj_d.as<HistJob>(),
-                                               static_cast<uint32_t>(hj.size()),
-                                               static_cast<uint32_t>(sigma),
-                                               occ_d.as<unsigned long long>());
-  EWT_LAUNCHED();
-  std::vector<uint64_t> occ(uint64_t(G) * sigma);
+  // ---- symbol counts of every text: the starts of its symbols
+  std::vector<uint64_t> c_host(uint64_t(G) * sigma + 1);
   uint32_t errs[4] = {0, 0, 0, 0};
-  EWT_CUDA(cudaMemcpyAsync(occ.data(), occ_d.get(), occ.size() * 8,
+  EWT_CUDA(cudaMemcpyAsync(c_host.data(), c_d.get(), c_host.size() * 8,
                            cudaMemcpyDeviceToHost, st));
   EWT_CUDA(cudaMemcpyAsync(errs, err.get(), 16, cudaMemcpyDeviceToHost, st));
   EWT_CUDA(cudaStreamSynchronize(st));
   EWT_REQUIRE(!(errs[0] & 1), EWT_ERR_ALPHABET,
               "a text holds a symbol above its alphabet's last symbol");
-  EWT_REQUIRE(errs[1] == 0, EWT_ERR_CUDA,
-              "internal consistency check failed while building levels (kind " +
-                  std::to_string(errs[1]) + ")");
   // ---- per-tree shape, counts and small tables
   std::vector<std::unique_ptr<ewt_tree>> trees(G);
   struct Slot {
@@ -338,10 +211,13 @@ void build_group(void const* const* texts, uint64_t const* lengths,
     t->alphabet.resize(sigma);
     for (uint64_t i = 0; i < sigma; ++i) t->alphabet[i] = i;
     set_tree_shape(*t);
-    t->occ.assign(occ.begin() + uint64_t(g) * sigma,
-                  occ.begin() + uint64_t(g + 1) * sigma);
-    t->counts.assign(sigma, 0);
-    for (uint64_t i = 1; i < sigma; ++i) t->counts[i] = t->counts[i - 1] + t->occ[i - 1];
+    uint64_t const* const cg = c_host.data() + uint64_t(g) * sigma;
+    t->counts.resize(sigma);
+    t->occ.resize(sigma);
+    for (uint64_t i = 0; i < sigma; ++i) {
+      t->counts[i] = cg[i] - cg[0];
+      t->occ[i] = cg[i + 1] - cg[i];
+    }
     t->level_bits.assign(L, t->n);
     Slot& s = slots[g];
     s.counts = tb; tb += round_up((sigma + 1) * 8);
@@ -462,11 +338,10 @@ void build_small_texts(void const* const* texts, uint64_t const* lengths,
                        std::vector<uint32_t> const& ids, int elem_size,
                        uint32_t L, int gpu, ewt_tree** out) {
   DeviceGuard g(gpu);
-  // groups of at most 2^(kPMaxStartLevel - start of the last pass) texts,
-  // so that every pass of the group tree starts at a supported level
-  uint32_t const span = last_pass_start(0, L);
-  uint32_t const max_a0 = kPMaxStartLevel >= span ? kPMaxStartLevel - span : 0;
-  size_t const per = size_t(1) << std::min<uint32_t>(max_a0, 16);
+  // at most 2^12 texts a group, fewer when the later passes would start with
+  // more than 2^16 nodes
+  uint32_t const last = L - 1 - plan_plane_passes(L).back();
+  size_t const per = size_t(1) << std::min<uint32_t>(12, 16 - last);
   for (size_t s0 = 0; s0 < ids.size(); s0 += per) {
     std::vector<uint32_t> part(ids.begin() + s0,
                                ids.begin() + std::min(ids.size(), s0 + per));

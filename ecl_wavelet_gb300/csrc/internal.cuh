@@ -60,12 +60,7 @@ void build_dense_samples(RSStore& rs, uint32_t shift, cudaStream_t stream);
 struct GroupStore {
   std::vector<ecl::detail::GroupLevel> levels;  // host copy
   DevBuf blocks, sb, ds, node_ranks, levels_d;
-  // transient, during a build: the symbols in level-`order_level` order as
-  // the first pass wrote them, for the octal group level starting there
-  DevBuf order;
-  uint32_t order_level = 0;
   uint32_t sel_shift = ecl::detail::kDefaultSelShift;
-  bool level0_built = false;  // octal level 0 written with the binary level 0
   ecl::detail::GroupView view() const;
   uint64_t bytes() const {
     return blocks.bytes() + sb.bytes() + ds.bytes() + node_ranks.bytes() +
@@ -270,18 +265,12 @@ bool groups_eligible(ewt_tree const& t);
 // Digit widths of the group levels of an L-level tree, top down: octal (3)
 // groups, then one or two quad (2) groups; they cover all L levels.
 std::vector<uint32_t> group_widths(uint32_t L);
-// sym: the tree's minimal symbols on the device (elem_size bytes each), or
-// null; level 0 is then built from them directly.
-void build_groups(ewt_tree& t, std::vector<uint64_t> const& C, void const* sym,
-                uint32_t elem_size, cudaStream_t st);
-// Octal level 0 from the minimal symbols (1- or 2-byte) before the other
-// levels exist: lays out the group levels, writes the octal level-0 blocks
-// and the binary level 0 (`level0`, its words) in one read of the symbols,
-// and reports symbols >= 2^L in err bit 0 when `check`; build_groups finishes
-// the level.
-bool octal_text_eligible(ewt_tree const& t, uint32_t elem_size);
-void build_octal_level0(ewt_tree& t, void const* sym, uint32_t elem_size,
-                        uint32_t* level0, bool check, uint32_t* err, cudaStream_t st);
+// The planes every group level needs below its first level: (level, planes).
+std::vector<std::pair<uint32_t, uint32_t>> group_planes(uint32_t L);
+// planes[i]: group level i's bit planes in the order of its first level, the
+// digit's highest bit (the binary level) first, zero past position n.
+void build_groups(ewt_tree& t, std::vector<uint64_t> const& C,
+                  std::vector<std::vector<uint32_t const*>> const& planes, cudaStream_t st);
 void build_group_samples(ewt_tree& t, uint32_t shift, cudaStream_t st);
 // Dense select samples of the binary and group levels at rate 2^shift (0:
 // none), and the tree's view updated.

@@ -9,8 +9,10 @@
 //   3. a non-minimal alphabet is remapped to 0..sigma-1 (:170-227); a
 //      non-power-of-two alphabet also gets a histogram (its short codes
 //      make level sizes depend on symbol counts, :776-790);
-//   4. level 0 bits are packed from the text; then for every level l:
-//      RankSelect counts of level l; the node kernel computes rank0 at every
+//   4. power-of-two alphabets of 1- and 2-byte symbols: all levels by
+//      bit-plane passes (planes.cuh), then the counts of all levels and the
+//      node-start ranks in one launch each.  Other alphabets: level 0 bits
+//      are packed from the text; then for every level l: RankSelect counts of level l; the node kernel computes rank0 at every
 //      node start of level l (precomputeRanksKernel, :332-352) and from it
 //      the count table C at each node's split point (zeros of a node =
 //      rank0(end) - rank0(start)), so no histogram pass is needed for
@@ -437,55 +439,76 @@ level_nodes_kernel(TreeView t, LevelNode const* __restrict__ nodes,
 }  // namespace
 }  // namespace ewt
 
+#include "planes.cuh"
 #include "split.cuh"
-#include "passes.cuh"
 
 namespace ewt {
 namespace {
 
-// Levels 1 .. L-1 of a power-of-two alphabet by multi-level passes (see
-// passes.cuh); level 0 is already written (or, with an ingested text,
-// written by the first pass).
+// rank0 at every node start of a power-of-two tree (nodes g = 1 .. 2^l - 1 of
+// level l = 1 + blockIdx.y start at symbol g << (L - l)), checked against the
+// count table: a node's zeros are the symbols below its split.
+__global__ void __launch_bounds__(128)
+pow2_node_ranks_kernel(TreeView t, uint64_t* __restrict__ ranks, uint32_t* __restrict__ err) {
+  uint32_t const l = 1 + blockIdx.y;
+  uint64_t const nodes = uint64_t(1) << l;
+  uint64_t const g = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
+  if (g >= nodes) return;
+  ArrayMeta const m = t.rs.meta[l];
+  uint32_t const sh = t.levels - l;
+  uint64_t const* C = t.counts;
+  uint64_t const ps = C[g << sh], pe = g + 1 < nodes ? C[(g + 1) << sh] : t.n;
+  uint64_t const r0 = ps - ecl::detail::rs_rank1<false>(t.rs, m, ps, nullptr);
+  uint64_t const r1 = pe - ecl::detail::rs_rank1<false>(t.rs, m, pe, nullptr);
+  if (r1 - r0 != C[(2 * g + 1) << (sh - 1)] - ps) atomicOr(err, 2u);
+  if (g) ranks[t.node_base[l] + g - 1] = r0;
+}
+
+// Planes l+1 .. l+count of a level order held as symbols (bits L-2-l ..),
+// 32 positions per warp and step.
 template <class T>
-void run_passes(ewt_tree& t, T const* sym, uint64_t n, uint32_t* err,
-                cudaStream_t st, T const* ingest_src = nullptr,
-                bool ingest_copy = false, bool group_order = false) {
-  uint32_t* const words = t.rs.words.as<uint32_t>();
-  uint64_t const w1 = t.rs.meta[1].word_off;
-  EWT_CUDA(cudaMemsetAsync(words + w1, 0, (t.rs.total_words - w1) * 4, st));
-  std::vector<uint64_t> off(t.L), bits(t.L);
-  for (uint32_t l = 0; l < t.L; ++l) {
-    off[l] = t.rs.meta[l].word_off;
-    bits[l] = t.rs.meta[l].bits;
-  }
-  // With octal group levels at 0 and 3 and at most four levels after level
-  // 3, the first pass covers levels 1-3 and hands its level-3 order to the
-  // group build, which reads octal level 3 straight from those symbols
-  // instead of routing levels 4 and 5 into level-3 order.
-  uint32_t first_k = 0;
-  DevBuf* keep = nullptr;
-  t.groups.order.reset();
-  t.groups.order_level = 0;
-  if (group_order) {
-    std::vector<uint32_t> const w = group_widths(t.L);
-    if (w.size() >= 2 && w[0] == 3 && w[1] == 3 && t.L >= 5 && t.L - 4 <= kPMaxK) {
-      first_k = 3;
-      keep = &t.groups.order;
+__global__ void __launch_bounds__(256)
+order_planes_kernel(T const* __restrict__ x, uint64_t n, uint32_t L, uint32_t l,
+                    uint32_t count, uint32_t* __restrict__ out, uint64_t stride) {
+  uint32_t const lane = threadIdx.x & 31;
+  uint64_t const words = (n + 31) / 32, step = uint64_t(gridDim.x) * (blockDim.x / 32);
+  for (uint64_t w = (blockIdx.x * uint64_t(blockDim.x) + threadIdx.x) / 32; w < words;
+       w += step) {
+    uint64_t const at = w * 32 + lane;
+    uint64_t const c = at < n ? uint64_t(x[at]) : 0;
+    for (uint32_t j = 0; j < count; ++j) {
+      uint32_t const v = __ballot_sync(0xffffffffu, (c >> (L - 2 - l - j)) & 1);
+      if (lane == 0) out[j * stride + w] = v;
     }
   }
-  run_pass_pipeline<T>(sym, n, t.L, 0, words, off.data(), bits.data(),
-                       t.counts_d.as<uint64_t>(), err, st, ingest_src,
-                       ingest_copy, first_k, keep);
-  if (keep && t.groups.order.get()) t.groups.order_level = 3;
+}
+
+// Levels 0 .. L-1 of a power-of-two alphabet of 1- or 2-byte symbols by
+// bit-plane passes (planes.cuh); returns the deeper planes that the group
+// levels read.
+template <class T>
+std::vector<OrderPlanes> run_passes(ewt_tree& t, PlaneText<T> const& x, bool groups,
+                                    uint32_t* err, cudaStream_t st) {
+  uint32_t* const words = t.rs.words.as<uint32_t>();
+  std::vector<uint32_t*> out(t.L);
+  std::vector<uint64_t> count(t.L);
+  for (uint32_t l = 0; l < t.L; ++l) {
+    out[l] = words + t.rs.meta[l].word_off;
+    count[l] = ceil_div(t.rs.meta[l].bits, 32);
+  }
+  if (t.L > 1) {
+    uint64_t const w1 = t.rs.meta[1].word_off;
+    EWT_CUDA(cudaMemsetAsync(words + w1, 0, (t.rs.total_words - w1) * 4, st));
+  }
+  return run_plane_passes<T>(x, out.data(), count.data(), t.counts_d.as<uint64_t>(),
+                             groups ? group_planes(t.L)
+                                    : std::vector<std::pair<uint32_t, uint32_t>>{},
+                             err, st);
 }
 
 thread_local bool t_texts_synced = false;
 thread_local bool t_batch_member = false;
 
-// Whether a host text goes straight to the first pass's ingest kernel
-// (kernels read the host text: a Grace host's pageable memory, or pinned
-// memory): 1- and 2-byte symbols, a given minimal power-of-two alphabet of at
-// least four symbols, a 16-byte aligned text.
 // A given alphabet 0 .. sigma-1 with sigma a power of two >= 4 (1- and
 // 2-byte symbols): the texts whose first pass can read them directly.
 template <class T>
@@ -501,6 +524,9 @@ bool minimal_pow2_alphabet(const void* alphabet, uint64_t sigma) {
   }
 }
 
+// Whether a host text goes straight to the ingest kernel (kernels read the
+// host text: a Grace host's pageable memory, or pinned memory): such an
+// alphabet and a 16-byte aligned text.
 template <class T>
 bool host_ingest(const void* data, uint64_t n, const void* alphabet, uint64_t sigma) {
   if constexpr (sizeof(T) > 2) {
@@ -527,8 +553,7 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
   // ---- text on the device
   DevBuf text_owned;
   T const* d_text;
-  T const* ingest = nullptr;  // text read by the first pass's ingest kernel
-  bool ingest_copy = false;   // ... a host text, copied by it
+  bool host_text = false;  // the ingest kernel reads the text in host memory
   bool const on_device = is_device_pointer(data);
   // The text may still be in flight on the caller's streams; the build runs
   // on its own stream, so order it after all prior device work (once per
@@ -543,11 +568,8 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
                              cudaMemcpyDeviceToDevice, st));
     d_text = text_owned.as<T>();
   } else if (host_ingest<T>(data, n, alphabet, sigma)) {
-    // read by the first pass's ingest kernel (see run_passes)
-    text_owned.alloc(n * sizeof(T) + 64);
-    d_text = text_owned.as<T>();
-    ingest = static_cast<T const*>(data);
-    ingest_copy = true;
+    d_text = static_cast<T const*>(data);
+    host_text = true;
   } else {
     text_owned.alloc(n * sizeof(T));
     PhaseTimer pt(EWT_PHASE_H2D, st);
@@ -596,7 +618,6 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
   // ---- shape
   set_tree_shape(t);
   uint32_t const L = t.L;
-  auto const level_nodes = make_level_nodes(sigma, L);
 
   // ---- device tables
   t.err_d.alloc(kTreeErrBytes);
@@ -605,19 +626,37 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
   uint32_t const grid_stream =
       static_cast<uint32_t>(std::min<uint64_t>(ceil_div(n, 256),
                                                uint64_t(sm_count()) * 8));
+  // Power-of-two alphabets of 1- and 2-byte symbols go through the bit-plane
+  // passes, which map symbols to codes as they read them.
+  bool const by_planes = sizeof(T) <= 2 && t.pow2;
+  auto const level_nodes = by_planes ? std::vector<std::vector<LevelNode>>{}
+                                     : make_level_nodes(sigma, L);
   DevBuf cur_buf;  // minimal symbols when the alphabet is not 0..sigma-1
+  DevBuf lut_d;
   T const* sym = d_text;
   if (!t.is_min) {
     std::vector<T> a(t.alphabet.begin(), t.alphabet.end());
     t.alphabet_d.alloc(sigma * sizeof(T));
     EWT_CUDA(cudaMemcpyAsync(t.alphabet_d.get(), a.data(), sigma * sizeof(T),
                              cudaMemcpyHostToDevice, st));
-    cur_buf.alloc(n * sizeof(T));
-    PhaseTimer pt(EWT_PHASE_HIST, st);
-    remap_kernel<T><<<grid_stream, 256, 0, st>>>(
-        d_text, n, t.alphabet_d.as<T>(), sigma, cur_buf.as<T>(), err_build);
-    EWT_LAUNCHED();
-    sym = cur_buf.as<T>();
+    if (by_planes) {
+      // symbol -> rank of the first alphabet symbol at or above it
+      std::vector<uint16_t> lut(sizeof(T) == 1 ? 256 : 65536, 0);
+      uint64_t v = 0;
+      for (uint64_t i = 0; i < sigma; ++i)
+        for (; v <= t.alphabet[i] && v < lut.size(); ++v) lut[v] = static_cast<uint16_t>(i);
+      lut_d.alloc(lut.size() * 2);
+      EWT_CUDA(cudaMemcpyAsync(lut_d.get(), lut.data(), lut.size() * 2,
+                               cudaMemcpyHostToDevice, st));
+      EWT_CUDA(cudaStreamSynchronize(st));  // `lut` leaves scope
+    } else {
+      cur_buf.alloc(n * sizeof(T));
+      PhaseTimer pt(EWT_PHASE_HIST, st);
+      remap_kernel<T><<<grid_stream, 256, 0, st>>>(
+          d_text, n, t.alphabet_d.as<T>(), sigma, cur_buf.as<T>(), err_build);
+      EWT_LAUNCHED();
+      sym = cur_buf.as<T>();
+    }
   }
   // Count table: exact histogram for non-power-of-two alphabets (their level
   // sizes need it); otherwise only C[0] = 0 and C[sigma] = n, the rest is
@@ -646,7 +685,7 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
     for (uint64_t i = 1; i <= sigma; ++i) c[i] = c[i - 1] + t.occ[i - 1];
     EWT_CUDA(cudaMemcpyAsync(t.counts_d.get(), c.data(), (sigma + 1) * 8,
                              cudaMemcpyHostToDevice, st));
-  } else {
+  } else if (!by_planes) {
     uint64_t const ends[2] = {0, n};
     EWT_CUDA(cudaMemcpyAsync(t.counts_d.get(), &ends[0], 8,
                              cudaMemcpyHostToDevice, st));
@@ -680,7 +719,7 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
                            cudaMemcpyHostToDevice, st));
   std::vector<LevelNode> flat;
   std::vector<uint64_t> lv_off(L + 1, 0);
-  for (uint32_t l = 0; l < L; ++l) {
+  for (uint32_t l = 0; l < L && !by_planes; ++l) {
     flat.insert(flat.end(), level_nodes[l].begin(), level_nodes[l].end());
     lv_off[l + 1] = flat.size();
   }
@@ -694,54 +733,49 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
   fill_tree_view(t);
   TreeView& v = t.view;
 
-  // ---- level 0 bits (with an ingested host text: written by the first pass)
   uint32_t* const words = t.rs.words.as<uint32_t>();
-  t.groups.level0_built = false;
   // Group query levels for power-of-two alphabets -- except for the short
   // texts of a batch build: the group build's launch latency would be most
   // of their build time; they get rank blocks on every level instead.
   bool const want_groups =
       groups_eligible(t) && !(t_batch_member && n < kBatchGroupMinSymbols);
-  if (!ingest && want_groups && octal_text_eligible(t, sizeof(T))) {
-    // level 0 is the octal level 0's top bit plane: both in one read
-    build_octal_level0(t, sym, sizeof(T), words + t.rs.meta[0].word_off, t.is_min,
-                       err_build, st);
-  } else if (!ingest) {
-    PhaseTimer pt(EWT_PHASE_FILL, st);
-    uint64_t const w0 = ceil_div(t.level_bits[0], 32);
-    uint32_t const blocks =
-        static_cast<uint32_t>(ceil_div(w0, uint64_t(256) * fill_words<T>()));
-    auto k = t.pow2 ? (t.is_min ? fill0_kernel<T, true, true>
-                                : fill0_kernel<T, true, false>)
-                    : (t.is_min ? fill0_kernel<T, false, true>
-                                : fill0_kernel<T, false, false>);
-    k<<<blocks, 256, 0, st>>>(sym, t.level_bits[0], L, sigma,
-                              words + t.rs.meta[0].word_off, err_build);
-    EWT_LAUNCHED();
-  }
-  // ---- levels
-  bool by_passes = false;
-  if constexpr (sizeof(T) <= 2) {
-    if (t.pow2 && L >= 2) {
-      run_passes<T>(t, sym, n, err_build, st, ingest, ingest_copy, want_groups);
-      by_passes = true;
+  std::vector<OrderPlanes> kept;  // deeper planes of the group levels' orders
+  if (by_planes) {
+    if constexpr (sizeof(T) <= 2) {
+      PlaneText<T> x;
+      x.sym = d_text;
+      x.n = n;
+      x.L = L;
+      if (!t.is_min) {
+        x.lut = lut_d.as<uint16_t>();
+        x.max_symbol = static_cast<uint32_t>(t.alphabet.back());
+      }
+      if (host_text) x.ingest_phase = EWT_PHASE_H2D;
+      kept = run_passes<T>(t, x, want_groups, err_build, st);
     }
-  }
-  if (by_passes) {
-    // All levels' bits came from the multi-level passes; now their counts
-    // and the node-start ranks (the count table is complete).
     build_rs_counts(t.rs, 0, L, st);
-    for (uint32_t l = 0; l < L; ++l) {
-      uint64_t const ncount = lv_off[l + 1] - lv_off[l];
-      if (ncount == 0) continue;
+    if (L > 1) {
       PhaseTimer pt(EWT_PHASE_NODE_RANKS, st);
-      level_nodes_kernel<<<static_cast<uint32_t>(ceil_div(ncount, 128)), 128,
-                           0, st>>>(v, lnodes_d.as<LevelNode>() + lv_off[l],
-                                    ncount, l, t.counts_d.as<uint64_t>(),
-                                    t.ranks_d.as<uint64_t>(), err_build);
+      dim3 const grid(static_cast<uint32_t>(ceil_div(uint64_t(1) << (L - 1), 128)), L - 1);
+      pow2_node_ranks_kernel<<<grid, 128, 0, st>>>(v, t.ranks_d.as<uint64_t>(), err_build);
       EWT_LAUNCHED();
     }
   } else {
+    {  // level 0 bits
+      PhaseTimer pt(EWT_PHASE_FILL, st);
+      uint64_t const w0 = ceil_div(t.level_bits[0], 32);
+      uint32_t const blocks =
+          static_cast<uint32_t>(ceil_div(w0, uint64_t(256) * fill_words<T>()));
+      auto k = t.pow2 ? (t.is_min ? fill0_kernel<T, true, true>
+                                  : fill0_kernel<T, true, false>)
+                      : (t.is_min ? fill0_kernel<T, false, true>
+                                  : fill0_kernel<T, false, false>);
+      k<<<blocks, 256, 0, st>>>(sym, t.level_bits[0], L, sigma,
+                                words + t.rs.meta[0].word_off, err_build);
+      EWT_LAUNCHED();
+    }
+    std::vector<std::pair<uint32_t, uint32_t>> const wanted =
+        want_groups ? group_planes(L) : std::vector<std::pair<uint32_t, uint32_t>>{};
     DevBuf ping, pong;
     if (L > 2) ping.alloc(n * sizeof(T));
     if (L > 3) pong.alloc(n * sizeof(T));
@@ -750,6 +784,20 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
     DevBuf slow_tiles((ceil_div(n, kSplitTile) + 1) * 4);
     T const* src = sym;
     for (uint32_t l = 0; l < L; ++l) {
+      for (auto const& w : wanted)
+        if (w.first == l) {  // a group level starts here
+          OrderPlanes o;
+          o.level = l;
+          o.first = l + 1;
+          o.count = w.second;
+          o.stride = ceil_div(ceil_div(n, 32), 32) * 32 + 32;
+          o.mem.alloc(o.count * o.stride * 4);
+          EWT_CUDA(cudaMemsetAsync(o.mem.get(), 0, o.count * o.stride * 4, st));
+          order_planes_kernel<T><<<grid_stream, 256, 0, st>>>(
+              src, n, L, l, o.count, o.mem.as<uint32_t>(), o.stride);
+          EWT_LAUNCHED();
+          kept.push_back(std::move(o));
+        }
       build_rs_counts(t.rs, l, l + 1, st);
       uint64_t const ncount = lv_off[l + 1] - lv_off[l];
       if (ncount > 0) {
@@ -805,7 +853,17 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
   t.counts.assign(c.begin(), c.begin() + sigma);
   t.occ.resize(sigma);
   for (uint64_t i = 0; i < sigma; ++i) t.occ[i] = c[i + 1] - c[i];
-  if (want_groups) build_groups(t, c, sym, sizeof(T), st);
+  if (want_groups) {
+    std::vector<std::vector<uint32_t const*>> planes;
+    for (auto const& w : group_planes(L)) {
+      std::vector<uint32_t const*> p{words + t.rs.meta[w.first].word_off};
+      for (OrderPlanes const& o : kept)
+        if (o.level == w.first)
+          for (uint32_t j = 1; j <= w.second; ++j) p.push_back(o.plane(w.first + j));
+      planes.push_back(std::move(p));
+    }
+    build_groups(t, c, planes, st);
+  }
   v.groups = t.groups.view();
 }
 

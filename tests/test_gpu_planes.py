@@ -1,0 +1,68 @@
+"""The bit-plane passes of the build (planes.cuh) where their bookkeeping can
+go wrong: texts ending at the edges of a tile (a CTA's slots of 128 symbols,
+less the slots that class runs may waste), for every pass plan; texts whose
+runs are all zeros, all ones, sorted or alternate, so that slots hold only one
+child's symbols and runs start at every bit offset; symbols mapped to codes on
+the way in.  Integer results: byte-identical to the oracle's."""
+import numpy as np
+import pytest
+
+from tests.test_gpu_parity import assert_same_tree, check_queries
+
+pytestmark = pytest.mark.gpu
+
+
+def tile(slots, k):
+    return (slots - ((5 << k) + 3) // 4) * 128
+
+
+# code bits -> slots and levels of the first pass
+FIRST = {1: (256, 0), 2: (256, 1), 3: (256, 2), 4: (256, 3), 5: (256, 4), 8: (256, 3),
+         9: (256, 4), 10: (128, 3), 16: (128, 3)}
+
+
+def same(ewt, oracle, text, alphabet, seed=1):
+    gt = ewt.WaveletTree(text, alphabet)
+    ot = oracle.OracleTree(text, alphabet)
+    assert_same_tree(gt, ot)
+    check_queries(gt, ot, text, np.asarray(alphabet, dtype=np.uint64), 1_000, seed=seed)
+
+
+@pytest.mark.parametrize("L", sorted(FIRST))
+@pytest.mark.parametrize("tiles,more", [(1, -1), (1, 0), (1, 1), (2, 127), (3, 33)])
+def test_tile_edges(ewt, oracle, L, tiles, more):
+    n = tiles * tile(*FIRST[L]) + more
+    dtype = np.uint8 if L <= 8 else np.uint16
+    rng = np.random.default_rng(1000 * L + tiles + more)
+    text = rng.integers(0, 1 << L, n, dtype=np.uint64).astype(dtype)
+    same(ewt, oracle, text, np.arange(1 << L))
+
+
+@pytest.mark.parametrize("shape", ["zeros", "ones", "sorted", "blocks", "rare"])
+@pytest.mark.parametrize("L", [5, 8, 12])
+def test_one_sided_slots(ewt, oracle, L, shape):
+    n, sigma = 70_001, 1 << L
+    dtype = np.uint8 if L <= 8 else np.uint16
+    rng = np.random.default_rng(L)
+    text = {"zeros": np.zeros(n, np.int64), "ones": np.full(n, sigma - 1),
+            "sorted": np.sort(rng.integers(0, sigma, n)),
+            "blocks": np.repeat(rng.integers(0, sigma, n // 37 + 1), 37)[:n],
+            "rare": np.where(rng.random(n) < 0.001, rng.integers(0, sigma, n), sigma // 2)}[shape]
+    same(ewt, oracle, text.astype(dtype), np.arange(sigma))
+
+
+@pytest.mark.parametrize("dtype,sigma", [(np.uint8, 2), (np.uint8, 64), (np.uint16, 512)])
+def test_mapped_symbols(ewt, oracle, dtype, sigma):
+    """Scattered alphabets of a power of two, detected from the text."""
+    rng = np.random.default_rng(sigma)
+    alphabet = np.sort(rng.choice(np.iinfo(dtype).max, sigma, replace=False)).astype(dtype)
+    text = alphabet[rng.integers(0, sigma, 50_021)]
+    text[:sigma] = alphabet
+    same(ewt, oracle, text, alphabet)
+    assert np.array_equal(ewt.WaveletTree(text).export("COUNTS"),
+                          ewt.WaveletTree(text, alphabet).export("COUNTS"))
+    if alphabet[-1] < np.iinfo(dtype).max:
+        bad = text.copy()
+        bad[-1] = np.iinfo(dtype).max
+        with pytest.raises(ewt.EwtError):
+            ewt.WaveletTree(bad, alphabet)
