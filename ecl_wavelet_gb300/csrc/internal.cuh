@@ -28,7 +28,10 @@ struct RSStore {
 
   // Lays out arrays of the given bit lengths and allocates words (zeroed),
   // L1, L2 and the device meta table.  Samples are allocated by build_rs.
-  void layout(std::vector<uint64_t> const& bits);
+  // With `stride` (a multiple of 32) array a starts at word a * stride of
+  // *filled, whose words are final (zero past every array's end) and are
+  // taken over.
+  void layout(std::vector<uint64_t> const& bits, uint64_t stride = 0, DevBuf* filled = nullptr);
   RSView view() const;
   uint64_t device_bytes() const {
     return words.bytes() + l1.bytes() + l2.bytes() + s0.bytes() + s1.bytes() + rb.bytes() +

@@ -25,7 +25,7 @@ struct BlockJob {
   uint64_t word_off, bits, l2_off, l1_off, num_l1, num_last_l2;
 };
 
-void RSStore::layout(std::vector<uint64_t> const& bits) {
+void RSStore::layout(std::vector<uint64_t> const& bits, uint64_t stride, DevBuf* filled) {
   meta.assign(bits.size(), ArrayMeta{});
   total_words = total_l1 = total_l2 = 0;
   for (size_t a = 0; a < bits.size(); ++a) {
@@ -33,7 +33,7 @@ void RSStore::layout(std::vector<uint64_t> const& bits) {
     m.bits = bits[a];
     uint64_t const w = ceil_div(bits[a], 32);
     m.word_off = total_words;
-    total_words += ceil_div(w, 32) * 32;  // 128-byte padding per array
+    total_words += filled ? stride : ceil_div(w, 32) * 32;  // 128-byte padding per array
     m.num_l1 = std::max<uint64_t>(1, ceil_div(bits[a], kL1Bits));
     m.num_last_l2 = ceil_div(bits[a] % kL1Bits, kL2Bits);
     if (m.num_last_l2 == 0) m.num_last_l2 = kL2PerL1;
@@ -44,7 +44,8 @@ void RSStore::layout(std::vector<uint64_t> const& bits) {
   }
   total_words += total_words % 2;
   // 16 words of slack: readers may fetch one word past an array's end
-  words.alloc(total_words * 4 + 64);
+  if (filled) words = std::move(*filled);
+  else words.alloc(total_words * 4 + 64);
   l1.alloc(total_l1 * 8);
   l2.alloc(total_l2 * 2);
   meta_d.alloc(meta.size() * sizeof(ArrayMeta));
@@ -62,6 +63,7 @@ void RSStore::layout(std::vector<uint64_t> const& bits) {
                            cudaMemcpyHostToDevice, st));
   // Zero the padding words behind every array (the arrays themselves are
   // written completely by their producer).
+  if (filled) return;
   for (auto const& m : meta) {
     uint64_t const w = ceil_div(m.bits, 32);
     uint64_t const padded = ceil_div(w, 32) * 32;

@@ -4,22 +4,24 @@
 //   1. alphabet: given, or detected (presence bitmap kernel for 1/2-byte
 //      symbols, host sort for wider ones) — wavelet_tree.cuh:590-614;
 //   2. shape on the host: minimal codes for non-power-of-two alphabets
-//      (:2100-2159), node starts (:2501-2532), nodes per level (:703-724),
-//      and the list of (start, split, end) symbol ranges of every node;
-//   3. a non-minimal alphabet is remapped to 0..sigma-1 (:170-227); a
-//      non-power-of-two alphabet also gets a histogram (its short codes
-//      make level sizes depend on symbol counts, :776-790);
-//   4. power-of-two alphabets of 1- and 2-byte symbols: all levels by
-//      bit-plane passes (planes.cuh), then the counts of all levels and the
-//      node-start ranks in one launch each.  Other alphabets: level 0 bits
-//      are packed from the text; then for every level l: RankSelect counts of level l; the node kernel computes rank0 at every
-//      node start of level l (precomputeRanksKernel, :332-352) and from it
-//      the count table C at each node's split point (zeros of a node =
-//      rank0(end) - rank0(start)), so no histogram pass is needed for
-//      power-of-two alphabets; the split kernel stably partitions every
-//      node of level l by its bit (the level l+1 order; the reference
-//      re-sorts the text on the top l+1 code bits, :806-818) and writes the
-//      bits of level l+1 directly;
+//      (:2100-2159), node starts (:2501-2532), nodes per level (:703-724);
+//   3. alphabets of up to 2^16 symbols: all levels by bit-plane passes
+//      (planes.cuh) over the symbols' codes.  Bytes and 16-bit symbols are
+//      mapped to codes as the passes read them, wider ones by remap_kernel
+//      (:170-227).  A short code of a non-power-of-two alphabet is padded
+//      with zero bits: codes are increasing, so the symbols whose code has
+//      ended are the end of every later order, their padding writes zeros
+//      there, and level l is the first part of that order (its size follows
+//      from the passes' symbol counts, :776-790).  Then the RankSelect counts
+//      of all levels and the node-start ranks (precomputeRanksKernel,
+//      :332-352) in one launch each;
+//   4. larger alphabets: level 0 bits are packed from the text; then for
+//      every level l: RankSelect counts of level l; the node kernel computes
+//      rank0 at every node start of level l and from it the count table C at
+//      each node's split point (zeros of a node = rank0(end) - rank0(start));
+//      the split kernel stably partitions every node of level l by its bit
+//      (the level l+1 order; the reference re-sorts the text on the top l+1
+//      code bits, :806-818) and writes the bits of level l+1 directly;
 //   5. select samples of all levels.
 // The split kernel has a fast path for tiles that lie inside one node of a
 // power-of-two alphabet: warp ballots rank the tile's zeros and ones, both
@@ -250,54 +252,72 @@ std::vector<uint64_t> detect_alphabet_wide(T const* d_text, uint64_t n,
   }
 }
 
-// Text -> minimal symbols (lower_bound in the sorted alphabet).
-template <class T>
-__global__ void __launch_bounds__(256)
+// Text -> minimal symbols (lower_bound in the sorted alphabet), or with
+// `codes` the code of each.  Smem: the alphabet is searched in shared memory.
+template <class T, class U, bool Smem>
+__global__ void __launch_bounds__(1024)
 remap_kernel(T const* __restrict__ text, uint64_t n,
-             T const* __restrict__ alphabet, uint64_t sigma,
-             T* __restrict__ cur, uint32_t* __restrict__ err) {
+             T const* __restrict__ alphabet, uint32_t sigma,
+             uint16_t const* __restrict__ codes, U* __restrict__ cur,
+             uint32_t* __restrict__ err) {
+  extern __shared__ __align__(16) unsigned char remap_smem[];
+  T* const sa = reinterpret_cast<T*>(remap_smem);
+  if constexpr (Smem) {
+    for (uint32_t i = threadIdx.x; i < sigma; i += blockDim.x) sa[i] = alphabet[i];
+    __syncthreads();
+  }
+  T const* const al = Smem ? sa : alphabet;
   uint64_t const stride = uint64_t(gridDim.x) * blockDim.x;
   uint32_t bad = 0;
   for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n;
        i += stride) {
     T const x = text[i];
-    uint64_t lo = 0, hi = sigma;
+    uint32_t lo = 0, hi = sigma;
     while (lo < hi) {
-      uint64_t const mid = (lo + hi) >> 1;
-      if (alphabet[mid] < x) lo = mid + 1; else hi = mid;
+      uint32_t const mid = (lo + hi) >> 1;
+      if (al[mid] < x) lo = mid + 1; else hi = mid;
     }
     if (lo >= sigma) {
       bad = 1;
       lo = 0;
     }
-    cur[i] = static_cast<T>(lo);
+    cur[i] = static_cast<U>(codes ? codes[lo] : lo);
   }
   if (bad) atomicOr(err, 1u);
 }
 
-// Histogram of minimal symbols (non-power-of-two alphabets only).
+// Searching in shared memory keeps two CTAs of 1024 threads on an SM up to
+// 96 KB of alphabet; above that the alphabet stays in the caches.
+template <class T, class U>
+void launch_remap(T const* text, uint64_t n, T const* alphabet, uint64_t sigma,
+                  uint16_t const* codes, U* out, uint32_t* err, cudaStream_t st) {
+  EWT_REQUIRE(sigma < UINT32_MAX, EWT_ERR_UNSUPPORTED, "alphabet too large");
+  uint32_t const grid = static_cast<uint32_t>(
+      std::min<uint64_t>(ceil_div(n, 1024), uint64_t(sm_count()) * 2));
+  constexpr size_t kMax = 96 * 1024;
+  if (sigma * sizeof(T) <= kMax) {
+    auto k = remap_kernel<T, U, true>;
+    set_smem_limit(k, kMax);
+    k<<<grid, 1024, sigma * sizeof(T), st>>>(text, n, alphabet, static_cast<uint32_t>(sigma),
+                                             codes, out, err);
+  } else {
+    remap_kernel<T, U, false><<<grid, 1024, 0, st>>>(
+        text, n, alphabet, static_cast<uint32_t>(sigma), codes, out, err);
+  }
+  EWT_LAUNCHED();
+}
+
+// Histogram of minimal symbols (non-power-of-two alphabets of more than
+// 2^16 symbols).
 template <class T>
 __global__ void __launch_bounds__(256)
 hist_kernel(T const* __restrict__ text, uint64_t n, uint64_t sigma,
-            unsigned long long* __restrict__ occ, uint32_t smem_bins) {
-  extern __shared__ uint32_t hist[];
-  bool const use_smem = smem_bins != 0;
-  if (use_smem) {
-    for (uint32_t i = threadIdx.x; i < smem_bins; i += blockDim.x) hist[i] = 0;
-    __syncthreads();
-  }
+            unsigned long long* __restrict__ occ) {
   uint64_t const stride = uint64_t(gridDim.x) * blockDim.x;
   for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n;
        i += stride) {
     uint64_t const c = text[i];
-    if (c >= sigma) continue;
-    if (use_smem) atomicAdd(&hist[c], 1u);
-    else atomicAdd(&occ[c], 1ull);
-  }
-  if (use_smem) {
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < smem_bins; i += blockDim.x)
-      if (hist[i]) atomicAdd(&occ[i], static_cast<unsigned long long>(hist[i]));
+    if (c < sigma) atomicAdd(&occ[c], 1ull);
   }
 }
 
@@ -445,23 +465,16 @@ level_nodes_kernel(TreeView t, LevelNode const* __restrict__ nodes,
 namespace ewt {
 namespace {
 
-// rank0 at every node start of a power-of-two tree (nodes g = 1 .. 2^l - 1 of
-// level l = 1 + blockIdx.y start at symbol g << (L - l)), checked against the
-// count table: a node's zeros are the symbols below its split.
+// rank0 at every node start (node i: first symbol and level, in the order the
+// ranks are stored in); the count table is complete.
 __global__ void __launch_bounds__(128)
-pow2_node_ranks_kernel(TreeView t, uint64_t* __restrict__ ranks, uint32_t* __restrict__ err) {
-  uint32_t const l = 1 + blockIdx.y;
-  uint64_t const nodes = uint64_t(1) << l;
-  uint64_t const g = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
-  if (g >= nodes) return;
-  ArrayMeta const m = t.rs.meta[l];
-  uint32_t const sh = t.levels - l;
-  uint64_t const* C = t.counts;
-  uint64_t const ps = C[g << sh], pe = g + 1 < nodes ? C[(g + 1) << sh] : t.n;
-  uint64_t const r0 = ps - ecl::detail::rs_rank1<false>(t.rs, m, ps, nullptr);
-  uint64_t const r1 = pe - ecl::detail::rs_rank1<false>(t.rs, m, pe, nullptr);
-  if (r1 - r0 != C[(2 * g + 1) << (sh - 1)] - ps) atomicOr(err, 2u);
-  if (g) ranks[t.node_base[l] + g - 1] = r0;
+node_ranks_kernel(TreeView t, NodeInfoH const* __restrict__ nodes, uint64_t count,
+                  uint64_t* __restrict__ ranks) {
+  uint64_t const i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
+  if (i >= count) return;
+  NodeInfoH const nd = nodes[i];
+  uint64_t const p = t.counts[nd.start];
+  ranks[i] = p - ecl::detail::rs_rank1<false>(t.rs, t.rs.meta[nd.level], p, nullptr);
 }
 
 // Planes l+1 .. l+count of a level order held as symbols (bits L-2-l ..),
@@ -483,25 +496,25 @@ order_planes_kernel(T const* __restrict__ x, uint64_t n, uint32_t L, uint32_t l,
   }
 }
 
-// Levels 0 .. L-1 of a power-of-two alphabet of 1- or 2-byte symbols by
-// bit-plane passes (planes.cuh); returns the deeper planes that the group
-// levels read.
-template <class T>
-std::vector<OrderPlanes> run_passes(ewt_tree& t, PlaneText<T> const& x, bool groups,
-                                    uint32_t* err, cudaStream_t st) {
-  uint32_t* const words = t.rs.words.as<uint32_t>();
-  std::vector<uint32_t*> out(t.L);
-  std::vector<uint64_t> count(t.L);
-  for (uint32_t l = 0; l < t.L; ++l) {
-    out[l] = words + t.rs.meta[l].word_off;
-    count[l] = ceil_div(t.rs.meta[l].bits, 32);
-  }
-  if (t.L > 1) {
-    uint64_t const w1 = t.rs.meta[1].word_off;
-    EWT_CUDA(cudaMemsetAsync(words + w1, 0, (t.rs.total_words - w1) * 4, st));
-  }
-  return run_plane_passes<T>(x, out.data(), count.data(), t.counts_d.as<uint64_t>(),
-                             groups ? group_planes(t.L)
+// Words of one level in the passes' store.
+uint64_t level_stride(uint64_t n) { return ceil_div(ceil_div(n, 32), 32) * 32; }
+
+// Levels 0 .. L-1 of codes of up to 16 bits by bit-plane passes (planes.cuh),
+// level l at words + l * level_stride(n); returns the deeper planes that the
+// group levels read.
+template <class U>
+std::vector<OrderPlanes> run_passes(ewt_tree& t, PlaneText<U> const& x, uint32_t* words,
+                                    uint64_t* starts, bool groups, uint32_t* err,
+                                    cudaStream_t st) {
+  uint64_t const stride = level_stride(x.n);
+  std::vector<uint32_t*> out(x.L);
+  std::vector<uint64_t> count(x.L, stride);
+  for (uint32_t l = 0; l < x.L; ++l) out[l] = words + l * stride;
+  // level 0 is written whole but for its padding
+  uint64_t const w0 = ceil_div(x.n, 32);
+  EWT_CUDA(cudaMemsetAsync(words + w0, 0, (x.L * stride - w0) * 4, st));
+  return run_plane_passes<U>(x, out.data(), count.data(), starts,
+                             groups ? group_planes(x.L)
                                     : std::vector<std::pair<uint32_t, uint32_t>>{},
                              err, st);
 }
@@ -509,32 +522,16 @@ std::vector<OrderPlanes> run_passes(ewt_tree& t, PlaneText<T> const& x, bool gro
 thread_local bool t_texts_synced = false;
 thread_local bool t_batch_member = false;
 
-// A given alphabet 0 .. sigma-1 with sigma a power of two >= 4 (1- and
-// 2-byte symbols): the texts whose first pass can read them directly.
+// Whether a host text goes straight to the ingest kernel, which is then its
+// only reader (kernels read the host text: a Grace host's pageable memory, or
+// pinned memory): 1- and 2-byte symbols, a given alphabet (one to be found is
+// another read), a 16-byte aligned text.
 template <class T>
-bool minimal_pow2_alphabet(const void* alphabet, uint64_t sigma) {
+bool host_ingest(const void* data, uint64_t n, uint64_t sigma) {
   if constexpr (sizeof(T) > 2) {
     return false;
   } else {
-    if (sigma < 4 || (sigma & (sigma - 1)) || !alphabet) return false;
-    T const* a = static_cast<T const*>(alphabet);
-    for (uint64_t i = 0; i < sigma; ++i)
-      if (uint64_t(a[i]) != i) return false;
-    return true;
-  }
-}
-
-// Whether a host text goes straight to the ingest kernel (kernels read the
-// host text: a Grace host's pageable memory, or pinned memory): such an
-// alphabet and a 16-byte aligned text.
-template <class T>
-bool host_ingest(const void* data, uint64_t n, const void* alphabet, uint64_t sigma) {
-  if constexpr (sizeof(T) > 2) {
-    return false;
-  } else {
-    if (!minimal_pow2_alphabet<T>(alphabet, sigma) || n == 0 ||
-        reinterpret_cast<uintptr_t>(data) % 16)
-      return false;
+    if (sigma < 2 || n == 0 || reinterpret_cast<uintptr_t>(data) % 16) return false;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return false;
     int pageable = 0;
@@ -567,7 +564,7 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
     EWT_CUDA(cudaMemcpyAsync(text_owned.get(), data, n * sizeof(T),
                              cudaMemcpyDeviceToDevice, st));
     d_text = text_owned.as<T>();
-  } else if (host_ingest<T>(data, n, alphabet, sigma)) {
+  } else if (host_ingest<T>(data, n, sigma)) {
     d_text = static_cast<T const*>(data);
     host_text = true;
   } else {
@@ -626,65 +623,121 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
   uint32_t const grid_stream =
       static_cast<uint32_t>(std::min<uint64_t>(ceil_div(n, 256),
                                                uint64_t(sm_count()) * 8));
-  // Power-of-two alphabets of 1- and 2-byte symbols go through the bit-plane
-  // passes, which map symbols to codes as they read them.
-  bool const by_planes = sizeof(T) <= 2 && t.pow2;
+  bool const by_planes = L <= kMaxPlanes;
   auto const level_nodes = by_planes ? std::vector<std::vector<LevelNode>>{}
                                      : make_level_nodes(sigma, L);
-  DevBuf cur_buf;  // minimal symbols when the alphabet is not 0..sigma-1
+  DevBuf cur_buf;  // minimal symbols (or codes) of a text the build cannot read as it is
   DevBuf lut_d;
   T const* sym = d_text;
-  if (!t.is_min) {
+  if (!t.is_min || (by_planes && sizeof(T) > 2)) {
     std::vector<T> a(t.alphabet.begin(), t.alphabet.end());
     t.alphabet_d.alloc(sigma * sizeof(T));
     EWT_CUDA(cudaMemcpyAsync(t.alphabet_d.get(), a.data(), sigma * sizeof(T),
                              cudaMemcpyHostToDevice, st));
-    if (by_planes) {
-      // symbol -> rank of the first alphabet symbol at or above it
+    EWT_CUDA(cudaStreamSynchronize(st));  // `a` leaves scope
+  }
+  // codes, padded with zero bits, by minimal symbol
+  std::vector<uint16_t> codes;
+  if (by_planes && (!t.pow2 || !t.is_min)) {
+    codes.resize(sigma);
+    for (uint64_t i = 0; i < sigma; ++i)
+      codes[i] = static_cast<uint16_t>(i < t.codes_start ? i : t.codes[i - t.codes_start].code);
+    if (sizeof(T) <= 2) {  // by symbol: that of the first alphabet symbol at or above it
       std::vector<uint16_t> lut(sizeof(T) == 1 ? 256 : 65536, 0);
       uint64_t v = 0;
       for (uint64_t i = 0; i < sigma; ++i)
-        for (; v <= t.alphabet[i] && v < lut.size(); ++v) lut[v] = static_cast<uint16_t>(i);
+        for (; v <= t.alphabet[i] && v < lut.size(); ++v) lut[v] = codes[i];
       lut_d.alloc(lut.size() * 2);
       EWT_CUDA(cudaMemcpyAsync(lut_d.get(), lut.data(), lut.size() * 2,
                                cudaMemcpyHostToDevice, st));
       EWT_CUDA(cudaStreamSynchronize(st));  // `lut` leaves scope
-    } else {
-      cur_buf.alloc(n * sizeof(T));
-      PhaseTimer pt(EWT_PHASE_HIST, st);
-      remap_kernel<T><<<grid_stream, 256, 0, st>>>(
-          d_text, n, t.alphabet_d.as<T>(), sigma, cur_buf.as<T>(), err_build);
-      EWT_LAUNCHED();
-      sym = cur_buf.as<T>();
+    } else if (!t.pow2) {
+      lut_d.alloc(sigma * 2);
+      EWT_CUDA(cudaMemcpyAsync(lut_d.get(), codes.data(), sigma * 2,
+                               cudaMemcpyHostToDevice, st));
     }
   }
-  // Count table: exact histogram for non-power-of-two alphabets (their level
-  // sizes need it); otherwise only C[0] = 0 and C[sigma] = n, the rest is
-  // derived level by level.
+  if (by_planes && sizeof(T) > 2) {
+    cur_buf.alloc(n * 2);
+    PhaseTimer pt(EWT_PHASE_HIST, st);
+    launch_remap<T, uint16_t>(d_text, n, t.alphabet_d.as<T>(), sigma, lut_d.as<uint16_t>(),
+                              cur_buf.as<uint16_t>(), err_build, st);
+  } else if (!by_planes && !t.is_min) {
+    cur_buf.alloc(n * sizeof(T));
+    PhaseTimer pt(EWT_PHASE_HIST, st);
+    launch_remap<T, T>(d_text, n, t.alphabet_d.as<T>(), sigma, nullptr, cur_buf.as<T>(),
+                       err_build, st);
+    sym = cur_buf.as<T>();
+  }
+  // Group query levels for power-of-two alphabets -- except for the short
+  // texts of a batch build: the group build's launch latency would be most
+  // of their build time; they get rank blocks on every level instead.
+  t.n = n;
+  bool const want_groups =
+      groups_eligible(t) && !(t_batch_member && n < kBatchGroupMinSymbols);
+  std::vector<OrderPlanes> kept;  // deeper planes of the group levels' orders
+  // The passes, given where level 0 and the class starts (2^L + 1) go.
+  auto passes = [&](uint32_t* words, uint64_t* starts) {
+    auto run = [&](auto x) {
+      x.n = n;
+      x.L = L;
+      kept = run_passes(t, x, words, starts, want_groups, err_build, st);
+    };
+    if constexpr (sizeof(T) <= 2) {
+      PlaneText<T> x;
+      x.sym = d_text;
+      if (!codes.empty()) {
+        x.lut = lut_d.as<uint16_t>();
+        x.max_symbol = static_cast<uint32_t>(t.alphabet.back());
+      }
+      if (host_text) x.ingest_phase = EWT_PHASE_H2D;
+      run(x);
+    } else {
+      PlaneText<uint16_t> x;
+      x.sym = cur_buf.as<uint16_t>();
+      run(x);
+    }
+  };
+  // Count table: for power-of-two alphabets the passes' class starts (or, of
+  // the split, C[0] = 0 and C[sigma] = n, the rest derived level by level);
+  // other alphabets need the symbol counts first, for their level sizes.
   t.counts_d.alloc((sigma + 1) * 8);
   t.level_bits.assign(L, n);
+  DevBuf words_early;  // the levels of passes that ran before the layout
   if (!t.pow2) {
-    DevBuf occ_d(sigma * 8);
-    EWT_CUDA(cudaMemsetAsync(occ_d.get(), 0, sigma * 8, st));
-    uint32_t const smem_bins = sigma <= 8192 ? static_cast<uint32_t>(sigma) : 0;
-    {
-      PhaseTimer pt(EWT_PHASE_HIST, st);
-      hist_kernel<T><<<grid_stream, 256, smem_bins * 4, st>>>(
-          sym, n, sigma, occ_d.as<unsigned long long>(), smem_bins);
-      EWT_LAUNCHED();
-    }
     t.occ.assign(sigma, 0);
-    EWT_CUDA(cudaMemcpyAsync(t.occ.data(), occ_d.get(), sigma * 8,
-                             cudaMemcpyDeviceToHost, st));
-    EWT_CUDA(cudaStreamSynchronize(st));
+    if (by_planes) {
+      uint64_t const slots = uint64_t(1) << L;
+      DevBuf starts((slots + 1) * 8);
+      words_early.alloc(L * level_stride(n) * 4 + 64);
+      passes(words_early.as<uint32_t>(), starts.as<uint64_t>());
+      std::vector<uint64_t> h(slots + 1);
+      EWT_CUDA(cudaMemcpyAsync(h.data(), starts.get(), (slots + 1) * 8,
+                               cudaMemcpyDeviceToHost, st));
+      EWT_CUDA(cudaStreamSynchronize(st));
+      for (uint64_t i = 0; i < sigma; ++i) t.occ[i] = h[codes[i] + 1] - h[codes[i]];
+    } else {
+      DevBuf occ_d(sigma * 8);
+      EWT_CUDA(cudaMemsetAsync(occ_d.get(), 0, sigma * 8, st));
+      {
+        PhaseTimer pt(EWT_PHASE_HIST, st);
+        hist_kernel<T><<<grid_stream, 256, 0, st>>>(
+            sym, n, sigma, occ_d.as<unsigned long long>());
+        EWT_LAUNCHED();
+      }
+      EWT_CUDA(cudaMemcpyAsync(t.occ.data(), occ_d.get(), sigma * 8,
+                               cudaMemcpyDeviceToHost, st));
+      EWT_CUDA(cudaStreamSynchronize(st));
+    }
     // Level sizes (wavelet_tree.cuh:776-790): drop symbols whose code ended.
-    for (uint32_t l = 0; l < L; ++l)
-      for (size_t j = 0; j < t.codes.size(); ++j)
-        if (t.codes[j].len <= l) t.level_bits[l] -= t.occ[t.codes_start + j];
+    for (size_t j = 0; j < t.codes.size(); ++j)
+      for (uint32_t l = static_cast<uint32_t>(t.codes[j].len); l < L; ++l)
+        t.level_bits[l] -= t.occ[t.codes_start + j];
     std::vector<uint64_t> c(sigma + 1, 0);
     for (uint64_t i = 1; i <= sigma; ++i) c[i] = c[i - 1] + t.occ[i - 1];
     EWT_CUDA(cudaMemcpyAsync(t.counts_d.get(), c.data(), (sigma + 1) * 8,
                              cudaMemcpyHostToDevice, st));
+    EWT_CUDA(cudaStreamSynchronize(st));  // `c` leaves scope
   } else if (!by_planes) {
     uint64_t const ends[2] = {0, n};
     EWT_CUDA(cudaMemcpyAsync(t.counts_d.get(), &ends[0], 8,
@@ -697,7 +750,20 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
     EWT_REQUIRE(t.level_bits[l] > 0, EWT_ERR_UNSUPPORTED,
                 "empty level: every symbol with a code this long is absent");
 
-  t.rs.layout(t.level_bits);
+  if (words_early.get()) {
+    uint64_t kept_bits = 0;
+    for (uint64_t b : t.level_bits) kept_bits += b;
+    // levels that short codes left mostly empty are packed
+    bool const pack = kept_bits * 8 < L * n * 7;
+    t.rs.layout(t.level_bits, pack ? 0 : level_stride(n), pack ? nullptr : &words_early);
+    for (uint32_t l = 0; pack && l < L; ++l)
+      EWT_CUDA(cudaMemcpyAsync(t.rs.words.as<uint32_t>() + t.rs.meta[l].word_off,
+                               words_early.as<uint32_t>() + l * level_stride(n),
+                               ceil_div(t.level_bits[l], 32) * 4, cudaMemcpyDeviceToDevice, st));
+    words_early.reset();
+  } else {
+    t.rs.layout(t.level_bits);
+  }
   t.ranks_d.alloc(std::max<size_t>(t.nodes.size(), 1) * 8);
   t.node_base_d.alloc((L + 1) * 8);
   EWT_CUDA(cudaMemcpyAsync(t.node_base_d.get(), t.node_base.data(), (L + 1) * 8,
@@ -723,41 +789,30 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
     flat.insert(flat.end(), level_nodes[l].begin(), level_nodes[l].end());
     lv_off[l + 1] = flat.size();
   }
+  DevBuf nodes_d;  // node starts (passes)
+  if (by_planes && !t.nodes.empty()) {
+    nodes_d.alloc(t.nodes.size() * sizeof(NodeInfoH));
+    EWT_CUDA(cudaMemcpyAsync(nodes_d.get(), t.nodes.data(), t.nodes.size() * sizeof(NodeInfoH),
+                             cudaMemcpyHostToDevice, st));
+  }
   DevBuf lnodes_d(std::max<size_t>(flat.size(), 1) * sizeof(LevelNode));
   EWT_CUDA(cudaMemcpyAsync(lnodes_d.get(), flat.data(),
                            flat.size() * sizeof(LevelNode),
                            cudaMemcpyHostToDevice, st));
   EWT_CUDA(cudaStreamSynchronize(st));  // host vectors above leave scope
 
-  t.n = n;
   fill_tree_view(t);
   TreeView& v = t.view;
 
   uint32_t* const words = t.rs.words.as<uint32_t>();
-  // Group query levels for power-of-two alphabets -- except for the short
-  // texts of a batch build: the group build's launch latency would be most
-  // of their build time; they get rank blocks on every level instead.
-  bool const want_groups =
-      groups_eligible(t) && !(t_batch_member && n < kBatchGroupMinSymbols);
-  std::vector<OrderPlanes> kept;  // deeper planes of the group levels' orders
   if (by_planes) {
-    if constexpr (sizeof(T) <= 2) {
-      PlaneText<T> x;
-      x.sym = d_text;
-      x.n = n;
-      x.L = L;
-      if (!t.is_min) {
-        x.lut = lut_d.as<uint16_t>();
-        x.max_symbol = static_cast<uint32_t>(t.alphabet.back());
-      }
-      if (host_text) x.ingest_phase = EWT_PHASE_H2D;
-      kept = run_passes<T>(t, x, want_groups, err_build, st);
-    }
+    if (t.pow2) passes(words, t.counts_d.as<uint64_t>());
+    if (t.is_min) t.alphabet_d.reset();  // only remap_kernel needed it
     build_rs_counts(t.rs, 0, L, st);
-    if (L > 1) {
+    if (!t.nodes.empty()) {
       PhaseTimer pt(EWT_PHASE_NODE_RANKS, st);
-      dim3 const grid(static_cast<uint32_t>(ceil_div(uint64_t(1) << (L - 1), 128)), L - 1);
-      pow2_node_ranks_kernel<<<grid, 128, 0, st>>>(v, t.ranks_d.as<uint64_t>(), err_build);
+      node_ranks_kernel<<<static_cast<uint32_t>(ceil_div(t.nodes.size(), 128)), 128, 0, st>>>(
+          v, nodes_d.as<NodeInfoH>(), t.nodes.size(), t.ranks_d.as<uint64_t>());
       EWT_LAUNCHED();
     }
   } else {

@@ -66,3 +66,39 @@ def test_mapped_symbols(ewt, oracle, dtype, sigma):
         bad[-1] = np.iinfo(dtype).max
         with pytest.raises(ewt.EwtError):
             ewt.WaveletTree(bad, alphabet)
+
+
+@pytest.mark.parametrize("dtype,sigma", [(np.uint8, 3), (np.uint8, 5), (np.uint8, 129),
+                                         (np.uint8, 255), (np.uint16, 257), (np.uint16, 1000),
+                                         (np.uint16, 40_001), (np.uint32, 300),
+                                         (np.uint32, 4096), (np.uint64, 5000)])
+@pytest.mark.parametrize("skew", ["uniform", "first", "last"])
+def test_short_codes(ewt, oracle, dtype, sigma, skew):
+    """Alphabets with short codes (their padding ends the levels) and wide
+    symbols, scattered and detected; texts dominated by the first (longest
+    code) or the last symbol (shortest: levels mostly empty, packed)."""
+    rng = np.random.default_rng(sigma)
+    top = min(np.iinfo(dtype).max, 1 << 62)
+    alphabet = np.sort(rng.choice(top, sigma, replace=False) if top < 1 << 17 else
+                       np.unique(rng.integers(0, top, 2 * sigma + 10))[:sigma]).astype(dtype)
+    n = max(61_003, 2 * sigma)
+    ids = rng.integers(0, sigma, n)
+    if skew != "uniform":
+        ids = np.where(rng.random(n) < 0.03, ids, 0 if skew == "first" else sigma - 1)
+    ids[rng.permutation(n)[:sigma]] = np.arange(sigma)
+    text = alphabet[ids]
+    same(ewt, oracle, text, alphabet)
+    detected = ewt.WaveletTree(text)
+    assert np.array_equal(detected.getAlphabet(), alphabet)
+    assert np.array_equal(detected.export("LEVEL_WORDS", 1),
+                          ewt.WaveletTree(text, alphabet).export("LEVEL_WORDS", 1))
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 13_823, 13_824, 13_825, 30_208 + 1])
+def test_short_codes_edges(ewt, oracle, n):
+    """Given minimal alphabets of no power of two; every code length present
+    (the last symbol of each length is appended)."""
+    for dtype, sigma in ((np.uint8, 75), (np.uint16, 2300)):
+        rng = np.random.default_rng(n + sigma)
+        text = np.concatenate([rng.integers(0, sigma, n), np.arange(sigma)]).astype(dtype)
+        same(ewt, oracle, text, np.arange(sigma))
