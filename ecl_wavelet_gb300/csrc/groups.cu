@@ -1,10 +1,15 @@
-// Group query levels of power-of-two trees: runs of w = 2 (quad) or 3
+// Group query levels: runs of w = 2 (quad) or 3
 // (octal) consecutive binary levels l .. l+w-1 become one level of w-bit
 // digits in level-l order, so a query resolves w binary levels per
 // dependent DRAM access.  The plan covers all L levels: as many octal
 // groups as fit, then one or two quad groups (L = 8: 3 + 3 + 2).  No
 // reference counterpart; the binary levels and their RankSelect stay the
 // source of truth for exports.
+//
+// Over an alphabet of no power of two they hold the minimal codes padded with
+// zero bits to L bits, for every position of the text on every level (the
+// passes carry ended codes to the end of the later orders), so the walks are
+// those of a power-of-two tree of 2^L codes.
 //
 // A digit's bits are the planes l .. l+w-1 of the level-l order: plane l is
 // the binary level l, the deeper ones come from the pass that wrote that
@@ -514,10 +519,42 @@ GroupView GroupStore::view() const {
   uint32_t covered = 0;
   for (auto const& ql : levels) covered += ql.width;
   v.covered = covered;
+  v.counts = counts.as<uint64_t>();
+  v.code = code.as<uint16_t>();
+  v.symbol = symbol.as<uint16_t>();
   return v;
 }
 
-bool groups_eligible(ewt_tree const& t) { return t.pow2 && t.L >= 2 && t.n >= 1; }
+bool groups_eligible(ewt_tree const& t) {
+  return (t.pow2 || t.L <= 16) && t.L >= 2 && t.n >= 1;
+}
+
+std::vector<uint64_t> code_counts(ewt_tree const& t) {
+  std::vector<uint64_t> C((uint64_t(1) << t.L) + 1, 0);
+  for (uint64_t i = 0; i < t.sigma; ++i) C[padded_code(t, i) + 1] = t.occ[i];
+  for (size_t i = 1; i < C.size(); ++i) C[i] += C[i - 1];
+  return C;
+}
+
+void upload_group_codes(ewt_tree& t, std::vector<uint64_t> const& C, cudaStream_t st) {
+  if (t.pow2) return;
+  std::vector<uint16_t> code(t.sigma), symbol(C.size() - 1, 0);
+  for (uint64_t i = 0; i < t.sigma; ++i) {
+    uint64_t const c = padded_code(t, i);
+    code[i] = static_cast<uint16_t>(c);
+    symbol[c] = static_cast<uint16_t>(i);
+  }
+  GroupStore& qs = t.groups;
+  qs.counts.alloc(C.size() * 8);
+  qs.code.alloc(code.size() * 2);
+  qs.symbol.alloc(symbol.size() * 2);
+  EWT_CUDA(cudaMemcpyAsync(qs.counts.get(), C.data(), C.size() * 8, cudaMemcpyHostToDevice, st));
+  EWT_CUDA(cudaMemcpyAsync(qs.code.get(), code.data(), code.size() * 2,
+                           cudaMemcpyHostToDevice, st));
+  EWT_CUDA(cudaMemcpyAsync(qs.symbol.get(), symbol.data(), symbol.size() * 2,
+                           cudaMemcpyHostToDevice, st));
+  EWT_CUDA(cudaStreamSynchronize(st));  // the host tables leave scope
+}
 
 namespace {
 
@@ -584,8 +621,9 @@ void build_groups(ewt_tree& t, std::vector<uint64_t> const& C,
   PhaseTimer pt(EWT_PHASE_QUAD, st);
   uint32_t const L = t.L;
   uint64_t const n = t.n;
-  EWT_REQUIRE(C.size() == t.sigma + 1 && C[t.sigma] == n, EWT_ERR_CUDA,
+  EWT_REQUIRE(C.size() == (uint64_t(1) << L) + 1 && C.back() == n, EWT_ERR_CUDA,
               "count table inconsistent");
+  upload_group_codes(t, C, st);
   layout_groups(t);
   EWT_REQUIRE(planes.size() == qs.levels.size(), EWT_ERR_CUDA, "group planes missing");
   // host: digit totals, node ranks

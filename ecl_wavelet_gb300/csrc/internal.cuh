@@ -59,15 +59,16 @@ uint64_t rank_block_starts(std::vector<ArrayMeta> const& meta,
 // (shift 0 drops them: select then uses the reference-format samples).
 void build_dense_samples(RSStore& rs, uint32_t shift, cudaStream_t stream);
 
-// Group (octal / quad) query levels of a power-of-two tree (groups.cu).
+// Group (octal / quad) query levels of a tree (groups.cu).
 struct GroupStore {
   std::vector<ecl::detail::GroupLevel> levels;  // host copy
   DevBuf blocks, sb, ds, node_ranks, levels_d;
+  DevBuf counts, code, symbol;  // padded codes (alphabets of no power of two)
   uint32_t sel_shift = ecl::detail::kDefaultSelShift;
   ecl::detail::GroupView view() const;
   uint64_t bytes() const {
     return blocks.bytes() + sb.bytes() + ds.bytes() + node_ranks.bytes() +
-           levels_d.bytes();
+           levels_d.bytes() + counts.bytes() + code.bytes() + symbol.bytes();
   }
 };
 
@@ -146,7 +147,7 @@ struct ewt_tree {
   std::vector<ewt::NodeInfoH> nodes;
   std::vector<uint64_t> nodes_at_level, node_base, level_bits;
   ewt::RSStore rs;
-  ewt::GroupStore groups;  // octal / quad query levels (power-of-two trees)
+  ewt::GroupStore groups;  // octal / quad query levels
   ewt::DevBuf counts_d, ranks_d, node_base_d, nodes_at_level_d, code_len_d,
       code_bits_d, alphabet_d, err_d;
   ecl::detail::TreeView view{};
@@ -260,11 +261,20 @@ void launch_serve_items(uint32_t elem_size, TreeView const* d_views,
                         void const* reqs, void const* items, uint32_t num_items,
                         uint32_t max_levels, uint32_t* req_err, cudaStream_t s);
 void prepare_serve_kernels(uint32_t elem_size);
-// Group query levels (groups.cu): whether a tree gets them (power-of-two
-// alphabet, two or more levels), their build from the finished binary levels
-// and count table C (sigma + 1 entries), and a rebuild of their dense select
-// samples at rate 2^shift (0: none).
+// Group query levels (groups.cu): whether a tree gets them (two or more
+// levels; power-of-two alphabets, or codes of up to 16 bits), their build from
+// the planes of the finished levels and the count table C over codes (2^L + 1
+// entries), and a rebuild of their dense select samples at rate 2^shift (0:
+// none).
 bool groups_eligible(ewt_tree const& t);
+// Code of minimal symbol i, a short one padded with zero bits to L bits.
+inline uint64_t padded_code(ewt_tree const& t, uint64_t i) {
+  return i < t.codes_start ? i : t.codes[i - t.codes_start].code;
+}
+// Symbols of a smaller code, 2^L + 1 entries, from the symbols' occurrences.
+std::vector<uint64_t> code_counts(ewt_tree const& t);
+// The code tables that the group walks of an alphabet of no power of two use.
+void upload_group_codes(ewt_tree& t, std::vector<uint64_t> const& C, cudaStream_t st);
 // Digit widths of the group levels of an L-level tree, top down: octal (3)
 // groups, then one or two quad (2) groups; they cover all L levels.
 std::vector<uint32_t> group_widths(uint32_t L);

@@ -132,7 +132,7 @@ extern "C" int ewt_save(const ewt_tree* t, const char* path) {
     dev_to_file(f, t->rs.ds.get(), t->rs.ds.bytes(), stage, s);
     dev_to_file(f, t->counts_d.get(), t->counts_d.bytes(), stage, s);
     dev_to_file(f, t->ranks_d.get(), t->ranks_d.bytes(), stage, s);
-    // group query levels (none for other alphabets)
+    // group query levels
     f.put_vec(t->groups.levels);
     f.put(t->groups.ds.get() ? t->groups.sel_shift : 0);
     if (!t->groups.levels.empty()) {
@@ -230,6 +230,16 @@ extern "C" int ewt_load(const char* path, int gpu_index, ewt_tree** out) {
         file_to_dev(f, t->groups.node_ranks, stage, s, big);
         upload(t->groups.levels_d, t->groups.levels, s);
         if (t->groups.sel_shift == 0) t->groups.ds.reset();
+        if (!t->pow2) {  // the code tables follow from the symbols' counts
+          EWT_REQUIRE(t->occ.size() == sig && t->codes_start + t->codes.size() == sig,
+                      EWT_ERR_INVALID_ARGUMENT, "index file is corrupt");
+          for (CodeH const& c : t->codes)
+            EWT_REQUIRE(c.code < (uint64_t(1) << t->L), EWT_ERR_INVALID_ARGUMENT,
+                        "index file is corrupt");
+          EWT_REQUIRE(t->codes_start <= (uint64_t(1) << t->L), EWT_ERR_INVALID_ARGUMENT,
+                      "index file is corrupt");
+          upload_group_codes(*t, code_counts(*t), s);
+        }
       }
       upload(t->rs.meta_d, t->rs.meta, s);
       upload(t->node_base_d, t->node_base, s);

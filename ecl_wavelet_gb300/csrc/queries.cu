@@ -38,15 +38,21 @@ struct StagePlan {
   size_t bytes;
 };
 
+// Count-table entries a walk reads: by code where codes are padded.
+inline uint64_t walk_entries(ewt_tree const& t) {
+  return !t.pow2 && !t.groups.levels.empty() ? (uint64_t(1) << t.L) + 1 : t.sigma;
+}
+
 inline StagePlan plan_stage(ewt_tree const& t) {
   StagePlan p{0, 0, 0};
   size_t b = t.L * sizeof(ArrayMeta) + (t.L + 1) * 8;
   b = (b + 15) & ~size_t(15);
-  if (b + t.sigma * 8 <= kStageLimitBytes / 2) {
+  if (b + walk_entries(t) * 8 <= kStageLimitBytes / 2) {
     p.stage_counts = 1;
-    b += t.sigma * 8;
+    b += walk_entries(t) * 8;
   }
-  if (b + t.nodes.size() * 8 <= kStageLimitBytes) {
+  // (the group walks read their own node ranks)
+  if (t.groups.levels.empty() && b + t.nodes.size() * 8 <= kStageLimitBytes) {
     p.stage_ranks = 1;
     b += t.nodes.size() * 8;
   }
@@ -67,6 +73,7 @@ query_kernel(TreeView t, uint8_t const* __restrict__ types,
   size_t off = L * sizeof(ArrayMeta) + (L + 1) * 8;
   off = (off + 15) & ~size_t(15);
   uint64_t const* counts = t.counts;
+  uint64_t const* walk = nullptr;
   uint64_t const* ranks = t.node_ranks;
   {
     uint64_t const* gm = reinterpret_cast<uint64_t const*>(t.rs.meta);
@@ -76,11 +83,13 @@ query_kernel(TreeView t, uint8_t const* __restrict__ types,
     for (uint32_t i = threadIdx.x; i <= L; i += blockDim.x)
       node_base[i] = t.node_base[i];
     if (stage_counts) {
+      bool const padded = padded_codes(t);
+      uint64_t const* from = padded ? t.groups.counts : t.counts;
+      uint64_t const entries = padded ? (uint64_t(1) << L) + 1 : t.sigma;
       uint64_t* sc = reinterpret_cast<uint64_t*>(smem + off);
-      for (uint64_t i = threadIdx.x; i < t.sigma; i += blockDim.x)
-        sc[i] = t.counts[i];
-      counts = sc;
-      off += t.sigma * 8;
+      for (uint64_t i = threadIdx.x; i < entries; i += blockDim.x) sc[i] = from[i];
+      (padded ? walk : counts) = sc;
+      off += entries * 8;
     }
     if (stage_ranks) {
       uint64_t* sr = reinterpret_cast<uint64_t*>(smem + off);
@@ -105,7 +114,7 @@ query_kernel(TreeView t, uint8_t const* __restrict__ types,
       T res = 0;
       if (idx < t.n)
         res = from_minimal<T>(
-            t, wt_access(t, meta, counts, ranks, node_base, idx));
+            t, wt_access(t, meta, counts, ranks, node_base, idx, walk));
       if (K == kMixed)
         static_cast<uint64_t*>(out)[i] = res;
       else
@@ -120,14 +129,14 @@ query_kernel(TreeView t, uint8_t const* __restrict__ types,
         res = UINT64_MAX;
         bad = 1;
       } else {
-        res = wt_rank(t, meta, counts, ranks, node_base, c, q.index);
+        res = wt_rank(t, meta, counts, ranks, node_base, c, q.index, walk);
       }
     } else if (kind == kSelect) {
       if (c >= t.sigma || q.index == 0) {
         res = UINT64_MAX;
         bad = 1;
       } else {
-        res = wt_select(t, meta, counts, ranks, node_base, c, q.index);
+        res = wt_select(t, meta, counts, ranks, node_base, c, q.index, walk);
       }
     } else {
       res = UINT64_MAX;
@@ -160,6 +169,7 @@ mixed_kernel(TreeView t, uint8_t const* __restrict__ types,
   size_t off = L * sizeof(ArrayMeta) + (L + 1) * 8;
   off = (off + 15) & ~size_t(15);
   uint64_t const* counts = t.counts;
+  uint64_t const* walk = nullptr;
   uint64_t const* ranks = t.node_ranks;
   {
     uint64_t const* gm = reinterpret_cast<uint64_t const*>(t.rs.meta);
@@ -169,11 +179,13 @@ mixed_kernel(TreeView t, uint8_t const* __restrict__ types,
     for (uint32_t i = threadIdx.x; i <= L; i += blockDim.x)
       node_base[i] = t.node_base[i];
     if (stage_counts) {
+      bool const padded = padded_codes(t);
+      uint64_t const* from = padded ? t.groups.counts : t.counts;
+      uint64_t const entries = padded ? (uint64_t(1) << L) + 1 : t.sigma;
       uint64_t* sc = reinterpret_cast<uint64_t*>(smem + off);
-      for (uint64_t i = threadIdx.x; i < t.sigma; i += blockDim.x)
-        sc[i] = t.counts[i];
-      counts = sc;
-      off += t.sigma * 8;
+      for (uint64_t i = threadIdx.x; i < entries; i += blockDim.x) sc[i] = from[i];
+      (padded ? walk : counts) = sc;
+      off += entries * 8;
     }
     if (stage_ranks) {
       uint64_t* sr = reinterpret_cast<uint64_t*>(smem + off);
@@ -214,7 +226,7 @@ mixed_kernel(TreeView t, uint8_t const* __restrict__ types,
       uint64_t const idx = in[q].index;
       out[q] = idx < t.n ? static_cast<uint64_t>(from_minimal<T>(
                                t, wt_access(t, meta, counts, ranks, node_base,
-                                            idx)))
+                                            idx, walk)))
                          : 0;
     }
     for (uint32_t i = threadIdx.x; i < list_len[1]; i += blockDim.x) {
@@ -225,7 +237,7 @@ mixed_kernel(TreeView t, uint8_t const* __restrict__ types,
         out[q] = UINT64_MAX;
         bad = 1;
       } else {
-        out[q] = wt_rank(t, meta, counts, ranks, node_base, sym, r.index);
+        out[q] = wt_rank(t, meta, counts, ranks, node_base, sym, r.index, walk);
       }
     }
     for (uint32_t i = threadIdx.x; i < list_len[2]; i += blockDim.x) {
@@ -236,7 +248,7 @@ mixed_kernel(TreeView t, uint8_t const* __restrict__ types,
         out[q] = UINT64_MAX;
         bad = 1;
       } else {
-        out[q] = wt_select(t, meta, counts, ranks, node_base, sym, r.index);
+        out[q] = wt_select(t, meta, counts, ranks, node_base, sym, r.index, walk);
       }
     }
     __syncthreads();  // lists are reused by the next chunk

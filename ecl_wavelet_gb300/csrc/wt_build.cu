@@ -641,7 +641,7 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
   if (by_planes && (!t.pow2 || !t.is_min)) {
     codes.resize(sigma);
     for (uint64_t i = 0; i < sigma; ++i)
-      codes[i] = static_cast<uint16_t>(i < t.codes_start ? i : t.codes[i - t.codes_start].code);
+      codes[i] = static_cast<uint16_t>(padded_code(t, i));
     if (sizeof(T) <= 2) {  // by symbol: that of the first alphabet symbol at or above it
       std::vector<uint16_t> lut(sizeof(T) == 1 ? 256 : 65536, 0);
       uint64_t v = 0;
@@ -669,9 +669,9 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
                        err_build, st);
     sym = cur_buf.as<T>();
   }
-  // Group query levels for power-of-two alphabets -- except for the short
-  // texts of a batch build: the group build's launch latency would be most
-  // of their build time; they get rank blocks on every level instead.
+  // Group query levels -- except for the short texts of a batch build: the
+  // group build's launch latency would be most of their build time; they get
+  // rank blocks on every level instead.
   t.n = n;
   bool const want_groups =
       groups_eligible(t) && !(t_batch_member && n < kBatchGroupMinSymbols);
@@ -704,6 +704,7 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
   t.counts_d.alloc((sigma + 1) * 8);
   t.level_bits.assign(L, n);
   DevBuf words_early;  // the levels of passes that ran before the layout
+  std::vector<uint64_t> code_starts;  // symbols of a smaller code (no power of two)
   if (!t.pow2) {
     t.occ.assign(sigma, 0);
     if (by_planes) {
@@ -711,7 +712,8 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
       DevBuf starts((slots + 1) * 8);
       words_early.alloc(L * level_stride(n) * 4 + 64);
       passes(words_early.as<uint32_t>(), starts.as<uint64_t>());
-      std::vector<uint64_t> h(slots + 1);
+      std::vector<uint64_t>& h = code_starts;
+      h.resize(slots + 1);
       EWT_CUDA(cudaMemcpyAsync(h.data(), starts.get(), (slots + 1) * 8,
                                cudaMemcpyDeviceToHost, st));
       EWT_CUDA(cudaStreamSynchronize(st));
@@ -760,7 +762,6 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
       EWT_CUDA(cudaMemcpyAsync(t.rs.words.as<uint32_t>() + t.rs.meta[l].word_off,
                                words_early.as<uint32_t>() + l * level_stride(n),
                                ceil_div(t.level_bits[l], 32) * 4, cudaMemcpyDeviceToDevice, st));
-    words_early.reset();
   } else {
     t.rs.layout(t.level_bits);
   }
@@ -911,13 +912,16 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
   if (want_groups) {
     std::vector<std::vector<uint32_t const*>> planes;
     for (auto const& w : group_planes(L)) {
-      std::vector<uint32_t const*> p{words + t.rs.meta[w.first].word_off};
+      // the whole order's bits also where a level was packed
+      std::vector<uint32_t const*> p{
+          words_early.get() ? words_early.as<uint32_t>() + w.first * level_stride(n)
+                            : words + t.rs.meta[w.first].word_off};
       for (OrderPlanes const& o : kept)
         if (o.level == w.first)
           for (uint32_t j = 1; j <= w.second; ++j) p.push_back(o.plane(w.first + j));
       planes.push_back(std::move(p));
     }
-    build_groups(t, c, planes, st);
+    build_groups(t, t.pow2 ? c : code_starts, planes, st);
   }
   v.groups = t.groups.view();
 }

@@ -88,8 +88,11 @@ struct RSView {
   uint32_t sel_shift;     // log2 of the dense sample rate; 0 = none
 };
 
-/* Group levels of power-of-two alphabets (query side, no reference
- * counterpart).  A group level covers w = 2 or 3 consecutive binary levels
+/* Group levels (query side, no reference counterpart).  They hold the symbols'
+ * L-bit codes: of a power-of-two alphabet the minimal symbols themselves, of
+ * another one the minimal codes padded with zero bits to L bits (increasing
+ * with the symbol, so every node of the padded tree is a range of symbols,
+ * and a code's padding bits lead to itself).  A group level covers w = 2 or 3 consecutive binary levels
  * starting at level l: in level-l order it holds each symbol's w-bit digit
  * (bits l .. l+w-1 counted from the top), so one read resolves w binary
  * levels.  Storage: 32-byte blocks; a block holds, before its digits, the
@@ -137,6 +140,10 @@ struct GroupView {
   const GroupLevel* levels;     // device array of num entries
   uint32_t num;                // group levels (0: the tree has none)
   uint32_t covered;            // binary levels they cover (the rest: binary)
+  /* alphabets of no power of two (null otherwise): */
+  const uint64_t* counts;      // symbols of a smaller code, 2^L + 1 entries
+  const uint16_t* code;        // padded code of each minimal symbol
+  const uint16_t* symbol;      // minimal symbol of each padded code
 };
 
 /* Everything a query walk needs; trivially copyable into a kernel. */
@@ -884,9 +891,13 @@ __device__ __forceinline__ uint64_t occurrences(const TreeView& t,
   return (c + 1 == t.sigma ? t.n : counts[c + 1]) - counts[c];
 }
 
-/* The three walks over group levels (power-of-two alphabets): the same
- * descent as the binary walks below, w binary levels per step; binary levels
- * past the groups (at most one) are walked as in the binary code. */
+/* The three walks over group levels: the same descent as the binary walks
+ * below, w binary levels per step, over codes (counts: symbols of a smaller
+ * code); binary levels past the groups (at most one) are walked as in the
+ * binary code. */
+__device__ __forceinline__ bool padded_codes(const TreeView& t) {
+  return t.groups.num && !t.is_pow2;
+}
 __device__ __forceinline__ uint64_t group_node_rank(const TreeView& t,
                                                    GroupLevel const& ql,
                                                    uint64_t g, uint32_t d) {
@@ -978,13 +989,18 @@ __device__ __forceinline__ uint64_t wt_select_groups(const TreeView& t,
 }
 
 /* Minimal symbol at text position idx < n (deviceAccess,
- * wavelet_tree.cuh:1815-1877). */
+ * wavelet_tree.cuh:1815-1877).  walk: a copy of GroupView::counts to use
+ * instead (padded codes; `counts` counts by minimal symbol). */
 __device__ __forceinline__ uint64_t wt_access(const TreeView& t,
                                               ArrayMeta const* meta,
                                               uint64_t const* counts,
                                               uint64_t const* ranks,
                                               uint64_t const* node_base,
-                                              uint64_t idx) {
+                                              uint64_t idx,
+                                              uint64_t const* walk = nullptr) {
+  if (padded_codes(t))
+    return __ldg(t.groups.symbol +
+                 wt_access_groups(t, meta, walk ? walk : t.groups.counts, idx));
   if (t.groups.num) return wt_access_groups(t, meta, counts, idx);
   uint64_t cs = 0, ce = t.sigma - 1;
   for (uint32_t l = 0; l < t.levels; ++l) {
@@ -1017,7 +1033,14 @@ __device__ __forceinline__ uint64_t wt_rank(const TreeView& t,
                                             uint64_t const* counts,
                                             uint64_t const* ranks,
                                             uint64_t const* node_base,
-                                            uint64_t c, uint64_t i) {
+                                            uint64_t c, uint64_t i,
+                                            uint64_t const* walk = nullptr) {
+  if (padded_codes(t)) {
+    uint64_t const* W = walk ? walk : t.groups.counts;
+    uint32_t const code = __ldg(t.groups.code + c);
+    if (W[code + 1] == W[code]) return 0;
+    return wt_rank_groups(t, meta, W, ranks, node_base, code, i);
+  }
   if (occurrences(t, counts, c) == 0) return 0;
   if (t.groups.num) return wt_rank_groups(t, meta, counts, ranks, node_base, c, i);
   uint64_t cs = 0, ce = t.sigma - 1, res = i;
@@ -1048,7 +1071,14 @@ __device__ __forceinline__ uint64_t wt_select(const TreeView& t,
                                               uint64_t const* counts,
                                               uint64_t const* ranks,
                                               uint64_t const* node_base,
-                                              uint64_t c, uint64_t k) {
+                                              uint64_t c, uint64_t k,
+                                              uint64_t const* walk = nullptr) {
+  if (padded_codes(t)) {
+    uint64_t const* W = walk ? walk : t.groups.counts;
+    uint32_t const code = __ldg(t.groups.code + c);
+    if (k == 0 || k > W[code + 1] - W[code]) return t.n;
+    return wt_select_groups(t, meta, W, ranks, node_base, code, k);
+  }
   if (k == 0 || k > occurrences(t, counts, c)) return t.n;
   if (t.groups.num) return wt_select_groups(t, meta, counts, ranks, node_base, c, k);
   uint32_t const L = t.levels;

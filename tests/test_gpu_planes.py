@@ -102,3 +102,25 @@ def test_short_codes_edges(ewt, oracle, n):
         rng = np.random.default_rng(n + sigma)
         text = np.concatenate([rng.integers(0, sigma, n), np.arange(sigma)]).astype(dtype)
         same(ewt, oracle, text, np.arange(sigma))
+
+
+@pytest.mark.parametrize("sigma", [5, 75, 200])
+@pytest.mark.parametrize("n", [43, 21_503, 21_505, 2 * 49_152 + 95])
+def test_padded_group_levels(ewt, oracle, sigma, n, tmp_path):
+    """Group query levels over padded codes at their superblock boundaries
+    (21,504 octal, 49,152 quad digits); again from an index file, and at other
+    select-sample rates."""
+    rng = np.random.default_rng(n + sigma)
+    alphabet = np.arange(sigma)
+    text = rng.integers(0, sigma, max(n, sigma)).astype(np.uint8)
+    text[rng.permutation(text.size)[:sigma]] = np.arange(sigma)
+    gt = ewt.WaveletTree(text, alphabet)
+    ot = oracle.OracleTree(text, alphabet)
+    al = alphabet.astype(np.uint64)
+    check_queries(gt, ot, text, al, 1_000, seed=n)
+    gt.save(str(tmp_path / "i"))
+    lt = ewt.WaveletTree.load(str(tmp_path / "i"))
+    check_queries(lt, ot, text, al, 1_000, seed=n + 1)
+    for rate in (0, 1024):
+        gt.set_select_samples(rate)
+        check_queries(gt, ot, text, al, 1_000, seed=rate)
