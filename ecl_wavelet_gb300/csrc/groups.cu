@@ -16,9 +16,10 @@
 // order (planes.cuh; the per-level split of larger alphabets extracts them
 // from the symbols of its level orders).  Per group level:
 //   1. group_counts_kernel (warp per superblock): its digit counts, by
-//      popcounts of the planes and of their intersections;
-//   2. group_scan_*: counts before every superblock (chunked scan);
-//   3. group_level_kernel (CTA per superblock, thread per block): block
+//      popcounts of the planes and of their intersections, added up per chunk
+//      of superblocks as well;
+//   2. group_scan_kernel: counts before every superblock (CTA per chunk);
+//   3. group_level_kernel (CTA per superblock, thread per two blocks): block
 //      headers from a CTA scan, blocks and dense select samples written;
 //      the superblock's totals are checked against pass 1, the level's
 //      against the count table.
@@ -44,7 +45,7 @@ constexpr uint64_t kOctSbDigits = uint64_t(kOctDigits) * kOctSbBlocks;
 
 namespace {
 
-constexpr uint32_t kScanChunk = 4096;   // superblock entries per scan CTA
+constexpr uint32_t kScanChunk = 512;   // superblock entries per scan CTA
 
 // Bits 2k of the result take bit k of x (k < 16).
 __device__ __forceinline__ uint32_t spread16(uint32_t x) {
@@ -56,117 +57,67 @@ __device__ __forceinline__ uint32_t spread16(uint32_t x) {
   return x;
 }
 
-// Block-wide exclusive scan of a uint64 (blockDim.x a multiple of 32, at
-// most 1024); *total receives the sum.
-__device__ __forceinline__ uint64_t cta_exclusive_scan(uint64_t x, uint64_t* total) {
-  __shared__ uint64_t warp_sums[32];
-  uint32_t const lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  uint64_t inc = x;
+// Inclusive warp scan.
+__device__ __forceinline__ uint32_t warp_inclusive(uint32_t x) {
 #pragma unroll
-  for (uint32_t o = 1; o < 32; o <<= 1) {
-    uint64_t const y = __shfl_up_sync(0xFFFFFFFFu, inc, o);
-    if (lane >= o) inc += y;
-  }
-  if (lane == 31) warp_sums[wid] = inc;
-  __syncthreads();
-  uint32_t const nwarps = blockDim.x >> 5;
-  if (wid == 0) {
-    uint64_t t = lane < nwarps ? warp_sums[lane] : 0;
-#pragma unroll
-    for (uint32_t o = 1; o < 32; o <<= 1) {
-      uint64_t const y = __shfl_up_sync(0xFFFFFFFFu, t, o);
-      if (lane >= o) t += y;
-    }
-    if (lane < nwarps) warp_sums[lane] = t;  // inclusive over warps
-  }
-  __syncthreads();
-  uint64_t const before = wid ? warp_sums[wid - 1] : 0;
-  *total = warp_sums[nwarps - 1];
-  __syncthreads();
-  return before + inc - x;
+  for (int o = 1; o < 32; o <<= 1)
+    asm volatile(
+        "{ .reg .pred p; .reg .u32 y;\n"
+        "shfl.sync.up.b32 y|p, %0, %1, 0, 0xffffffff;\n"
+        "@p add.u32 %0, %0, y; }"
+        : "+r"(x)
+        : "r"(o));
+  return x;
 }
 
-// Scan 1: per chunk of kScanChunk superblock entries (S digits each), the
-// S sums.
+// Pass 2: counts before every superblock, in place (a thread per entry of S
+// digits, each below 2^16; chunk[c] = the digits of chunk c).  A CTA adds up
+// the chunks before its own, so the scan is one launch: 6 Gi symbols have 586
+// chunks.  (Three launches over chunks of 4,096 entries took 53 us a level at
+// 2^28 symbols, this one 6 us.)
 template <uint32_t S>
-__global__ void __launch_bounds__(256)
-group_scan_partial_kernel(uint64_t const* __restrict__ sb, uint64_t count,
-                          uint64_t* __restrict__ chunk) {
-  uint64_t const first = uint64_t(blockIdx.x) * kScanChunk;
-  uint64_t c[S];
+__global__ void __launch_bounds__(kScanChunk)
+group_scan_kernel(uint64_t* __restrict__ sb, uint64_t count,
+                  uint64_t const* __restrict__ chunk) {
+  constexpr uint32_t kWarps = kScanChunk / 32;
+  __shared__ uint64_t part[kWarps][32];
+  __shared__ uint32_t warp_tot[S][kWarps];
+  uint32_t const tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  // lane l of every warp: digit l % S of chunks (l / S) + (32 / S) * (wid + kWarps * i)
+  uint64_t sum = 0;
+  for (uint32_t c = wid * (32 / S) + lane / S; c < blockIdx.x; c += kWarps * (32 / S))
+    sum += chunk[uint64_t(c) * S + lane % S];
+  part[wid][lane] = sum;
+  uint64_t const i = uint64_t(blockIdx.x) * kScanChunk + tid;
+  uint32_t x[S], inc[S];
 #pragma unroll
-  for (uint32_t d = 0; d < S; ++d) c[d] = 0;
-  for (uint64_t i = first + threadIdx.x; i < min(count, first + kScanChunk);
-       i += blockDim.x)
-#pragma unroll
-    for (uint32_t d = 0; d < S; ++d) c[d] += sb[i * S + d];
+  for (uint32_t k = 0; k < S / 2; ++k) {
+    uint4 const a = i < count ? reinterpret_cast<uint4 const*>(sb + i * S)[k]
+                              : make_uint4(0, 0, 0, 0);
+    x[2 * k] = a.x;
+    x[2 * k + 1] = a.z;
+  }
 #pragma unroll
   for (uint32_t d = 0; d < S; ++d) {
-    uint64_t tot = 0;
-    cta_exclusive_scan(c[d], &tot);
-    if (threadIdx.x == 0) chunk[blockIdx.x * S + d] = tot;
+    inc[d] = warp_inclusive(x[d]);
+    if (lane == 31) warp_tot[d][wid] = inc[d];
   }
-}
-
-// Scan 2: exclusive prefix of the chunk sums (one thread per digit).
-template <uint32_t S>
-__global__ void group_scan_chunks_kernel(uint64_t* __restrict__ chunk,
-                                         uint64_t chunks) {
-  uint32_t const d = threadIdx.x;
-  if (d >= S) return;
-  uint64_t run = 0;
-  for (uint64_t i = 0; i < chunks; ++i) {
-    uint64_t const x = chunk[i * S + d];
-    chunk[i * S + d] = run;
-    run += x;
+  __syncthreads();
+  uint64_t carry = 0;  // digit lane % S before the chunk
+  if (wid == 0) {
+    for (uint32_t w = 0; w < kWarps; ++w) carry += part[w][lane];
+    for (uint32_t o = S; o < 32; o <<= 1) carry += __shfl_xor_sync(0xffffffffu, carry, o);
   }
-}
-
-// Scan 3: exclusive prefix of every entry, in place (1024 threads; two
-// digits packed per 64-bit scan: every entry is below 2^16, a round's sums
-// below 2^32).
-template <uint32_t S>
-__global__ void __launch_bounds__(1024)
-group_scan_apply_kernel(uint64_t* __restrict__ sb, uint64_t count,
-                        uint64_t const* __restrict__ chunk) {
-  uint64_t const first = uint64_t(blockIdx.x) * kScanChunk;
-  uint64_t const end = min(count, first + kScanChunk);
-  uint64_t carry[S];
-  for (uint32_t d = 0; d < S; ++d) carry[d] = chunk ? chunk[blockIdx.x * S + d] : 0;
-  for (uint64_t base = first; base < end; base += blockDim.x) {
-    uint64_t const i = base + threadIdx.x;
-    bool const in = i < end;
+  __syncthreads();
+  if (wid == 0) part[0][lane] = carry;
+  __syncthreads();
+  if (i >= count) return;
 #pragma unroll
-    for (uint32_t k = 0; k < S / 2; ++k) {
-      uint4 const a = in ? reinterpret_cast<uint4 const*>(sb + i * S)[k]
-                         : make_uint4(0, 0, 0, 0);
-      uint64_t tot = 0;
-      uint64_t const e = cta_exclusive_scan(uint64_t(a.x) | (uint64_t(a.z) << 32), &tot);
-      if (in) {
-        sb[i * S + 2 * k] = carry[2 * k] + (e & 0xFFFFFFFFu);
-        sb[i * S + 2 * k + 1] = carry[2 * k + 1] + (e >> 32);
-      }
-      carry[2 * k] += tot & 0xFFFFFFFFu;
-      carry[2 * k + 1] += tot >> 32;
-    }
+  for (uint32_t d = 0; d < S; ++d) {
+    uint32_t before = inc[d] - x[d];
+    for (uint32_t w = 0; w < wid; ++w) before += warp_tot[d][w];
+    sb[i * S + d] = part[0][d] + before;
   }
-}
-
-// Counts before every superblock of one level's table (nsb + 1 entries of
-// S digits, the last one zero before and the totals after).
-template <uint32_t S>
-void scan_superblocks(uint64_t* sb, uint64_t entries, DevBuf& chunk, cudaStream_t st) {
-  uint64_t const chunks = ceil_div(entries, kScanChunk);
-  if (chunks > 1) {
-    group_scan_partial_kernel<S><<<static_cast<uint32_t>(chunks), 256, 0, st>>>(
-        sb, entries, chunk.as<uint64_t>());
-    EWT_LAUNCHED();
-    group_scan_chunks_kernel<S><<<1, 32, 0, st>>>(chunk.as<uint64_t>(), chunks);
-    EWT_LAUNCHED();
-  }
-  group_scan_apply_kernel<S><<<static_cast<uint32_t>(chunks), 1024, 0, st>>>(
-      sb, entries, chunks > 1 ? chunk.as<uint64_t>() : nullptr);
-  EWT_LAUNCHED();
 }
 
 // Dense samples of one block: entry k of digit d names the block holding
@@ -189,14 +140,6 @@ __device__ __forceinline__ void put_group_samples(uint32_t* __restrict__ ds,
     uint64_t k = (before[d] + off) >> sh;
     for (uint32_t o = off; o < c[d]; o += rm + 1, ++k) S_[k] = static_cast<uint32_t>(blk);
   }
-}
-
-// 64 bits of a plane from bit q on (the arrays have slack behind their end).
-__device__ __forceinline__ uint64_t bits64(uint32_t const* __restrict__ w, uint64_t q) {
-  uint64_t const i = q >> 5;
-  uint32_t const s = static_cast<uint32_t>(q) & 31u;
-  uint32_t const a = __ldg(w + i), b = __ldg(w + i + 1), c = __ldg(w + i + 2);
-  return uint64_t(__funnelshift_r(a, b, s)) | (uint64_t(__funnelshift_r(b, c, s)) << 32);
 }
 
 // The planes of a group level, the digit's highest bit first.
@@ -229,12 +172,12 @@ __device__ __forceinline__ void digit_counts(uint32_t const* s, uint32_t n, uint
 // planes hold zeros past position n.  Bound by reading the planes once.
 template <int W>
 __global__ void __launch_bounds__(256)
-group_counts_kernel(GroupPlanes g, uint64_t n, uint64_t nsb, uint64_t* __restrict__ sb) {
+group_counts_kernel(GroupPlanes g, uint64_t n, uint64_t nsb, uint64_t* __restrict__ sb,
+                    unsigned long long* __restrict__ chunk) {
   constexpr uint32_t S = 1u << W, K = S - 1;
   constexpr uint32_t kWords = GroupShape<W>::kDigits * GroupShape<W>::kSbBlocks / 32;
   uint64_t const s = (blockIdx.x * uint64_t(blockDim.x) + threadIdx.x) >> 5;
   uint32_t const lane = threadIdx.x & 31;
-  if (s > nsb) return;
   uint32_t acc[K];
 #pragma unroll
   for (uint32_t i = 0; i < K; ++i) acc[i] = 0;
@@ -260,136 +203,183 @@ group_counts_kernel(GroupPlanes g, uint64_t n, uint64_t nsb, uint64_t* __restric
   }
 #pragma unroll
   for (uint32_t i = 0; i < K; ++i) acc[i] = __reduce_add_sync(0xFFFFFFFFu, acc[i]);
-  uint32_t c[S];
+  uint32_t c[S], own = 0;
   digit_counts<W>(acc, total, c);
 #pragma unroll
   for (uint32_t d = 0; d < S; ++d)
-    if (lane == d) sb[s * S + d] = c[d];  // entry nsb: zeros
-}
-
-// Exclusive scan of four uint32 over a CTA of 512 threads.
-__device__ __forceinline__ uint4 cta_exclusive_scan4(uint4 x, uint4* total) {
-  __shared__ uint4 ws[16];
-  uint32_t const lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  uint4 inc = x;
-#pragma unroll
-  for (uint32_t o = 1; o < 32; o <<= 1) {
-    uint32_t const a = __shfl_up_sync(0xFFFFFFFFu, inc.x, o);
-    uint32_t const b = __shfl_up_sync(0xFFFFFFFFu, inc.y, o);
-    uint32_t const c = __shfl_up_sync(0xFFFFFFFFu, inc.z, o);
-    uint32_t const d = __shfl_up_sync(0xFFFFFFFFu, inc.w, o);
-    if (lane >= o) { inc.x += a; inc.y += b; inc.z += c; inc.w += d; }
-  }
-  if (lane == 31) ws[wid] = inc;
-  __syncthreads();
-  if (wid == 0) {
-    uint4 t = lane < 16 ? ws[lane] : make_uint4(0, 0, 0, 0);
-#pragma unroll
-    for (uint32_t o = 1; o < 16; o <<= 1) {
-      uint32_t const a = __shfl_up_sync(0xFFFFFFFFu, t.x, o);
-      uint32_t const b = __shfl_up_sync(0xFFFFFFFFu, t.y, o);
-      uint32_t const c = __shfl_up_sync(0xFFFFFFFFu, t.z, o);
-      uint32_t const d = __shfl_up_sync(0xFFFFFFFFu, t.w, o);
-      if (lane >= o) { t.x += a; t.y += b; t.z += c; t.w += d; }
-    }
-    if (lane < 16) ws[lane] = t;
+    if (lane == d) own = c[d];
+  __shared__ uint32_t sum[8][S];  // the CTA's eight superblocks are of one chunk
+  uint32_t const wid = threadIdx.x >> 5;
+  if (lane < S) {
+    if (s <= nsb) sb[s * S + lane] = own;  // entry nsb: zeros
+    sum[wid][lane] = own;
   }
   __syncthreads();
-  uint4 const before = wid ? ws[wid - 1] : make_uint4(0, 0, 0, 0);
-  *total = ws[15];
-  return make_uint4(before.x + inc.x - x.x, before.y + inc.y - x.y,
-                    before.z + inc.z - x.z, before.w + inc.w - x.w);
+  if (threadIdx.x < S) {
+    uint32_t tot = 0;
+    for (uint32_t w = 0; w < 8; ++w) tot += sum[w][threadIdx.x];
+    if (tot) atomicAdd(chunk + s / kScanChunk * S + threadIdx.x, tot);
+  }
 }
 
-// Pass 3: a CTA of 512 threads per superblock, thread t its block t: the
-// block's bits of every plane, digit counts by popcounts, the header from a
-// CTA scan of them (two 16-bit counts per word: a superblock holds fewer
-// than 2^16 digits), and the dense samples.
+// Pass 3: a CTA of 256 threads per superblock, thread t its blocks 2t and
+// 2t + 1: their bits of every plane, digit counts by popcounts, the headers
+// from one CTA scan (two 16-bit counts per word: a superblock holds fewer than
+// 2^16 digits), and the dense samples with 32-bit arithmetic from the
+// superblock's own first entry and remainder.  Bound by instructions.  All
+// group levels of 2^30 symbols of 256 (counts, scans, blocks, samples): 1.17
+// ms, 1.56 ms with a thread per block, three scan launches and a loop of
+// 64-bit sample ranks.
 template <int W>
-__global__ void __launch_bounds__(512, 3)
+__global__ void __launch_bounds__(256, 5)
 group_level_kernel(GroupPlanes g, uint64_t n, GroupLevel ql, uint4* __restrict__ blocks,
                    uint64_t const* __restrict__ sb, uint64_t nsb,
                    uint32_t* __restrict__ ds, uint32_t* __restrict__ err) {
   constexpr uint32_t S = 1u << W, kD = GroupShape<W>::kDigits, kSb = GroupShape<W>::kSbBlocks;
+  constexpr uint32_t kWarps = 8, kP = S / 2;  // packed count words
+  static_assert(kSb == 512, "two blocks per thread");
+  __shared__ uint32_t warp_tot[kWarps][4];
+  __shared__ uint32_t* entry[S];  // the sample of the superblock's next multiple of R
+  __shared__ uint32_t remainder[S];
   uint64_t const sbi = blockIdx.x;
-  uint32_t const t = threadIdx.x;
-  uint64_t const blk = sbi * kSb + t;
-  bool const mine = blk < ql.num_blocks;
-  uint64_t const p = blk * kD;
-  uint32_t const valid =
-      mine && p < n ? static_cast<uint32_t>(min(uint64_t(kD), n - p)) : 0u;
-  uint32_t c[S];
-  uint64_t H = 0, M = 0, B = 0;          // octal: 42 bits of each plane
-  uint32_t h[3] = {0, 0, 0}, b[3] = {0, 0, 0};  // quad: three words of each
-  if constexpr (W == 3) {
-    if (valid) {
-      uint64_t const vm = (1ull << valid) - 1;
-      H = bits64(g.p[0], p) & vm;
-      M = bits64(g.p[1], p) & vm;
-      B = bits64(g.p[2], p) & vm;
-    }
-    uint32_t const s[7] = {uint32_t(__popcll(H)),     uint32_t(__popcll(M)),
-                           uint32_t(__popcll(B)),     uint32_t(__popcll(H & M)),
-                           uint32_t(__popcll(H & B)), uint32_t(__popcll(M & B)),
-                           uint32_t(__popcll(H & M & B))};
-    digit_counts<3>(s, valid, c);
-  } else {
-    uint32_t s[3] = {0, 0, 0};
-#pragma unroll
-    for (uint32_t k = 0; k < 3; ++k) {
-      uint32_t const v = valid > 32 * k ? min(32u, valid - 32 * k) : 0u;
-      if (v) {
-        uint32_t const vm = v == 32 ? ~0u : (1u << v) - 1u;
-        h[k] = __ldg(g.p[0] + blk * 3 + k) & vm;
-        b[k] = __ldg(g.p[1] + blk * 3 + k) & vm;
-      }
-      s[0] += __popc(h[k]);
-      s[1] += __popc(b[k]);
-      s[2] += __popc(h[k] & b[k]);
-    }
-    digit_counts<2>(s, valid, c);
-  }
-  uint4 x = make_uint4(c[0] | (c[1] << 16), c[2] | (c[3] << 16), 0, 0);
-  if constexpr (W == 3) {
-    x.z = c[4] | (c[5] << 16);
-    x.w = c[6] | (c[7] << 16);
-  }
-  uint4 tot;
-  uint4 const e = cta_exclusive_scan4(x, &tot);
+  uint32_t const t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  uint64_t const blk = sbi * kSb + 2 * t, p = blk * kD;
   uint64_t const* sbe = sb + sbi * S;
-  if (t < S) {  // pass 1's counts must agree, and the level's totals
-    uint32_t const w4[4] = {tot.x, tot.y, tot.z, tot.w};
-    uint32_t const own = (w4[t >> 1] >> (16 * (t & 1))) & 0xFFFFu;
-    if (sbe[S + t] - sbe[t] != own) atomicOr(err, 2u);
-    if (sbi == 0 && sb[nsb * S + t] != ql.total[t]) atomicOr(err, 4u);
+  uint32_t const sh = ql.sel_shift, rm = (1u << sh) - 1u;
+  if (t < S) {
+    entry[t] = ds + ql.ds_off[t] + (sbe[t] >> sh);
+    remainder[t] = static_cast<uint32_t>(sbe[t]) & rm;
   }
-  if (!mine) return;
-  uint4* out = blocks + blk * 2;
+  uint32_t valid[2];
+  valid[0] = p < n ? static_cast<uint32_t>(min(uint64_t(kD), n - p)) : 0u;
+  valid[1] = p + kD < n ? static_cast<uint32_t>(min(uint64_t(kD), n - p - kD)) : 0u;
+  uint32_t c[2][S];
+  uint64_t H[2], M[2], B[2];     // octal: 42 bits of each plane
+  uint32_t h[2][3], b[2][3];     // quad: three words of each
   if constexpr (W == 3) {
-    // planes H, M, B in words 1..3, counts of digits 4..6 above them
-    uint64_t const w1 = H | (uint64_t(e.z & 0xFFFFu) << 42);
-    uint64_t const w2 = M | (uint64_t(e.z >> 16) << 42);
-    uint64_t const w3 = B | (uint64_t(e.w & 0xFFFFu) << 42);
-    out[0] = make_uint4(e.x, e.y, static_cast<uint32_t>(w1), static_cast<uint32_t>(w1 >> 32));
-    out[1] = make_uint4(static_cast<uint32_t>(w2), static_cast<uint32_t>(w2 >> 32),
-                        static_cast<uint32_t>(w3), static_cast<uint32_t>(w3 >> 32));
-  } else {
-    uint32_t dw[6];
+    uint64_t const i = p >> 5;
+    uint32_t const s = static_cast<uint32_t>(p) & 31u, s2 = s + kD;
+    auto bits = [&](uint32_t const* __restrict__ w, uint64_t& x, uint64_t& y) {
+      uint32_t a[4];
 #pragma unroll
-    for (uint32_t k = 0; k < 3; ++k) {
-      dw[2 * k] = spread16(b[k]) | (spread16(h[k]) << 1);
-      dw[2 * k + 1] = spread16(b[k] >> 16) | (spread16(h[k] >> 16) << 1);
+      for (int u = 0; u < 4; ++u) a[u] = valid[0] ? __ldg(w + i + u) : 0u;
+      x = (uint64_t(__funnelshift_r(a[1], a[2], s)) << 32) | __funnelshift_r(a[0], a[1], s);
+      uint32_t const b0 = s2 < 64 ? a[1] : a[2], b1 = s2 < 64 ? a[2] : a[3],
+                     b2 = s2 < 64 ? a[3] : 0u;
+      y = (uint64_t(__funnelshift_r(b1, b2, s2)) << 32) | __funnelshift_r(b0, b1, s2);
+      x &= (1ull << valid[0]) - 1;
+      y &= (1ull << valid[1]) - 1;
+    };
+    bits(g.p[0], H[0], H[1]);
+    bits(g.p[1], M[0], M[1]);
+    bits(g.p[2], B[0], B[1]);
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      uint64_t const hm = H[u] & M[u];
+      uint32_t const s7[7] = {uint32_t(__popcll(H[u])),        uint32_t(__popcll(M[u])),
+                              uint32_t(__popcll(B[u])),        uint32_t(__popcll(hm)),
+                              uint32_t(__popcll(H[u] & B[u])), uint32_t(__popcll(M[u] & B[u])),
+                              uint32_t(__popcll(hm & B[u]))};
+      digit_counts<3>(s7, valid[u], c[u]);
     }
-    out[0] = make_uint4(e.x, e.y & 0xFFFFu, dw[0], dw[1]);
-    out[1] = make_uint4(dw[2], dw[3], dw[4], dw[5]);
-  }
-  if (ds && ql.sel_shift) {
-    uint32_t const hd[8] = {e.x & 0xFFFFu, e.x >> 16, e.y & 0xFFFFu, e.y >> 16,
-                            e.z & 0xFFFFu, e.z >> 16, e.w & 0xFFFFu, e.w >> 16};
-    uint64_t before[S];
+  } else {
 #pragma unroll
-    for (uint32_t d = 0; d < S; ++d) before[d] = sbe[d] + hd[d];
-    put_group_samples<S>(ds, ql, blk, before, c);
+    for (int u = 0; u < 2; ++u) {
+      uint32_t s3[3] = {0, 0, 0};
+#pragma unroll
+      for (uint32_t k = 0; k < 3; ++k) {
+        uint32_t const v = valid[u] > 32 * k ? min(32u, valid[u] - 32 * k) : 0u;
+        uint32_t const vm = v == 32 ? ~0u : (1u << v) - 1u;
+        h[u][k] = v ? __ldg(g.p[0] + (blk + u) * 3 + k) & vm : 0u;
+        b[u][k] = v ? __ldg(g.p[1] + (blk + u) * 3 + k) & vm : 0u;
+        s3[0] += __popc(h[u][k]);
+        s3[1] += __popc(b[u][k]);
+        s3[2] += __popc(h[u][k] & b[u][k]);
+      }
+      digit_counts<2>(s3, valid[u], c[u]);
+    }
+  }
+  uint32_t e[kP];  // packed counts before block 2t
+  {
+    uint32_t x[kP];
+#pragma unroll
+    for (uint32_t k = 0; k < kP; ++k) {
+      x[k] = (c[0][2 * k] + c[1][2 * k]) | ((c[0][2 * k + 1] + c[1][2 * k + 1]) << 16);
+      e[k] = warp_inclusive(x[k]);
+      if (lane == 31) warp_tot[wid][k] = e[k];
+    }
+    __syncthreads();
+    uint32_t tot[kP];
+#pragma unroll
+    for (uint32_t k = 0; k < kP; ++k) {
+      tot[k] = 0;
+      e[k] -= x[k];
+    }
+#pragma unroll
+    for (uint32_t w = 0; w < kWarps; ++w)
+#pragma unroll
+      for (uint32_t k = 0; k < kP; ++k) {
+        uint32_t const y = warp_tot[w][k];
+        if (w < wid) e[k] += y;
+        tot[k] += y;
+      }
+    if (t == 0) {  // pass 1's counts must agree, and the level's totals
+      bool ok = true, all = true;
+#pragma unroll
+      for (uint32_t d = 0; d < S; ++d) {
+        uint32_t const own = (tot[d >> 1] >> (16 * (d & 1))) & 0xFFFFu;
+        ok = ok && sbe[S + d] - sbe[d] == own;
+        if (sbi == 0) all = all && sb[nsb * S + d] == ql.total[d];
+      }
+      if (!ok) atomicOr(err, 2u);
+      if (!all) atomicOr(err, 4u);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    if (blk + u >= ql.num_blocks) return;
+    if (u)
+#pragma unroll
+      for (uint32_t k = 0; k < kP; ++k) e[k] += c[0][2 * k] | (c[0][2 * k + 1] << 16);
+    uint4* out = blocks + (blk + u) * 2;
+    if constexpr (W == 3) {
+      // planes H, M, B in words 1..3, counts of digits 4..6 above them
+      uint64_t const w1 = H[u] | (uint64_t(e[2] & 0xFFFFu) << 42);
+      uint64_t const w2 = M[u] | (uint64_t(e[2] >> 16) << 42);
+      uint64_t const w3 = B[u] | (uint64_t(e[3] & 0xFFFFu) << 42);
+      out[0] = make_uint4(e[0], e[1], static_cast<uint32_t>(w1), static_cast<uint32_t>(w1 >> 32));
+      out[1] = make_uint4(static_cast<uint32_t>(w2), static_cast<uint32_t>(w2 >> 32),
+                          static_cast<uint32_t>(w3), static_cast<uint32_t>(w3 >> 32));
+    } else {
+      uint32_t dw[6];
+#pragma unroll
+      for (uint32_t k = 0; k < 3; ++k) {
+        dw[2 * k] = spread16(b[u][k]) | (spread16(h[u][k]) << 1);
+        dw[2 * k + 1] = spread16(b[u][k] >> 16) | (spread16(h[u][k] >> 16) << 1);
+      }
+      out[0] = make_uint4(e[0], e[1] & 0xFFFFu, dw[0], dw[1]);
+      out[1] = make_uint4(dw[2], dw[3], dw[4], dw[5]);
+    }
+    if (ds && sh) {
+      // entry k of a digit names the block holding its (k R + 1)-th
+      // occurrence: the block's first entry of a digit by a predicated store
+      uint32_t most = 0;
+#pragma unroll
+      for (uint32_t d = 0; d < S; ++d) {
+        uint32_t const x = remainder[d] + ((e[d >> 1] >> (16 * (d & 1))) & 0xFFFFu);
+        uint32_t const off = (0u - x) & rm;  // occurrences of the block before an entry
+        if (off < c[u][d]) entry[d][(x + rm) >> sh] = static_cast<uint32_t>(blk + u);
+        most = max(most, c[u][d]);
+      }
+      if (most > rm + 1)  // only then can there be more than one
+#pragma unroll
+        for (uint32_t d = 0; d < S; ++d) {
+          uint32_t const x = remainder[d] + ((e[d >> 1] >> (16 * (d & 1))) & 0xFFFFu);
+          uint32_t k = (x + rm) >> sh;
+          for (uint32_t o = ((0u - x) & rm) + rm + 1; o < c[u][d]; o += rm + 1)
+            entry[d][++k] = static_cast<uint32_t>(blk + u);
+        }
+    }
   }
 }
 
@@ -590,11 +580,15 @@ void build_group_level(GroupStore& qs, GroupLevel const& ql, GroupPlanes const& 
                        DevBuf& chunk, uint32_t* err, cudaStream_t st) {
   uint64_t const nsb = ceil_div(ql.num_blocks, uint64_t(GroupShape<W>::kSbBlocks));
   uint64_t* const sb = qs.sb.as<uint64_t>() + ql.sb_off;
+  constexpr uint32_t S = 1u << W;
+  uint32_t const chunks = static_cast<uint32_t>(ceil_div(nsb + 1, kScanChunk));
+  EWT_CUDA(cudaMemsetAsync(chunk.get(), 0, uint64_t(chunks) * S * 8, st));
   group_counts_kernel<W><<<static_cast<uint32_t>(ceil_div(nsb + 1, 8)), 256, 0, st>>>(
-      g, n, nsb, sb);
+      g, n, nsb, sb, chunk.as<unsigned long long>());
   EWT_LAUNCHED();
-  scan_superblocks<(1u << W)>(sb, nsb + 1, chunk, st);
-  group_level_kernel<W><<<static_cast<uint32_t>(nsb), 512, 0, st>>>(
+  group_scan_kernel<S><<<chunks, kScanChunk, 0, st>>>(sb, nsb + 1, chunk.as<uint64_t>());
+  EWT_LAUNCHED();
+  group_level_kernel<W><<<static_cast<uint32_t>(nsb), 256, 0, st>>>(
       g, n, ql, qs.blocks.as<uint4>() + ql.blk_off * 2, sb, nsb,
       qs.ds.get() ? qs.ds.as<uint32_t>() : nullptr, err);
   EWT_LAUNCHED();

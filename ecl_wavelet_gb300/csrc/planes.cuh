@@ -832,6 +832,12 @@ plane_pass_kernel(const __grid_constant__ PlanePass p) {
           store_slot<W>(buf + 8 + (j - 1) * kPS + tid * W, zero);
         }
       }
+      // the chunk's next tile, on its way to L2 (1.7 % of the pass)
+      if (ti + 1 < tiles && (ti + 1) * p.g.tile + tid * kSlotBits < len_c) {
+        uint64_t const at = (ts + p.g.tile + uint64_t(tid) * kSlotBits) >> 5;
+        for (uint32_t j = 0; j <= np; ++j)
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(p.src[j] + at));
+      }
       // ---- class tables
       if (wid == 0) {  // prefix of the tile's digit counts
         uint32_t const own =
