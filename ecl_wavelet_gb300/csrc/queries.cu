@@ -147,18 +147,22 @@ query_kernel(TreeView t, uint8_t const* __restrict__ types,
   if (bad) atomicOr(err, 1u);
 }
 
-// Batched mixed form: CTAs take 2048-query chunks of the interleaved batch,
-// sort each chunk's query numbers by type in shared memory (warp ballots),
-// then walk the access, rank and select lists in turn, so every warp runs
-// one kind of walk.  Results go straight to their original slots.
+// Batched mixed form: CTAs take chunks of up to 2048 queries of the interleaved
+// batch, sort each chunk's query numbers by type in shared memory (warp
+// ballots), then walk the access, rank and select lists one after the other,
+// each from a warp boundary on, so every warp runs one kind of walk and the
+// kinds run side by side.  Results go straight to their original slots.
 constexpr uint32_t kMixChunk = 2048;
+// Smallest chunk: with fewer queries the staged tables cost more than the walks.
+constexpr uint32_t kMixChunkMin = 64;
 
 template <class T>
 __global__ void __launch_bounds__(kMaxQueryThreads)
 mixed_kernel(TreeView t, uint8_t const* __restrict__ types,
              QueryRec<T> const* __restrict__ in, uint64_t m,
              uint64_t* __restrict__ out, uint32_t* __restrict__ err,
-             uint32_t stage_counts, uint32_t stage_ranks, uint32_t* queue) {
+             uint32_t stage_counts, uint32_t stage_ranks, uint32_t* queue,
+             uint32_t chunk) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ uint16_t lists[3][kMixChunk];
   __shared__ uint32_t list_len[3];
@@ -197,13 +201,13 @@ mixed_kernel(TreeView t, uint8_t const* __restrict__ types,
   uint32_t const lane = threadIdx.x & 31;
   uint32_t const lt = (1u << lane) - 1u;
   uint32_t bad = 0;
-  uint64_t const chunks = (m + kMixChunk - 1) / kMixChunk;
+  uint64_t const chunks = (m + chunk - 1) / chunk;
   for (uint64_t c = wq_take(queue, &next_chunk, 0, true); c < chunks;
        c = wq_take(queue, &next_chunk, c, false)) {
-    uint64_t const base = c * kMixChunk;
+    uint64_t const base = c * chunk;
     if (threadIdx.x < 3) list_len[threadIdx.x] = 0;
     __syncthreads();
-    for (uint32_t j = threadIdx.x; j < kMixChunk; j += blockDim.x) {
+    for (uint32_t j = threadIdx.x; j < chunk; j += blockDim.x) {
       uint64_t const q = base + j;
       uint32_t const ty = q < m ? types[q] : 3u;
 #pragma unroll
@@ -221,35 +225,31 @@ mixed_kernel(TreeView t, uint8_t const* __restrict__ types,
       }
     }
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < list_len[0]; i += blockDim.x) {
-      uint64_t const q = base + lists[0][i];
-      uint64_t const idx = in[q].index;
-      out[q] = idx < t.n ? static_cast<uint64_t>(from_minimal<T>(
-                               t, wt_access(t, meta, counts, ranks, node_base,
-                                            idx, walk)))
-                         : 0;
-    }
-    for (uint32_t i = threadIdx.x; i < list_len[1]; i += blockDim.x) {
-      uint64_t const q = base + lists[1][i];
+    // selects first: their walks are the longest
+    uint32_t const e2 = (list_len[2] + 31) & ~31u, e1 = e2 + ((list_len[1] + 31) & ~31u);
+    uint32_t const e0 = e1 + list_len[0];
+    for (uint32_t i = threadIdx.x; i < e0; i += blockDim.x) {
+      uint32_t const k = i < e2 ? 2u : i < e1 ? 1u : 0u;
+      uint32_t const at = i - (k == 2 ? 0u : k == 1 ? e2 : e1);
+      if (at >= list_len[k]) continue;
+      uint64_t const q = base + lists[k][at];
+      if (k == 0) {
+        uint64_t const idx = in[q].index;
+        out[q] = idx < t.n ? static_cast<uint64_t>(from_minimal<T>(
+                                 t, wt_access(t, meta, counts, ranks, node_base, idx, walk)))
+                           : 0;
+        continue;
+      }
       QueryRec<T> const r = in[q];
       uint64_t const sym = to_minimal<T>(t, r.symbol);
-      if (sym >= t.sigma || r.index > t.n) {
-        out[q] = UINT64_MAX;
+      uint64_t res = UINT64_MAX;
+      if (sym >= t.sigma || (k == 1 ? r.index > t.n : r.index == 0))
         bad = 1;
-      } else {
-        out[q] = wt_rank(t, meta, counts, ranks, node_base, sym, r.index, walk);
-      }
-    }
-    for (uint32_t i = threadIdx.x; i < list_len[2]; i += blockDim.x) {
-      uint64_t const q = base + lists[2][i];
-      QueryRec<T> const r = in[q];
-      uint64_t const sym = to_minimal<T>(t, r.symbol);
-      if (sym >= t.sigma || r.index == 0) {
-        out[q] = UINT64_MAX;
-        bad = 1;
-      } else {
-        out[q] = wt_select(t, meta, counts, ranks, node_base, sym, r.index, walk);
-      }
+      else if (k == 1)
+        res = wt_rank(t, meta, counts, ranks, node_base, sym, r.index, walk);
+      else
+        res = wt_select(t, meta, counts, ranks, node_base, sym, r.index, walk);
+      out[q] = res;
     }
     __syncthreads();  // lists are reused by the next chunk
   }
@@ -314,14 +314,19 @@ void launch_mixed_kernel(ewt_tree& t, uint8_t const* types, void const* in,
                                                          p.bytes));
   per_sm = std::max(per_sm, 1);
   if (t.tune_blocks[kMixed]) per_sm = std::min<int>(per_sm, t.tune_blocks[kMixed]);
-  uint64_t const chunks = ceil_div(m, kMixChunk);
-  uint32_t const blocks = static_cast<uint32_t>(
-      std::min<uint64_t>(chunks, uint64_t(per_sm) * sm_count()));
+  // chunks small enough that a batch occupies all the CTAs that fit (device
+  // batches over 16 Mi symbols of 256: 1 Ki queries 26.7 -> 14.5 us, 128 Ki
+  // 46 -> 18.6 us, 4 Mi 226 -> 197 us, the last by the lists side by side)
+  uint64_t const full = uint64_t(per_sm) * sm_count();
+  uint32_t const chunk = static_cast<uint32_t>(std::min<uint64_t>(
+      kMixChunk, std::max<uint64_t>(kMixChunkMin, ceil_div(ceil_div(m, full), 32) * 32)));
+  uint64_t const chunks = ceil_div(m, chunk);
+  uint32_t const blocks = static_cast<uint32_t>(std::min<uint64_t>(chunks, full));
   PhaseTimer pt(EWT_PHASE_QUERY, s);
   mk<<<blocks, threads, p.bytes, s>>>(t.view, types,
                                       static_cast<QueryRec<T> const*>(in), m,
                                       out, err, p.stage_counts, p.stage_ranks,
-                                      queue);
+                                      queue, chunk);
   EWT_LAUNCHED();
 }
 
