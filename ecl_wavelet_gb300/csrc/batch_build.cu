@@ -132,7 +132,6 @@ void build_group(void const* const* texts, uint64_t const* lengths,
                            cudaMemcpyHostToDevice, st));
   uint64_t const stride_w = ceil_div(N, 32) + 64;  // words per group level
   DevBuf lw(L * stride_w * 4);
-  EWT_CUDA(cudaMemsetAsync(lw.get(), 0, L * stride_w * 4, st));
   DevBuf err(16);
   EWT_CUDA(cudaMemsetAsync(err.get(), 0, 16, st));
   uint32_t* const words = lw.as<uint32_t>();

@@ -45,11 +45,12 @@ struct RSStore {
 void build_rs_counts(RSStore& rs, uint32_t first, uint32_t last,
                      cudaStream_t stream);
 // Allocates and fills the select samples of every array (needs counts of
-// all arrays) and uploads the final meta table.
+// all arrays).  Asynchronous.
 void build_rs_samples(RSStore& rs, cudaStream_t stream);
-// Builds the query-side rank blocks of every array (needs the counts) and,
-// when rs.sel_shift > 0, the dense select samples in the same pass; uploads
-// the meta table with their offsets.
+// Takes the arrays' totals of ones over to the host meta table, builds the
+// query-side rank blocks of every array (needs the counts) and, when
+// rs.sel_shift > 0, the dense select samples in the same pass; uploads the
+// meta table with their offsets.
 void build_rank_blocks(RSStore& rs, cudaStream_t stream);
 // Rank-block start of every array (running totals; arrays without blocks
 // add none) and the total block count.

@@ -41,7 +41,7 @@
 // The reference re-sorts the whole text with a radix sort per level and
 // fills each level from it (wavelet_tree.cuh:806-818, 2422-2493); the bits
 // written here are identical.  Words shared by two runs are combined with
-// atomicOr into levels that are zeroed beforehand; all writes are
+// atomicOr, cleared beforehand (clear_edges_kernel); all writes are
 // bounds-checked.
 #pragma once
 
@@ -219,7 +219,7 @@ constexpr uint32_t kIngestThreads = 256;
 // of every plane out (128 bytes per warp and plane).  Map: codes come from a
 // table (256 entries in shared memory for bytes).
 template <class T, bool Map>
-__global__ void __launch_bounds__(kIngestThreads)
+__global__ void __launch_bounds__(kIngestThreads, sizeof(T) == 1 ? 6 : 2)
 ingest_planes_kernel(T const* __restrict__ text, IngestArgs a) {
   __shared__ uint32_t cnt[kMaxDigits * 32];
   __shared__ uint16_t lut_s[Map && sizeof(T) == 1 ? 256 : 1];
@@ -391,7 +391,7 @@ __device__ __forceinline__ void tally(uint32_t m, uint32_t const (&x)[D],
 constexpr uint32_t kCountThreads = 128;
 
 template <int D>
-__global__ void __launch_bounds__(kCountThreads)
+__global__ void __launch_bounds__(kCountThreads, 10)
 plane_counts_kernel(const __grid_constant__ PlaneSources src, TileGrid g) {
   __shared__ uint32_t sum[1 << D];
   uint32_t const tid = threadIdx.x, lane = tid & 31;
@@ -405,7 +405,7 @@ plane_counts_kernel(const __grid_constant__ PlaneSources src, TileGrid g) {
     uint32_t acc[1 << D];
 #pragma unroll
     for (int i = 0; i < (1 << D); ++i) acc[i] = 0;
-#pragma unroll 2
+#pragma unroll 1
     for (uint32_t w = tid; w * 32 < len; w += kCountThreads) {
       uint64_t const p0 = s + uint64_t(w) * 32;
       uint32_t const valid = min(32u, len - w * 32);
@@ -573,6 +573,46 @@ struct PlanePass {
   uint32_t ext_mask[kMaxPassK + 1];      // bit j: ext[r][j] is wanted
   uint32_t ext_words;
 };
+
+// Clears the words of a pass's outputs that two runs may share, into which
+// the pass ORs: every word that holds the start of a tile's class run, and the
+// arrays' ends (all other words are written whole by one thread).  A warp per
+// chunk, lane per digit: the chunk's digit positions, stepped from tile to
+// tile and added up per class.  (Clearing the outputs whole took 1.4 ms per
+// build of 6 Gi symbols of 256.)
+__global__ void __launch_bounds__(128)
+clear_edges_kernel(const __grid_constant__ PlanePass p) {
+  uint32_t const lane = threadIdx.x & 31, D = p.g.D, digits = 1u << D;
+  uint32_t const chunks = p.g.chunk_first[p.g.nodes];
+  uint64_t const w_end = p.g.n >> 5;
+  auto clear = [&](uint32_t r, uint64_t w) {
+    if (w < p.out_words[r]) p.out[r][w] = 0;
+    for (uint32_t mask = p.ext_mask[r]; mask; mask &= mask - 1)
+      if (w < p.ext_words) p.ext[r][__ffs(mask) - 1][w] = 0;
+  };
+  if (blockIdx.x == 0)
+    for (uint32_t r = 1; r <= p.k; ++r) {
+      uint64_t const lim = max(p.out_words[r], p.ext_mask[r] ? p.ext_words : 0u);
+      for (uint64_t w = w_end + threadIdx.x; w < lim; w += blockDim.x) clear(r, w);
+    }
+  for (uint32_t c = blockIdx.x * 4 + (threadIdx.x >> 5); c < chunks; c += gridDim.x * 4) {
+    uint32_t const N = owner_node(p.g.chunk_first, p.g.nodes, c);
+    uint32_t const t0 = p.g.tile_first[N] + (c - p.g.chunk_first[N]) * p.g.ct;
+    uint32_t const t1 = min(t0 + p.g.ct, p.g.tile_first[N + 1]);
+    bool const on = lane < digits;
+    uint64_t const start = on ? p.g.starts_next[(uint64_t(N) << D) + lane] : 0;
+    uint64_t pre = on ? p.g.chunk_pre[(uint64_t(c) << D) + lane] : 0;
+    for (uint32_t t = t0; t < t1; ++t) {
+      uint64_t sum = pre;  // of the lane's class
+      for (uint32_t r = D; r > 0; --r) {
+        uint32_t const h = 1u << (D - r);  // digits of a level-r class
+        if (h > 1) sum += __shfl_xor_sync(0xffffffffu, sum, h >> 1);
+        if (r <= p.k && on && (lane & (h - 1)) == 0) clear(r, (start + sum) >> 5);
+      }
+      if (on) pre += p.g.tile_cnt[(uint64_t(t) << D) + lane];
+    }
+  }
+}
 
 // Swap masks of the five in-word stages for one word of the mask plane with
 // r0 ones before it in the slot: c[s] holds the positions q of the left
@@ -1095,8 +1135,8 @@ struct PlaneText {
   int ingest_phase = EWT_PHASE_FILL;
 };
 
-// Levels 0 .. L-1 of a text: level l at words[l] (word_count[l] words; levels
-// above 0 zeroed beforehand), and starts_out, (nodes << L) + 1 entries: the
+// Levels 0 .. L-1 of a text: level l at words[l] (word_count[l] words, zero
+// past the text's end on levels above 0), and starts_out, (nodes << L) + 1 entries: the
 // start of every code's symbols.  `wanted`: (level, planes) pairs, the planes
 // that many levels below `level` in its order are kept and returned.
 template <class T>
@@ -1116,19 +1156,16 @@ std::vector<OrderPlanes> run_plane_passes(
     return 0;
   };
   std::vector<OrderPlanes> kept;
-  auto make_order = [&](uint32_t level, uint32_t count, bool zero) {
+  auto make_order = [&](uint32_t level, uint32_t count) {
     OrderPlanes o;
     o.level = level;
     o.first = level + 1;
     o.count = count;
     o.stride = stride;
-    if (count) {
-      o.mem.alloc(count * stride * 4);
-      if (zero) EWT_CUDA(cudaMemsetAsync(o.mem.get(), 0, count * stride * 4, st));
-    }
+    if (count) o.mem.alloc(count * stride * 4);
     return o;
   };
-  OrderPlanes cur = make_order(0, L - 1, false);
+  OrderPlanes cur = make_order(0, L - 1);
   DevBuf starts_buf[2], tile_first, chunk_first, range_first, tile_cnt, chunk_pre, range_tot;
   uint32_t nodes = x.nodes;
   uint64_t* starts = x.starts;
@@ -1247,7 +1284,7 @@ std::vector<OrderPlanes> run_plane_passes(
       bool const whole = r == k && !final;  // the next pass's input
       uint32_t const count = whole ? np - k : std::min(wants(a + r), np - r);
       if (!count) continue;
-      OrderPlanes o = make_order(a + r, count, true);
+      OrderPlanes o = make_order(a + r, count);
       for (uint32_t j = 1; j <= count; ++j) {
         p.ext[r][r + j] = o.plane(a + r + j);
         p.ext_mask[r] |= 1u << (r + j);
@@ -1257,6 +1294,10 @@ std::vector<OrderPlanes> run_plane_passes(
     }
     {
       PhaseTimer pt(EWT_PHASE_SPLIT, st);
+      clear_edges_kernel<<<static_cast<uint32_t>(std::min<uint64_t>(
+                               ceil_div(max_chunks, 4), uint64_t(sms) * 8)),
+                           128, 0, st>>>(p);
+      EWT_LAUNCHED();
       launch_plane_pass(p, slots, max_chunks, st);
     }
     if (wants(a)) kept.push_back(std::move(cur));

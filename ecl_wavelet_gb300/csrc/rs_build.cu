@@ -7,8 +7,8 @@
 //   s1[k]  = position of the (k+1)*4096-th one, s0 likewise for zeros.
 // Kernels: one CTA per 65,536-bit L1 block counts its 128 L2 blocks with
 // 128-bit coalesced loads and a CTA scan; one CTA per array scans the L1
-// block totals; one thread per 512-bit block emits the (at most one) one-
-// and zero-sample that falls inside it.  No kernel waits on another CTA.
+// block totals; a warp per L1 block emits the (at most one) one- and
+// zero-sample of each of its 512-bit blocks.  No kernel waits on another CTA.
 #include <algorithm>
 
 #include "internal.cuh"
@@ -27,7 +27,7 @@ struct BlockJob {
 
 void RSStore::layout(std::vector<uint64_t> const& bits, uint64_t stride, DevBuf* filled) {
   meta.assign(bits.size(), ArrayMeta{});
-  total_words = total_l1 = total_l2 = 0;
+  total_words = total_l1 = total_l2 = total_s1 = 0;
   for (size_t a = 0; a < bits.size(); ++a) {
     ArrayMeta& m = meta[a];
     m.bits = bits[a];
@@ -41,7 +41,12 @@ void RSStore::layout(std::vector<uint64_t> const& bits, uint64_t stride, DevBuf*
     m.l2_off = total_l2;
     total_l1 += m.num_l1;
     total_l2 += (m.num_l1 - 1) * kL2PerL1 + m.num_last_l2;
+    // room for the samples of an array of zeros or ones alone in either list,
+    // so that their places do not depend on the counts
+    m.s0_off = m.s1_off = total_s1;
+    total_s1 += m.bits / kSampleRate;
   }
+  total_s0 = total_s1;
   total_words += total_words % 2;
   // 16 words of slack: readers may fetch one word past an array's end
   if (filled) words = std::move(*filled);
@@ -194,21 +199,6 @@ rs_l1_scan_kernel(BlockJob const* jobs, uint32_t first_array,
   if (t == 0) meta[first_array + blockIdx.x].ones = carry_s;
 }
 
-struct SampleJob {
-  uint64_t word_off, bits, l1_off, l2_off, num_l1, num_l2, ones, s0_off,
-      s1_off;
-};
-
-__device__ __forceinline__ uint32_t find_sjob(SampleJob const* jobs,
-                                              uint32_t count, uint64_t g) {
-  uint32_t lo = 0, hi = count - 1;
-  while (lo < hi) {
-    uint32_t const mid = (lo + hi + 1) >> 1;
-    if (jobs[mid].l2_off <= g) lo = mid; else hi = mid - 1;
-  }
-  return lo;
-}
-
 // Position inside the 512-bit block of the r-th (1-based) `value` bit.
 __device__ __forceinline__ uint32_t select_in_block(uint32_t const* blk,
                                                     uint32_t r, int value) {
@@ -221,40 +211,59 @@ __device__ __forceinline__ uint32_t select_in_block(uint32_t const* blk,
   return kL2Bits;  // not reached
 }
 
-// One thread per L2 block of every array.
+// Select samples of every array: a warp per L1 block, four L2 blocks per
+// lane, so the array is looked up once for 65,536 bits and only lanes whose
+// blocks hold a sample read bits.  (A thread per L2 block that looked its
+// array up took 1.28 ms for the eight levels of 6 Gi symbols.)
 __global__ void __launch_bounds__(256)
 rs_samples_kernel(uint32_t const* __restrict__ words,
                   uint64_t const* __restrict__ l1,
-                  uint16_t const* __restrict__ l2, SampleJob const* jobs,
-                  uint32_t num_jobs, uint64_t total_l2,
+                  uint16_t const* __restrict__ l2, BlockJob const* jobs,
+                  ArrayMeta const* __restrict__ meta, uint32_t num_jobs, uint64_t total_l1,
                   uint64_t* __restrict__ s0, uint64_t* __restrict__ s1) {
-  uint64_t const g = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
-  if (g >= total_l2) return;
-  SampleJob const job = jobs[find_sjob(jobs, num_jobs, g)];
-  uint64_t const k = g - job.l2_off;  // L2 block inside the array
-  uint64_t const b = k / kL2PerL1;
-  uint64_t const l1v = l1[job.l1_off + b];
-  uint64_t const before1 = l1v + l2[g];
-  uint64_t after1;
-  if ((k + 1) % kL2PerL1 != 0 && k + 1 < job.num_l2)
-    after1 = l1v + l2[g + 1];
-  else if (b + 1 < job.num_l1)
-    after1 = l1[job.l1_off + b + 1];
-  else
-    after1 = job.ones;
-  uint64_t const bit0 = k * kL2Bits;
-  uint64_t const nbits = min(job.bits - bit0, kL2Bits);
-  uint64_t const before0 = bit0 - before1;
-  uint64_t const after0 = bit0 + nbits - after1;
-  uint32_t const* blk = words + job.word_off + k * kL2Words;
-  uint64_t const t1 = (before1 / kSampleRate + 1) * kSampleRate;
-  if (t1 <= after1)
-    s1[job.s1_off + t1 / kSampleRate - 1] =
-        bit0 + select_in_block(blk, static_cast<uint32_t>(t1 - before1), 1);
-  uint64_t const t0 = (before0 / kSampleRate + 1) * kSampleRate;
-  if (t0 <= after0)
-    s0[job.s0_off + t0 / kSampleRate - 1] =
-        bit0 + select_in_block(blk, static_cast<uint32_t>(t0 - before0), 0);
+  uint64_t const g = (blockIdx.x * uint64_t(blockDim.x) + threadIdx.x) >> 5;
+  uint32_t const lane = threadIdx.x & 31;
+  if (g >= total_l1) return;
+  uint32_t const a = find_job(jobs, num_jobs, g);
+  BlockJob const job = jobs[a];
+  ArrayMeta const& m = meta[a];
+  uint64_t const b = g - job.l1_off;  // L1 block inside the array
+  bool const last = b + 1 == job.num_l1;
+  uint64_t const bit_b = b * kL1Bits, end_b = last ? job.bits : bit_b + kL1Bits;
+  uint64_t const ones_b = l1[g], ones_e = last ? m.ones : l1[g + 1];
+  uint32_t const nblk = static_cast<uint32_t>((end_b - bit_b + kL2Bits - 1) / kL2Bits);
+  uint16_t const* const c = l2 + job.l2_off + b * kL2PerL1;
+  // ones of the L1 block before L2 block 4 lane + i; the block's end past nblk
+  uint32_t const all = static_cast<uint32_t>(ones_e - ones_b);
+  uint32_t x[5];
+#pragma unroll
+  for (uint32_t i = 0; i < 4; ++i) {
+    uint32_t const k = lane * 4 + i;
+    x[i] = k < nblk ? c[k] : all;
+  }
+  uint32_t const next = __shfl_down_sync(0xffffffffu, x[0], 1);
+  x[4] = lane == 31 ? all : next;
+  uint32_t const* const blk = words + job.word_off + b * (kL1Bits / 32);
+  uint64_t const zeros_b = bit_b - ones_b;
+#pragma unroll
+  for (uint32_t i = 0; i < 4; ++i) {
+    uint32_t const k = lane * 4 + i;
+    if (k >= nblk) break;
+    uint64_t const bit0 = bit_b + uint64_t(k) * kL2Bits;
+    uint64_t const bit1 = min(bit0 + kL2Bits, end_b);
+    // the next sample at or below the block's end
+    uint64_t const o0 = ones_b + x[i], o1 = ones_b + x[i + 1];
+    uint64_t const z0 = zeros_b + (bit0 - bit_b) - x[i], z1 = zeros_b + (bit1 - bit_b) - x[i + 1];
+    uint64_t const t1 = o1 / kSampleRate, t0 = z1 / kSampleRate;
+    if (t1 > o0 / kSampleRate)
+      s1[m.s1_off + t1 - 1] =
+          bit0 + select_in_block(blk + k * kL2Words,
+                                 static_cast<uint32_t>(t1 * kSampleRate - o0), 1);
+    if (t0 > z0 / kSampleRate)
+      s0[m.s0_off + t0 - 1] =
+          bit0 + select_in_block(blk + k * kL2Words,
+                                 static_cast<uint32_t>(t0 * kSampleRate - z0), 0);
+  }
 }
 
 }  // namespace
@@ -280,51 +289,16 @@ void build_rs_counts(RSStore& rs, uint32_t first, uint32_t last,
 }
 
 void build_rs_samples(RSStore& rs, cudaStream_t stream) {
-  uint32_t const count = static_cast<uint32_t>(rs.meta.size());
-  // Totals of ones were written on the device by the L1 scans.
-  std::vector<ArrayMeta> dm(count);
-  EWT_CUDA(cudaMemcpyAsync(dm.data(), rs.meta_d.get(), count * sizeof(ArrayMeta),
-                           cudaMemcpyDeviceToHost, stream));
-  EWT_CUDA(cudaStreamSynchronize(stream));
-  for (uint32_t a = 0; a < count; ++a) rs.meta[a].ones = dm[a].ones;
-  rs.total_s0 = rs.total_s1 = 0;
-  for (auto& m : rs.meta) {
-    m.s1_off = rs.total_s1;
-    m.s0_off = rs.total_s0;
-    rs.total_s1 += m.ones / kSampleRate;
-    rs.total_s0 += (m.bits - m.ones) / kSampleRate;
-  }
   rs.s0.alloc(rs.total_s0 * 8);
   rs.s1.alloc(rs.total_s1 * 8);
-  EWT_CUDA(cudaMemcpyAsync(rs.meta_d.get(), rs.meta.data(),
-                           count * sizeof(ArrayMeta), cudaMemcpyHostToDevice,
-                           stream));
-  if (rs.total_s0 + rs.total_s1 > 0) {
-    std::vector<SampleJob> jobs(count);
-    for (uint32_t a = 0; a < count; ++a) {
-      ArrayMeta const& m = rs.meta[a];
-      jobs[a] = {m.word_off, m.bits, m.l1_off, m.l2_off, m.num_l1,
-                 (m.num_l1 - 1) * kL2PerL1 + m.num_last_l2, m.ones, m.s0_off,
-                 m.s1_off};
-    }
-    DevBuf jobs_d(count * sizeof(SampleJob));
-    EWT_CUDA(cudaMemcpyAsync(jobs_d.get(), jobs.data(),
-                             count * sizeof(SampleJob), cudaMemcpyHostToDevice,
-                             stream));
-    uint64_t const total_l2 = rs.meta.back().l2_off +
-                              (rs.meta.back().num_l1 - 1) * kL2PerL1 +
-                              rs.meta.back().num_last_l2;
-    uint64_t const blocks = ceil_div(total_l2, 256);
-    PhaseTimer pt(EWT_PHASE_SAMPLES, stream);
-    rs_samples_kernel<<<static_cast<uint32_t>(blocks), 256, 0, stream>>>(
-        rs.words.as<uint32_t>(), rs.l1.as<uint64_t>(), rs.l2.as<uint16_t>(),
-        jobs_d.as<SampleJob>(), count, total_l2, rs.s0.as<uint64_t>(),
-        rs.s1.as<uint64_t>());
-    EWT_LAUNCHED();
-    EWT_CUDA(cudaStreamSynchronize(stream));
-  } else {
-    EWT_CUDA(cudaStreamSynchronize(stream));
-  }
+  if (rs.total_s1 == 0) return;
+  PhaseTimer pt(EWT_PHASE_SAMPLES, stream);
+  rs_samples_kernel<<<static_cast<uint32_t>(ceil_div(rs.total_l1, 8)), 256, 0, stream>>>(
+      rs.words.as<uint32_t>(), rs.l1.as<uint64_t>(), rs.l2.as<uint16_t>(),
+      rs.jobs_d.as<BlockJob>(), rs.meta_d.as<ArrayMeta>(),
+      static_cast<uint32_t>(rs.meta.size()), rs.total_l1, rs.s0.as<uint64_t>(),
+      rs.s1.as<uint64_t>());
+  EWT_LAUNCHED();
 }
 
 namespace {
@@ -459,6 +433,13 @@ uint64_t rank_block_starts(std::vector<ArrayMeta> const& meta,
 
 void build_rank_blocks(RSStore& rs, cudaStream_t stream) {
   uint32_t const count = static_cast<uint32_t>(rs.meta.size());
+  {  // the totals of ones that the L1 scans left on the device
+    std::vector<ArrayMeta> dm(count);
+    EWT_CUDA(cudaMemcpyAsync(dm.data(), rs.meta_d.get(), count * sizeof(ArrayMeta),
+                             cudaMemcpyDeviceToHost, stream));
+    EWT_CUDA(cudaStreamSynchronize(stream));
+    for (uint32_t a = 0; a < count; ++a) rs.meta[a].ones = dm[a].ones;
+  }
   std::vector<uint64_t> start(count);
   uint64_t total = 0, highs = 0;
   for (uint32_t a = 0; a < count; ++a) {

@@ -512,7 +512,7 @@ std::vector<OrderPlanes> run_passes(ewt_tree& t, PlaneText<U> const& x, uint32_t
   for (uint32_t l = 0; l < x.L; ++l) out[l] = words + l * stride;
   // level 0 is written whole but for its padding
   uint64_t const w0 = ceil_div(x.n, 32);
-  EWT_CUDA(cudaMemsetAsync(words + w0, 0, (x.L * stride - w0) * 4, st));
+  if (stride > w0) EWT_CUDA(cudaMemsetAsync(words + w0, 0, (stride - w0) * 4, st));
   return run_plane_passes<U>(x, out.data(), count.data(), starts,
                              groups ? group_planes(x.L)
                                     : std::vector<std::pair<uint32_t, uint32_t>>{},
