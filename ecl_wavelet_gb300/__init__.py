@@ -494,8 +494,8 @@ class RankSelect:
 
     def __init__(self, words_per_array, bits, gpu_index: int = 0):
         bits = np.ascontiguousarray(bits, dtype=np.uint64)
-        words = np.concatenate([np.asarray(w, dtype=np.uint32)
-                                for w in words_per_array]).astype(np.uint32)
+        parts = [np.ascontiguousarray(w, dtype=np.uint32) for w in words_per_array]
+        words = parts[0] if len(parts) == 1 else np.concatenate(parts)
         self._h = C.c_void_p()
         _check(lib().ewt_rs_build(_ptr(words), bits.ctypes.data_as(_U64P),
                                   bits.size, gpu_index, C.byref(self._h)),

@@ -46,7 +46,7 @@ struct SharedStore {
   ~SharedStore() {
     DeviceGuard g(device);
     for (DevBuf* b : {&rs.words, &rs.l1, &rs.l2, &rs.s0, &rs.s1, &rs.meta_d,
-                      &rs.jobs_d, &rs.rb, &rs.ds, &tables})
+                      &rs.rb, &rs.ds, &tables})
       b->reset();  // stream-ordered frees, then the stream goes
     if (stream) {
       cudaStreamSynchronize(stream);
@@ -180,7 +180,6 @@ void build_group(void const* const* texts, uint64_t const* lengths,
   uint32_t const arrays = G * L;
   build_rs_counts(rs, 0, arrays, st);
   build_rs_samples(rs, st);
-  rs.skip_blocks.assign(arrays, 0);
   build_rank_blocks(rs, st);
   // ---- symbol counts of every text: the starts of its symbols
   std::vector<uint64_t> c_host(uint64_t(G) * sigma + 1);

@@ -134,37 +134,26 @@ void ensure(DevBuf& b, size_t& cap, size_t bytes) {
   cap = bytes;
 }
 
-// Reads and clears the tree's invalid-query word.
-int take_query_status(DevBuf& err, cudaStream_t s) {
+__global__ void status_kernel(uint32_t* err, uint32_t* host) {
+  *host = *err;
+  *err = 0;
+}
+
+// Reads and clears the invalid-query word `err`; on a GPU that can write the
+// host's memory a kernel hands it over (two microseconds; a copy to pageable
+// memory and a memset took ten), into a word of the tree's own.
+int take_query_status(DevBuf& err, uint32_t* word, int dev, cudaStream_t s) {
+  if (word && pageable_access(dev)) {
+    status_kernel<<<1, 1, 0, s>>>(err.as<uint32_t>(), word);
+    EWT_LAUNCHED();
+    EWT_CUDA(cudaStreamSynchronize(s));
+    return *const_cast<uint32_t volatile*>(word) ? EWT_ERR_QUERY : EWT_OK;
+  }
   uint32_t e = 0;
   EWT_CUDA(cudaMemcpyAsync(&e, err.get(), 4, cudaMemcpyDeviceToHost, s));
   EWT_CUDA(cudaMemsetAsync(err.get(), 0, 4, s));
   EWT_CUDA(cudaStreamSynchronize(s));
   return e ? EWT_ERR_QUERY : EWT_OK;
-}
-
-__global__ void mask_tails_kernel(uint32_t* words, ArrayMeta const* meta,
-                                  uint32_t count) {
-  uint32_t const a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a >= count) return;
-  ArrayMeta const m = meta[a];
-  if (m.bits % 32)
-    words[m.word_off + m.bits / 32] &= (1u << (m.bits % 32)) - 1u;
-}
-
-// Bits past each array's end -- in its last word and in the padding words
-// up to the next 32-word boundary -- set to zero (arrays filled by callers).
-__global__ void clear_tails_kernel(uint32_t* words, ArrayMeta const* meta,
-                                   uint32_t count) {
-  uint32_t const a = blockIdx.x;
-  if (a >= count) return;
-  ArrayMeta const m = meta[a];
-  uint64_t const w = (m.bits + 31) / 32;
-  uint64_t const padded = (w + 31) / 32 * 32;
-  uint32_t const t = threadIdx.x;  // 32 threads
-  if (t == 0 && m.bits % 32)
-    words[m.word_off + m.bits / 32] &= (1u << (m.bits % 32)) - 1u;
-  if (w + t < padded) words[m.word_off + w + t] = 0u;
 }
 
 }  // namespace
@@ -221,7 +210,6 @@ int host_batch(ewt_tree* t, void const* in, size_t in_rec, uint8_t const* types,
       // large batches: copies in and out overlap the kernels chunk by chunk
       // (copy engines reach the C2C bandwidth; the kernel then works on
       // device memory only)
-      populate_for_write(out, m * out_rec);
       QueryPipe& P = t->pipe;
       P.init();
       uint64_t const chunk = std::max<uint64_t>(kPipeMin / 4, ceil_div(m, 8));
@@ -248,12 +236,14 @@ int host_batch(ewt_tree* t, void const* in, size_t in_rec, uint8_t const* types,
         launch(P.types[x].as<uint8_t>(), P.in[x].get(), k, P.out[x].get(), s);
         EWT_CUDA(cudaEventRecord(P.k_done[x], s));
         EWT_CUDA(cudaStreamWaitEvent(P.s_out, P.k_done[x], 0));
+        // pages of the chunk's results, while the GPU works on it
+        populate_for_write(static_cast<char*>(out) + b * out_rec, k * out_rec);
         EWT_CUDA(cudaMemcpyAsync(static_cast<char*>(out) + b * out_rec, P.out[x].get(),
                                  k * out_rec, cudaMemcpyDefault, P.s_out));
         EWT_CUDA(cudaEventRecord(P.out_done[x], P.s_out));
       }
       EWT_CUDA(cudaStreamWaitEvent(s, P.out_done[(i - 1) & 1], 0));
-      int const st = take_query_status(t->err_d, s);
+      int const st = take_query_status(t->err_d, &t->status_word, t->device, s);
       if (st != EWT_OK)
         throw Error(st, "the batch held invalid queries (their results are "
                         "UINT64_MAX)");
@@ -264,7 +254,7 @@ int host_batch(ewt_tree* t, void const* in, size_t in_rec, uint8_t const* types,
       // place (host page tables): no staging copies
       populate_for_write(out, m * out_rec);
       launch(types, in, m, out, s);
-      int const st = take_query_status(t->err_d, s);
+      int const st = take_query_status(t->err_d, &t->status_word, t->device, s);
       if (st != EWT_OK)
         throw Error(st, "the batch held invalid queries (their results are "
                         "UINT64_MAX)");
@@ -288,7 +278,7 @@ int host_batch(ewt_tree* t, void const* in, size_t in_rec, uint8_t const* types,
                                sc.out.get(), k * out_rec, cudaMemcpyDefault,
                                s));
     }
-    int const st = take_query_status(t->err_d, s);
+    int const st = take_query_status(t->err_d, &t->status_word, t->device, s);
     if (st != EWT_OK)
       throw Error(st, "the batch held invalid queries (their results are "
                       "UINT64_MAX)");
@@ -309,7 +299,7 @@ int rs_host_batch(ewt_rs* r, uint64_t const* in, uint64_t m, uint64_t* out,
     if (pageable_access(r->device)) {  // in place, as host_batch
       populate_for_write(out, m * 8);
       launch(in, m, out, r->stream);
-      int const st = take_query_status(r->err_d, r->stream);
+      int const st = take_query_status(r->err_d, &r->status_word, r->device, r->stream);
       if (st != EWT_OK)
         throw Error(st, "the batch held invalid queries (their results are "
                         "UINT64_MAX)");
@@ -327,7 +317,7 @@ int rs_host_batch(ewt_rs* r, uint64_t const* in, uint64_t m, uint64_t* out,
       EWT_CUDA(cudaMemcpyAsync(out + b, sc.out.get(), k * 8, cudaMemcpyDefault,
                                s));
     }
-    int const st = take_query_status(r->err_d, s);
+    int const st = take_query_status(r->err_d, &r->status_word, r->device, s);
     if (st != EWT_OK)
       throw Error(st, "the batch held invalid queries (their results are "
                       "UINT64_MAX)");
@@ -455,10 +445,7 @@ int ewt_free(ewt_tree* t) {
       cudaStream_t const st = t->stream;
       if (st) cudaStreamSynchronize(st);
       delete t;  // device buffers are freed in the stream's order
-      if (st) {
-        cudaStreamSynchronize(st);
-        cudaStreamDestroy(st);
-      }
+      if (st) cudaStreamDestroy(st);  // (goes once they are)
     }
   });
 }
@@ -604,7 +591,7 @@ int ewt_query_status(ewt_tree* t, void* stream) {
     DeviceGuard dg(t->device);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     EWT_CUDA(cudaStreamSynchronize(s));
-    st = take_query_status(t->err_d, t->stream);
+    st = take_query_status(t->err_d, nullptr, t->device, t->stream);
   });
   if (g != EWT_OK) return g;
   if (st != EWT_OK) set_last_error("a batch held invalid queries");
@@ -649,12 +636,7 @@ int ewt_rs_build(const uint32_t* words, const uint64_t* bits,
                                  words + off, w * 4, cudaMemcpyDefault, st));
         off += w;
       }
-      EWT_CUDA(cudaMemcpyAsync(r->rs.meta_d.get(), r->rs.meta.data(),
-                               num_arrays * sizeof(ArrayMeta),
-                               cudaMemcpyHostToDevice, st));
-      mask_tails_kernel<<<ceil_div(num_arrays, 128), 128, 0, st>>>(
-          r->rs.words.as<uint32_t>(), r->rs.meta_d.as<ArrayMeta>(), num_arrays);
-      EWT_LAUNCHED();
+      clear_tails(r->rs, st);
       build_rs_counts(r->rs, 0, num_arrays, st);
       build_rs_samples(r->rs, st);
       build_rank_blocks(r->rs, st);
@@ -720,11 +702,8 @@ int ewt_rs_build_in_place(ewt_rs* r) {
     EWT_CUDA(cudaDeviceSynchronize());
     cudaStream_t const st = r->stream;
     AllocStream as(st);
-    uint32_t const count = static_cast<uint32_t>(r->rs.meta.size());
-    clear_tails_kernel<<<count, 32, 0, st>>>(r->rs.words.as<uint32_t>(),
-                                             r->rs.meta_d.as<ArrayMeta>(), count);
-    EWT_LAUNCHED();
-    build_rs_counts(r->rs, 0, count, st);
+    clear_tails(r->rs, st);
+    build_rs_counts(r->rs, 0, static_cast<uint32_t>(r->rs.meta.size()), st);
     build_rs_samples(r->rs, st);
     build_rank_blocks(r->rs, st);
     EWT_CUDA(cudaStreamSynchronize(st));

@@ -20,11 +20,11 @@ using ecl::detail::TreeView;
 // do: arrays padded to 32-word multiples, total word count even.
 struct RSStore {
   std::vector<ArrayMeta> meta;  // host copy
-  DevBuf words, l1, l2, s0, s1, meta_d, jobs_d, rb, ds;
+  DevBuf words, l1, l2, s0, s1, meta_d, rb, ds;
   uint64_t total_words = 0, total_l1 = 0, total_l2 = 0;
   uint64_t total_s0 = 0, total_s1 = 0;
   uint32_t sel_shift = ecl::detail::kDefaultSelShift;  // dense sample rate
-  std::vector<uint8_t> skip_blocks;  // arrays built without rank blocks
+  std::vector<uint8_t> skip_blocks;  // arrays built without rank blocks (set before layout)
 
   // Lays out arrays of the given bit lengths and allocates words (zeroed),
   // L1, L2 and the device meta table.  Samples are allocated by build_rs.
@@ -39,6 +39,8 @@ struct RSStore {
   }
 };
 
+// Clears the bits past every array's end, up to its padding's end.
+void clear_tails(RSStore& rs, cudaStream_t st);
 // Builds L2/L1/total counts for arrays [first, last) of `rs` on `stream`
 // (the words must be final); totals land in the device meta table only.
 // Asynchronous: no host synchronisation.
@@ -149,12 +151,14 @@ struct ewt_tree {
   std::vector<uint64_t> nodes_at_level, node_base, level_bits;
   ewt::RSStore rs;
   ewt::GroupStore groups;  // octal / quad query levels
+  ewt::DevBuf tables_d;  // node_base_d .. code_bits_d are parts of it (passes)
   ewt::DevBuf counts_d, ranks_d, node_base_d, nodes_at_level_d, code_len_d,
       code_bits_d, alphabet_d, err_d;
   ecl::detail::TreeView view{};
   std::mutex query_mu;  // host batch calls share scratch buffers
   ewt::QueryScratch scratch;
   ewt::QueryPipe pipe;
+  uint32_t status_word = 0;       // written by status_kernel (host calls)
   cudaStream_t stream = nullptr;  // library-owned stream for host calls
   // Trees of a batch build's short texts: their rank/select arrays and small
   // tables are views into a store shared by the batch's group, kept alive by
@@ -174,6 +178,7 @@ struct ewt_rs {
   ewt::DevBuf err_d;
   std::mutex query_mu;
   ewt::QueryScratch scratch;
+  uint32_t status_word = 0;
   cudaStream_t stream = nullptr;
 };
 

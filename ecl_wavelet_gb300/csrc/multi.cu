@@ -665,8 +665,15 @@ extern "C" int ewt_build_batch(const void* const* texts, const uint64_t* lengths
       uint64_t need = 0;
       for (uint32_t i = 0; i < count; ++i)
         need += lengths[i] * uint64_t(elem_size > 0 ? elem_size : 1) * 4 + (uint64_t(2) << 20);
+      uint64_t held = 0, used = 0;
+      bool const grown =  // an earlier batch's pool already has room
+          cudaMemPoolGetAttribute(lib_pool(), cudaMemPoolAttrReservedMemCurrent, &held) ==
+              cudaSuccess &&
+          cudaMemPoolGetAttribute(lib_pool(), cudaMemPoolAttrUsedMemCurrent, &used) ==
+              cudaSuccess &&
+          held - used >= need;
       size_t free_b = 0, total_b = 0;
-      if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && need < free_b / 2) {
+      if (!grown && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && need < free_b / 2) {
         void* p = nullptr;
         if (cudaMallocFromPoolAsync(&p, need, lib_pool(), nullptr) == cudaSuccess) {
           cudaFreeAsync(p, nullptr);
@@ -724,21 +731,29 @@ extern "C" int ewt_build_batch(const void* const* texts, const uint64_t* lengths
         std::min<uint32_t>({static_cast<uint32_t>(rest.size()), kBuildWorkers, hw});
     std::vector<std::thread> pool;
     for (uint32_t w = 0; w < workers; ++w) pool.emplace_back(work);
+    // The group builds of the alphabet sizes run side by side, one thread and
+    // stream each (mostly launches and short waits), the last on this thread.
     std::vector<uint32_t> retry;  // texts of groups that failed as a group
-    for (uint32_t L = 0; L < small.size(); ++L) {
-      if (small[L].empty()) continue;
+    auto build_size = [&](uint32_t L) {
       try {
         build_small_texts(texts, lengths, small[L], elem_size, L, gpu_index, out);
         if (statuses)
           for (uint32_t i : small[L]) statuses[i] = EWT_OK;
       } catch (...) {
+        std::lock_guard<std::mutex> lk(mu);
         for (uint32_t i : small[L]) {
           if (out[i]) ewt_free(out[i]);
           out[i] = nullptr;
           retry.push_back(i);
         }
       }
-    }
+    };
+    std::vector<uint32_t> sizes;
+    for (uint32_t L = 0; L < small.size(); ++L)
+      if (!small[L].empty()) sizes.push_back(L);
+    for (size_t i = 0; i + 1 < sizes.size(); ++i)
+      pool.emplace_back([&build_size, L = sizes[i]] { build_size(L); });
+    if (!sizes.empty()) build_size(sizes.back());
     for (auto& th : pool) th.join();
     // one by one, so that each failing text reports its own status
     set_texts_synchronized(true);

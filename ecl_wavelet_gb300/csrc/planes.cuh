@@ -1166,7 +1166,7 @@ std::vector<OrderPlanes> run_plane_passes(
     return o;
   };
   OrderPlanes cur = make_order(0, L - 1);
-  DevBuf starts_buf[2], tile_first, chunk_first, range_first, tile_cnt, chunk_pre, range_tot;
+  DevBuf starts_buf[2], scratch;
   uint32_t nodes = x.nodes;
   uint64_t* starts = x.starts;
   if (nodes == 1) {
@@ -1192,12 +1192,18 @@ std::vector<OrderPlanes> run_plane_passes(
                 "text too long");
     g.rc = ceil_div(64, g.ct);  // 64 tiles a range
     uint64_t const max_ranges = max_chunks / g.rc + nodes;
-    tile_first.alloc((uint64_t(nodes) + 1) * 4);
-    chunk_first.alloc((uint64_t(nodes) + 1) * 4);
-    tile_cnt.alloc((max_tiles << g.D) * 2);
-    chunk_pre.alloc((max_chunks << g.D) * 8);
-    range_first.alloc((uint64_t(nodes) + 1) * 4);
-    range_tot.alloc((max_ranges << g.D) * 8);
+    // one allocation for the pass's tables
+    size_t bytes = 0;
+    auto room = [&](uint64_t b) {
+      size_t const at = bytes;
+      bytes += (b + 255) / 256 * 256;
+      return at;
+    };
+    size_t const at_tf = room((uint64_t(nodes) + 1) * 4), at_cf = room((uint64_t(nodes) + 1) * 4),
+                 at_rf = room((uint64_t(nodes) + 1) * 4), at_cnt = room((max_tiles << g.D) * 2),
+                 at_pre = room((max_chunks << g.D) * 8), at_tot = room((max_ranges << g.D) * 8);
+    scratch.alloc(bytes);
+    unsigned char* const base = scratch.as<unsigned char>();
     uint64_t* next_starts = starts_out;
     if (!final) {
       DevBuf& sb = starts_buf[(i + 1) & 1];
@@ -1205,12 +1211,12 @@ std::vector<OrderPlanes> run_plane_passes(
       next_starts = sb.as<uint64_t>();
     }
     g.starts = starts;
-    g.tile_first = tile_first.as<uint32_t>();
-    g.chunk_first = chunk_first.as<uint32_t>();
-    g.range_first = range_first.as<uint32_t>();
-    g.tile_cnt = tile_cnt.as<uint16_t>();
-    g.chunk_pre = chunk_pre.as<uint64_t>();
-    g.range_tot = range_tot.as<uint64_t>();
+    g.tile_first = reinterpret_cast<uint32_t*>(base + at_tf);
+    g.chunk_first = reinterpret_cast<uint32_t*>(base + at_cf);
+    g.range_first = reinterpret_cast<uint32_t*>(base + at_rf);
+    g.tile_cnt = reinterpret_cast<uint16_t*>(base + at_cnt);
+    g.chunk_pre = reinterpret_cast<uint64_t*>(base + at_pre);
+    g.range_tot = reinterpret_cast<uint64_t*>(base + at_tot);
     g.starts_next = next_starts;
     uint32_t const scan_grid = static_cast<uint32_t>(
         std::min<uint64_t>(max_tiles, uint64_t(sms) * 6));

@@ -21,9 +21,25 @@ using ecl::detail::kL2PerL1;
 using ecl::detail::kL2Words;
 using ecl::detail::kSampleRate;
 
-struct BlockJob {
-  uint64_t word_off, bits, l2_off, l1_off, num_l1, num_last_l2;
-};
+namespace {
+// Bits past each array's end -- in its last word and in the padding words up
+// to the next 32-word boundary -- set to zero (a CTA of 32 threads each).
+__global__ void clear_tails_kernel(uint32_t* words, ArrayMeta const* meta) {
+  ArrayMeta const& m = meta[blockIdx.x];
+  uint64_t const w = (m.bits + 31) / 32;
+  uint64_t const padded = (w + 31) / 32 * 32;
+  uint32_t const t = threadIdx.x;
+  if (t == 0 && m.bits % 32)
+    words[m.word_off + m.bits / 32] &= (1u << (m.bits % 32)) - 1u;
+  if (w + t < padded) words[m.word_off + w + t] = 0u;
+}
+}  // namespace
+
+void clear_tails(RSStore& rs, cudaStream_t st) {
+  clear_tails_kernel<<<static_cast<uint32_t>(rs.meta.size()), 32, 0, st>>>(
+      rs.words.as<uint32_t>(), rs.meta_d.as<ArrayMeta>());
+  EWT_LAUNCHED();
+}
 
 void RSStore::layout(std::vector<uint64_t> const& bits, uint64_t stride, DevBuf* filled) {
   meta.assign(bits.size(), ArrayMeta{});
@@ -45,6 +61,8 @@ void RSStore::layout(std::vector<uint64_t> const& bits, uint64_t stride, DevBuf*
     // so that their places do not depend on the counts
     m.s0_off = m.s1_off = total_s1;
     total_s1 += m.bits / kSampleRate;
+    if (a < skip_blocks.size() && skip_blocks[a])
+      m.rb_off = m.rbh_off = m.ds0_off = m.ds1_off = ecl::detail::kNoBlocks;
   }
   total_s0 = total_s1;
   total_words += total_words % 2;
@@ -58,24 +76,10 @@ void RSStore::layout(std::vector<uint64_t> const& bits, uint64_t stride, DevBuf*
   EWT_CUDA(cudaMemcpyAsync(meta_d.get(), meta.data(),
                            meta.size() * sizeof(ArrayMeta),
                            cudaMemcpyHostToDevice, st));
-  std::vector<BlockJob> jobs(meta.size());
-  for (size_t a = 0; a < meta.size(); ++a)
-    jobs[a] = {meta[a].word_off, meta[a].bits, meta[a].l2_off, meta[a].l1_off,
-               meta[a].num_l1, meta[a].num_last_l2};
-  jobs_d.alloc(jobs.size() * sizeof(BlockJob));
-  EWT_CUDA(cudaMemcpyAsync(jobs_d.get(), jobs.data(),
-                           jobs.size() * sizeof(BlockJob),
-                           cudaMemcpyHostToDevice, st));
-  // Zero the padding words behind every array (the arrays themselves are
-  // written completely by their producer).
   if (filled) return;
-  for (auto const& m : meta) {
-    uint64_t const w = ceil_div(m.bits, 32);
-    uint64_t const padded = ceil_div(w, 32) * 32;
-    if (padded > w)
-      EWT_CUDA(cudaMemsetAsync(words.as<uint32_t>() + m.word_off + w, 0,
-                               (padded - w) * 4, st));
-  }
+  // The padding words behind every array are zero (the arrays themselves are
+  // written completely by their producer).
+  clear_tails(*this, st);
   if (total_words > 0 && total_words % 32)  // the even-rounding word
     EWT_CUDA(cudaMemsetAsync(words.as<uint32_t>() + total_words - 1, 0, 4, st));
 }
@@ -105,7 +109,7 @@ RSView RSStore::view() const {
 namespace {
 
 // Finds the array owning global L1 block g among jobs[0..count).
-__device__ __forceinline__ uint32_t find_job(BlockJob const* jobs,
+__device__ __forceinline__ uint32_t find_job(ArrayMeta const* __restrict__ jobs,
                                              uint32_t count, uint64_t g) {
   uint32_t lo = 0, hi = count - 1;
   while (lo < hi) {
@@ -117,12 +121,12 @@ __device__ __forceinline__ uint32_t find_job(BlockJob const* jobs,
 
 // One CTA of 128 threads per L1 block; thread k owns L2 block k.
 __global__ void __launch_bounds__(128)
-rs_block_kernel(uint32_t const* __restrict__ words, BlockJob const* jobs,
+rs_block_kernel(uint32_t const* __restrict__ words, ArrayMeta const* __restrict__ jobs,
                 uint32_t num_jobs, uint64_t l1_base,
                 uint16_t* __restrict__ l2, uint64_t* __restrict__ l1) {
   uint64_t const g = l1_base + blockIdx.x;
   uint32_t const j = find_job(jobs, num_jobs, g);
-  BlockJob const job = jobs[j];
+  ArrayMeta const& job = jobs[j];
   uint64_t const b = g - job.l1_off;
   uint32_t const k = threadIdx.x;
   uint64_t const nblk = (b + 1 == job.num_l1) ? job.num_last_l2 : kL2PerL1;
@@ -168,18 +172,17 @@ rs_block_kernel(uint32_t const* __restrict__ words, BlockJob const* jobs,
 // One CTA per array: in-place exclusive scan of the L1 block totals; the
 // grand total goes straight into the array's device meta entry.
 __global__ void __launch_bounds__(1024)
-rs_l1_scan_kernel(BlockJob const* jobs, uint32_t first_array,
-                  uint64_t* __restrict__ l1, ArrayMeta* __restrict__ meta) {
-  BlockJob const job = jobs[blockIdx.x];
-  uint64_t* p = l1 + job.l1_off;
+rs_l1_scan_kernel(ArrayMeta* __restrict__ meta, uint64_t* __restrict__ l1) {
+  uint64_t const num_l1 = meta[blockIdx.x].num_l1;
+  uint64_t* p = l1 + meta[blockIdx.x].l1_off;
   __shared__ uint64_t warp_tot[32];
   __shared__ uint64_t carry_s;
   uint32_t const t = threadIdx.x, lane = t & 31, wid = t >> 5;
   if (t == 0) carry_s = 0;
   __syncthreads();
-  for (uint64_t base = 0; base < job.num_l1; base += blockDim.x) {
+  for (uint64_t base = 0; base < num_l1; base += blockDim.x) {
     uint64_t const i = base + t;
-    uint64_t const v = i < job.num_l1 ? p[i] : 0;
+    uint64_t const v = i < num_l1 ? p[i] : 0;
     uint64_t inc = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -191,12 +194,12 @@ rs_l1_scan_kernel(BlockJob const* jobs, uint32_t first_array,
     uint64_t wb = 0;
     for (uint32_t w = 0; w < wid; ++w) wb += warp_tot[w];
     uint64_t const carry = carry_s;
-    if (i < job.num_l1) p[i] = carry + wb + inc - v;
+    if (i < num_l1) p[i] = carry + wb + inc - v;
     __syncthreads();
     if (t == blockDim.x - 1) carry_s = carry + wb + inc;
     __syncthreads();
   }
-  if (t == 0) meta[first_array + blockIdx.x].ones = carry_s;
+  if (t == 0) meta[blockIdx.x].ones = carry_s;
 }
 
 // Position inside the 512-bit block of the r-th (1-based) `value` bit.
@@ -218,19 +221,17 @@ __device__ __forceinline__ uint32_t select_in_block(uint32_t const* blk,
 __global__ void __launch_bounds__(256)
 rs_samples_kernel(uint32_t const* __restrict__ words,
                   uint64_t const* __restrict__ l1,
-                  uint16_t const* __restrict__ l2, BlockJob const* jobs,
-                  ArrayMeta const* __restrict__ meta, uint32_t num_jobs, uint64_t total_l1,
+                  uint16_t const* __restrict__ l2, ArrayMeta const* __restrict__ jobs,
+                  uint32_t num_jobs, uint64_t total_l1,
                   uint64_t* __restrict__ s0, uint64_t* __restrict__ s1) {
   uint64_t const g = (blockIdx.x * uint64_t(blockDim.x) + threadIdx.x) >> 5;
   uint32_t const lane = threadIdx.x & 31;
   if (g >= total_l1) return;
-  uint32_t const a = find_job(jobs, num_jobs, g);
-  BlockJob const job = jobs[a];
-  ArrayMeta const& m = meta[a];
+  ArrayMeta const& job = jobs[find_job(jobs, num_jobs, g)];
   uint64_t const b = g - job.l1_off;  // L1 block inside the array
   bool const last = b + 1 == job.num_l1;
   uint64_t const bit_b = b * kL1Bits, end_b = last ? job.bits : bit_b + kL1Bits;
-  uint64_t const ones_b = l1[g], ones_e = last ? m.ones : l1[g + 1];
+  uint64_t const ones_b = l1[g], ones_e = last ? job.ones : l1[g + 1];
   uint32_t const nblk = static_cast<uint32_t>((end_b - bit_b + kL2Bits - 1) / kL2Bits);
   uint16_t const* const c = l2 + job.l2_off + b * kL2PerL1;
   // ones of the L1 block before L2 block 4 lane + i; the block's end past nblk
@@ -256,11 +257,11 @@ rs_samples_kernel(uint32_t const* __restrict__ words,
     uint64_t const z0 = zeros_b + (bit0 - bit_b) - x[i], z1 = zeros_b + (bit1 - bit_b) - x[i + 1];
     uint64_t const t1 = o1 / kSampleRate, t0 = z1 / kSampleRate;
     if (t1 > o0 / kSampleRate)
-      s1[m.s1_off + t1 - 1] =
+      s1[job.s1_off + t1 - 1] =
           bit0 + select_in_block(blk + k * kL2Words,
                                  static_cast<uint32_t>(t1 * kSampleRate - o0), 1);
     if (t0 > z0 / kSampleRate)
-      s0[m.s0_off + t0 - 1] =
+      s0[job.s0_off + t0 - 1] =
           bit0 + select_in_block(blk + k * kL2Words,
                                  static_cast<uint32_t>(t0 * kSampleRate - z0), 0);
   }
@@ -272,19 +273,18 @@ void build_rs_counts(RSStore& rs, uint32_t first, uint32_t last,
                      cudaStream_t stream) {
   if (first >= last) return;
   uint32_t const count = last - first;
-  BlockJob const* jobs = rs.jobs_d.as<BlockJob>() + first;
+  ArrayMeta* const meta = rs.meta_d.as<ArrayMeta>() + first;
   PhaseTimer pt(EWT_PHASE_RS_COUNTS, stream);
   uint64_t const l1_first = rs.meta[first].l1_off;
   uint64_t const l1_end = rs.meta[last - 1].l1_off + rs.meta[last - 1].num_l1;
   for (uint64_t base = l1_first; base < l1_end; base += (1u << 30)) {
     uint64_t const nb = std::min<uint64_t>(l1_end - base, 1u << 30);
     rs_block_kernel<<<static_cast<uint32_t>(nb), 128, 0, stream>>>(
-        rs.words.as<uint32_t>(), jobs, count, base, rs.l2.as<uint16_t>(),
+        rs.words.as<uint32_t>(), meta, count, base, rs.l2.as<uint16_t>(),
         rs.l1.as<uint64_t>());
     EWT_LAUNCHED();
   }
-  rs_l1_scan_kernel<<<count, 1024, 0, stream>>>(
-      jobs, first, rs.l1.as<uint64_t>(), rs.meta_d.as<ArrayMeta>());
+  rs_l1_scan_kernel<<<count, 1024, 0, stream>>>(meta, rs.l1.as<uint64_t>());
   EWT_LAUNCHED();
 }
 
@@ -295,9 +295,8 @@ void build_rs_samples(RSStore& rs, cudaStream_t stream) {
   PhaseTimer pt(EWT_PHASE_SAMPLES, stream);
   rs_samples_kernel<<<static_cast<uint32_t>(ceil_div(rs.total_l1, 8)), 256, 0, stream>>>(
       rs.words.as<uint32_t>(), rs.l1.as<uint64_t>(), rs.l2.as<uint16_t>(),
-      rs.jobs_d.as<BlockJob>(), rs.meta_d.as<ArrayMeta>(),
-      static_cast<uint32_t>(rs.meta.size()), rs.total_l1, rs.s0.as<uint64_t>(),
-      rs.s1.as<uint64_t>());
+      rs.meta_d.as<ArrayMeta>(), static_cast<uint32_t>(rs.meta.size()), rs.total_l1,
+      rs.s0.as<uint64_t>(), rs.s1.as<uint64_t>());
   EWT_LAUNCHED();
 }
 
@@ -433,13 +432,10 @@ uint64_t rank_block_starts(std::vector<ArrayMeta> const& meta,
 
 void build_rank_blocks(RSStore& rs, cudaStream_t stream) {
   uint32_t const count = static_cast<uint32_t>(rs.meta.size());
-  {  // the totals of ones that the L1 scans left on the device
-    std::vector<ArrayMeta> dm(count);
-    EWT_CUDA(cudaMemcpyAsync(dm.data(), rs.meta_d.get(), count * sizeof(ArrayMeta),
-                             cudaMemcpyDeviceToHost, stream));
-    EWT_CUDA(cudaStreamSynchronize(stream));
-    for (uint32_t a = 0; a < count; ++a) rs.meta[a].ones = dm[a].ones;
-  }
+  // (the totals of ones that the L1 scans left on the device)
+  EWT_CUDA(cudaMemcpyAsync(rs.meta.data(), rs.meta_d.get(), count * sizeof(ArrayMeta),
+                           cudaMemcpyDeviceToHost, stream));
+  EWT_CUDA(cudaStreamSynchronize(stream));
   std::vector<uint64_t> start(count);
   uint64_t total = 0, highs = 0;
   for (uint32_t a = 0; a < count; ++a) {

@@ -466,13 +466,22 @@ namespace ewt {
 namespace {
 
 // rank0 at every node start (node i: first symbol and level, in the order the
-// ranks are stored in); the count table is complete.
+// ranks are stored in; null: a power-of-two tree's); the count table is
+// complete.
 __global__ void __launch_bounds__(128)
 node_ranks_kernel(TreeView t, NodeInfoH const* __restrict__ nodes, uint64_t count,
                   uint64_t* __restrict__ ranks) {
   uint64_t const i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
   if (i >= count) return;
-  NodeInfoH const nd = nodes[i];
+  NodeInfoH nd;
+  if (nodes) {
+    nd = nodes[i];
+  } else {  // power of two: level l's nodes 1 .. 2^l - 1 follow 2^l - 1 - l others
+    uint32_t l = 1;
+    while (i >= (uint64_t(2) << l) - 2 - l) ++l;
+    nd.level = l;
+    nd.start = (i - ((uint64_t(1) << l) - 1 - l) + 1) << (t.levels - l);
+  }
   uint64_t const p = t.counts[nd.start];
   ranks[i] = p - ecl::detail::rs_rank1<false>(t.rs, t.rs.meta[nd.level], p, nullptr);
 }
@@ -547,6 +556,19 @@ bool host_ingest(const void* data, uint64_t n, uint64_t sigma) {
 template <class T>
 void build_typed(ewt_tree& t, const void* data, uint64_t n,
                  const void* alphabet, uint64_t sigma, cudaStream_t st) {
+  // Host tables that copies to the device read: they outlive the copies (also
+  // when the build throws: the guard below them waits first).
+  std::vector<T> alphabet_h;
+  std::vector<uint16_t> codes, lut;  // padded codes by minimal symbol, by symbol
+  std::vector<uint64_t> tables, c_h;
+  std::vector<LevelNode> flat;
+  struct Drain {
+    cudaStream_t s;
+    bool on = true;
+    ~Drain() {
+      if (on) cudaStreamSynchronize(s);
+    }
+  } drain{st};
   // ---- text on the device
   DevBuf text_owned;
   T const* d_text;
@@ -630,27 +652,23 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
   DevBuf lut_d;
   T const* sym = d_text;
   if (!t.is_min || (by_planes && sizeof(T) > 2)) {
-    std::vector<T> a(t.alphabet.begin(), t.alphabet.end());
+    alphabet_h.assign(t.alphabet.begin(), t.alphabet.end());
     t.alphabet_d.alloc(sigma * sizeof(T));
-    EWT_CUDA(cudaMemcpyAsync(t.alphabet_d.get(), a.data(), sigma * sizeof(T),
+    EWT_CUDA(cudaMemcpyAsync(t.alphabet_d.get(), alphabet_h.data(), sigma * sizeof(T),
                              cudaMemcpyHostToDevice, st));
-    EWT_CUDA(cudaStreamSynchronize(st));  // `a` leaves scope
   }
-  // codes, padded with zero bits, by minimal symbol
-  std::vector<uint16_t> codes;
   if (by_planes && (!t.pow2 || !t.is_min)) {
     codes.resize(sigma);
     for (uint64_t i = 0; i < sigma; ++i)
       codes[i] = static_cast<uint16_t>(padded_code(t, i));
     if (sizeof(T) <= 2) {  // by symbol: that of the first alphabet symbol at or above it
-      std::vector<uint16_t> lut(sizeof(T) == 1 ? 256 : 65536, 0);
+      lut.assign(sizeof(T) == 1 ? 256 : 65536, 0);
       uint64_t v = 0;
       for (uint64_t i = 0; i < sigma; ++i)
         for (; v <= t.alphabet[i] && v < lut.size(); ++v) lut[v] = codes[i];
       lut_d.alloc(lut.size() * 2);
       EWT_CUDA(cudaMemcpyAsync(lut_d.get(), lut.data(), lut.size() * 2,
                                cudaMemcpyHostToDevice, st));
-      EWT_CUDA(cudaStreamSynchronize(st));  // `lut` leaves scope
     } else if (!t.pow2) {
       lut_d.alloc(sigma * 2);
       EWT_CUDA(cudaMemcpyAsync(lut_d.get(), codes.data(), sigma * 2,
@@ -735,11 +753,10 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
     for (size_t j = 0; j < t.codes.size(); ++j)
       for (uint32_t l = static_cast<uint32_t>(t.codes[j].len); l < L; ++l)
         t.level_bits[l] -= t.occ[t.codes_start + j];
-    std::vector<uint64_t> c(sigma + 1, 0);
-    for (uint64_t i = 1; i <= sigma; ++i) c[i] = c[i - 1] + t.occ[i - 1];
-    EWT_CUDA(cudaMemcpyAsync(t.counts_d.get(), c.data(), (sigma + 1) * 8,
+    c_h.assign(sigma + 1, 0);
+    for (uint64_t i = 1; i <= sigma; ++i) c_h[i] = c_h[i - 1] + t.occ[i - 1];
+    EWT_CUDA(cudaMemcpyAsync(t.counts_d.get(), c_h.data(), (sigma + 1) * 8,
                              cudaMemcpyHostToDevice, st));
-    EWT_CUDA(cudaStreamSynchronize(st));  // `c` leaves scope
   } else if (!by_planes) {
     uint64_t const ends[2] = {0, n};
     EWT_CUDA(cudaMemcpyAsync(t.counts_d.get(), &ends[0], 8,
@@ -752,6 +769,13 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
     EWT_REQUIRE(t.level_bits[l] > 0, EWT_ERR_UNSUPPORTED,
                 "empty level: every symbol with a code this long is absent");
 
+  // binary levels that group levels cover get no rank blocks
+  t.rs.skip_blocks.assign(L, 0);
+  if (want_groups) {
+    uint32_t covered = 0;
+    for (uint32_t w : group_widths(L)) covered += w;
+    for (uint32_t l = 0; l < covered; ++l) t.rs.skip_blocks[l] = 1;
+  }
   if (words_early.get()) {
     uint64_t kept_bits = 0;
     for (uint64_t b : t.level_bits) kept_bits += b;
@@ -766,41 +790,41 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
     t.rs.layout(t.level_bits);
   }
   t.ranks_d.alloc(std::max<size_t>(t.nodes.size(), 1) * 8);
-  t.node_base_d.alloc((L + 1) * 8);
-  EWT_CUDA(cudaMemcpyAsync(t.node_base_d.get(), t.node_base.data(), (L + 1) * 8,
-                           cudaMemcpyHostToDevice, st));
-  t.nodes_at_level_d.alloc(L * 8);
-  EWT_CUDA(cudaMemcpyAsync(t.nodes_at_level_d.get(), t.nodes_at_level.data(),
-                           L * 8, cudaMemcpyHostToDevice, st));
+  // node bases, nodes per level, short codes: one block, one copy
   size_t const nc = std::max<size_t>(t.codes.size(), 1);
-  std::vector<uint64_t> cl(nc, 0), cb(nc, 0);
+  tables.assign(t.node_base.begin(), t.node_base.end());
+  tables.insert(tables.end(), t.nodes_at_level.begin(), t.nodes_at_level.end());
+  size_t const at_len = tables.size(), at_code = at_len + nc;
+  tables.resize(at_code + nc, 0);
   for (size_t i = 0; i < t.codes.size(); ++i) {
-    cl[i] = t.codes[i].len;
-    cb[i] = t.codes[i].code;
+    tables[at_len + i] = t.codes[i].len;
+    tables[at_code + i] = t.codes[i].code;
   }
-  t.code_len_d.alloc(nc * 8);
-  t.code_bits_d.alloc(nc * 8);
-  EWT_CUDA(cudaMemcpyAsync(t.code_len_d.get(), cl.data(), nc * 8,
+  t.tables_d.alloc(tables.size() * 8);
+  EWT_CUDA(cudaMemcpyAsync(t.tables_d.get(), tables.data(), tables.size() * 8,
                            cudaMemcpyHostToDevice, st));
-  EWT_CUDA(cudaMemcpyAsync(t.code_bits_d.get(), cb.data(), nc * 8,
-                           cudaMemcpyHostToDevice, st));
-  std::vector<LevelNode> flat;
+  uint64_t* const tab = t.tables_d.as<uint64_t>();
+  t.node_base_d.view(tab, (L + 1) * 8);
+  t.nodes_at_level_d.view(tab + L + 1, L * 8);
+  t.code_len_d.view(tab + at_len, nc * 8);
+  t.code_bits_d.view(tab + at_code, nc * 8);
   std::vector<uint64_t> lv_off(L + 1, 0);
   for (uint32_t l = 0; l < L && !by_planes; ++l) {
     flat.insert(flat.end(), level_nodes[l].begin(), level_nodes[l].end());
     lv_off[l + 1] = flat.size();
   }
-  DevBuf nodes_d;  // node starts (passes)
-  if (by_planes && !t.nodes.empty()) {
+  DevBuf nodes_d;  // node starts (passes; of a power of two they follow from the index)
+  if (by_planes && !t.pow2 && !t.nodes.empty()) {
     nodes_d.alloc(t.nodes.size() * sizeof(NodeInfoH));
     EWT_CUDA(cudaMemcpyAsync(nodes_d.get(), t.nodes.data(), t.nodes.size() * sizeof(NodeInfoH),
                              cudaMemcpyHostToDevice, st));
   }
-  DevBuf lnodes_d(std::max<size_t>(flat.size(), 1) * sizeof(LevelNode));
-  EWT_CUDA(cudaMemcpyAsync(lnodes_d.get(), flat.data(),
-                           flat.size() * sizeof(LevelNode),
-                           cudaMemcpyHostToDevice, st));
-  EWT_CUDA(cudaStreamSynchronize(st));  // host vectors above leave scope
+  DevBuf lnodes_d;
+  if (!flat.empty()) {
+    lnodes_d.alloc(flat.size() * sizeof(LevelNode));
+    EWT_CUDA(cudaMemcpyAsync(lnodes_d.get(), flat.data(), flat.size() * sizeof(LevelNode),
+                             cudaMemcpyHostToDevice, st));
+  }
 
   fill_tree_view(t);
   TreeView& v = t.view;
@@ -884,16 +908,15 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
     }
   }
   build_rs_samples(t.rs, st);
-  // binary levels that group levels cover get no rank blocks
-  t.rs.skip_blocks.assign(L, 0);
-  if (want_groups) {
-    uint32_t covered = 0;
-    for (uint32_t w : group_widths(L)) covered += w;
-    for (uint32_t l = 0; l < covered; ++l) t.rs.skip_blocks[l] = 1;
+  if (want_groups && std::count(t.rs.skip_blocks.begin(), t.rs.skip_blocks.end(), 0) == 0) {
+    // no rank blocks: only the totals of ones come over (below)
+    t.rs.rb.alloc(0);
+    t.rs.ds.alloc(0);
+    EWT_CUDA(cudaMemcpyAsync(t.rs.meta.data(), t.rs.meta_d.get(), L * sizeof(ArrayMeta),
+                             cudaMemcpyDeviceToHost, st));
+  } else {
+    build_rank_blocks(t.rs, st);
   }
-  build_rank_blocks(t.rs, st);
-  v.rs = t.rs.view();
-  v.groups = ecl::detail::GroupView{};
   uint32_t build_err = 0;
   EWT_CUDA(cudaMemcpyAsync(&build_err, err_build, 4, cudaMemcpyDeviceToHost,
                            st));
@@ -923,7 +946,9 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
     }
     build_groups(t, t.pow2 ? c : code_starts, planes, st);
   }
+  v.rs = t.rs.view();
   v.groups = t.groups.view();
+  drain.on = false;  // the stream was waited for above
 }
 
 }  // namespace
