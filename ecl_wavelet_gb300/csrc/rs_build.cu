@@ -5,8 +5,8 @@
 //   L1[j]  = ones in [0, j * 65536)                           (uint64)
 //   ones   = total ones
 //   s1[k]  = position of the (k+1)*4096-th one, s0 likewise for zeros.
-// Kernels: one CTA per 65,536-bit L1 block counts its 128 L2 blocks with
-// 128-bit coalesced loads and a CTA scan; one CTA per array scans the L1
+// Kernels: a CTA counts the 128 L2 blocks of a few 65,536-bit L1 blocks with
+// 128-bit loads and CTA scans; one CTA per array scans the L1
 // block totals; a warp per L1 block emits the (at most one) one- and
 // zero-sample of each of its 512-bit blocks.  No kernel waits on another CTA.
 #include <algorithm>
@@ -119,54 +119,84 @@ __device__ __forceinline__ uint32_t find_job(ArrayMeta const* __restrict__ jobs,
   return lo;
 }
 
-// One CTA of 128 threads per L1 block; thread k owns L2 block k.
+// A CTA of 128 threads counts kBlocksPerCta L1 blocks, thread k L2 block k of
+// each; all their words are asked for before the first count, and an array is
+// looked up once for the blocks that follow each other in it.
+constexpr uint32_t kBlocksPerCta = 4;
+
 __global__ void __launch_bounds__(128)
 rs_block_kernel(uint32_t const* __restrict__ words, ArrayMeta const* __restrict__ jobs,
-                uint32_t num_jobs, uint64_t l1_base,
+                uint32_t num_jobs, uint64_t l1_base, uint64_t l1_end,
                 uint16_t* __restrict__ l2, uint64_t* __restrict__ l1) {
-  uint64_t const g = l1_base + blockIdx.x;
-  uint32_t const j = find_job(jobs, num_jobs, g);
-  ArrayMeta const& job = jobs[j];
-  uint64_t const b = g - job.l1_off;
-  uint32_t const k = threadIdx.x;
-  uint64_t const nblk = (b + 1 == job.num_l1) ? job.num_last_l2 : kL2PerL1;
-  uint32_t cnt = 0;
-  if (k < nblk) {
-    uint64_t const kb = b * kL2PerL1 + k;  // L2 block inside the array
-    uint64_t const bit0 = kb * kL2Bits;
-    uint64_t const valid = min(job.bits - bit0, kL2Bits);
-    uint4 const* p = reinterpret_cast<uint4 const*>(words + job.word_off +
-                                                    kb * kL2Words);
+  __shared__ uint32_t warp_tot[kBlocksPerCta][4];
+  uint32_t const k = threadIdx.x, lane = k & 31, wid = k >> 5;
+  uint64_t const g0 = l1_base + uint64_t(blockIdx.x) * kBlocksPerCta;
+  uint32_t j = find_job(jobs, num_jobs, g0);
+  uint64_t first = jobs[j].l1_off, num = jobs[j].num_l1, bits = jobs[j].bits;
+  uint64_t word_off = jobs[j].word_off, l2_off = jobs[j].l2_off;
+  uint4 v[kBlocksPerCta][4];
+  uint32_t valid[kBlocksPerCta];     // bits of the thread's L2 block
+  uint64_t l2_at[kBlocksPerCta];     // its entry
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      uint4 v = p[q];
-      uint32_t w[4] = {v.x, v.y, v.z, v.w};
+  for (uint32_t u = 0; u < kBlocksPerCta; ++u) {
+    uint64_t const g = g0 + u;
+    valid[u] = 0;
+    l2_at[u] = 0;
+    if (g < l1_end && g >= first + num && j + 1 < num_jobs) {
+      ++j;  // every array has at least one L1 block
+      first = jobs[j].l1_off;
+      num = jobs[j].num_l1;
+      bits = jobs[j].bits;
+      word_off = jobs[j].word_off;
+      l2_off = jobs[j].l2_off;
+    }
+    uint64_t const kb = (g - first) * kL2PerL1 + k, bit0 = kb * kL2Bits;
+    if (g < l1_end && bit0 < bits) {
+      valid[u] = static_cast<uint32_t>(min(bits - bit0, kL2Bits));
+      l2_at[u] = l2_off + kb;
+      uint4 const* p = reinterpret_cast<uint4 const*>(words + word_off + kb * kL2Words);
 #pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        uint32_t const lo = (q * 4 + t) * 32;
-        uint32_t x = w[t];
-        if (lo >= valid) x = 0;
-        else if (valid - lo < 32) x &= (1u << (valid - lo)) - 1u;
-        cnt += __popc(x);
-      }
+      for (int q = 0; q < 4; ++q) v[u][q] = __ldg(p + q);
     }
   }
-  // CTA exclusive scan of 128 counts.
-  __shared__ uint32_t warp_tot[4];
-  uint32_t const lane = k & 31, wid = k >> 5;
-  uint32_t inc = cnt;
+  uint32_t inc[kBlocksPerCta], cnt[kBlocksPerCta];
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    uint32_t const y = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= o) inc += y;
+  for (uint32_t u = 0; u < kBlocksPerCta; ++u) {
+    uint32_t c = 0;
+    if (valid[u] == kL2Bits) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        c += __popc(v[u][q].x) + __popc(v[u][q].y) + __popc(v[u][q].z) + __popc(v[u][q].w);
+    } else if (valid[u]) {  // an array's last block
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        uint32_t const w[4] = {v[u][q].x, v[u][q].y, v[u][q].z, v[u][q].w};
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          uint32_t const lo = (q * 4 + t) * 32;
+          uint32_t const m = lo >= valid[u] ? 0u
+                             : valid[u] - lo < 32 ? (1u << (valid[u] - lo)) - 1u
+                                                  : ~0u;
+          c += __popc(w[t] & m);
+        }
+      }
+    }
+    cnt[u] = inc[u] = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      uint32_t const y = __shfl_up_sync(0xffffffffu, inc[u], o);
+      if (lane >= o) inc[u] += y;
+    }
+    if (lane == 31) warp_tot[u][wid] = inc[u];
   }
-  if (lane == 31) warp_tot[wid] = inc;
   __syncthreads();
-  uint32_t base = 0;
-  for (uint32_t w = 0; w < wid; ++w) base += warp_tot[w];
-  uint32_t const excl = base + inc - cnt;
-  if (k < nblk) l2[job.l2_off + b * kL2PerL1 + k] = static_cast<uint16_t>(excl);
-  if (k == 127) l1[job.l1_off + b] = base + inc;  // block total for now
+#pragma unroll
+  for (uint32_t u = 0; u < kBlocksPerCta; ++u) {
+    uint32_t base = 0;
+    for (uint32_t w = 0; w < wid; ++w) base += warp_tot[u][w];
+    if (valid[u]) l2[l2_at[u]] = static_cast<uint16_t>(base + inc[u] - cnt[u]);
+    if (k == 127 && g0 + u < l1_end) l1[g0 + u] = base + inc[u];  // block total for now
+  }
 }
 
 // One CTA per array: in-place exclusive scan of the L1 block totals; the
@@ -277,11 +307,12 @@ void build_rs_counts(RSStore& rs, uint32_t first, uint32_t last,
   PhaseTimer pt(EWT_PHASE_RS_COUNTS, stream);
   uint64_t const l1_first = rs.meta[first].l1_off;
   uint64_t const l1_end = rs.meta[last - 1].l1_off + rs.meta[last - 1].num_l1;
-  for (uint64_t base = l1_first; base < l1_end; base += (1u << 30)) {
-    uint64_t const nb = std::min<uint64_t>(l1_end - base, 1u << 30);
-    rs_block_kernel<<<static_cast<uint32_t>(nb), 128, 0, stream>>>(
-        rs.words.as<uint32_t>(), meta, count, base, rs.l2.as<uint16_t>(),
-        rs.l1.as<uint64_t>());
+  constexpr uint64_t kLaunch = uint64_t(kBlocksPerCta) << 30;  // L1 blocks per launch
+  for (uint64_t base = l1_first; base < l1_end; base += kLaunch) {
+    uint64_t const end = std::min(l1_end, base + kLaunch);
+    rs_block_kernel<<<static_cast<uint32_t>(ceil_div(end - base, kBlocksPerCta)), 128, 0,
+                      stream>>>(rs.words.as<uint32_t>(), meta, count, base, end,
+                                rs.l2.as<uint16_t>(), rs.l1.as<uint64_t>());
     EWT_LAUNCHED();
   }
   rs_l1_scan_kernel<<<count, 1024, 0, stream>>>(meta, rs.l1.as<uint64_t>());
