@@ -125,8 +125,50 @@ void populate_for_write(void* p, size_t bytes) {
 
 // Largest batch moved through the device scratch in one piece.
 constexpr uint64_t kChunk = uint64_t(1) << 25;
-// Host batches from this size on run pipelined (QueryPipe).
-constexpr uint64_t kPipeMin = uint64_t(1) << 21;
+// Host batches from this size on run pipelined (QueryPipe): where a kernel
+// can copy pageable host memory from 2^19 queries on (1 Mi mixed queries: in
+// place 458 us, pipelined 300 us; 128 Ki: in place 79 us, and eight chunks of
+// copies alone cost as much in launches), else from 2^21.
+constexpr uint64_t kPipeMin = uint64_t(1) << 21, kPipeMinKernel = uint64_t(1) << 19;
+
+// Copies between host and device memory by a kernel, V bytes a step (both
+// ends and the size multiples of V): copies of pageable memory by the driver
+// hold the calling thread until they are done, which left nothing to overlap
+// with (3 M rank queries: 279 us in and 140 us out, one after the other and
+// after the pages of the results).  Bound by the C2C link: 195 GB/s in, 160
+// GB/s out from 16 CTAs on, so 32 CTAs leave the SMs to the queries.
+template <class V>
+__global__ void __launch_bounds__(512)
+copy_kernel(V const* __restrict__ src, V* __restrict__ dst, uint64_t count) {
+  uint64_t const step = uint64_t(gridDim.x) * blockDim.x;
+  uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
+  for (; i + 3 * step < count; i += 4 * step) {
+    V const a = src[i], b = src[i + step], c = src[i + 2 * step], d = src[i + 3 * step];
+    dst[i] = a;
+    dst[i + step] = b;
+    dst[i + 2 * step] = c;
+    dst[i + 3 * step] = d;
+  }
+  for (; i < count; i += step) dst[i] = src[i];
+}
+
+void copy_async(void* dst, void const* src, uint64_t bytes, bool by_kernel, cudaStream_t s) {
+  if (!by_kernel) {
+    EWT_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, s));
+    return;
+  }
+  uintptr_t const low = reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src) | bytes;
+  auto run = [&](auto v) {
+    using V = decltype(v);
+    copy_kernel<V><<<32, 512, 0, s>>>(static_cast<V const*>(src), static_cast<V*>(dst),
+                                      bytes / sizeof(V));
+  };
+  if (low % 16 == 0) run(uint4{});
+  else if (low % 8 == 0) run(uint64_t{});
+  else if (low % 4 == 0) run(uint32_t{});
+  else run(uint8_t{});
+  EWT_LAUNCHED();
+}
 
 void ensure(DevBuf& b, size_t& cap, size_t bytes) {
   if (bytes <= cap && b.get()) return;
@@ -206,13 +248,21 @@ int host_batch(ewt_tree* t, void const* in, size_t in_rec, uint8_t const* types,
     DeviceGuard g(t->device);
     AllocStream as(t->stream);
     cudaStream_t s = t->stream;
-    if (m >= kPipeMin) {
+    bool const by_kernel = pageable_access(t->device);
+    if (m >= (by_kernel ? kPipeMinKernel : kPipeMin)) {
       // large batches: copies in and out overlap the kernels chunk by chunk
-      // (copy engines reach the C2C bandwidth; the kernel then works on
-      // device memory only)
+      // (which then work on device memory only)
+      // (below the driver copies' size the caller's buffers are held to the
+      // alignment that the kernels ask of buffers they use in place)
+      EWT_REQUIRE(m >= kPipeMin ||
+                      (reinterpret_cast<uintptr_t>(in) % 8 == 0 &&
+                       (in_rec == 8 || reinterpret_cast<uintptr_t>(out) % 8 == 0)),
+                  EWT_ERR_INVALID_ARGUMENT,
+                  "query and result buffers must be 8-byte aligned");
       QueryPipe& P = t->pipe;
       P.init();
-      uint64_t const chunk = std::max<uint64_t>(kPipeMin / 4, ceil_div(m, 8));
+      uint64_t const chunk = std::max<uint64_t>(
+          (by_kernel ? kPipeMinKernel : kPipeMin) / 4, ceil_div(ceil_div(m, 8), 16) * 16);
       for (int x = 0; x < 2; ++x) {  // allocated on s, before the copy streams start
         ensure(P.in[x], P.cap_in[x], chunk * in_rec);
         ensure(P.out[x], P.cap_out[x], chunk * out_rec);
@@ -225,11 +275,9 @@ int host_batch(ewt_tree* t, void const* in, size_t in_rec, uint8_t const* types,
         int const x = static_cast<int>(i & 1);
         uint64_t const k = std::min(chunk, m - b);
         if (i >= 2) EWT_CUDA(cudaStreamWaitEvent(P.s_in, P.k_done[x], 0));
-        EWT_CUDA(cudaMemcpyAsync(P.in[x].get(), static_cast<char const*>(in) + b * in_rec,
-                                 k * in_rec, cudaMemcpyDefault, P.s_in));
-        if (types)
-          EWT_CUDA(cudaMemcpyAsync(P.types[x].get(), types + b, k, cudaMemcpyDefault,
-                                   P.s_in));
+        copy_async(P.in[x].get(), static_cast<char const*>(in) + b * in_rec, k * in_rec,
+                   by_kernel, P.s_in);
+        if (types) copy_async(P.types[x].get(), types + b, k, by_kernel, P.s_in);
         EWT_CUDA(cudaEventRecord(P.in_done[x], P.s_in));
         EWT_CUDA(cudaStreamWaitEvent(s, P.in_done[x], 0));
         if (i >= 2) EWT_CUDA(cudaStreamWaitEvent(s, P.out_done[x], 0));
@@ -238,8 +286,8 @@ int host_batch(ewt_tree* t, void const* in, size_t in_rec, uint8_t const* types,
         EWT_CUDA(cudaStreamWaitEvent(P.s_out, P.k_done[x], 0));
         // pages of the chunk's results, while the GPU works on it
         populate_for_write(static_cast<char*>(out) + b * out_rec, k * out_rec);
-        EWT_CUDA(cudaMemcpyAsync(static_cast<char*>(out) + b * out_rec, P.out[x].get(),
-                                 k * out_rec, cudaMemcpyDefault, P.s_out));
+        copy_async(static_cast<char*>(out) + b * out_rec, P.out[x].get(), k * out_rec,
+                   by_kernel, P.s_out);
         EWT_CUDA(cudaEventRecord(P.out_done[x], P.s_out));
       }
       EWT_CUDA(cudaStreamWaitEvent(s, P.out_done[(i - 1) & 1], 0));
