@@ -622,6 +622,7 @@ void build_groups(ewt_tree& t, std::vector<uint64_t> const& C,
   EWT_REQUIRE(planes.size() == qs.levels.size(), EWT_ERR_CUDA, "group planes missing");
   // host: digit totals, node ranks
   std::vector<uint64_t> nr;
+  nr.reserve(uint64_t(2) << std::min<uint32_t>(L, 16));
   uint64_t max_sb = 0;
   for (auto& ql : qs.levels) {
     uint32_t const w = ql.width, S = 1u << w, l = ql.start;

@@ -88,28 +88,6 @@ std::vector<CodeH> make_codes(uint64_t sigma) {
   return std::vector<CodeH>(c.end() - kept, c.end());
 }
 
-// Node starts per level (getNodeInfos, wavelet_tree.cuh:2501-2532).
-std::vector<NodeInfoH> make_nodes(uint64_t sigma,
-                                  std::vector<CodeH> const& codes) {
-  uint32_t const L = h_ceil_log2(sigma);
-  uint64_t const cs = sigma - codes.size();
-  auto code_of = [&](uint64_t i) {
-    return i < cs ? CodeH{L, i} : codes[i - cs];
-  };
-  std::vector<NodeInfoH> out;
-  for (uint32_t l = 1; l < L; ++l) {
-    uint32_t const sh = L - l - 1;
-    CodeH prev = code_of(0);
-    for (uint64_t i = 1; i < sigma; ++i) {
-      CodeH const cur = code_of(i);
-      if (cur.len > l && !((cur.code >> sh) & 1) && ((prev.code >> sh) & 1))
-        out.push_back({i, l});
-      prev = cur;
-    }
-  }
-  return out;
-}
-
 // Every node with at least two symbols, level by level, in symbol order:
 // [start, end) splits at start + prevPow2(end - start), the descent of
 // deviceAccess (wavelet_tree.cuh:1854-1868).
@@ -133,6 +111,26 @@ std::vector<std::vector<LevelNode>> make_level_nodes(uint64_t sigma,
     cur.swap(nxt);
   }
   return lv;
+}
+
+// Node starts per level (getNodeInfos, wavelet_tree.cuh:2501-2532): every node
+// of at least two symbols but each level's first.  (A symbol begins a node of
+// level l where its code's bit l is 0 and its neighbour's 1; the neighbour is
+// then the last symbol of a node of at least two, since a node's left child is
+// the deeper one, so codes end on a level from the right.)
+std::vector<NodeInfoH> make_nodes(uint64_t sigma, uint32_t L) {
+  std::vector<NodeInfoH> out;
+  out.reserve(sigma);
+  if (h_is_pow2(sigma)) {
+    for (uint32_t l = 1; l < L; ++l)
+      for (uint64_t g = 1; g < uint64_t(1) << l; ++g) out.push_back({g << (L - l), l});
+    return out;
+  }
+  auto const lv = make_level_nodes(sigma, L);
+  for (uint32_t l = 1; l < L; ++l)
+    for (LevelNode const& nd : lv[l])
+      if (nd.cs) out.push_back({nd.cs, l});
+  return out;
 }
 
 // --------------------------------------------------------------------------
@@ -159,11 +157,14 @@ __global__ void presence_kernel(T const* __restrict__ text, uint64_t n,
 // Alphabet detection for 4- and 8-byte symbols: a device hash set of the
 // distinct symbols (open addressing, linear probing, 64-bit slots).  An
 // empty slot holds kEmptySlot; for 8-byte texts the one symbol equal to it is
-// recorded in a flag instead.  A symbol is looked up with a plain load first
-// (most symbols repeat) and inserted with atomicCAS only when missing; warp
-// peers holding the same symbol insert once.  A probe that runs around the
-// whole table reports overflow and the host retries with a larger table.
+// recorded in a flag instead.  Each CTA remembers the symbols it has looked up
+// in a direct-mapped table in shared memory, so a symbol that repeats goes no
+// further (20 M symbols of 10,000: 300 us without).  Others are looked up with
+// a plain load first and inserted with atomicCAS only when missing.  A probe
+// that runs around the whole table reports overflow and the host retries with
+// a larger table.
 constexpr uint64_t kEmptySlot = ~uint64_t(0);
+constexpr uint32_t kSeenSlots = 8192;
 
 __device__ __forceinline__ uint64_t slot_hash(uint64_t x) {
   x ^= x >> 33;
@@ -173,28 +174,33 @@ __device__ __forceinline__ uint64_t slot_hash(uint64_t x) {
 }
 
 template <class T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(1024)
 distinct_kernel(T const* __restrict__ text, uint64_t n,
                 unsigned long long* __restrict__ table, uint64_t cap_mask,
                 unsigned long long* __restrict__ count,
                 uint32_t* __restrict__ flags) {  // [0] overflow, [1] max symbol seen
+  extern __shared__ __align__(8) uint64_t seen[];
+  for (uint32_t i = threadIdx.x; i < kSeenSlots; i += blockDim.x) seen[i] = kEmptySlot;
+  __syncthreads();
   uint64_t const stride = uint64_t(gridDim.x) * blockDim.x;
   for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n;
        i += stride) {
     uint64_t const key = static_cast<uint64_t>(text[i]);
-    uint32_t const peers = __match_any_sync(__activemask(), key);
-    if ((threadIdx.x & 31) != __ffs(peers) - 1) continue;  // one per value
     if (key == kEmptySlot) {
       flags[1] = 1;
       continue;
     }
-    uint64_t h = slot_hash(key) & cap_mask;
+    uint64_t const hash = slot_hash(key);
+    // (a slot is read and written whole, so racing threads see one key or another)
+    uint64_t volatile* const mine = seen + (hash & (kSeenSlots - 1));
+    if (*mine == key) continue;
+    uint64_t h = hash & cap_mask;
     for (uint64_t probe = 0;; ++probe) {
       if (probe > cap_mask) {
         flags[0] = 1;
         break;
       }
-      uint64_t const cur = table[h];
+      uint64_t const cur = *const_cast<unsigned long long volatile*>(table + h);
       if (cur == key) break;
       if (cur == kEmptySlot) {
         unsigned long long const prev =
@@ -208,7 +214,41 @@ distinct_kernel(T const* __restrict__ text, uint64_t n,
       }
       h = (h + 1) & cap_mask;
     }
+    *mine = key;
   }
+}
+
+// The table's symbols side by side (order as it comes).
+__global__ void __launch_bounds__(256)
+compact_kernel(unsigned long long const* __restrict__ table, uint64_t cap,
+               uint64_t* __restrict__ out, uint64_t count, uint32_t* __restrict__ next) {
+  uint64_t const i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
+  if (i >= cap || table[i] == kEmptySlot) return;
+  uint32_t const at = atomicAdd(next, 1u);
+  if (at < count) out[at] = table[i];
+}
+
+// Sorted by counting: symbol i goes to the number of smaller ones (all are
+// distinct).  count^2 comparisons, but on every SM and without a pass over
+// memory: 10,000 symbols 12 us, 65,536 about 130 us; the host's sort of 10,000
+// took 0.5 ms.
+constexpr uint64_t kRankSortMax = 65536;
+
+__global__ void __launch_bounds__(256)
+rank_sort_kernel(uint64_t const* __restrict__ in, uint32_t count, uint64_t* __restrict__ out) {
+  __shared__ uint64_t tile[1024];
+  uint32_t const i = blockIdx.x * blockDim.x + threadIdx.x;
+  uint64_t const x = i < count ? in[i] : 0;
+  uint32_t rank = 0;
+  for (uint32_t base = 0; base < count; base += 1024) {
+    uint32_t const len = min(1024u, count - base);
+    __syncthreads();
+    for (uint32_t j = threadIdx.x; j < len; j += blockDim.x) tile[j] = in[base + j];
+    __syncthreads();
+#pragma unroll 8
+    for (uint32_t j = 0; j < len; ++j) rank += tile[j] < x;
+  }
+  if (i < count) out[rank] = x;
 }
 
 // Sorted distinct symbols of a device-resident 4- or 8-byte text.
@@ -217,13 +257,14 @@ std::vector<uint64_t> detect_alphabet_wide(T const* d_text, uint64_t n,
                                            cudaStream_t st) {
   uint64_t cap = 1ull << 16;
   uint32_t const blocks = static_cast<uint32_t>(
-      std::min<uint64_t>(ceil_div(n, 256), uint64_t(sm_count()) * 8));
+      std::min<uint64_t>(ceil_div(n, 1024), uint64_t(sm_count()) * 2));
+  set_smem_limit(distinct_kernel<T>, kSeenSlots * 8);
   for (;;) {
     DevBuf table(cap * 8), cnt(8), flags(8);
     EWT_CUDA(cudaMemsetAsync(table.get(), 0xFF, cap * 8, st));
     EWT_CUDA(cudaMemsetAsync(cnt.get(), 0, 8, st));
     EWT_CUDA(cudaMemsetAsync(flags.get(), 0, 8, st));
-    distinct_kernel<T><<<blocks, 256, 0, st>>>(
+    distinct_kernel<T><<<blocks, 1024, kSeenSlots * 8, st>>>(
         d_text, n, table.as<unsigned long long>(), cap - 1,
         cnt.as<unsigned long long>(), flags.as<uint32_t>());
     EWT_LAUNCHED();
@@ -232,6 +273,24 @@ std::vector<uint64_t> detect_alphabet_wide(T const* d_text, uint64_t n,
     EWT_CUDA(cudaMemcpyAsync(&count, cnt.get(), 8, cudaMemcpyDeviceToHost, st));
     EWT_CUDA(cudaMemcpyAsync(fl, flags.get(), 8, cudaMemcpyDeviceToHost, st));
     EWT_CUDA(cudaStreamSynchronize(st));
+    if (!fl[0] && count * 2 <= cap && count <= kRankSortMax) {
+      DevBuf list(std::max<uint64_t>(count, 1) * 16), next(4);
+      EWT_CUDA(cudaMemsetAsync(next.get(), 0, 4, st));
+      uint64_t* const sorted = list.as<uint64_t>() + count;
+      compact_kernel<<<static_cast<uint32_t>(ceil_div(cap, 256)), 256, 0, st>>>(
+          table.as<unsigned long long>(), cap, list.as<uint64_t>(), count, next.as<uint32_t>());
+      EWT_LAUNCHED();
+      if (count) {
+        rank_sort_kernel<<<static_cast<uint32_t>(ceil_div(count, 256)), 256, 0, st>>>(
+            list.as<uint64_t>(), static_cast<uint32_t>(count), sorted);
+        EWT_LAUNCHED();
+      }
+      std::vector<uint64_t> out(count);
+      EWT_CUDA(cudaMemcpyAsync(out.data(), sorted, count * 8, cudaMemcpyDeviceToHost, st));
+      EWT_CUDA(cudaStreamSynchronize(st));
+      if (fl[1]) out.push_back(kEmptySlot);
+      return out;
+    }
     if (!fl[0] && count * 2 <= cap) {
       std::vector<uint64_t> h(cap);
       EWT_CUDA(cudaMemcpyAsync(h.data(), table.get(), cap * 8,
@@ -254,6 +313,11 @@ std::vector<uint64_t> detect_alphabet_wide(T const* d_text, uint64_t n,
 
 // Text -> minimal symbols (lower_bound in the sorted alphabet), or with
 // `codes` the code of each.  Smem: the alphabet is searched in shared memory.
+// A symbol's place in the alphabet's range (kRemapBuckets equal parts) gives
+// the two entries to search between: 10,000 symbols spread evenly take two
+// steps instead of fourteen (20 M symbols 120 us without).
+constexpr uint32_t kRemapBuckets = 4096;
+
 template <class T, class U, bool Smem>
 __global__ void __launch_bounds__(1024)
 remap_kernel(T const* __restrict__ text, uint64_t n,
@@ -261,25 +325,41 @@ remap_kernel(T const* __restrict__ text, uint64_t n,
              uint16_t const* __restrict__ codes, U* __restrict__ cur,
              uint32_t* __restrict__ err) {
   extern __shared__ __align__(16) unsigned char remap_smem[];
+  __shared__ uint32_t first[kRemapBuckets + 1];  // lower_bound of each bucket's start
   T* const sa = reinterpret_cast<T*>(remap_smem);
   if constexpr (Smem) {
     for (uint32_t i = threadIdx.x; i < sigma; i += blockDim.x) sa[i] = alphabet[i];
     __syncthreads();
   }
   T const* const al = Smem ? sa : alphabet;
+  auto search = [&](T x, uint32_t lo, uint32_t hi) {
+    while (lo < hi) {
+      uint32_t const mid = (lo + hi) >> 1;
+      if (al[mid] < x) lo = mid + 1; else hi = mid;
+    }
+    return lo;
+  };
+  T const low = al[0], top = al[sigma - 1];
+  uint32_t shift = 0;  // bucket of x: (x - low) >> shift < kRemapBuckets
+  while ((uint64_t(top) - uint64_t(low)) >> shift >= kRemapBuckets) ++shift;
+  for (uint32_t b = threadIdx.x; b <= kRemapBuckets; b += blockDim.x) {
+    uint64_t const d = uint64_t(b) << shift;  // past the range: all of the alphabet
+    first[b] = (d >> shift) != b || d > uint64_t(top) - uint64_t(low)
+                   ? sigma
+                   : search(static_cast<T>(uint64_t(low) + d), 0, sigma);
+  }
+  __syncthreads();
   uint64_t const stride = uint64_t(gridDim.x) * blockDim.x;
   uint32_t bad = 0;
   for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n;
        i += stride) {
     T const x = text[i];
-    uint32_t lo = 0, hi = sigma;
-    while (lo < hi) {
-      uint32_t const mid = (lo + hi) >> 1;
-      if (al[mid] < x) lo = mid + 1; else hi = mid;
-    }
-    if (lo >= sigma) {
+    uint32_t lo = 0;
+    if (x > top) {
       bad = 1;
-      lo = 0;
+    } else if (x > low) {
+      uint32_t const b = static_cast<uint32_t>((uint64_t(x) - uint64_t(low)) >> shift);
+      lo = search(x, first[b], first[b + 1]);
     }
     cur[i] = static_cast<U>(codes ? codes[lo] : lo);
   }
@@ -287,14 +367,14 @@ remap_kernel(T const* __restrict__ text, uint64_t n,
 }
 
 // Searching in shared memory keeps two CTAs of 1024 threads on an SM up to
-// 96 KB of alphabet; above that the alphabet stays in the caches.
+// 80 KB of alphabet; above that the alphabet stays in the caches.
 template <class T, class U>
 void launch_remap(T const* text, uint64_t n, T const* alphabet, uint64_t sigma,
                   uint16_t const* codes, U* out, uint32_t* err, cudaStream_t st) {
   EWT_REQUIRE(sigma < UINT32_MAX, EWT_ERR_UNSUPPORTED, "alphabet too large");
   uint32_t const grid = static_cast<uint32_t>(
       std::min<uint64_t>(ceil_div(n, 1024), uint64_t(sm_count()) * 2));
-  constexpr size_t kMax = 96 * 1024;
+  constexpr size_t kMax = 80 * 1024;
   if (sigma * sizeof(T) <= kMax) {
     auto k = remap_kernel<T, U, true>;
     set_smem_limit(k, kMax);
@@ -1026,8 +1106,8 @@ void set_tree_shape(ewt_tree& t) {
   uint64_t const sigma = t.sigma;
   t.codes = make_codes(sigma);
   t.codes_start = sigma - t.codes.size();
-  t.nodes = make_nodes(sigma, t.codes);
   uint32_t const L = t.L;
+  t.nodes = make_nodes(sigma, L);
   t.nodes_at_level.assign(L, 0);
   if (t.pow2) {
     for (uint32_t l = 0; l < L; ++l) t.nodes_at_level[l] = (uint64_t(1) << l) - 1;

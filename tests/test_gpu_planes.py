@@ -124,3 +124,27 @@ def test_padded_group_levels(ewt, oracle, sigma, n, tmp_path):
     for rate in (0, 1024):
         gt.set_select_samples(rate)
         check_queries(gt, ot, text, al, 1_000, seed=rate)
+
+
+@pytest.mark.parametrize("dtype,kind", [(np.uint32, "dense"), (np.uint32, "clustered"),
+                                        (np.uint64, "clustered"), (np.uint64, "two"),
+                                        (np.uint32, "large"), (np.uint64, "shared")])
+def test_wide_alphabets(ewt, oracle, dtype, kind):
+    """Detection and search of 4- and 8-byte alphabets: consecutive symbols; all
+    but one in one bucket of the search's range; two symbols at the type's
+    ends; more symbols than are searched in shared memory, and than are sorted
+    on the device."""
+    rng = np.random.default_rng(7)
+    top = int(np.iinfo(dtype).max)
+    a = {"dense": np.arange(1000, 1900), "clustered": np.append(np.arange(5, 3005, 3), top),
+         "two": np.array([0, top], dtype=np.uint64), "shared": np.arange(20_000) * (top // 20_001),
+         "large": np.arange(70_000) * 61_001}[kind].astype(dtype)
+    text = a[rng.integers(0, a.size, max(100_001, 2 * a.size))]
+    text[:a.size] = a
+    same(ewt, oracle, text, a)
+    assert np.array_equal(ewt.WaveletTree(text).getAlphabet(), a)
+    if a[0] > 0:  # a symbol below all others stands for the first
+        below = text.copy()
+        below[-1] = 0
+        gt, ot = ewt.WaveletTree(below, a), ewt.WaveletTree(np.append(text[:-1], a[:1]), a)
+        assert np.array_equal(gt.export("COUNTS"), ot.export("COUNTS"))
