@@ -13,7 +13,7 @@
 //      of the first pass, in one read of the text;
 //   2. plane_counts_kernel (later passes, and passes that start with many
 //      nodes): the digit counts of every tile from the planes, a digit being
-//      the D bits below the node;
+//      the k bits below the node;
 //   3. range_totals / digit_starts / chunk_starts kernels: where every
 //      digit class starts, and the digits of a node before every chunk of
 //      tiles;
@@ -25,7 +25,7 @@
 // instruction per symbol and level and 1/8 byte of shared memory, where
 // moving the symbols as bytes took about 20 instructions and a byte store per
 // symbol and level.  6 Gi uint8 symbols, sigma 256 (one GB300): passes 38.6 ->
-// 19.4 ms, digit counts 3.6 -> 2.6 ms, whole build 57.6 -> 33.3 ms.
+// 19.4 ms, digit counts 3.6 -> 1.7 ms, whole build 57.6 -> 32.5 ms.
 //
 // The partition of one slot (128 or 256 consecutive positions of one class)
 // by its mask m: an inverse butterfly of stages of distance 1, 2, 4, .. brings
@@ -56,7 +56,7 @@ namespace {
 
 constexpr uint32_t kMaxPlanes = 16;  // code bits
 constexpr uint32_t kMaxPassK = 4;    // levels per pass
-constexpr uint32_t kMaxDigits = 32;  // digits of a tile count (up to 5 bits)
+constexpr uint32_t kMaxDigits = 16;  // digits of a tile count (up to 4 bits)
 
 // The tiles of one pass: every node [starts[N], starts[N+1]) of the level-a
 // order is cut into tiles of `tile` symbols, `ct` consecutive tiles of a
@@ -65,6 +65,7 @@ constexpr uint32_t kMaxDigits = 32;  // digits of a tile count (up to 5 bits)
 struct TileGrid {
   uint64_t n;
   uint32_t nodes, D, tile, ct, rc;
+  uint32_t halves;          // 1: starts_next has two entries per digit (below)
   uint64_t* starts;         // nodes + 1
   uint32_t* tile_first;     // nodes + 1
   uint32_t* chunk_first;    // nodes + 1
@@ -72,8 +73,18 @@ struct TileGrid {
   uint16_t* tile_cnt;       // [tile][1 << D]
   uint64_t* chunk_pre;      // [chunk][1 << D]: the digit in the node before
   uint64_t* range_tot;      // [range][1 << D]
-  uint64_t* starts_next;    // (nodes << D) + 1
+  uint64_t* starts_next;    // (nodes << D << halves) + 1
 };
+
+// Where digit d of node N starts.  The last pass's digits are the classes of
+// the last level, of which plane_pass_kernel counts the ones on its way: the
+// second entry of a digit, the start of its ones, begins as the digit's end
+// and is lowered by them.  (Counting digits of one bit more beforehand, a
+// popcount for each of twice as many classes: digit counts of 6 Gi symbols of
+// 256 2.63 -> 1.66 ms.)
+__device__ __forceinline__ uint64_t* digit_start(TileGrid const& g, uint32_t N, uint32_t d) {
+  return g.starts_next + ((uint64_t(N) << g.D | d) << g.halves);
+}
 
 // The node owning entry i of a non-decreasing table first[0 .. nodes]: the
 // last one whose first entry is <= i.
@@ -470,7 +481,7 @@ range_totals_kernel(TileGrid g) {
 // digit's start position (node start + smaller digits).
 __device__ __forceinline__ uint64_t node_digit_starts(TileGrid const& g, uint32_t N,
                                                       uint64_t own) {
-  __shared__ uint64_t part[32][kMaxDigits];
+  __shared__ uint64_t part[32][32];
   uint32_t const lane = threadIdx.x & 31, wid = threadIdx.x >> 5, warps = blockDim.x >> 5;
   part[wid][lane] = own;
   __syncthreads();
@@ -488,9 +499,10 @@ __device__ __forceinline__ uint64_t node_digit_starts(TileGrid const& g, uint32_
     }
     if (lane < (1u << g.D)) {
       uint64_t const at = g.starts[N] + inc - tot;
-      g.starts_next[(uint64_t(N) << g.D) + lane] = at;
-      if (N == g.nodes - 1 && lane == (1u << g.D) - 1)
-        g.starts_next[uint64_t(g.nodes) << g.D] = at + tot;
+      uint64_t* const s = digit_start(g, N, lane);
+      s[0] = at;
+      if (g.halves || (N == g.nodes - 1 && lane == (1u << g.D) - 1)) s[1] = at + tot;
+      if (g.halves && N == g.nodes - 1 && lane == (1u << g.D) - 1) s[2] = at + tot;
     }
   }
   return before;
@@ -601,7 +613,7 @@ clear_edges_kernel(const __grid_constant__ PlanePass p) {
     uint32_t const t0 = p.g.tile_first[N] + (c - p.g.chunk_first[N]) * p.g.ct;
     uint32_t const t1 = min(t0 + p.g.ct, p.g.tile_first[N + 1]);
     bool const on = lane < digits;
-    uint64_t const start = on ? p.g.starts_next[(uint64_t(N) << D) + lane] : 0;
+    uint64_t const start = on ? *digit_start(p.g, N, lane) : 0;
     uint64_t pre = on ? p.g.chunk_pre[(uint64_t(c) << D) + lane] : 0;
     for (uint32_t t = t0; t < t1; ++t) {
       uint64_t sum = pre;  // of the lane's class
@@ -801,6 +813,7 @@ plane_pass_kernel(const __grid_constant__ PlanePass p) {
   __shared__ uint8_t warp_cls[kMaxPassK + 1][kWarps];  // class of a warp's first slot
   __shared__ uint32_t nslots[kMaxPassK + 1];
   __shared__ uint32_t warp_tot[kWarps];
+  __shared__ uint32_t half_ones[1 << kMaxPassK];  // last pass: ones of every class, last plane
   __shared__ uint64_t ck_start;
   __shared__ uint32_t ck_node, ck_tile, ck_len;
 
@@ -838,8 +851,9 @@ plane_pass_kernel(const __grid_constant__ PlanePass p) {
     for (uint32_t i = 2 + tid; i < (2u << k); i += NT) {
       uint32_t const r = 31 - __clz(i), q = i - (1u << r);
       uint32_t const d0 = q << (D - r), d1 = (q + 1) << (D - r);
-      gpos[i] = p.g.starts_next[(uint64_t(ck_node) << D) + d0] + pre_s[d1] - pre_s[d0];
+      gpos[i] = *digit_start(p.g, ck_node, d0) + pre_s[d1] - pre_s[d0];
     }
+    if (tid < (1u << kMaxPassK)) half_ones[tid] = 0;
     uint32_t const len_c = ck_len;
     uint32_t const tiles = (len_c + p.g.tile - 1) / p.g.tile;
     for (uint32_t ti = 0; ti < tiles; ++ti) {
@@ -980,7 +994,15 @@ plane_pass_kernel(const __grid_constant__ PlanePass p) {
             put(y, p.ext[r][j], p.ext_words);
           }
         }
-        if (r == k) break;
+        if (r == k) {
+          if (p.g.halves && act) {
+            uint32_t c = 0;
+#pragma unroll
+            for (uint32_t u = 0; u < W; ++u) c += __popc(m[u]);
+            atomicAdd(&half_ones[q], c);
+          }
+          break;
+        }
         // -- zeros before every slot in its class
         uint32_t ones[W];  // of the slot, before word u
         uint32_t c = 0;
@@ -1071,6 +1093,9 @@ plane_pass_kernel(const __grid_constant__ PlanePass p) {
       __syncthreads();  // the tile is out
       for (uint32_t i = 2 + tid; i < (2u << k); i += NT) gpos[i] += rec[i].x >> 16;
     }
+    if (p.g.halves && tid < (1u << k) && half_ones[tid])
+      atomicAdd(reinterpret_cast<unsigned long long*>(digit_start(p.g, ck_node, tid) + 1),
+                0ull - half_ones[tid]);
     __syncthreads();  // gpos and the chunk's words are rewritten next
   }
 }
@@ -1186,7 +1211,8 @@ std::vector<OrderPlanes> run_plane_passes(
     TileGrid g{};
     g.n = n;
     g.nodes = nodes;
-    g.D = final ? k + 1 : k;
+    g.halves = final && k;
+    g.D = std::max(k, 1u);
     g.tile = pass_tile(slots, kSlotWords, k);
     // chunks of up to 8 tiles while every CTA still gets several
     g.ct = static_cast<uint32_t>(std::min<uint64_t>(
@@ -1256,8 +1282,7 @@ std::vector<OrderPlanes> run_plane_passes(
         auto kern = g.D == 1   ? plane_counts_kernel<1>
                     : g.D == 2 ? plane_counts_kernel<2>
                     : g.D == 3 ? plane_counts_kernel<3>
-                    : g.D == 4 ? plane_counts_kernel<4>
-                               : plane_counts_kernel<5>;
+                               : plane_counts_kernel<4>;
         kern<<<static_cast<uint32_t>(std::min<uint64_t>(max_tiles, uint64_t(sms) * 12)),
                kCountThreads, 0, st>>>(src, g);
         EWT_LAUNCHED();
@@ -1314,7 +1339,7 @@ std::vector<OrderPlanes> run_plane_passes(
     if (wants(a)) kept.push_back(std::move(cur));
     cur = std::move(next);
     starts = next_starts;
-    nodes <<= g.D;
+    nodes <<= k;
     a = b;
   }
   return kept;
