@@ -57,6 +57,12 @@ __device__ __forceinline__ uint32_t spread16(uint32_t x) {
   return x;
 }
 
+// A block in one 32-byte store.
+__device__ __forceinline__ void store_block(uint4* p, uint4 a, uint4 b) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(a.x),
+               "r"(a.y), "r"(a.z), "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w));
+}
+
 // Inclusive warp scan.
 __device__ __forceinline__ uint32_t warp_inclusive(uint32_t x) {
 #pragma unroll
@@ -168,6 +174,15 @@ __device__ __forceinline__ void digit_counts(uint32_t const* s, uint32_t n, uint
   }
 }
 
+// The same, two counts to a word.
+template <int W>
+__device__ __forceinline__ void packed_counts(uint32_t const* s, uint32_t n, uint32_t* c) {
+  uint32_t x[1 << W];
+  digit_counts<W>(s, n, x);
+#pragma unroll
+  for (uint32_t k = 0; k < (1u << W) / 2; ++k) c[k] = x[2 * k] | x[2 * k + 1] << 16;
+}
+
 // Pass 1: digit counts of every superblock (a warp each; whole words).  The
 // planes hold zeros past position n.  Bound by reading the planes once.
 template <int W>
@@ -222,14 +237,22 @@ group_counts_kernel(GroupPlanes g, uint64_t n, uint64_t nsb, uint64_t* __restric
   }
 }
 
+// A build samples at the default rate R (group_samples_kernel writes others
+// later): a superblock's counts and twice R stay within 16 bits.
+constexpr uint32_t kBuildRate = 1u << ecl::detail::kDefaultSelShift;
+static_assert(ecl::detail::kDefaultSelShift > 0 && kQuadSbDigits + 2 * kBuildRate <= 65536 &&
+              kOctSbDigits + 2 * kBuildRate <= 65536);
+
 // Pass 3: a CTA of 256 threads per superblock, thread t its blocks 2t and
 // 2t + 1: their bits of every plane, digit counts by popcounts, the headers
 // from one CTA scan (two 16-bit counts per word: a superblock holds fewer than
-// 2^16 digits), and the dense samples with 32-bit arithmetic from the
-// superblock's own first entry and remainder.  Bound by instructions.  All
-// group levels of 2^30 symbols of 256 (counts, scans, blocks, samples): 1.17
-// ms, 1.56 ms with a thread per block, three scan launches and a loop of
-// 64-bit sample ranks.
+// 2^16 digits), and the dense samples, two digits at a time, from the
+// superblock's own first entry and remainder.  A block goes out in one store
+// of 32 bytes.  Bound by instructions (a quarter of them for the samples).
+// All group levels of 2^30 symbols of 256 (counts, scans, blocks, samples):
+// 1.02 ms; 1.06 with the samples digit by digit, 1.17 with two stores of 16
+// bytes as well, 1.56 with a thread per block, three scan launches and a loop
+// of 64-bit sample ranks.
 template <int W>
 __global__ void __launch_bounds__(256, 5)
 group_level_kernel(GroupPlanes g, uint64_t n, GroupLevel ql, uint4* __restrict__ blocks,
@@ -240,20 +263,20 @@ group_level_kernel(GroupPlanes g, uint64_t n, GroupLevel ql, uint4* __restrict__
   static_assert(kSb == 512, "two blocks per thread");
   __shared__ uint32_t warp_tot[kWarps][4];
   __shared__ uint32_t* entry[S];  // the sample of the superblock's next multiple of R
-  __shared__ uint32_t remainder[S];
+  __shared__ uint32_t rem[kP];   // R - 1 + the occurrences since the one before it
   uint64_t const sbi = blockIdx.x;
   uint32_t const t = threadIdx.x, lane = t & 31, wid = t >> 5;
   uint64_t const blk = sbi * kSb + 2 * t, p = blk * kD;
   uint64_t const* sbe = sb + sbi * S;
-  uint32_t const sh = ql.sel_shift, rm = (1u << sh) - 1u;
-  if (t < S) {
-    entry[t] = ds + ql.ds_off[t] + (sbe[t] >> sh);
-    remainder[t] = static_cast<uint32_t>(sbe[t]) & rm;
-  }
+  uint32_t const sh = ql.sel_shift, rm = (1u << sh) - 1u, rm2 = rm * 0x10001u;
+  if (ds && t < S) entry[t] = ds + ql.ds_off[t] + (sbe[t] >> sh);
+  if (ds && t < kP)
+    rem[t] = ((static_cast<uint32_t>(sbe[2 * t]) & rm) |
+              (static_cast<uint32_t>(sbe[2 * t + 1]) & rm) << 16) + rm2;
   uint32_t valid[2];
   valid[0] = p < n ? static_cast<uint32_t>(min(uint64_t(kD), n - p)) : 0u;
   valid[1] = p + kD < n ? static_cast<uint32_t>(min(uint64_t(kD), n - p - kD)) : 0u;
-  uint32_t c[2][S];
+  uint32_t c[2][kP];
   uint64_t H[2], M[2], B[2];     // octal: 42 bits of each plane
   uint32_t h[2][3], b[2][3];     // quad: three words of each
   if constexpr (W == 3) {
@@ -280,7 +303,7 @@ group_level_kernel(GroupPlanes g, uint64_t n, GroupLevel ql, uint4* __restrict__
                               uint32_t(__popcll(B[u])),        uint32_t(__popcll(hm)),
                               uint32_t(__popcll(H[u] & B[u])), uint32_t(__popcll(M[u] & B[u])),
                               uint32_t(__popcll(hm & B[u]))};
-      digit_counts<3>(s7, valid[u], c[u]);
+      packed_counts<3>(s7, valid[u], c[u]);
     }
   } else {
 #pragma unroll
@@ -296,7 +319,7 @@ group_level_kernel(GroupPlanes g, uint64_t n, GroupLevel ql, uint4* __restrict__
         s3[1] += __popc(b[u][k]);
         s3[2] += __popc(h[u][k] & b[u][k]);
       }
-      digit_counts<2>(s3, valid[u], c[u]);
+      packed_counts<2>(s3, valid[u], c[u]);
     }
   }
   uint32_t e[kP];  // packed counts before block 2t
@@ -304,7 +327,7 @@ group_level_kernel(GroupPlanes g, uint64_t n, GroupLevel ql, uint4* __restrict__
     uint32_t x[kP];
 #pragma unroll
     for (uint32_t k = 0; k < kP; ++k) {
-      x[k] = (c[0][2 * k] + c[1][2 * k]) | ((c[0][2 * k + 1] + c[1][2 * k + 1]) << 16);
+      x[k] = c[0][k] + c[1][k];
       e[k] = warp_inclusive(x[k]);
       if (lane == 31) warp_tot[wid][k] = e[k];
     }
@@ -340,16 +363,18 @@ group_level_kernel(GroupPlanes g, uint64_t n, GroupLevel ql, uint4* __restrict__
     if (blk + u >= ql.num_blocks) return;
     if (u)
 #pragma unroll
-      for (uint32_t k = 0; k < kP; ++k) e[k] += c[0][2 * k] | (c[0][2 * k + 1] << 16);
+      for (uint32_t k = 0; k < kP; ++k) e[k] += c[0][k];
     uint4* out = blocks + (blk + u) * 2;
     if constexpr (W == 3) {
       // planes H, M, B in words 1..3, counts of digits 4..6 above them
       uint64_t const w1 = H[u] | (uint64_t(e[2] & 0xFFFFu) << 42);
       uint64_t const w2 = M[u] | (uint64_t(e[2] >> 16) << 42);
       uint64_t const w3 = B[u] | (uint64_t(e[3] & 0xFFFFu) << 42);
-      out[0] = make_uint4(e[0], e[1], static_cast<uint32_t>(w1), static_cast<uint32_t>(w1 >> 32));
-      out[1] = make_uint4(static_cast<uint32_t>(w2), static_cast<uint32_t>(w2 >> 32),
-                          static_cast<uint32_t>(w3), static_cast<uint32_t>(w3 >> 32));
+      store_block(out,
+                  make_uint4(e[0], e[1], static_cast<uint32_t>(w1),
+                             static_cast<uint32_t>(w1 >> 32)),
+                  make_uint4(static_cast<uint32_t>(w2), static_cast<uint32_t>(w2 >> 32),
+                             static_cast<uint32_t>(w3), static_cast<uint32_t>(w3 >> 32)));
     } else {
       uint32_t dw[6];
 #pragma unroll
@@ -357,27 +382,28 @@ group_level_kernel(GroupPlanes g, uint64_t n, GroupLevel ql, uint4* __restrict__
         dw[2 * k] = spread16(b[u][k]) | (spread16(h[u][k]) << 1);
         dw[2 * k + 1] = spread16(b[u][k] >> 16) | (spread16(h[u][k] >> 16) << 1);
       }
-      out[0] = make_uint4(e[0], e[1] & 0xFFFFu, dw[0], dw[1]);
-      out[1] = make_uint4(dw[2], dw[3], dw[4], dw[5]);
+      store_block(out, make_uint4(e[0], e[1] & 0xFFFFu, dw[0], dw[1]),
+                  make_uint4(dw[2], dw[3], dw[4], dw[5]));
     }
-    if (ds && sh) {
+    if (ds) {
       // entry k of a digit names the block holding its (k R + 1)-th
-      // occurrence: the block's first entry of a digit by a predicated store
-      uint32_t most = 0;
+      // occurrence: the entries below the block's end, less those below its
+      // start, are the block's own
+      uint32_t more = 0;
 #pragma unroll
-      for (uint32_t d = 0; d < S; ++d) {
-        uint32_t const x = remainder[d] + ((e[d >> 1] >> (16 * (d & 1))) & 0xFFFFu);
-        uint32_t const off = (0u - x) & rm;  // occurrences of the block before an entry
-        if (off < c[u][d]) entry[d][(x + rm) >> sh] = static_cast<uint32_t>(blk + u);
-        most = max(most, c[u][d]);
+      for (uint32_t k = 0; k < kP; ++k) {
+        uint32_t const z = e[k] + rem[k], hit = (z ^ (z + c[u][k])) & ~rm2;
+        if (hit & 0xFFFFu) entry[2 * k][(z & 0xFFFFu) >> sh] = static_cast<uint32_t>(blk + u);
+        if (hit >> 16) entry[2 * k + 1][z >> 16 >> sh] = static_cast<uint32_t>(blk + u);
+        more |= c[u][k] + 0x7FFF7FFFu - rm2 - 0x10001u;
       }
-      if (most > rm + 1)  // only then can there be more than one
+      if (rm + 1 < kD && (more & 0x80008000u))  // a digit more than R times
 #pragma unroll
         for (uint32_t d = 0; d < S; ++d) {
-          uint32_t const x = remainder[d] + ((e[d >> 1] >> (16 * (d & 1))) & 0xFFFFu);
-          uint32_t k = (x + rm) >> sh;
-          for (uint32_t o = ((0u - x) & rm) + rm + 1; o < c[u][d]; o += rm + 1)
-            entry[d][++k] = static_cast<uint32_t>(blk + u);
+          uint32_t const z = ((e[d >> 1] + rem[d >> 1]) >> (16 * (d & 1))) & 0xFFFFu;
+          uint32_t const end = z + ((c[u][d >> 1] >> (16 * (d & 1))) & 0xFFFFu);
+          for (uint32_t k = (z >> sh) + 1; k < end >> sh; ++k)
+            entry[d][k] = static_cast<uint32_t>(blk + u);
         }
     }
   }
@@ -590,7 +616,7 @@ void build_group_level(GroupStore& qs, GroupLevel const& ql, GroupPlanes const& 
   EWT_LAUNCHED();
   group_level_kernel<W><<<static_cast<uint32_t>(nsb), 256, 0, st>>>(
       g, n, ql, qs.blocks.as<uint4>() + ql.blk_off * 2, sb, nsb,
-      qs.ds.get() ? qs.ds.as<uint32_t>() : nullptr, err);
+      qs.ds.as<uint32_t>(), err);
   EWT_LAUNCHED();
 }
 

@@ -25,7 +25,7 @@
 // instruction per symbol and level and 1/8 byte of shared memory, where
 // moving the symbols as bytes took about 20 instructions and a byte store per
 // symbol and level.  6 Gi uint8 symbols, sigma 256 (one GB300): passes 38.6 ->
-// 19.4 ms, digit counts 3.6 -> 1.7 ms, whole build 57.6 -> 32.5 ms.
+// 19.4 ms, digit counts 3.6 -> 1.7 ms, whole build 57.6 -> 31.6 ms.
 //
 // The partition of one slot (128 or 256 consecutive positions of one class)
 // by its mask m: an inverse butterfly of stages of distance 1, 2, 4, .. brings
