@@ -48,6 +48,7 @@ struct MultiItem {
 
 constexpr uint32_t kMultiChunk = 2048;
 constexpr uint32_t kMultiThreads = 256;
+constexpr uint32_t kMultiPerSm = 4;    // resident CTAs
 constexpr uint32_t kPlanThreads = 1024;
 constexpr uint32_t kMaxMultiTrees = 1u << 16;  // trees in one call
 constexpr uint32_t kBuildWorkers = 16;          // host threads of a batch build
@@ -118,8 +119,8 @@ tree_scatter_smem_kernel(uint32_t const* __restrict__ tree_of, uint64_t m,
 // One CTA: tree starts in the tree-ordered batch (cursor) and the work list.
 __global__ void __launch_bounds__(kPlanThreads)
 tree_plan_kernel(uint32_t const* __restrict__ cnt, uint32_t num_trees,
-                 uint64_t* __restrict__ cursor, MultiItem* __restrict__ items,
-                 uint32_t* __restrict__ num_items) {
+                 uint32_t chunk, uint64_t* __restrict__ cursor,
+                 MultiItem* __restrict__ items, uint32_t* __restrict__ num_items) {
   __shared__ uint64_t warp_q[32];
   __shared__ uint32_t warp_i[32];
   __shared__ uint64_t carry_q;
@@ -133,7 +134,7 @@ tree_plan_kernel(uint32_t const* __restrict__ cnt, uint32_t num_trees,
   for (uint32_t base = 0; base < num_trees; base += kPlanThreads) {
     uint32_t const t = base + tid;
     uint32_t const c = t < num_trees ? cnt[t] : 0u;
-    uint32_t const ni = (c + kMultiChunk - 1) / kMultiChunk;
+    uint32_t const ni = (c + chunk - 1) / chunk;
     uint64_t iq = c;
     uint32_t ii = ni;
 #pragma unroll
@@ -161,8 +162,7 @@ tree_plan_kernel(uint32_t const* __restrict__ cnt, uint32_t num_trees,
     if (t < num_trees) {
       cursor[t] = q0;
       for (uint32_t j = 0; j < ni; ++j)
-        items[i0 + j] = MultiItem{t, min(kMultiChunk, c - j * kMultiChunk),
-                                  q0 + uint64_t(j) * kMultiChunk};
+        items[i0 + j] = MultiItem{t, min(chunk, c - j * chunk), q0 + uint64_t(j) * chunk};
     }
     __syncthreads();
     if (tid == kPlanThreads - 1) {
@@ -199,8 +199,54 @@ tree_scatter_kernel(uint32_t const* __restrict__ tree_of, uint64_t m,
   }
 }
 
+// The queries of one item, listed by type (0 access, 1 rank, 2 select), a
+// thread a query.  A list begins at the warp behind the one before it, so that
+// short lists run side by side.
+template <class T, class Slot>
+__device__ __forceinline__ void answer_item(
+    TreeView const& tv, ArrayMeta const* meta, uint64_t const* node_base,
+    uint16_t const (*lists)[kMultiChunk], uint32_t const* list_len, Slot const& slot,
+    MultiRec<T> const* __restrict__ in, uint64_t* __restrict__ out, uint32_t* bad) {
+  static_assert((kMultiThreads & (kMultiThreads - 1)) == 0);
+  uint32_t first = 0;  // thread of the list's first query
+  auto begin = [&](uint32_t k) {
+    uint32_t const i = (threadIdx.x - first) & (kMultiThreads - 1);
+    first += (list_len[k] + 31) & ~31u;
+    return i;
+  };
+  for (uint32_t i = begin(0); i < list_len[0]; i += kMultiThreads) {
+    uint64_t const q = slot(lists[0][i]);
+    uint64_t const idx = in[q].index;
+    out[q] = idx < tv.n ? static_cast<uint64_t>(from_minimal<T>(
+                              tv, wt_access(tv, meta, tv.counts, tv.node_ranks, node_base, idx)))
+                        : 0;
+  }
+  for (uint32_t i = begin(1); i < list_len[1]; i += kMultiThreads) {
+    uint64_t const q = slot(lists[1][i]);
+    MultiRec<T> const r = in[q];
+    uint64_t const sym = to_minimal<T>(tv, r.symbol);
+    if (sym >= tv.sigma || r.index > tv.n) {
+      out[q] = UINT64_MAX;
+      *bad = 1;
+    } else {
+      out[q] = wt_rank(tv, meta, tv.counts, tv.node_ranks, node_base, sym, r.index);
+    }
+  }
+  for (uint32_t i = begin(2); i < list_len[2]; i += kMultiThreads) {
+    uint64_t const q = slot(lists[2][i]);
+    MultiRec<T> const r = in[q];
+    uint64_t const sym = to_minimal<T>(tv, r.symbol);
+    if (sym >= tv.sigma || r.index == 0) {
+      out[q] = UINT64_MAX;
+      *bad = 1;
+    } else {
+      out[q] = wt_select(tv, meta, tv.counts, tv.node_ranks, node_base, sym, r.index);
+    }
+  }
+}
+
 template <class T>
-__global__ void __launch_bounds__(kMultiThreads)
+__global__ void __launch_bounds__(kMultiThreads, kMultiPerSm)
 multi_kernel(TreeView const* __restrict__ views,
              MultiItem const* __restrict__ items,
              uint32_t const* __restrict__ num_items_d, uint32_t num_items_h,
@@ -243,7 +289,7 @@ multi_kernel(TreeView const* __restrict__ views,
       for (uint32_t i = tid; i <= L; i += blockDim.x) node_base[i] = tv.node_base[i];
     }
     // sort the item's query slots by type (warp ballots)
-    for (uint32_t j = tid; j < kMultiChunk; j += blockDim.x) {
+    for (uint32_t j = tid; j < ((item.count + 31) & ~31u); j += blockDim.x) {
       uint32_t ty = 3u;
       uint64_t q = 0;
       if (j < item.count) {
@@ -268,36 +314,7 @@ multi_kernel(TreeView const* __restrict__ views,
     auto slot = [&](uint32_t j) -> uint64_t {
       return perm ? perm[item.start + j] : item.start + j;
     };
-    for (uint32_t i = tid; i < list_len[0]; i += blockDim.x) {
-      uint64_t const q = slot(lists[0][i]);
-      uint64_t const idx = in[q].index;
-      out[q] = idx < tv.n ? static_cast<uint64_t>(from_minimal<T>(
-                                tv, wt_access(tv, meta, tv.counts, tv.node_ranks,
-                                              node_base, idx)))
-                          : 0;
-    }
-    for (uint32_t i = tid; i < list_len[1]; i += blockDim.x) {
-      uint64_t const q = slot(lists[1][i]);
-      MultiRec<T> const r = in[q];
-      uint64_t const sym = to_minimal<T>(tv, r.symbol);
-      if (sym >= tv.sigma || r.index > tv.n) {
-        out[q] = UINT64_MAX;
-        bad = 1;
-      } else {
-        out[q] = wt_rank(tv, meta, tv.counts, tv.node_ranks, node_base, sym, r.index);
-      }
-    }
-    for (uint32_t i = tid; i < list_len[2]; i += blockDim.x) {
-      uint64_t const q = slot(lists[2][i]);
-      MultiRec<T> const r = in[q];
-      uint64_t const sym = to_minimal<T>(tv, r.symbol);
-      if (sym >= tv.sigma || r.index == 0) {
-        out[q] = UINT64_MAX;
-        bad = 1;
-      } else {
-        out[q] = wt_select(tv, meta, tv.counts, tv.node_ranks, node_base, sym, r.index);
-      }
-    }
+    answer_item<T>(tv, meta, node_base, lists, list_len, slot, in, out, &bad);
     __syncthreads();  // tv, meta and lists are reused by the next item
   }
   wq_finish(queue);
@@ -320,7 +337,7 @@ struct ServeItemD {
 };
 
 template <class T>
-__global__ void __launch_bounds__(kMultiThreads)
+__global__ void __launch_bounds__(kMultiThreads, kMultiPerSm)
 serve_kernel(TreeView const* __restrict__ views, ServeReq const* __restrict__ reqs,
              ServeItemD const* __restrict__ items, uint32_t n_items,
              uint32_t* __restrict__ req_err) {
@@ -359,7 +376,7 @@ serve_kernel(TreeView const* __restrict__ views, ServeReq const* __restrict__ re
       for (uint32_t i = tid; i <= L; i += blockDim.x) node_base[i] = tv.node_base[i];
     }
     uint32_t bad = 0;
-    for (uint32_t j = tid; j < kMultiChunk; j += blockDim.x) {
+    for (uint32_t j = tid; j < ((item.count + 31) & ~31u); j += blockDim.x) {
       uint32_t const ty = j < item.count ? types[j] : 3u;
 #pragma unroll
       for (uint32_t k = 0; k < 3; ++k) {
@@ -376,36 +393,8 @@ serve_kernel(TreeView const* __restrict__ views, ServeReq const* __restrict__ re
       }
     }
     __syncthreads();
-    for (uint32_t i = tid; i < list_len[0]; i += blockDim.x) {
-      uint32_t const j = lists[0][i];
-      uint64_t const idx = in[j].index;
-      out[j] = idx < tv.n ? static_cast<uint64_t>(from_minimal<T>(
-                                tv, wt_access(tv, meta, tv.counts, tv.node_ranks,
-                                              node_base, idx)))
-                          : 0;
-    }
-    for (uint32_t i = tid; i < list_len[1]; i += blockDim.x) {
-      uint32_t const j = lists[1][i];
-      MultiRec<T> const r = in[j];
-      uint64_t const sym = to_minimal<T>(tv, r.symbol);
-      if (sym >= tv.sigma || r.index > tv.n) {
-        out[j] = UINT64_MAX;
-        bad = 1;
-      } else {
-        out[j] = wt_rank(tv, meta, tv.counts, tv.node_ranks, node_base, sym, r.index);
-      }
-    }
-    for (uint32_t i = tid; i < list_len[2]; i += blockDim.x) {
-      uint32_t const j = lists[2][i];
-      MultiRec<T> const r = in[j];
-      uint64_t const sym = to_minimal<T>(tv, r.symbol);
-      if (sym >= tv.sigma || r.index == 0) {
-        out[j] = UINT64_MAX;
-        bad = 1;
-      } else {
-        out[j] = wt_select(tv, meta, tv.counts, tv.node_ranks, node_base, sym, r.index);
-      }
-    }
+    auto slot = [](uint32_t j) -> uint64_t { return j; };
+    answer_item<T>(tv, meta, node_base, lists, list_len, slot, in, out, &bad);
     if (bad) req_err[item.req] = 1u;  // the same value from every writer
     __syncthreads();  // tv, rq, meta and lists are reused by the next item
   }
@@ -506,7 +495,16 @@ void multi_device(ViewSet const& vs, uint32_t num_trees, uint32_t const* d_tree_
                   uint64_t* d_out, uint32_t* d_err, cudaStream_t s) {
   EWT_REQUIRE(m < (uint64_t(1) << 32), EWT_ERR_TOO_LARGE,
               "a multi-tree batch holds fewer than 2^32 queries");
-  uint64_t const max_items = m / kMultiChunk + num_trees + 1;
+  // items as small as keeps them, a part-filled one per tree, within the
+  // CTAs that fit at a time (64 trees, 1 Ki queries: 60 -> 45 us, 128 Ki: 151
+  // -> 64 us; 4 Mi, items of the full size: 683, 687 us)
+  uint64_t const full = uint64_t(sm_count()) * kMultiPerSm;
+  uint32_t const chunk = static_cast<uint32_t>(std::min<uint64_t>(
+      kMultiChunk,
+      std::max<uint64_t>(kMultiThreads,
+                         ceil_div(ceil_div(m, full - std::min<uint64_t>(num_trees, full / 2)),
+                                  32) * 32)));
+  uint64_t const max_items = m / chunk + num_trees + 1;
   DevBuf cnt((num_trees + 1) * 4), cursor(num_trees * 8),
       items(max_items * sizeof(MultiItem)), nitems(4), perm(std::max<uint64_t>(m, 1) * 4),
       queue(8);
@@ -521,7 +519,7 @@ void multi_device(ViewSet const& vs, uint32_t num_trees, uint32_t const* d_tree_
   else
     tree_hist_kernel<<<grid, 256, 0, s>>>(d_tree_of, m, num_trees, cnt.as<uint32_t>());
   EWT_LAUNCHED();
-  tree_plan_kernel<<<1, kPlanThreads, 0, s>>>(cnt.as<uint32_t>(), num_trees,
+  tree_plan_kernel<<<1, kPlanThreads, 0, s>>>(cnt.as<uint32_t>(), num_trees, chunk,
                                               cursor.as<uint64_t>(),
                                               items.as<MultiItem>(),
                                               nitems.as<uint32_t>());
