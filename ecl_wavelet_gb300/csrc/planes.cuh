@@ -581,10 +581,10 @@ struct PlanePass {
   uint32_t k, np;                        // levels written; planes behind plane a
   uint32_t const* src[kMaxPlanes];       // src[j]: plane a + j, j = 0 .. np
   uint32_t* out[kMaxPassK + 1];          // out[r]: level a + r, r = 1 .. k
-  uint32_t out_words[kMaxPassK + 1];
+  uint64_t out_words[kMaxPassK + 1];
   uint32_t* ext[kMaxPassK + 1][kMaxPlanes];  // plane a + j in level-(a+r) order
   uint32_t ext_mask[kMaxPassK + 1];      // bit j: ext[r][j] is wanted
-  uint32_t ext_words;
+  uint64_t ext_words;
 };
 
 // Clears the words of a pass's outputs that two runs may share, into which
@@ -605,7 +605,7 @@ clear_edges_kernel(const __grid_constant__ PlanePass p) {
   };
   if (blockIdx.x == 0)
     for (uint32_t r = 1; r <= p.k; ++r) {
-      uint64_t const lim = max(p.out_words[r], p.ext_mask[r] ? p.ext_words : 0u);
+      uint64_t const lim = max(p.out_words[r], p.ext_mask[r] ? p.ext_words : uint64_t(0));
       for (uint64_t w = w_end + threadIdx.x; w < lim; w += blockDim.x) clear(r, w);
     }
   for (uint32_t c = blockIdx.x * 4 + (threadIdx.x >> 5); c < chunks; c += gridDim.x * 4) {
@@ -798,9 +798,10 @@ __device__ __forceinline__ void store_slot(uint32_t* p, uint32_t const* y) {
 // (one pass of 7 levels) runs waste a third of the slots, 36 against 20 ms.
 // A class run is laid out at the bit offset of its place in the
 // level's words, so that going out is a copy of whole words.
-template <uint32_t NT, uint32_t W>
+template <uint32_t NT, uint32_t W, class Index>
 __global__ void __launch_bounds__(NT, NT == 256 ? 3 : 4)
 plane_pass_kernel(const __grid_constant__ PlanePass p) {
+  using Words = std::make_unsigned_t<Index>;
   constexpr uint32_t kWarps = NT / 32, kSlotBits = 32 * W;
   extern __shared__ __align__(16) uint32_t buf[];
   __shared__ __align__(16) uint2 rec[2 << kMaxPassK];  // class q of level r at (1 << r) + q:
@@ -962,19 +963,19 @@ plane_pass_kernel(const __grid_constant__ PlanePass p) {
           // [w0, w1) are the run's own and whole; a slot's part of the run's
           // first (before w0) and last word (at w1) is ORed (rev: the other
           // way round)
-          uint32_t const base =
-              rev ? static_cast<uint32_t>((gs + end - 1) >> 5) - (b0 >> 5) - (W - 1)
-                  : static_cast<uint32_t>((gs - off) >> 5) + (b0 >> 5);
+          Words const base = rev ? static_cast<Words>((gs + end - 1) >> 5) - (b0 >> 5) - (W - 1)
+                                 : static_cast<Words>((gs - off) >> 5) + (b0 >> 5);
           uint32_t const f0 = b0 < off ? 1u : 0u, f1 = min(W, (end - b0) / 32);
           bool const tail = f1 < W && b0 + 32 * f1 < end;
           uint32_t const w0 = rev ? W - f1 : f0, w1 = rev ? W - f0 : f1;
           uint32_t const ua = rev ? W - 1 : 0, ub = rev ? W - 1 - f1 : f1;
-          auto put = [&](uint32_t const* y, uint32_t* __restrict__ o, uint32_t nw) {
+          auto put = [&](uint32_t const* y, uint32_t* __restrict__ o, Words nw) {
             uint32_t x[W];
 #pragma unroll
             for (uint32_t u = 0; u < W; ++u) x[u] = rev ? __brev(y[W - 1 - u]) : y[u];
-            o += static_cast<int>(base);  // rev: may start before the array
-            int const lim = min(static_cast<int>(w1), static_cast<int>(nw - base));
+            o += static_cast<Index>(base);  // rev: may start before the array
+            int const lim = static_cast<int>(
+                min(static_cast<Index>(w1), static_cast<Index>(nw - base)));
 #pragma unroll
             for (uint32_t u = 0; u < W; ++u)
               if (u >= w0 && static_cast<int>(u) < lim) o[u] = x[u];
@@ -986,12 +987,12 @@ plane_pass_kernel(const __grid_constant__ PlanePass p) {
               atomicOr(o + ub, e);
             }
           };
-          put(m, p.out[r], p.out_words[r]);
+          put(m, p.out[r], static_cast<Words>(p.out_words[r]));
           for (uint32_t mask = p.ext_mask[r]; mask; mask &= mask - 1) {
             uint32_t const j = __ffs(mask) - 1;
             uint32_t y[W];
             load_slot<W>(cur + (j - 1) * kPS, y);
-            put(y, p.ext[r][j], p.ext_words);
+            put(y, p.ext[r][j], static_cast<Words>(p.ext_words));
           }
         }
         if (r == k) {
@@ -1102,17 +1103,26 @@ plane_pass_kernel(const __grid_constant__ PlanePass p) {
 
 // ---- the pipeline ---------------------------------------------------------------
 
-// Deeper planes of one level's order that outlive the pass writing them:
-// plane(j), first <= j < first + count, is code bit L - 1 - j in level
-// `level`'s order.
+// Deeper planes of one level's order: plane(j), first <= j < first + count, is
+// code bit L - 1 - j in level `level`'s order.  The first `kept` of them
+// outlive the pass that reads the order; the first `front` are in `mem`.
 struct OrderPlanes {
-  uint32_t level = 0, first = 0, count = 0;
+  uint32_t level = 0, first = 0, count = 0, kept = 0, front = 0;
   uint64_t stride = 0;  // words per plane
-  DevBuf mem;
+  DevBuf mem, rest;
   uint32_t* plane(uint32_t j) const {
-    return mem.as<uint32_t>() + uint64_t(j - first) * stride;
+    uint32_t const i = j - first;
+    return i < front ? mem.as<uint32_t>() + uint64_t(i) * stride
+                     : rest.as<uint32_t>() + uint64_t(i - front) * stride;
   }
 };
+
+// Orders of more bytes than this hold the planes that go with their pass in
+// an allocation of their own, so that they make room for the group levels (6
+// Gi symbols of 256: 3.8 bytes per symbol at the peak instead of 4.7).  The
+// pool gives such pieces back in other pieces than it gave them out, which
+// costs more than it saves where memory is not short (6 Gi: 2.7 ms).
+constexpr uint64_t kSplitOrderBytes = uint64_t(32) << 30;
 
 // Levels per pass: as few passes of at most 4 levels as cover the L - 1 below
 // level 0; the first of 3 where that takes no pass more (a group level's
@@ -1136,9 +1146,9 @@ constexpr uint32_t kSlotWords = 4;  // words of a slot: a thread's work
 // The largest CTA of which three fit an SM's shared memory (128: four).
 inline uint32_t pass_slots(uint32_t np) { return np <= 8 ? 256 : 128; }
 
-template <uint32_t NT>
+template <uint32_t NT, class Index>
 void launch_plane_pass_as(PlanePass const& p, uint64_t max_chunks, cudaStream_t st) {
-  auto kern = plane_pass_kernel<NT, kSlotWords>;
+  auto kern = plane_pass_kernel<NT, kSlotWords, Index>;
   set_smem_limit(kern, static_cast<int>(pass_smem(NT, kSlotWords, NT == 256 ? 8 : 15)));
   uint32_t const grid = static_cast<uint32_t>(std::max<uint64_t>(
       1, std::min<uint64_t>(max_chunks, uint64_t(sm_count()) * (NT == 256 ? 3 : 4))));
@@ -1148,8 +1158,12 @@ void launch_plane_pass_as(PlanePass const& p, uint64_t max_chunks, cudaStream_t 
 
 inline void launch_plane_pass(PlanePass const& p, uint32_t slots, uint64_t max_chunks,
                               cudaStream_t st) {
-  if (slots == 256) launch_plane_pass_as<256>(p, max_chunks, st);
-  else launch_plane_pass_as<128>(p, max_chunks, st);
+  // 32-bit word indices while a level's words allow it (2^36 symbols)
+  bool const narrow = p.ext_words < uint64_t(INT32_MAX);
+  if (slots == 256 && narrow) launch_plane_pass_as<256, int32_t>(p, max_chunks, st);
+  else if (slots == 256) launch_plane_pass_as<256, int64_t>(p, max_chunks, st);
+  else if (narrow) launch_plane_pass_as<128, int32_t>(p, max_chunks, st);
+  else launch_plane_pass_as<128, int64_t>(p, max_chunks, st);
 }
 
 // The text of a build (or the concatenated texts of a batch, one node each).
@@ -1191,8 +1205,11 @@ std::vector<OrderPlanes> run_plane_passes(
     o.level = level;
     o.first = level + 1;
     o.count = count;
+    o.kept = std::min(wants(level), count);
+    o.front = count * stride * 4 > kSplitOrderBytes ? o.kept : count;
     o.stride = stride;
-    if (count) o.mem.alloc(count * stride * 4);
+    if (o.front) o.mem.alloc(o.front * stride * 4);
+    if (count > o.front) o.rest.alloc((count - o.front) * stride * 4);
     return o;
   };
   OrderPlanes cur = make_order(0, L - 1);
@@ -1219,8 +1236,7 @@ std::vector<OrderPlanes> run_plane_passes(
         8, std::max<uint64_t>(1, n / g.tile / (uint64_t(sms) * 12))));
     uint64_t const max_tiles = n / g.tile + nodes;
     uint64_t const max_chunks = n / (uint64_t(g.tile) * g.ct) + nodes;
-    EWT_REQUIRE(max_tiles < INT32_MAX && stride < INT32_MAX, EWT_ERR_UNSUPPORTED,
-                "text too long");
+    EWT_REQUIRE(max_tiles < INT32_MAX, EWT_ERR_UNSUPPORTED, "text too long");
     g.rc = ceil_div(64, g.ct);  // 64 tiles a range
     uint64_t const max_ranges = max_chunks / g.rc + nodes;
     // one allocation for the pass's tables
@@ -1310,13 +1326,13 @@ std::vector<OrderPlanes> run_plane_passes(
     p.g = g;
     p.k = k;
     p.np = np;
-    p.ext_words = static_cast<uint32_t>(stride);
+    p.ext_words = stride;
     p.src[0] = words[a];
     for (uint32_t j = 1; j <= np; ++j) p.src[j] = cur.plane(a + j);
     OrderPlanes next;
     for (uint32_t r = 1; r <= k; ++r) {
       p.out[r] = words[a + r];
-      p.out_words[r] = static_cast<uint32_t>(word_count[a + r]);
+      p.out_words[r] = word_count[a + r];
       bool const whole = r == k && !final;  // the next pass's input
       uint32_t const count = whole ? np - k : std::min(wants(a + r), np - r);
       if (!count) continue;
@@ -1336,7 +1352,11 @@ std::vector<OrderPlanes> run_plane_passes(
       EWT_LAUNCHED();
       launch_plane_pass(p, slots, max_chunks, st);
     }
-    if (wants(a)) kept.push_back(std::move(cur));
+    if (cur.kept) {  // the rest makes room for what is built next
+      cur.rest.reset();
+      cur.count = cur.kept;
+      kept.push_back(std::move(cur));
+    }
     cur = std::move(next);
     starts = next_starts;
     nodes <<= k;

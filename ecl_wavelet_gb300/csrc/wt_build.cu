@@ -949,7 +949,7 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
           OrderPlanes o;
           o.level = l;
           o.first = l + 1;
-          o.count = w.second;
+          o.count = o.front = w.second;
           o.stride = ceil_div(ceil_div(n, 32), 32) * 32 + 32;
           o.mem.alloc(o.count * o.stride * 4);
           EWT_CUDA(cudaMemsetAsync(o.mem.get(), 0, o.count * o.stride * 4, st));
