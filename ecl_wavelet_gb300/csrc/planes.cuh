@@ -156,6 +156,20 @@ tile_table_kernel(TileGrid g) {
   }
 }
 
+// Inclusive warp scan (a shuffle's predicate says whether its source lane
+// exists).
+__device__ __forceinline__ uint32_t warp_inclusive(uint32_t x) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1)
+    asm volatile(
+        "{ .reg .pred p; .reg .u32 y;\n"
+        "shfl.sync.up.b32 y|p, %0, %1, 0, 0xffffffff;\n"
+        "@p add.u32 %0, %0, y; }"
+        : "+r"(x)
+        : "r"(o));
+  return x;
+}
+
 // ---- transposes ------------------------------------------------------------
 
 // Four words (a, b, c, d): out[i] = byte i of each, in that order.
@@ -450,6 +464,69 @@ plane_counts_kernel(const __grid_constant__ PlaneSources src, TileGrid g) {
 
 // ---- 3. scans ------------------------------------------------------------------
 
+// One pass: its tiles, input planes and outputs.
+struct PlanePass {
+  TileGrid g;
+  uint32_t k, np;                        // levels written; planes behind plane a
+  uint32_t const* src[kMaxPlanes];       // src[j]: plane a + j, j = 0 .. np
+  uint32_t* out[kMaxPassK + 1];          // out[r]: level a + r, r = 1 .. k
+  uint64_t out_words[kMaxPassK + 1];
+  uint32_t* ext[kMaxPassK + 1][kMaxPlanes];  // plane a + j in level-(a+r) order
+  uint32_t ext_mask[kMaxPassK + 1];      // bit j: ext[r][j] is wanted
+  uint64_t ext_words;
+};
+
+// Clears word w of level a + r and of the deeper planes of its order.
+__device__ __forceinline__ void clear_word(PlanePass const& p, uint32_t r, uint64_t w) {
+  if (w < p.out_words[r]) p.out[r][w] = 0;
+  for (uint32_t mask = p.ext_mask[r]; mask; mask &= mask - 1)
+    if (w < p.ext_words) p.ext[r][__ffs(mask) - 1][w] = 0;
+}
+
+// The words of a pass's outputs that two runs may share, into which the pass
+// ORs, are cleared first: every word that holds the start of a tile's class
+// run, and the arrays' ends (all other words are written whole by one
+// thread).  A warp takes tiles t0 .. t1 - 1 of a node, lane per digit: the
+// digit positions (start: the digit's own, pre: the node's before t0), stepped
+// from tile to tile and added up per class.  (Clearing the outputs whole took
+// 1.4 ms per build of 6 Gi symbols of 256.)
+__device__ __forceinline__ void clear_tile_edges(PlanePass const& p, uint64_t start,
+                                                 uint64_t pre, uint32_t t0, uint32_t t1) {
+  uint32_t const lane = threadIdx.x & 31, D = p.g.D;
+  bool const on = lane < (1u << D);
+  for (uint32_t t = t0; t < t1; ++t) {
+    uint64_t sum = pre;  // of the lane's class
+    for (uint32_t r = D; r > 0; --r) {
+      uint32_t const h = 1u << (D - r);  // digits of a level-r class
+      if (h > 1) sum += __shfl_xor_sync(0xffffffffu, sum, h >> 1);
+      if (r <= p.k && on && (lane & (h - 1)) == 0) clear_word(p, r, (start + sum) >> 5);
+    }
+    if (on) pre += p.g.tile_cnt[(uint64_t(t) << D) + lane];
+  }
+}
+__device__ __forceinline__ void clear_ends(PlanePass const& p) {
+  for (uint32_t r = 1; r <= p.k; ++r) {
+    uint64_t const lim = max(p.out_words[r], p.ext_mask[r] ? p.ext_words : uint64_t(0));
+    for (uint64_t w = (p.g.n >> 5) + threadIdx.x; w < lim; w += blockDim.x) clear_word(p, r, w);
+  }
+}
+
+// ... a warp per chunk.
+__global__ void __launch_bounds__(128)
+clear_edges_kernel(const __grid_constant__ PlanePass p) {
+  uint32_t const lane = threadIdx.x & 31, D = p.g.D;
+  uint32_t const chunks = p.g.chunk_first[p.g.nodes];
+  bool const on = lane < (1u << D);
+  if (blockIdx.x == 0) clear_ends(p);
+  for (uint32_t c = blockIdx.x * 4 + (threadIdx.x >> 5); c < chunks; c += gridDim.x * 4) {
+    uint32_t const N = owner_node(p.g.chunk_first, p.g.nodes, c);
+    uint32_t const t0 = p.g.tile_first[N] + (c - p.g.chunk_first[N]) * p.g.ct;
+    clear_tile_edges(p, on ? *digit_start(p.g, N, lane) : 0,
+                     on ? p.g.chunk_pre[(uint64_t(c) << D) + lane] : 0, t0,
+                     min(t0 + p.g.ct, p.g.tile_first[N + 1]));
+  }
+}
+
 // Range r: its node and tiles [t0, t1) (whole chunks).
 __device__ __forceinline__ uint32_t range_tiles(TileGrid const& g, uint32_t r, uint32_t* t0,
                                                 uint32_t* t1) {
@@ -533,9 +610,12 @@ digit_starts_kernel(TileGrid g) {
 }
 
 // All of the scan in one launch for orders of few tiles: a CTA per node, lane
-// per digit, a stretch of chunks per warp.
+// per digit, a stretch of chunks per warp.  With p.k > 0 the outputs' shared
+// words are cleared as well; with next.nodes > 0 (a single node) the next
+// pass's tables are made.
 __global__ void __launch_bounds__(1024)
-node_scan_kernel(TileGrid g) {
+node_scan_kernel(const __grid_constant__ PlanePass p, const __grid_constant__ TileGrid next) {
+  TileGrid const& g = p.g;
   uint32_t const d = threadIdx.x & 31, wid = threadIdx.x >> 5, warps = blockDim.x >> 5;
   uint32_t const N = blockIdx.x;
   bool const on = d < (1u << g.D);
@@ -547,12 +627,34 @@ node_scan_kernel(TileGrid g) {
   uint64_t own = 0;
 #pragma unroll 8
   for (uint32_t t = t0; t < t1; ++t) own += on ? c[uint64_t(t) << g.D] : 0;
-  uint64_t run = node_digit_starts(g, N, own);
+  uint64_t const before = node_digit_starts(g, N, own);
+  uint64_t run = before;
 #pragma unroll 8
   for (uint32_t t = t0; t < t1; ++t) {
     if (on && (t - f) % g.ct == 0)
       g.chunk_pre[(uint64_t(c0 + (t - f) / g.ct) << g.D) + d] = run;
     run += on ? c[uint64_t(t) << g.D] : 0;
+  }
+  __syncthreads();  // the digit starts are written
+  if (p.k) {
+    if (N == 0) clear_ends(p);
+    clear_tile_edges(p, on ? *digit_start(g, N, d) : 0, before, t0, t1);
+  }
+  if (next.nodes && wid == 0) {  // as many as this pass has digits
+    uint32_t x[3] = {0, 0, 0};
+    if (on) {
+      uint64_t const len = g.starts_next[d + 1] - g.starts_next[d];
+      x[0] = static_cast<uint32_t>((len + next.tile - 1) / next.tile);
+      x[1] = (x[0] + next.ct - 1) / next.ct;
+      x[2] = (x[1] + next.rc - 1) / next.rc;
+    }
+    uint32_t* const first[3] = {next.tile_first, next.chunk_first, next.range_first};
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      uint32_t const inc = warp_inclusive(x[i]);
+      if (on) first[i][d] = inc - x[i];
+      if (on && d == next.nodes - 1) first[i][next.nodes] = inc;
+    }
   }
 }
 
@@ -576,56 +678,6 @@ chunk_starts_kernel(TileGrid g) {
 
 // ---- 4. the pass ------------------------------------------------------------------
 
-struct PlanePass {
-  TileGrid g;
-  uint32_t k, np;                        // levels written; planes behind plane a
-  uint32_t const* src[kMaxPlanes];       // src[j]: plane a + j, j = 0 .. np
-  uint32_t* out[kMaxPassK + 1];          // out[r]: level a + r, r = 1 .. k
-  uint64_t out_words[kMaxPassK + 1];
-  uint32_t* ext[kMaxPassK + 1][kMaxPlanes];  // plane a + j in level-(a+r) order
-  uint32_t ext_mask[kMaxPassK + 1];      // bit j: ext[r][j] is wanted
-  uint64_t ext_words;
-};
-
-// Clears the words of a pass's outputs that two runs may share, into which
-// the pass ORs: every word that holds the start of a tile's class run, and the
-// arrays' ends (all other words are written whole by one thread).  A warp per
-// chunk, lane per digit: the chunk's digit positions, stepped from tile to
-// tile and added up per class.  (Clearing the outputs whole took 1.4 ms per
-// build of 6 Gi symbols of 256.)
-__global__ void __launch_bounds__(128)
-clear_edges_kernel(const __grid_constant__ PlanePass p) {
-  uint32_t const lane = threadIdx.x & 31, D = p.g.D, digits = 1u << D;
-  uint32_t const chunks = p.g.chunk_first[p.g.nodes];
-  uint64_t const w_end = p.g.n >> 5;
-  auto clear = [&](uint32_t r, uint64_t w) {
-    if (w < p.out_words[r]) p.out[r][w] = 0;
-    for (uint32_t mask = p.ext_mask[r]; mask; mask &= mask - 1)
-      if (w < p.ext_words) p.ext[r][__ffs(mask) - 1][w] = 0;
-  };
-  if (blockIdx.x == 0)
-    for (uint32_t r = 1; r <= p.k; ++r) {
-      uint64_t const lim = max(p.out_words[r], p.ext_mask[r] ? p.ext_words : uint64_t(0));
-      for (uint64_t w = w_end + threadIdx.x; w < lim; w += blockDim.x) clear(r, w);
-    }
-  for (uint32_t c = blockIdx.x * 4 + (threadIdx.x >> 5); c < chunks; c += gridDim.x * 4) {
-    uint32_t const N = owner_node(p.g.chunk_first, p.g.nodes, c);
-    uint32_t const t0 = p.g.tile_first[N] + (c - p.g.chunk_first[N]) * p.g.ct;
-    uint32_t const t1 = min(t0 + p.g.ct, p.g.tile_first[N + 1]);
-    bool const on = lane < digits;
-    uint64_t const start = on ? *digit_start(p.g, N, lane) : 0;
-    uint64_t pre = on ? p.g.chunk_pre[(uint64_t(c) << D) + lane] : 0;
-    for (uint32_t t = t0; t < t1; ++t) {
-      uint64_t sum = pre;  // of the lane's class
-      for (uint32_t r = D; r > 0; --r) {
-        uint32_t const h = 1u << (D - r);  // digits of a level-r class
-        if (h > 1) sum += __shfl_xor_sync(0xffffffffu, sum, h >> 1);
-        if (r <= p.k && on && (lane & (h - 1)) == 0) clear(r, (start + sum) >> 5);
-      }
-      if (on) pre += p.g.tile_cnt[(uint64_t(t) << D) + lane];
-    }
-  }
-}
 
 // Swap masks of the five in-word stages for one word of the mask plane with
 // r0 ones before it in the slot: c[s] holds the positions q of the left
@@ -745,20 +797,6 @@ __host__ __device__ __forceinline__ void swap_words(uint32_t* x, WordSwaps<W> co
         x[b + u] ^= t;
         x[b + h + u] ^= t;
       }
-}
-
-// Inclusive warp scan (a shuffle's predicate says whether its source lane
-// exists).
-__device__ __forceinline__ uint32_t warp_inclusive(uint32_t x) {
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1)
-    asm volatile(
-        "{ .reg .pred p; .reg .u32 y;\n"
-        "shfl.sync.up.b32 y|p, %0, %1, 0, 0xffffffff;\n"
-        "@p add.u32 %0, %0, y; }"
-        : "+r"(x)
-        : "r"(o));
-  return x;
 }
 
 template <uint32_t W>
@@ -1220,35 +1258,55 @@ std::vector<OrderPlanes> run_plane_passes(
     starts_buf[0].alloc(16);
     starts = starts_buf[0].as<uint64_t>();
   }
+  // ---- every pass's tiles, and one allocation for the nodes' tables
+  std::vector<TileGrid> grids(ks.size());
+  DevBuf tables;
+  {
+    size_t bytes = 0;
+    std::vector<size_t> at;
+    uint64_t nd = nodes;
+    for (size_t i = 0, a = 0; i < ks.size(); a += ks[i], nd <<= ks[i], ++i) {
+      TileGrid& g = grids[i];
+      g.n = n;
+      g.nodes = static_cast<uint32_t>(nd);
+      g.halves = i + 1 == ks.size() && ks[i];
+      g.D = std::max(ks[i], 1u);
+      g.tile = pass_tile(pass_slots(static_cast<uint32_t>(L - 1 - a)), kSlotWords, ks[i]);
+      // chunks of up to 8 tiles while every CTA still gets several
+      g.ct = static_cast<uint32_t>(std::min<uint64_t>(
+          8, std::max<uint64_t>(1, n / g.tile / (uint64_t(sms) * 12))));
+      g.rc = ceil_div(64, g.ct);  // 64 tiles a range
+      at.push_back(bytes);
+      bytes += 3 * ((nd + 1) * 4 + 255) / 256 * 256;
+    }
+    tables.alloc(bytes);
+    for (size_t i = 0; i < grids.size(); ++i) {
+      uint32_t* const first = reinterpret_cast<uint32_t*>(tables.as<unsigned char>() + at[i]);
+      grids[i].tile_first = first;
+      grids[i].chunk_first = first + grids[i].nodes + 1;
+      grids[i].range_first = first + 2 * (uint64_t(grids[i].nodes) + 1);
+    }
+  }
   uint32_t a = 0;
+  bool tables_made = false;  // of this pass, by the one before
   for (size_t i = 0; i < ks.size(); ++i) {
     uint32_t const k = ks[i], b = a + k, np = L - 1 - a;
     bool const final = i + 1 == ks.size();
     uint32_t const slots = pass_slots(np);
-    TileGrid g{};
-    g.n = n;
-    g.nodes = nodes;
-    g.halves = final && k;
-    g.D = std::max(k, 1u);
-    g.tile = pass_tile(slots, kSlotWords, k);
-    // chunks of up to 8 tiles while every CTA still gets several
-    g.ct = static_cast<uint32_t>(std::min<uint64_t>(
-        8, std::max<uint64_t>(1, n / g.tile / (uint64_t(sms) * 12))));
+    TileGrid& g = grids[i];
     uint64_t const max_tiles = n / g.tile + nodes;
     uint64_t const max_chunks = n / (uint64_t(g.tile) * g.ct) + nodes;
     EWT_REQUIRE(max_tiles < INT32_MAX, EWT_ERR_UNSUPPORTED, "text too long");
-    g.rc = ceil_div(64, g.ct);  // 64 tiles a range
     uint64_t const max_ranges = max_chunks / g.rc + nodes;
-    // one allocation for the pass's tables
+    // one allocation for the pass's counts
     size_t bytes = 0;
     auto room = [&](uint64_t b) {
       size_t const at = bytes;
       bytes += (b + 255) / 256 * 256;
       return at;
     };
-    size_t const at_tf = room((uint64_t(nodes) + 1) * 4), at_cf = room((uint64_t(nodes) + 1) * 4),
-                 at_rf = room((uint64_t(nodes) + 1) * 4), at_cnt = room((max_tiles << g.D) * 2),
-                 at_pre = room((max_chunks << g.D) * 8), at_tot = room((max_ranges << g.D) * 8);
+    size_t const at_cnt = room((max_tiles << g.D) * 2), at_pre = room((max_chunks << g.D) * 8),
+                 at_tot = room((max_ranges << g.D) * 8);
     scratch.alloc(bytes);
     unsigned char* const base = scratch.as<unsigned char>();
     uint64_t* next_starts = starts_out;
@@ -1258,9 +1316,6 @@ std::vector<OrderPlanes> run_plane_passes(
       next_starts = sb.as<uint64_t>();
     }
     g.starts = starts;
-    g.tile_first = reinterpret_cast<uint32_t*>(base + at_tf);
-    g.chunk_first = reinterpret_cast<uint32_t*>(base + at_cf);
-    g.range_first = reinterpret_cast<uint32_t*>(base + at_rf);
     g.tile_cnt = reinterpret_cast<uint16_t*>(base + at_cnt);
     g.chunk_pre = reinterpret_cast<uint64_t*>(base + at_pre);
     g.range_tot = reinterpret_cast<uint64_t*>(base + at_tot);
@@ -1285,43 +1340,7 @@ std::vector<OrderPlanes> run_plane_passes(
       kern<<<scan_grid, kIngestThreads, 0, st>>>(x.sym, ia);
       EWT_LAUNCHED();
     }
-    {
-      PhaseTimer pt(EWT_PHASE_HIST, st);
-      if (nodes > 1) {
-        tile_table_kernel<<<1, 1024, 0, st>>>(g);
-        EWT_LAUNCHED();
-      }
-      if (i > 0 || nodes > 1) {
-        PlaneSources src{};
-        src.p[0] = words[a];
-        for (uint32_t j = 1; j < g.D; ++j) src.p[j] = cur.plane(a + j);
-        auto kern = g.D == 1   ? plane_counts_kernel<1>
-                    : g.D == 2 ? plane_counts_kernel<2>
-                    : g.D == 3 ? plane_counts_kernel<3>
-                               : plane_counts_kernel<4>;
-        kern<<<static_cast<uint32_t>(std::min<uint64_t>(max_tiles, uint64_t(sms) * 12)),
-               kCountThreads, 0, st>>>(src, g);
-        EWT_LAUNCHED();
-      }
-      // One launch while the tiles are few enough for the warps of one CTA,
-      // should a single node hold them all (16 Mi symbols, 520 tiles: 7 us
-      // against 17 us by three launches).
-      uint32_t const range_grid = static_cast<uint32_t>(ceil_div(max_ranges, kRangeWarps));
-      if (max_tiles <= 2048) {
-        node_scan_kernel<<<nodes, nodes == 1 ? 1024 : nodes <= 64 ? 512 : 128, 0, st>>>(g);
-        EWT_LAUNCHED();
-      } else {
-        range_totals_kernel<<<range_grid, kRangeWarps * 32, 0, st>>>(g);
-        EWT_LAUNCHED();
-        digit_starts_kernel<<<nodes, nodes <= 64 ? 1024 : 128, 0, st>>>(g);
-        EWT_LAUNCHED();
-        if (k) {
-          chunk_starts_kernel<<<range_grid, kRangeWarps * 32, 0, st>>>(g);
-          EWT_LAUNCHED();
-        }
-      }
-    }
-    if (k == 0) break;
+    // ---- the pass's outputs
     PlanePass p{};
     p.g = g;
     p.k = k;
@@ -1344,12 +1363,60 @@ std::vector<OrderPlanes> run_plane_passes(
       if (whole) next = std::move(o);
       else kept.push_back(std::move(o));
     }
+    bool const few_tiles = max_tiles <= 2048;
+    bool const clears = few_tiles && k && n / g.tile <= 256;
+    {
+      PhaseTimer pt(EWT_PHASE_HIST, st);
+      if (nodes > 1 && !tables_made) {
+        tile_table_kernel<<<1, 1024, 0, st>>>(g);
+        EWT_LAUNCHED();
+      }
+      if (i > 0 || nodes > 1) {
+        PlaneSources src{};
+        src.p[0] = words[a];
+        for (uint32_t j = 1; j < g.D; ++j) src.p[j] = cur.plane(a + j);
+        auto kern = g.D == 1   ? plane_counts_kernel<1>
+                    : g.D == 2 ? plane_counts_kernel<2>
+                    : g.D == 3 ? plane_counts_kernel<3>
+                               : plane_counts_kernel<4>;
+        kern<<<static_cast<uint32_t>(std::min<uint64_t>(max_tiles, uint64_t(sms) * 12)),
+               kCountThreads, 0, st>>>(src, g);
+        EWT_LAUNCHED();
+      }
+      // One launch while the tiles are few enough for the warps of one CTA,
+      // should a single node hold them all (16 Mi symbols, 520 tiles: 7 us
+      // against 17 us by three launches); it clears the outputs' shared words
+      // up to eight tiles a warp (about 3 us, as long as a launch takes).
+      uint32_t const range_grid = static_cast<uint32_t>(ceil_div(max_ranges, kRangeWarps));
+      tables_made = few_tiles && nodes == 1 && !final;
+      if (few_tiles) {
+        PlanePass scanned = p;
+        scanned.k = clears ? k : 0;
+        TileGrid following{};
+        if (tables_made) following = grids[i + 1];
+        node_scan_kernel<<<nodes, nodes == 1 ? 1024 : nodes <= 64 ? 512 : 128, 0, st>>>(
+            scanned, following);
+        EWT_LAUNCHED();
+      } else {
+        range_totals_kernel<<<range_grid, kRangeWarps * 32, 0, st>>>(g);
+        EWT_LAUNCHED();
+        digit_starts_kernel<<<nodes, nodes <= 64 ? 1024 : 128, 0, st>>>(g);
+        EWT_LAUNCHED();
+        if (k) {
+          chunk_starts_kernel<<<range_grid, kRangeWarps * 32, 0, st>>>(g);
+          EWT_LAUNCHED();
+        }
+      }
+    }
+    if (k == 0) break;
     {
       PhaseTimer pt(EWT_PHASE_SPLIT, st);
-      clear_edges_kernel<<<static_cast<uint32_t>(std::min<uint64_t>(
-                               ceil_div(max_chunks, 4), uint64_t(sms) * 8)),
-                           128, 0, st>>>(p);
-      EWT_LAUNCHED();
+      if (!clears) {
+        clear_edges_kernel<<<static_cast<uint32_t>(std::min<uint64_t>(
+                                 ceil_div(max_chunks, 4), uint64_t(sms) * 8)),
+                             128, 0, st>>>(p);
+        EWT_LAUNCHED();
+      }
       launch_plane_pass(p, slots, max_chunks, st);
     }
     if (cur.kept) {  // the rest makes room for what is built next
