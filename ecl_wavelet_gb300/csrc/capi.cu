@@ -125,10 +125,12 @@ void populate_for_write(void* p, size_t bytes) {
 
 // Largest batch moved through the device scratch in one piece.
 constexpr uint64_t kChunk = uint64_t(1) << 25;
-// Host batches from this size on run pipelined (QueryPipe): where a kernel
-// can copy pageable host memory from 2^19 queries on (1 Mi mixed queries: in
+// Host batches from this size on run pipelined (QueryPipe): pageable buffers,
+// where a kernel can copy them, from 2^19 queries on (1 Mi mixed queries: in
 // place 458 us, pipelined 300 us; 128 Ki: in place 79 us, and eight chunks of
-// copies alone cost as much in launches), else from 2^21.
+// copies alone cost as much in launches), else from 2^21.  Buffers that CUDA
+// knows keep to the copy engines, which hold nobody up (2^22 mixed queries from
+// pinned memory: 551 us, by kernels 696; 1 Mi in place 299, by kernels 322).
 constexpr uint64_t kPipeMin = uint64_t(1) << 21, kPipeMinKernel = uint64_t(1) << 19;
 
 // Copies between host and device memory by a kernel, V bytes a step (both
@@ -168,6 +170,16 @@ void copy_async(void* dst, void const* src, uint64_t bytes, bool by_kernel, cuda
   else if (low % 4 == 0) run(uint32_t{});
   else run(uint8_t{});
   EWT_LAUNCHED();
+}
+
+// Whether p is ordinary host memory that CUDA knows nothing of.
+bool is_pageable(void const* p) {
+  cudaPointerAttributes a{};
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeUnregistered;
 }
 
 void ensure(DevBuf& b, size_t& cap, size_t bytes) {
@@ -248,7 +260,8 @@ int host_batch(ewt_tree* t, void const* in, size_t in_rec, uint8_t const* types,
     DeviceGuard g(t->device);
     AllocStream as(t->stream);
     cudaStream_t s = t->stream;
-    bool const by_kernel = pageable_access(t->device);
+    bool const by_kernel = m >= kPipeMinKernel && pageable_access(t->device) &&
+                           is_pageable(in) && is_pageable(out) && (!types || is_pageable(types));
     if (m >= (by_kernel ? kPipeMinKernel : kPipeMin)) {
       // large batches: copies in and out overlap the kernels chunk by chunk
       // (which then work on device memory only)

@@ -44,3 +44,19 @@ def test_odd_addresses(ewt, tree, shift):
     assert ewt.lib().ewt_access(t.handle, room_in.ctypes.data + a, m, room_out.ctypes.data + b) == 0
     assert np.array_equal(room_out[b:b + m], text[idx.astype(np.int64)])
     assert not room_out[:b].any() and not room_out[b + m:].any()
+
+
+@pytest.mark.parametrize("m", [MIN + 7, 4 * MIN + 33])
+@pytest.mark.parametrize("pinned", [(True, True), (True, False), (False, True)])
+def test_pinned_buffers(ewt, tree, m, pinned):
+    torch = pytest.importorskip("torch")
+    text, t = tree
+    rng = np.random.default_rng(m)
+
+    def room(count, dtype, pin):
+        return torch.zeros(count * dtype().itemsize, dtype=torch.uint8, pin_memory=pin).numpy().view(dtype)
+
+    idx, out = room(m, np.uint64, pinned[0]), room(m, np.uint8, pinned[1])
+    idx[:] = rng.integers(0, text.size, m)
+    assert ewt.lib().ewt_access(t.handle, idx.ctypes.data, m, out.ctypes.data) == 0
+    assert np.array_equal(out, text[idx.astype(np.int64)])
