@@ -267,8 +267,50 @@ def reference_gpu(n, sigma, m, reps=2, timeout=900):
     return out
 
 
+def plane_pass_plan(L):
+    """Levels written by each bit-plane pass of a build, as the library plans
+    them (planes.cuh plan_plane_passes): as few passes of at most four levels
+    as cover the L - 1 below level 0, the first of three where that takes no
+    pass more, the others of near-equal size."""
+    rest = L - 1
+    if rest <= 4:
+        return [rest] if rest else []
+    plan = []
+    if -(-(rest - 3) // 4) + 1 == -(-rest // 4):
+        plan, rest = [3], rest - 3
+    np_ = -(-rest // 4)
+    return plan + [rest // np_ + (1 if i < rest % np_ else 0) for i in range(np_)]
+
+
+def plane_pass_bytes_per_launch(n, L):
+    """Algorithmic HBM bytes of one bit-plane pass over n symbols, averaged
+    over the passes.  A pass from level a to b reads planes a .. L-1 of the
+    level-a order and writes levels a+1 .. b, the deeper planes of the level-b
+    order unless it is the last pass, and those of the other orders that a
+    group level reads."""
+    plan = plane_pass_plan(L)
+    if not plan:
+        return 0.0
+    # group levels: as many of three levels as fit, then one or two of two
+    quads = (0, 2, 1)[L % 3] if L > 1 else 0
+    wanted, l = {}, 0
+    for w in [3] * ((L - 2 * quads) // 3) + [2] * quads:
+        wanted[l] = w - 1
+        l += w
+    planes, a = 0, 0
+    for k in plan:
+        b = a + k
+        planes += L - a + k
+        for j in range(a + 1, b + 1):
+            whole = j == b and b < L - 1
+            planes += L - 1 - j if whole else min(wanted.get(j, 0), L - 1 - j)
+        a = b
+    return planes * n / 8.0 / len(plan)
+
+
 def pass_plan(L):
-    """Levels emitted by each build pass, as the library plans them: with
+    """Levels emitted by each pass over the symbols themselves (the form of
+    the build before it kept its orders as bit planes): with
     octal group levels at 0 and 3 and at most four levels below level 3
     (L = 6 or 8) a first pass of levels 1-3 and one of the rest (its level-3
     order feeds octal level 3); else the L - 1 levels below level 0 in
@@ -738,14 +780,15 @@ def run_ours(args, world, rank, local):
     dom_ms, dom_launches = build_phases[dom]
     L = int(tree.getNumLevels())
     per_launch_bytes = {
-        # split: the multi-level passes (power-of-two alphabet, uint8)
-        "split": pass_bytes_per_launch(n, L),
-        # fill: read the level order, write one bit per symbol
-        "fill": n + n / 8.0,
-        # rank/select counts: read one level's bits, write L2 + L1
-        "rs_counts": n / 8.0 + 2.0 * n / 512 + 8.0 * n / 65536,
-        # digit counts of each pass: read the level order
-        "hist": float(n),
+        # split: the bit-plane passes
+        "split": plane_pass_bytes_per_launch(n, L),
+        # fill: read the text, write its bit planes
+        "fill": n + L * n / 8.0,
+        # rank/select counts: read the levels' bits, write L2 + L1
+        "rs_counts": L * (n / 8.0 + 2.0 * n / 512 + 8.0 * n / 65536),
+        # digit counts of the second pass: read its top planes (the first
+        # pass's come from the fill)
+        "hist": (plane_pass_plan(L) or [0])[-1] * n / 8.0,
         "samples": 2.0 * L * n / 512 + 16.0 * L * n / 4096,
         "node_ranks": 0.0,
     }

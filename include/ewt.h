@@ -305,9 +305,9 @@ int ewt_probe_random_reads(int gpu_index, uint64_t bytes, uint32_t depth,
  * them (select then runs the reference's sample -> L1 -> L2 search, or on
  * group levels a search of the superblock table), else a
  * power of two in [32, 65536]; each entry costs 4 bytes.  Built at 256 by
- * default.  Octal group levels (3-bit digits) of power-of-two trees sample
- * eight times as densely (rate / 8, at least 16).  Refused (EWT_ERR_INVALID_ARGUMENT) once the device view was
- * copied out.  No reference counterpart (rank_select.cuh:44-64 fixes one
+ * default.  Octal group levels (3-bit digits) sample eight times as densely
+ * (rate / 8, at least 16).  Refused (EWT_ERR_INVALID_ARGUMENT) once the device
+ * view was copied out.  No reference counterpart (rank_select.cuh:44-64 fixes one
  * sample per 4096 at compile time). */
 int ewt_set_select_samples(ewt_tree* tree, uint32_t rate);
 int ewt_rs_set_select_samples(ewt_rs* rs, uint32_t rate);
