@@ -823,13 +823,13 @@ __device__ __forceinline__ void store_slot(uint32_t* p, uint32_t const* y) {
 // a chunk's tiles in order (the run positions carry from tile to tile).
 // Per tile: class tables of all levels from the tile's digit counts (warp r
 // builds level r's); then per level r: every slot finds its class and writes
-// its 64 bits of level a+r (and of the wanted deeper planes) out, a scan of
+// its 128 bits of level a+r (and of the wanted deeper planes) out, a scan of
 // the slots' zero counts gives each slot's place in its class's two
 // children, and every deeper plane is swapped and ORed into the next order's
 // buffer.
 //
-// Bound by the ALU pipe (two thirds busy, three quarters of the issue slots
-// used; 3 CTAs of 256 threads per SM by shared memory).  128-bit slots: a
+// Bound by the ALU pipe (73 % busy, 62 % of the issue slots used; 3 CTAs of
+// 256 threads per SM by shared memory).  128-bit slots: a
 // slot's bookkeeping costs about as much as three plane moves, so 64-bit
 // slots took 28 % more instructions; 256-bit slots leave 3 warps per
 // scheduler (18 % slower).  Passes of at most 4 levels: with 128 classes

@@ -149,14 +149,20 @@ query_kernel(TreeView t, uint8_t const* __restrict__ types,
 
 // Batched mixed form: CTAs take chunks of up to 2048 queries of the interleaved
 // batch, sort each chunk's query numbers by type in shared memory (warp
-// ballots), then walk the access, rank and select lists one after the other,
-// each from a warp boundary on, so every warp runs one kind of walk and the
-// kinds run side by side.  Results go straight to their original slots.
+// ballots), then walk the select, rank and access lists.  A list begins at the
+// warp behind the one before it, so every warp runs one kind of walk and short
+// lists run side by side.  Results go straight to their original slots.
+//
+// Joined: one loop over the three lists, which keeps all warps busy at the
+// lists' ends (4 Mi queries over 16 Mi symbols of 256: 198 us, 218 list by
+// list, 226 with every list from the CTA's first warp on).  Over an index that
+// is read from DRAM the kinds' own loops are the faster ones: 2^26 queries over
+// 6 Gi symbols of 256 in 7.41 ms, 7.50 joined.
 constexpr uint32_t kMixChunk = 2048;
 // Smallest chunk: with fewer queries the staged tables cost more than the walks.
 constexpr uint32_t kMixChunkMin = 64;
 
-template <class T>
+template <class T, bool Joined>
 __global__ void __launch_bounds__(kMaxQueryThreads)
 mixed_kernel(TreeView t, uint8_t const* __restrict__ types,
              QueryRec<T> const* __restrict__ in, uint64_t m,
@@ -225,31 +231,51 @@ mixed_kernel(TreeView t, uint8_t const* __restrict__ types,
       }
     }
     __syncthreads();
-    // selects first: their walks are the longest
-    uint32_t const e2 = (list_len[2] + 31) & ~31u, e1 = e2 + ((list_len[1] + 31) & ~31u);
-    uint32_t const e0 = e1 + list_len[0];
-    for (uint32_t i = threadIdx.x; i < e0; i += blockDim.x) {
-      uint32_t const k = i < e2 ? 2u : i < e1 ? 1u : 0u;
-      uint32_t const at = i - (k == 2 ? 0u : k == 1 ? e2 : e1);
-      if (at >= list_len[k]) continue;
-      uint64_t const q = base + lists[k][at];
-      if (k == 0) {
-        uint64_t const idx = in[q].index;
-        out[q] = idx < t.n ? static_cast<uint64_t>(from_minimal<T>(
-                                 t, wt_access(t, meta, counts, ranks, node_base, idx, walk)))
-                           : 0;
-        continue;
-      }
+    auto answer_access = [&](uint64_t q) {
+      uint64_t const idx = in[q].index;
+      out[q] = idx < t.n ? static_cast<uint64_t>(from_minimal<T>(
+                               t, wt_access(t, meta, counts, ranks, node_base, idx, walk)))
+                         : 0;
+    };
+    auto answer = [&](uint64_t q, bool rank) {
       QueryRec<T> const r = in[q];
       uint64_t const sym = to_minimal<T>(t, r.symbol);
       uint64_t res = UINT64_MAX;
-      if (sym >= t.sigma || (k == 1 ? r.index > t.n : r.index == 0))
+      if (sym >= t.sigma || (rank ? r.index > t.n : r.index == 0))
         bad = 1;
-      else if (k == 1)
+      else if (rank)
         res = wt_rank(t, meta, counts, ranks, node_base, sym, r.index, walk);
       else
         res = wt_select(t, meta, counts, ranks, node_base, sym, r.index, walk);
       out[q] = res;
+    };
+    if constexpr (Joined) {  // selects first: their walks are the longest
+      uint32_t const e2 = (list_len[2] + 31) & ~31u, e1 = e2 + ((list_len[1] + 31) & ~31u);
+      uint32_t const e0 = e1 + list_len[0];
+      for (uint32_t i = threadIdx.x; i < e0; i += blockDim.x) {
+        uint32_t const k = i < e2 ? 2u : i < e1 ? 1u : 0u;
+        uint32_t const at = i - (k == 2 ? 0u : k == 1 ? e2 : e1);
+        if (at >= list_len[k]) continue;
+        uint64_t const q = base + lists[k][at];
+        if (k == 0)
+          answer_access(q);
+        else
+          answer(q, k == 1);
+      }
+    } else {
+      uint32_t first = 0;  // thread of the list's first query
+      auto begin = [&](uint32_t k) {
+        uint32_t const i = threadIdx.x >= first ? threadIdx.x - first
+                                                : threadIdx.x + blockDim.x - first;
+        first = (first + ((list_len[k] + 31) & ~31u)) % blockDim.x;
+        return i;
+      };
+      for (uint32_t i = begin(0); i < list_len[0]; i += blockDim.x)
+        answer_access(base + lists[0][i]);
+      for (uint32_t i = begin(1); i < list_len[1]; i += blockDim.x)
+        answer(base + lists[1][i], true);
+      for (uint32_t i = begin(2); i < list_len[2]; i += blockDim.x)
+        answer(base + lists[2][i], false);
     }
     __syncthreads();  // lists are reused by the next chunk
   }
@@ -296,6 +322,11 @@ rs_select_kernel(RSView v, uint32_t array, uint64_t const* __restrict__ idx,
 
 namespace {
 
+// Level bits up to which mixed_kernel joins its lists: 16 Mi queries over 2^28,
+// 2^30, 2^31 symbols of 256 take 1394, 1580, 1662 us joined and 1412, 1580, 1665
+// us list by list.
+constexpr uint64_t kJoinedBytes = uint64_t(1) << 30;
+
 // One mixed_kernel launch with the tree's tuned shape (threads x CTAs per SM
 // when the autotuner chose them), timed as a query phase; invalid queries
 // set *err.
@@ -305,7 +336,7 @@ void launch_mixed_kernel(ewt_tree& t, uint8_t const* types, void const* in,
                          StagePlan const& p, cudaStream_t s,
                          uint32_t* queue) {
   RelaxedCapture relaxed;
-  auto mk = mixed_kernel<T>;
+  auto mk = t.n * t.L / 8 <= kJoinedBytes ? mixed_kernel<T, true> : mixed_kernel<T, false>;
   set_smem_limit(mk, static_cast<int>(kStageLimitBytes + 4096));
   uint32_t const threads =
       t.tune_threads[kMixed] ? t.tune_threads[kMixed] : kQueryThreads;
@@ -459,7 +490,7 @@ random_chain_kernel(uint4 const* __restrict__ a, uint64_t units, uint32_t depth,
 
 int kernel_binary_version() {
   cudaFuncAttributes a{};
-  EWT_CUDA(cudaFuncGetAttributes(&a, mixed_kernel<uint8_t>));
+  EWT_CUDA(cudaFuncGetAttributes(&a, mixed_kernel<uint8_t, true>));
   return a.binaryVersion;
 }
 
