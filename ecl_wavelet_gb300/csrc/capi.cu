@@ -274,6 +274,7 @@ int host_batch(ewt_tree* t, void const* in, size_t in_rec, uint8_t const* types,
                   "query and result buffers must be 8-byte aligned");
       QueryPipe& P = t->pipe;
       P.init();
+      DrainOnError drain(P.s_in, s, P.s_out);
       uint64_t const chunk = std::max<uint64_t>(
           (by_kernel ? kPipeMinKernel : kPipeMin) / 4, ceil_div(ceil_div(m, 8), 16) * 16);
       for (int x = 0; x < 2; ++x) {  // allocated on s, before the copy streams start
@@ -305,6 +306,7 @@ int host_batch(ewt_tree* t, void const* in, size_t in_rec, uint8_t const* types,
       }
       EWT_CUDA(cudaStreamWaitEvent(s, P.out_done[(i - 1) & 1], 0));
       int const st = take_query_status(t->err_d, &t->status_word, t->device, s);
+      drain.dismiss();
       if (st != EWT_OK)
         throw Error(st, "the batch held invalid queries (their results are "
                         "UINT64_MAX)");
@@ -314,8 +316,10 @@ int host_batch(ewt_tree* t, void const* in, size_t in_rec, uint8_t const* types,
       // the kernel reads the caller's queries and writes its results in
       // place (host page tables): no staging copies
       populate_for_write(out, m * out_rec);
+      DrainOnError drain(s);
       launch(types, in, m, out, s);
       int const st = take_query_status(t->err_d, &t->status_word, t->device, s);
+      drain.dismiss();
       if (st != EWT_OK)
         throw Error(st, "the batch held invalid queries (their results are "
                         "UINT64_MAX)");
@@ -326,6 +330,7 @@ int host_batch(ewt_tree* t, void const* in, size_t in_rec, uint8_t const* types,
     ensure(sc.in, sc.in_cap, chunk * in_rec);
     ensure(sc.out, sc.out_cap, chunk * out_rec);
     if (types) ensure(sc.types, sc.types_cap, chunk);
+    DrainOnError drain(s);
     for (uint64_t b = 0; b < m; b += chunk) {
       uint64_t const k = std::min(chunk, m - b);
       EWT_CUDA(cudaMemcpyAsync(sc.in.get(),
@@ -340,6 +345,7 @@ int host_batch(ewt_tree* t, void const* in, size_t in_rec, uint8_t const* types,
                                s));
     }
     int const st = take_query_status(t->err_d, &t->status_word, t->device, s);
+    drain.dismiss();
     if (st != EWT_OK)
       throw Error(st, "the batch held invalid queries (their results are "
                       "UINT64_MAX)");
@@ -359,8 +365,10 @@ int rs_host_batch(ewt_rs* r, uint64_t const* in, uint64_t m, uint64_t* out,
     AllocStream as(r->stream);
     if (pageable_access(r->device)) {  // in place, as host_batch
       populate_for_write(out, m * 8);
+      DrainOnError drain(r->stream);
       launch(in, m, out, r->stream);
       int const st = take_query_status(r->err_d, &r->status_word, r->device, r->stream);
+      drain.dismiss();
       if (st != EWT_OK)
         throw Error(st, "the batch held invalid queries (their results are "
                         "UINT64_MAX)");
@@ -371,6 +379,7 @@ int rs_host_batch(ewt_rs* r, uint64_t const* in, uint64_t m, uint64_t* out,
     ensure(sc.in, sc.in_cap, chunk * 8);
     ensure(sc.out, sc.out_cap, chunk * 8);
     cudaStream_t s = r->stream;
+    DrainOnError drain(s);
     for (uint64_t b = 0; b < m; b += chunk) {
       uint64_t const k = std::min(chunk, m - b);
       EWT_CUDA(cudaMemcpyAsync(sc.in.get(), in + b, k * 8, cudaMemcpyDefault, s));
@@ -379,6 +388,7 @@ int rs_host_batch(ewt_rs* r, uint64_t const* in, uint64_t m, uint64_t* out,
                                s));
     }
     int const st = take_query_status(r->err_d, &r->status_word, r->device, s);
+    drain.dismiss();
     if (st != EWT_OK)
       throw Error(st, "the batch held invalid queries (their results are "
                       "UINT64_MAX)");

@@ -205,6 +205,26 @@ class DeviceGuard {
   int prev_ = 0;
 };
 
+// Waits for the streams when a call leaves by an exception: what it queued on
+// them reads and writes the caller's buffers (or host tables of the call),
+// which are the caller's again once it returns.  dismiss() after the call's
+// own wait.
+class DrainOnError {
+ public:
+  explicit DrainOnError(cudaStream_t a, cudaStream_t b = nullptr, cudaStream_t c = nullptr)
+      : s_{a, b, c} {}
+  ~DrainOnError() {
+    for (cudaStream_t s : s_)
+      if (s) cudaStreamSynchronize(s);
+  }
+  DrainOnError(DrainOnError const&) = delete;
+  DrainOnError& operator=(DrainOnError const&) = delete;
+  void dismiss() { s_[0] = s_[1] = s_[2] = nullptr; }
+
+ private:
+  cudaStream_t s_[3];
+};
+
 inline bool is_device_pointer(const void* p) {
   cudaPointerAttributes a;
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {

@@ -642,13 +642,7 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
   std::vector<uint16_t> codes, lut;  // padded codes by minimal symbol, by symbol
   std::vector<uint64_t> tables, c_h;
   std::vector<LevelNode> flat;
-  struct Drain {
-    cudaStream_t s;
-    bool on = true;
-    ~Drain() {
-      if (on) cudaStreamSynchronize(s);
-    }
-  } drain{st};
+  DrainOnError drain(st);
   // ---- text on the device
   DevBuf text_owned;
   T const* d_text;
@@ -1028,7 +1022,7 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
   }
   v.rs = t.rs.view();
   v.groups = t.groups.view();
-  drain.on = false;  // the stream was waited for above
+  drain.dismiss();  // the stream was waited for above
 }
 
 }  // namespace
