@@ -18,8 +18,10 @@
 // own stream; each result is a tree of its own.
 #include <algorithm>
 #include <atomic>
+#include <functional>
 #include <mutex>
 #include <string>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -727,11 +729,10 @@ extern "C" int ewt_build_batch(const void* const* texts, const uint64_t* lengths
     uint32_t const hw = std::max(1u, std::thread::hardware_concurrency());
     uint32_t const workers =
         std::min<uint32_t>({static_cast<uint32_t>(rest.size()), kBuildWorkers, hw});
-    std::vector<std::thread> pool;
-    for (uint32_t w = 0; w < workers; ++w) pool.emplace_back(work);
     // The group builds of the alphabet sizes run side by side, one thread and
     // stream each (mostly launches and short waits), the last on this thread.
     std::vector<uint32_t> retry;  // texts of groups that failed as a group
+    retry.reserve(count);
     auto build_size = [&](uint32_t L) {
       try {
         build_small_texts(texts, lengths, small[L], elem_size, L, gpu_index, out);
@@ -749,10 +750,32 @@ extern "C" int ewt_build_batch(const void* const* texts, const uint64_t* lengths
     std::vector<uint32_t> sizes;
     for (uint32_t L = 0; L < small.size(); ++L)
       if (!small[L].empty()) sizes.push_back(L);
-    for (size_t i = 0; i + 1 < sizes.size(); ++i)
-      pool.emplace_back([&build_size, L = sizes[i]] { build_size(L); });
-    if (!sizes.empty()) build_size(sizes.back());
-    for (auto& th : pool) th.join();
+    // Where the system refuses a thread, its work is left to the others or done
+    // here.  All are joined whatever happens.
+    struct Threads {
+      std::vector<std::thread> pool;
+      bool start(std::function<void()> f) {
+        try {
+          pool.emplace_back(std::move(f));
+        } catch (std::system_error const&) {
+          return false;
+        }
+        return true;
+      }
+      void join() {
+        for (auto& th : pool) th.join();
+        pool.clear();
+      }
+      ~Threads() { join(); }
+    } threads;
+    threads.pool.reserve(workers + small.size());
+    uint32_t started = 0;
+    while (started < workers && threads.start(work)) ++started;
+    for (size_t i = 0; i < sizes.size(); ++i)
+      if (i + 1 == sizes.size() || !threads.start([&build_size, L = sizes[i]] { build_size(L); }))
+        build_size(sizes[i]);
+    if (started == 0) work();
+    threads.join();
     // one by one, so that each failing text reports its own status
     set_texts_synchronized(true);
     for (uint32_t i : retry) build_one(i);
