@@ -1181,16 +1181,22 @@ inline std::vector<uint32_t> plan_plane_passes(uint32_t L) {
 
 constexpr uint32_t kSlotWords = 4;  // words of a slot: a thread's work
 
-// The largest CTA of which three fit an SM's shared memory (128: four).
+// The largest CTA of which three fit an SM's shared memory (128: four, three
+// from 14 planes on).
 inline uint32_t pass_slots(uint32_t np) { return np <= 8 ? 256 : 128; }
 
 template <uint32_t NT, class Index>
 void launch_plane_pass_as(PlanePass const& p, uint64_t max_chunks, cudaStream_t st) {
   auto kern = plane_pass_kernel<NT, kSlotWords, Index>;
   set_smem_limit(kern, static_cast<int>(pass_smem(NT, kSlotWords, NT == 256 ? 8 : 15)));
+  // one wave: chunks are dealt out by CTA number, so a CTA that started when
+  // others had ended would have its share done on a nearly empty GPU
+  size_t const smem = pass_smem(NT, kSlotWords, p.np);
+  int per_sm = 0;
+  EWT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, smem));
   uint32_t const grid = static_cast<uint32_t>(std::max<uint64_t>(
-      1, std::min<uint64_t>(max_chunks, uint64_t(sm_count()) * (NT == 256 ? 3 : 4))));
-  kern<<<grid, NT, pass_smem(NT, kSlotWords, p.np), st>>>(p);
+      1, std::min<uint64_t>(max_chunks, uint64_t(sm_count()) * std::max(per_sm, 1))));
+  kern<<<grid, NT, smem, st>>>(p);
   EWT_LAUNCHED();
 }
 
