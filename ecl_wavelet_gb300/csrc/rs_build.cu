@@ -541,7 +541,8 @@ uint64_t rs_bytes_bound(uint64_t bits, uint32_t arrays, bool with_support) {
   uint64_t const l2 = (ceil_div(bits, kL2Bits) + 1) * 2;
   uint64_t per = words + l1 + l2 + sizeof(ArrayMeta) + 64;
   if (with_support) {
-    uint64_t const samples = (bits / kSampleRate + 2) * 8;
+    uint64_t const samples = 2 * (bits / kSampleRate + 2) * 8;  // zeros and ones, each with
+                                                                // room for all of the bits
     uint64_t const blocks = (ceil_div(bits, 224) + 1) * 32 + 8;
     uint64_t const dense = (bits / 32 + 2) * 4;  // densest rate (32)
     per += samples + blocks + dense;
