@@ -298,8 +298,8 @@ void build_group(void const* const* texts, uint64_t const* lengths,
     for (ArrayMeta const& m : r.meta) {
       share += ceil_div(ceil_div(m.bits, 32), 32) * 128 + m.num_l1 * 8 +
                ((m.num_l1 - 1) * 128 + m.num_last_l2) * 2 +
-               (m.bits / 4096 + 1) * 8 + ceil_div(m.bits, 224) * 32 +
-               sizeof(ArrayMeta);
+               2 * (m.bits / ecl::detail::kSampleRate) * 8 +
+               ceil_div(m.bits, 224) * 32 + 8 + sizeof(ArrayMeta);
       if (rs.ds.get() && rs.sel_shift)
         share += (m.bits >> rs.sel_shift) * 4 + 8;
     }

@@ -37,3 +37,29 @@ def test_rank_select_bound(L, bits, arrays, rate):
     held = L.fake_live() - before - 16
     assert L.ewt_rs_free(out) == 0
     assert held <= needed(L, RANKSELECT, bits, arrays)
+
+
+def test_batch_shares(L):
+    """The trees of a batch build that share a store count all of it between
+    them (their small tables are padded to 256 bytes: seven per tree)."""
+    rng = np.random.default_rng(3)
+    texts = [np.zeros(n, np.uint8) for n in rng.integers(1 << 21, 1 << 22, 6)]
+    al = np.arange(16, dtype=np.uint8)
+    ptr = lambda arrays: (C.c_void_p * len(arrays))(*[a.ctypes.data for a in arrays])
+    lens = np.array([t.size for t in texts], np.uint64)
+    sigmas = np.full(len(texts), 16, np.uint64)
+    out = (C.c_void_p * len(texts))()
+    L.fake_reset()
+    before = L.fake_live()
+    assert L.ewt_build_batch(ptr(texts), lens.ctypes.data, len(texts), 1, ptr([al] * len(texts)),
+                             sigmas.ctypes.data, 0, out, None) == 0
+    held = L.fake_live() - before
+    from ecl_wavelet_gb300 import Info
+    total = 0
+    for t in out:
+        i = Info()
+        assert L.ewt_get_info(t, C.byref(i)) == 0
+        total += i.device_bytes
+    for t in out:
+        assert L.ewt_free(t) == 0
+    assert held - 7 * 256 * len(texts) <= total <= held + held // 100
