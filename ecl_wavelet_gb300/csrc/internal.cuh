@@ -32,6 +32,9 @@ struct RSStore {
   // *filled, whose words are final (zero past every array's end) and are
   // taken over.
   void layout(std::vector<uint64_t> const& bits, uint64_t stride = 0, DevBuf* filled = nullptr);
+  // Moves finished arrays side by side, as a layout without stride has them.
+  // Returns when that is done.
+  void pack(cudaStream_t st);
   RSView view() const;
   uint64_t device_bytes() const {
     return words.bytes() + l1.bytes() + l2.bytes() + s0.bytes() + s1.bytes() + rb.bytes() +

@@ -84,6 +84,28 @@ void RSStore::layout(std::vector<uint64_t> const& bits, uint64_t stride, DevBuf*
     EWT_CUDA(cudaMemsetAsync(words.as<uint32_t>() + total_words - 1, 0, 4, st));
 }
 
+void RSStore::pack(cudaStream_t st) {
+  std::vector<uint64_t> off;
+  uint64_t total = 0;
+  for (ArrayMeta const& m : meta) {
+    off.push_back(total);
+    total += ceil_div(ceil_div(m.bits, 32), 32) * 32;
+  }
+  total += total % 2;
+  DevBuf packed(total * 4 + 64);
+  for (size_t a = 0; a < meta.size(); ++a) {  // the padding's zeros go with the words
+    EWT_CUDA(cudaMemcpyAsync(packed.as<uint32_t>() + off[a], words.as<uint32_t>() + meta[a].word_off,
+                             ceil_div(ceil_div(meta[a].bits, 32), 32) * 128,
+                             cudaMemcpyDeviceToDevice, st));
+    meta[a].word_off = off[a];
+  }
+  total_words = total;
+  words = std::move(packed);
+  EWT_CUDA(cudaMemcpyAsync(meta_d.get(), meta.data(), meta.size() * sizeof(ArrayMeta),
+                           cudaMemcpyHostToDevice, st));
+  EWT_CUDA(cudaStreamSynchronize(st));
+}
+
 RSView RSStore::view() const {
   RSView v{};
   v.words = words.as<uint32_t>();

@@ -725,6 +725,11 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
   DevBuf cur_buf;  // minimal symbols (or codes) of a text the build cannot read as it is
   DevBuf lut_d;
   T const* sym = d_text;
+  // A large copy that was read for the last time makes room for what is built
+  // next (as the planes of large orders do, planes.cuh).
+  auto release = [](DevBuf& b) {
+    if (b.bytes() > kSplitOrderBytes) b.reset();
+  };
   if (!t.is_min || (by_planes && sizeof(T) > 2)) {
     alphabet_h.assign(t.alphabet.begin(), t.alphabet.end());
     t.alphabet_d.alloc(sigma * sizeof(T));
@@ -754,6 +759,7 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
     PhaseTimer pt(EWT_PHASE_HIST, st);
     launch_remap<T, uint16_t>(d_text, n, t.alphabet_d.as<T>(), sigma, lut_d.as<uint16_t>(),
                               cur_buf.as<uint16_t>(), err_build, st);
+    release(text_owned);
   } else if (!by_planes && !t.is_min) {
     cur_buf.alloc(n * sizeof(T));
     PhaseTimer pt(EWT_PHASE_HIST, st);
@@ -774,6 +780,8 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
       x.n = n;
       x.L = L;
       kept = run_passes(t, x, words, starts, want_groups, err_build, st);
+      release(text_owned);
+      release(cur_buf);
     };
     if constexpr (sizeof(T) <= 2) {
       PlaneText<T> x;
@@ -851,15 +859,7 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
     for (uint32_t l = 0; l < covered; ++l) t.rs.skip_blocks[l] = 1;
   }
   if (words_early.get()) {
-    uint64_t kept_bits = 0;
-    for (uint64_t b : t.level_bits) kept_bits += b;
-    // levels that short codes left mostly empty are packed
-    bool const pack = kept_bits * 8 < L * n * 7;
-    t.rs.layout(t.level_bits, pack ? 0 : level_stride(n), pack ? nullptr : &words_early);
-    for (uint32_t l = 0; pack && l < L; ++l)
-      EWT_CUDA(cudaMemcpyAsync(t.rs.words.as<uint32_t>() + t.rs.meta[l].word_off,
-                               words_early.as<uint32_t>() + l * level_stride(n),
-                               ceil_div(t.level_bits[l], 32) * 4, cudaMemcpyDeviceToDevice, st));
+    t.rs.layout(t.level_bits, level_stride(n), &words_early);
   } else {
     t.rs.layout(t.level_bits);
   }
@@ -1009,16 +1009,21 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
   if (want_groups) {
     std::vector<std::vector<uint32_t const*>> planes;
     for (auto const& w : group_planes(L)) {
-      // the whole order's bits also where a level was packed
-      std::vector<uint32_t const*> p{
-          words_early.get() ? words_early.as<uint32_t>() + w.first * level_stride(n)
-                            : words + t.rs.meta[w.first].word_off};
+      std::vector<uint32_t const*> p{words + t.rs.meta[w.first].word_off};
       for (OrderPlanes const& o : kept)
         if (o.level == w.first)
           for (uint32_t j = 1; j <= w.second; ++j) p.push_back(o.plane(w.first + j));
       planes.push_back(std::move(p));
     }
     build_groups(t, t.pow2 ? c : code_starts, planes, st);
+    kept.clear();
+  }
+  if (by_planes && !t.pow2) {
+    // levels that short codes left mostly empty are packed (when the planes are
+    // gone: the build's peak is the group levels')
+    uint64_t bits = 0;
+    for (uint64_t b : t.level_bits) bits += b;
+    if (bits * 8 < L * n * 7) t.rs.pack(st);
   }
   v.rs = t.rs.view();
   v.groups = t.groups.view();

@@ -63,3 +63,48 @@ def test_batch_shares(L):
     for t in out:
         assert L.ewt_free(t) == 0
     assert held - 7 * 256 * len(texts) <= total <= held + held // 100
+
+
+def zeros(nbytes, shift=0):
+    """Reserved, untouched address space, `shift` bytes past a page."""
+    import mmap
+    m = mmap.mmap(-1, nbytes + shift, flags=mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS | 0x4000)
+    return np.frombuffer(m, np.uint8)[shift:]
+
+
+def build_peak(L, dtype, sigma, n, copied, short):
+    """Device bytes at the peak of a build; copied: the text starts off a
+    16-byte boundary, so that the device gets a copy; short: but for 1,000 symbols of
+    the longest code the text holds the first of the short ones."""
+    size = np.dtype(dtype).itemsize
+    text = zeros(n * size, size if copied else 0)
+    al = np.arange(sigma, dtype=np.uint64).astype(dtype)
+    bits = max(1, (sigma - 1).bit_length())
+    L.fake_reset()
+    for entries in {(1 << bits) + 1, sigma + 1}:
+        if short:
+            L.fake_patch(entries * 8, 1, 1000)
+        L.fake_patch(entries * 8, (1 << bits) // 2 + 1 if short else entries - 1, n)
+    out = C.c_void_p()
+    before = L.fake_live()
+    assert L.ewt_build(text.ctypes.data, n, size, al.ctypes.data, sigma, 0, C.byref(out)) == 0, \
+        L.ewt_last_error()
+    peak = L.fake_peak() - before
+    assert L.ewt_free(out) == 0
+    return peak
+
+
+GPU_BYTES = 284_208 << 20
+
+
+@pytest.mark.parametrize("dtype,sigma,n,copied,short", [
+    (np.uint8, 96, 73_000_000_000, 1, 0), (np.uint8, 96, 73_000_000_000, 1, 1),
+    (np.uint8, 129, 72_000_000_000, 1, 0), (np.uint8, 129, 72_000_000_000, 0, 1),
+    (np.uint8, 256, 57_000_000_000, 1, 0), (np.uint16, 1000, 40_000_000_000, 1, 0),
+    (np.uint16, 33_024, 36_000_000_000, 1, 0), (np.uint16, 33_024, 36_000_000_000, 0, 1),
+    (np.uint16, 65_536, 35_000_000_000, 0, 0), (np.uint32, 10_000, 21_000_000_000, 1, 1),
+    (np.uint32, 65_536, 21_000_000_000, 0, 0), (np.uint64, 40_000, 11_000_000_000, 0, 0)])
+def test_largest_builds_fit(L, dtype, sigma, n, copied, short):
+    """Texts from the host that fill one GPU: text copies, planes and levels
+    that are no longer needed make room for what is built next."""
+    assert build_peak(L, dtype, sigma, n, copied, short) <= GPU_BYTES
