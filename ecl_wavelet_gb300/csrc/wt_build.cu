@@ -160,11 +160,15 @@ __global__ void presence_kernel(T const* __restrict__ text, uint64_t n,
 // recorded in a flag instead.  Each CTA remembers the symbols it has looked up
 // in a direct-mapped table in shared memory, so a symbol that repeats goes no
 // further (20 M symbols of 10,000: 300 us without).  Others are looked up with
-// a plain load first and inserted with atomicCAS only when missing.  A probe
-// that runs around the whole table reports overflow and the host retries with
-// a larger table.
+// a plain load first and inserted with atomicCAS only when missing.  A table
+// that is more than half full is too small: the host retries with a larger one,
+// and every thread ends early, asking for that where it inserts and every
+// kAskProbes probes (chains of a table that is large enough are shorter;
+// without, each of the text's symbols ran around the full table: 20 M symbols
+// of a million took 21 s).
 constexpr uint64_t kEmptySlot = ~uint64_t(0);
 constexpr uint32_t kSeenSlots = 8192;
+constexpr uint64_t kAskProbes = 16;
 
 __device__ __forceinline__ uint64_t slot_hash(uint64_t x) {
   x ^= x >> 33;
@@ -178,7 +182,7 @@ __global__ void __launch_bounds__(1024)
 distinct_kernel(T const* __restrict__ text, uint64_t n,
                 unsigned long long* __restrict__ table, uint64_t cap_mask,
                 unsigned long long* __restrict__ count,
-                uint32_t* __restrict__ flags) {  // [0] overflow, [1] max symbol seen
+                uint32_t* flags) {  // [0] overflow, [1] max symbol seen
   extern __shared__ __align__(8) uint64_t seen[];
   for (uint32_t i = threadIdx.x; i < kSeenSlots; i += blockDim.x) seen[i] = kEmptySlot;
   __syncthreads();
@@ -195,10 +199,10 @@ distinct_kernel(T const* __restrict__ text, uint64_t n,
     uint64_t volatile* const mine = seen + (hash & (kSeenSlots - 1));
     if (*mine == key) continue;
     uint64_t h = hash & cap_mask;
-    for (uint64_t probe = 0;; ++probe) {
-      if (probe > cap_mask) {
-        flags[0] = 1;
-        break;
+    for (uint64_t probe = 1;; ++probe) {
+      if (probe % kAskProbes == 0) {
+        if (probe > cap_mask) flags[0] = 1;
+        if (*static_cast<uint32_t volatile*>(flags)) return;
       }
       uint64_t const cur = *const_cast<unsigned long long volatile*>(table + h);
       if (cur == key) break;
@@ -207,7 +211,8 @@ distinct_kernel(T const* __restrict__ text, uint64_t n,
             atomicCAS(&table[h], static_cast<unsigned long long>(kEmptySlot),
                       static_cast<unsigned long long>(key));
         if (prev == kEmptySlot) {
-          atomicAdd(count, 1ull);
+          if ((atomicAdd(count, 1ull) + 1) * 2 > cap_mask + 1) flags[0] = 1;
+          if (*static_cast<uint32_t volatile*>(flags)) return;
           break;
         }
         if (prev == key) break;
