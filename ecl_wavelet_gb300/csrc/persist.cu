@@ -58,9 +58,7 @@ struct File {
   }
 };
 
-void dev_to_file(File& f, void const* d, uint64_t bytes, PinnedBuf& stage,
-                 cudaStream_t s) {
-  f.put(bytes);
+void piece_to_file(File& f, void const* d, uint64_t bytes, PinnedBuf& stage, cudaStream_t s) {
   for (uint64_t o = 0; o < bytes; o += kPiece) {
     size_t const k = static_cast<size_t>(std::min<uint64_t>(kPiece, bytes - o));
     EWT_CUDA(cudaMemcpyAsync(stage.get(), static_cast<char const*>(d) + o, k,
@@ -68,6 +66,29 @@ void dev_to_file(File& f, void const* d, uint64_t bytes, PinnedBuf& stage,
     EWT_CUDA(cudaStreamSynchronize(s));
     f.write(stage.get(), k);
   }
+}
+
+// A device array.  Its bytes from `used` on were never written: zeros go out in
+// their place, so that a file holds nothing of what was in that memory before.
+void dev_to_file(File& f, DevBuf const& d, uint64_t used, PinnedBuf& stage, cudaStream_t s) {
+  uint64_t const bytes = d.bytes();
+  used = std::min(used, bytes);
+  f.put(bytes);
+  piece_to_file(f, d.get(), used, stage, s);
+  std::vector<char> const zeros(std::min<uint64_t>(kPiece, bytes - used), 0);
+  for (uint64_t o = used; o < bytes; o += zeros.size())
+    f.write(zeros.data(), std::min<uint64_t>(zeros.size(), bytes - o));
+}
+void dev_to_file(File& f, DevBuf const& d, PinnedBuf& stage, cudaStream_t s) {
+  dev_to_file(f, d, d.bytes(), stage, s);
+}
+
+// Whether any array has rank blocks (and with them dense samples); without, a
+// store holds a stub of each.
+bool has_blocks(RSStore const& rs) {
+  for (ArrayMeta const& m : rs.meta)
+    if (m.rb_off != ecl::detail::kNoBlocks) return true;
+  return false;
 }
 
 void file_to_dev(File& f, DevBuf& d, PinnedBuf& stage, cudaStream_t s,
@@ -116,30 +137,46 @@ extern "C" int ewt_save(const ewt_tree* t, const char* path) {
     f.put_vec(t->nodes_at_level);
     f.put_vec(t->node_base);
     f.put_vec(t->level_bits);
-    f.put_vec(t->rs.meta);
-    for (uint64_t v : {t->rs.total_words, t->rs.total_l1, t->rs.total_l2,
-                       t->rs.total_s0, t->rs.total_s1,
+    // the select samples go out side by side: on the device each list has room
+    // for an array of zeros or ones alone
+    std::vector<ArrayMeta> meta = t->rs.meta;
+    uint64_t s0 = 0, s1 = 0;
+    for (ArrayMeta& m : meta) {
+      m.s0_off = s0;
+      m.s1_off = s1;
+      s0 += (m.bits - m.ones) / ecl::detail::kSampleRate;
+      s1 += m.ones / ecl::detail::kSampleRate;
+    }
+    f.put_vec(meta);
+    for (uint64_t v : {t->rs.total_words, t->rs.total_l1, t->rs.total_l2, s0, s1,
                        uint64_t(t->rs.ds.get() ? t->rs.sel_shift : 0)})
       f.put(v);
     PinnedBuf stage;
     stage.ensure(kPiece);
-    dev_to_file(f, t->rs.words.get(), t->rs.words.bytes(), stage, s);
-    dev_to_file(f, t->rs.l1.get(), t->rs.l1.bytes(), stage, s);
-    dev_to_file(f, t->rs.l2.get(), t->rs.l2.bytes(), stage, s);
-    dev_to_file(f, t->rs.s0.get(), t->rs.s0.bytes(), stage, s);
-    dev_to_file(f, t->rs.s1.get(), t->rs.s1.bytes(), stage, s);
-    dev_to_file(f, t->rs.rb.get(), t->rs.rb.bytes(), stage, s);
-    dev_to_file(f, t->rs.ds.get(), t->rs.ds.bytes(), stage, s);
-    dev_to_file(f, t->counts_d.get(), t->counts_d.bytes(), stage, s);
-    dev_to_file(f, t->ranks_d.get(), t->ranks_d.bytes(), stage, s);
+    RSStore const& rs = t->rs;
+    dev_to_file(f, rs.words, rs.total_words * 4, stage, s);
+    dev_to_file(f, rs.l1, stage, s);
+    dev_to_file(f, rs.l2, stage, s);
+    f.put(s0 * 8);
+    for (ArrayMeta const& m : rs.meta)
+      piece_to_file(f, rs.s0.as<uint64_t>() + m.s0_off,
+                    (m.bits - m.ones) / ecl::detail::kSampleRate * 8, stage, s);
+    f.put(s1 * 8);
+    for (ArrayMeta const& m : rs.meta)
+      piece_to_file(f, rs.s1.as<uint64_t>() + m.s1_off, m.ones / ecl::detail::kSampleRate * 8,
+                    stage, s);
+    dev_to_file(f, rs.rb, has_blocks(rs) ? rs.rb.bytes() : 0, stage, s);
+    dev_to_file(f, rs.ds, has_blocks(rs) && rs.sel_shift ? rs.ds.bytes() : 0, stage, s);
+    dev_to_file(f, t->counts_d, stage, s);
+    dev_to_file(f, t->ranks_d, t->nodes.size() * 8, stage, s);
     // group query levels
     f.put_vec(t->groups.levels);
     f.put(t->groups.ds.get() ? t->groups.sel_shift : 0);
     if (!t->groups.levels.empty()) {
-      dev_to_file(f, t->groups.blocks.get(), t->groups.blocks.bytes(), stage, s);
-      dev_to_file(f, t->groups.sb.get(), t->groups.sb.bytes(), stage, s);
-      dev_to_file(f, t->groups.ds.get(), t->groups.ds.bytes(), stage, s);
-      dev_to_file(f, t->groups.node_ranks.get(), t->groups.node_ranks.bytes(), stage, s);
+      dev_to_file(f, t->groups.blocks, stage, s);
+      dev_to_file(f, t->groups.sb, stage, s);
+      dev_to_file(f, t->groups.ds, stage, s);
+      dev_to_file(f, t->groups.node_ranks, stage, s);
     }
   });
 }
