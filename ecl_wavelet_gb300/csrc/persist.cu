@@ -2,7 +2,8 @@
 // rebuilding (ewt_save / ewt_load).  The reference has no serialisation; a
 // serving process uses this to admit prebuilt indexes.
 //
-// Layout (little-endian): the magic "EWTIDX03", a header of 64-bit fields,
+// Layout (little-endian): the magic "EWTIDX03" ("EWTIDX04" for the group levels
+// of an alphabet of no power of two, below), a header of 64-bit fields,
 // the host-side shape (alphabet, count table, codes, node starts, nodes per
 // level, node bases, level sizes, per-array metadata), then the device arrays
 // in a fixed order (level words, L1, L2, samples of zeros and ones, rank
@@ -19,7 +20,12 @@
 namespace ewt {
 namespace {
 
+// Group levels over padded codes (alphabets of no power of two) are walked with
+// counts by code; a reader that knows only group levels over symbols would take
+// such a file and answer wrongly, so it has a tag of its own.  Some files with
+// such levels carry the older tag; they are read all the same.
 constexpr char kMagic[8] = {'E', 'W', 'T', 'I', 'D', 'X', '0', '3'};
+constexpr char kMagicPadded[8] = {'E', 'W', 'T', 'I', 'D', 'X', '0', '4'};
 constexpr size_t kPiece = size_t(64) << 20;
 
 struct File {
@@ -124,7 +130,7 @@ extern "C" int ewt_save(const ewt_tree* t, const char* path) {
     DeviceGuard g(t->device);
     cudaStream_t const s = t->stream;
     File f(path, "wb");
-    f.write(kMagic, 8);
+    f.write(!t->pow2 && !t->groups.levels.empty() ? kMagicPadded : kMagic, 8);
     for (uint64_t v : {uint64_t(t->elem_size), t->n, t->sigma, uint64_t(t->L),
                        uint64_t(t->is_min), uint64_t(t->pow2), t->codes_start,
                        t->nodes_until_last})
@@ -188,8 +194,8 @@ extern "C" int ewt_load(const char* path, int gpu_index, ewt_tree** out) {
     File f(path, "rb");
     char magic[8];
     f.read(magic, 8);
-    EWT_REQUIRE(std::memcmp(magic, kMagic, 8) == 0, EWT_ERR_INVALID_ARGUMENT,
-                "not an index file (bad magic)");
+    EWT_REQUIRE(std::memcmp(magic, kMagic, 8) == 0 || std::memcmp(magic, kMagicPadded, 8) == 0,
+                EWT_ERR_INVALID_ARGUMENT, "not an index file (bad magic)");
     DeviceGuard g(gpu_index);
     auto t = std::make_unique<ewt_tree>();
     t->device = gpu_index;

@@ -53,3 +53,26 @@ def test_saved_again(ewt, tmp_path):
     for l in range(2):
         for part in ("SAMPLES0", "SAMPLES1"):
             assert np.array_equal(batch[1].export(part, l), v.export(part, l))
+
+
+@pytest.mark.parametrize("dtype,sigma,tag", [(np.uint8, 2, b"EWTIDX03"), (np.uint8, 256, b"EWTIDX03"),
+                                             (np.uint8, 5, b"EWTIDX04"), (np.uint16, 1000, b"EWTIDX04"),
+                                             (np.uint32, 70_000, b"EWTIDX03")])
+def test_tags(ewt, tmp_path, dtype, sigma, tag):
+    """Group levels over padded codes have a tag of their own, which readers of
+    the older form refuse; the older tag before such levels is still read."""
+    rng = np.random.default_rng(sigma)
+    text = rng.integers(0, sigma, 150_001).astype(dtype)
+    text[:sigma] = np.arange(sigma)
+    t = ewt.WaveletTree(text, np.arange(sigma))
+    t.save(str(tmp_path / "i"))
+    raw = (tmp_path / "i").read_bytes()
+    assert raw[:8] == tag
+    idx = rng.integers(0, text.size, 1000).astype(np.uint64)
+    for magic in (tag, b"EWTIDX03"):
+        (tmp_path / "j").write_bytes(magic + raw[8:])
+        u = ewt.WaveletTree.load(str(tmp_path / "j"))
+        assert np.array_equal(u.access(idx), text[idx])
+    (tmp_path / "j").write_bytes(b"EWTIDX05" + raw[8:])
+    with pytest.raises(ewt.EwtError):
+        ewt.WaveletTree.load(str(tmp_path / "j"))
