@@ -1,6 +1,7 @@
 // Split kernels of the wavelet-tree level pipeline: the stable partition
 // of every node of level l by the level's bit, which produces the level
-// l+1 order and that level's bits.  Included by wt_build.cu after the node
+// l+1 order and that level's bits, for alphabets of more than 2^16 symbols (4-
+// and 8-byte texts).  Included by wt_build.cu after the node
 // helpers (node_of, level_bit) and views these kernels use.
 #pragma once
 
@@ -177,36 +178,19 @@ split_kernel(T const* __restrict__ src, T* __restrict__ dst, uint64_t n,
 }
 
 // Copies `len` staged symbols (shared memory, 32-byte aligned) to
-// dst[pos, pos + len).  Bytes move as 4-byte words: a few head and tail
-// bytes singly, the body with funnel shifts from two staged words.
+// dst[pos, pos + len).
 template <class T>
 __device__ __forceinline__ void copy_run(T* __restrict__ dst, uint64_t n,
                                          uint64_t pos, uint32_t len,
                                          T const* src) {
   if (len == 0 || pos + len > n) return;  // corrupt position: never write past
   uint32_t const tid = threadIdx.x;
-  if constexpr (sizeof(T) == 1) {
-    uint32_t const head = min(len, static_cast<uint32_t>((4 - (pos & 3)) & 3));
-    if (tid < head) dst[pos + tid] = src[tid];
-    uint32_t const body = (len - head) >> 2;
-    uint32_t const* s32 = reinterpret_cast<uint32_t const*>(src);
-    uint32_t* d32 = reinterpret_cast<uint32_t*>(dst + pos + head);
-    uint32_t const shift = head * 8;
-    for (uint32_t i = tid; i < body; i += kSplitThreads) {
-      uint32_t const lo = s32[i], hi = s32[i + 1];
-      d32[i] = head ? __funnelshift_r(lo, hi, shift) : lo;
-    }
-    uint32_t const tail = (len - head) & 3;
-    uint32_t const t0 = head + 4 * body;
-    if (tid < tail) dst[pos + t0 + tid] = src[t0 + tid];
-  } else {
-    for (uint32_t i = tid; i < len; i += kSplitThreads) dst[pos + i] = src[i];
-  }
+  for (uint32_t i = tid; i < len; i += kSplitThreads) dst[pos + i] = src[i];
 }
 
 template <class T>
 __host__ __device__ constexpr uint32_t split_stages() {
-  return sizeof(T) <= 2 ? 4 : (sizeof(T) == 4 ? 3 : 2);
+  return sizeof(T) == 4 ? 3 : 2;
 }
 
 // Bytes of the output staging area: the zero run at offset 0, the one run
@@ -221,25 +205,8 @@ __host__ __device__ constexpr uint32_t split_stage_bytes() {
 template <class T>
 __device__ __forceinline__ uint32_t pack_bits32(T const* run, uint32_t b) {
   uint32_t w = 0;
-  if constexpr (sizeof(T) == 1) {
-    uint4 const* q = reinterpret_cast<uint4 const*>(run);
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      uint4 const v = q[h];
-      uint32_t const x[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        // bit b of each byte -> bits 0, 8, 16, 24; the multiply gathers
-        // them into bits 21..24 without carries.
-        uint32_t const t = (x[i] >> b) & 0x01010101u;
-        w |= (((t * 0x00204081u) >> 21) & 0xFu) << (16 * h + 4 * i);
-      }
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < 32; ++i)
-      w |= uint32_t((uint64_t(run[i]) >> b) & 1u) << i;
-  }
+  for (int i = 0; i < 32; ++i) w |= uint32_t((uint64_t(run[i]) >> b) & 1u) << i;
   return w;
 }
 
@@ -252,7 +219,7 @@ __device__ __forceinline__ uint32_t pack_bits32(T const* run, uint32_t b) {
 // (C[start], C[split], rank0 at start) is cached while consecutive tiles
 // stay in one node.  Per tile:
 //   1. each thread takes 16 consecutive symbols (blocked), checks that they
-//      share the node prefix, and packs their level bits (SWAR for bytes);
+//      share the node prefix, and packs their level bits;
 //   2. one CTA scan of the per-thread zero counts;
 //   3. symbols are staged in output order: the tile's zeros, then (from the
 //      next 32-symbol boundary) its ones;
@@ -345,22 +312,10 @@ split_fast_kernel(T const* __restrict__ src, T* __restrict__ dst, uint64_t n,
     }
     uint32_t bits = 0;
     bool same = true;
-    if constexpr (sizeof(T) == 1) {
-      uint32_t const* w = reinterpret_cast<uint32_t const*>(e);
-      uint32_t const pre_mask = 0x01010101u * (0xFFu >> (sh + 1));
-      uint32_t const pre_key = 0x01010101u * static_cast<uint32_t>(key);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        same &= ((w[i] >> (sh + 1)) & pre_mask) == pre_key;
-        uint32_t const tb = (w[i] >> sh) & 0x01010101u;
-        bits |= (((tb * 0x00204081u) >> 21) & 0xFu) << (4 * i);
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < int(kSplitItems); ++i) {
-        same &= (uint64_t(e[i]) >> (sh + 1)) == key;
-        bits |= uint32_t((uint64_t(e[i]) >> sh) & 1u) << i;
-      }
+    for (int i = 0; i < int(kSplitItems); ++i) {
+      same &= (uint64_t(e[i]) >> (sh + 1)) == key;
+      bits |= uint32_t((uint64_t(e[i]) >> sh) & 1u) << i;
     }
     uint32_t const z = kSplitItems - __popc(bits);
     // 2. CTA exclusive scan of the zero counts

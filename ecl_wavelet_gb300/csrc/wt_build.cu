@@ -442,78 +442,37 @@ __device__ __forceinline__ bool level_bit(uint64_t c, uint32_t l, uint32_t L,
   return c >= node_of<false>(c, l, L, sigma).split;
 }
 
-// Level 0 bits: each thread writes fill_words<T>() output words (words
-// blockIdx.x * 256 * fill_words + threadIdx.x + 256 * j), with all their
-// symbol loads (128 bytes) issued before any is used.  Check = validate
-// symbols of a minimal alphabet (c < sigma).
-template <class T>
-__host__ __device__ constexpr uint32_t fill_words() {
-  return sizeof(T) == 1 ? 4u : (sizeof(T) == 2 ? 2u : 1u);
-}
-
+// Level 0 bits of an alphabet of more than 2^16 symbols: a thread per output
+// word.  Check = validate symbols of a minimal alphabet (c < sigma).
 template <class T, bool Pow2, bool Check>
 __global__ void __launch_bounds__(256)
 fill0_kernel(T const* __restrict__ src, uint64_t size0, uint32_t L,
              uint64_t sigma, uint32_t* __restrict__ out,
              uint32_t* __restrict__ err) {
-  constexpr uint32_t kFillWords = fill_words<T>();
-  constexpr int kVec = 32 * sizeof(T) / 16;
-  uint64_t const base = uint64_t(blockIdx.x) * 256 * kFillWords + threadIdx.x;
-  uint4 buf[kFillWords][kVec];
-#pragma unroll
-  for (uint32_t j = 0; j < kFillWords; ++j) {
-    uint64_t const p0 = (base + 256 * j) * 32;
-    if (p0 + 32 <= size0) {
-      uint4 const* s = reinterpret_cast<uint4 const*>(src + p0);
-#pragma unroll
-      for (int q = 0; q < kVec; ++q) buf[j][q] = __ldg(s + q);
-    }
-  }
+  uint64_t const w = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x, p0 = w * 32;
+  if (p0 >= size0) return;
   bool bad = false;
+  uint32_t word = 0;
+  if (p0 + 32 <= size0) {  // all loads before their first use
+    constexpr int kVec = 32 * sizeof(T) / 16;
+    uint4 buf[kVec];
 #pragma unroll
-  for (uint32_t j = 0; j < kFillWords; ++j) {
-    uint64_t const w = base + 256 * j;
-    uint64_t const p0 = w * 32;
-    if (p0 >= size0) break;
-    uint32_t word = 0;
-    if (p0 + 32 <= size0) {
-      if constexpr (Pow2 && sizeof(T) <= 2) {
-        // SWAR: bit L-1 of four bytes (two 16-bit symbols) per operation;
-        // a symbol is >= sigma = 2^L iff it has a bit at or above L.
-        uint32_t const* w32 = reinterpret_cast<uint32_t const*>(buf[j]);
-        uint32_t const b = L - 1;
-        uint32_t const hi = sizeof(T) == 1
-                                ? 0x01010101u * ((0xFFu << L) & 0xFFu)
-                                : 0x00010001u * ((0xFFFFu << L) & 0xFFFFu);
+    for (int q = 0; q < kVec; ++q) buf[q] = __ldg(reinterpret_cast<uint4 const*>(src + p0) + q);
+    T const* e = reinterpret_cast<T const*>(buf);
 #pragma unroll
-        for (int i = 0; i < 8 * int(sizeof(T)); ++i) {
-          if (Check) bad |= (w32[i] & hi) != 0;
-          if constexpr (sizeof(T) == 1) {
-            uint32_t const t = (w32[i] >> b) & 0x01010101u;
-            word |= (((t * 0x00204081u) >> 21) & 0xFu) << (4 * i);
-          } else {
-            uint32_t const t = (w32[i] >> b) & 0x00010001u;
-            word |= ((t | (t >> 15)) & 3u) << (2 * i);
-          }
-        }
-      } else {
-        T const* e = reinterpret_cast<T const*>(buf[j]);
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          uint64_t const c = e[i];
-          if (Check) bad |= c >= sigma;
-          word |= uint32_t(level_bit<Pow2>(c, 0, L, sigma)) << i;
-        }
-      }
-    } else {
-      for (uint32_t i = 0; p0 + i < size0; ++i) {
-        uint64_t const c = src[p0 + i];
-        if (Check) bad |= c >= sigma;
-        word |= uint32_t(level_bit<Pow2>(c, 0, L, sigma)) << i;
-      }
+    for (int i = 0; i < 32; ++i) {
+      uint64_t const c = e[i];
+      if (Check) bad |= c >= sigma;
+      word |= uint32_t(level_bit<Pow2>(c, 0, L, sigma)) << i;
     }
-    out[w] = word;
+  } else {
+    for (uint32_t i = 0; p0 + i < size0; ++i) {
+      uint64_t const c = src[p0 + i];
+      if (Check) bad |= c >= sigma;
+      word |= uint32_t(level_bit<Pow2>(c, 0, L, sigma)) << i;
+    }
   }
+  out[w] = word;
   if (Check && bad) atomicOr(err, 1u);
 }
 
@@ -724,7 +683,7 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
   uint32_t const grid_stream =
       static_cast<uint32_t>(std::min<uint64_t>(ceil_div(n, 256),
                                                uint64_t(sm_count()) * 8));
-  bool const by_planes = L <= kMaxPlanes;
+  bool const by_planes = sizeof(T) <= 2 || L <= kMaxPlanes;
   auto const level_nodes = by_planes ? std::vector<std::vector<LevelNode>>{}
                                      : make_level_nodes(sigma, L);
   DevBuf cur_buf;  // minimal symbols (or codes) of a text the build cannot read as it is
@@ -759,18 +718,20 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
                                cudaMemcpyHostToDevice, st));
     }
   }
-  if (by_planes && sizeof(T) > 2) {
-    cur_buf.alloc(n * 2);
-    PhaseTimer pt(EWT_PHASE_HIST, st);
-    launch_remap<T, uint16_t>(d_text, n, t.alphabet_d.as<T>(), sigma, lut_d.as<uint16_t>(),
-                              cur_buf.as<uint16_t>(), err_build, st);
-    release(text_owned);
-  } else if (!by_planes && !t.is_min) {
-    cur_buf.alloc(n * sizeof(T));
-    PhaseTimer pt(EWT_PHASE_HIST, st);
-    launch_remap<T, T>(d_text, n, t.alphabet_d.as<T>(), sigma, nullptr, cur_buf.as<T>(),
-                       err_build, st);
-    sym = cur_buf.as<T>();
+  if constexpr (sizeof(T) > 2) {
+    if (by_planes) {
+      cur_buf.alloc(n * 2);
+      PhaseTimer pt(EWT_PHASE_HIST, st);
+      launch_remap<T, uint16_t>(d_text, n, t.alphabet_d.as<T>(), sigma, lut_d.as<uint16_t>(),
+                                cur_buf.as<uint16_t>(), err_build, st);
+      release(text_owned);
+    } else if (!t.is_min) {
+      cur_buf.alloc(n * sizeof(T));
+      PhaseTimer pt(EWT_PHASE_HIST, st);
+      launch_remap<T, T>(d_text, n, t.alphabet_d.as<T>(), sigma, nullptr, cur_buf.as<T>(),
+                         err_build, st);
+      sym = cur_buf.as<T>();
+    }
   }
   // Group query levels -- except for the short texts of a batch build: the
   // group build's launch latency would be most of their build time; they get
@@ -823,7 +784,7 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
                                cudaMemcpyDeviceToHost, st));
       EWT_CUDA(cudaStreamSynchronize(st));
       for (uint64_t i = 0; i < sigma; ++i) t.occ[i] = h[codes[i] + 1] - h[codes[i]];
-    } else {
+    } else if constexpr (sizeof(T) > 2) {
       DevBuf occ_d(sigma * 8);
       EWT_CUDA(cudaMemsetAsync(occ_d.get(), 0, sigma * 8, st));
       {
@@ -919,12 +880,12 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
           v, nodes_d.as<NodeInfoH>(), t.nodes.size(), t.ranks_d.as<uint64_t>());
       EWT_LAUNCHED();
     }
-  } else {
+  } else if constexpr (sizeof(T) > 2) {
     {  // level 0 bits
       PhaseTimer pt(EWT_PHASE_FILL, st);
       uint64_t const w0 = ceil_div(t.level_bits[0], 32);
       uint32_t const blocks =
-          static_cast<uint32_t>(ceil_div(w0, uint64_t(256) * fill_words<T>()));
+          static_cast<uint32_t>(ceil_div(w0, 256));
       auto k = t.pow2 ? (t.is_min ? fill0_kernel<T, true, true>
                                   : fill0_kernel<T, true, false>)
                       : (t.is_min ? fill0_kernel<T, false, true>
