@@ -1162,6 +1162,14 @@ struct OrderPlanes {
 // costs more than it saves where memory is not short (6 Gi: 2.7 ms).
 constexpr uint64_t kSplitOrderBytes = uint64_t(32) << 30;
 
+// Where the forms for large texts begin (tests take them at small sizes): orders
+// of more than split_bytes in two allocations, levels of wide_words 32-bit words
+// with 64-bit word indices (2^36 symbols).
+struct PlaneLimits {
+  uint64_t split_bytes = kSplitOrderBytes;
+  uint64_t wide_words = INT32_MAX;
+};
+
 // Levels per pass: as few passes of at most 4 levels as cover the L - 1 below
 // level 0; the first of 3 where that takes no pass more (a group level's
 // planes start at level 3, and the first pass carries the most planes), the
@@ -1201,9 +1209,8 @@ void launch_plane_pass_as(PlanePass const& p, uint64_t max_chunks, cudaStream_t 
 }
 
 inline void launch_plane_pass(PlanePass const& p, uint32_t slots, uint64_t max_chunks,
-                              cudaStream_t st) {
-  // 32-bit word indices while a level's words allow it (2^36 symbols)
-  bool const narrow = p.ext_words < uint64_t(INT32_MAX);
+                              uint64_t wide_words, cudaStream_t st) {
+  bool const narrow = p.ext_words < wide_words;
   if (slots == 256 && narrow) launch_plane_pass_as<256, int32_t>(p, max_chunks, st);
   else if (slots == 256) launch_plane_pass_as<256, int64_t>(p, max_chunks, st);
   else if (narrow) launch_plane_pass_as<128, int32_t>(p, max_chunks, st);
@@ -1231,7 +1238,7 @@ template <class T>
 std::vector<OrderPlanes> run_plane_passes(
     PlaneText<T> const& x, uint32_t* const* words, uint64_t const* word_count,
     uint64_t* starts_out, std::vector<std::pair<uint32_t, uint32_t>> const& wanted,
-    uint32_t* err, cudaStream_t st) {
+    uint32_t* err, cudaStream_t st, PlaneLimits const& limits = {}) {
   uint64_t const n = x.n;
   uint32_t const L = x.L;
   EWT_REQUIRE(L >= 1 && L <= kMaxPlanes, EWT_ERR_UNSUPPORTED, "too many levels for plane passes");
@@ -1250,7 +1257,7 @@ std::vector<OrderPlanes> run_plane_passes(
     o.first = level + 1;
     o.count = count;
     o.kept = std::min(wants(level), count);
-    o.front = count * stride * 4 > kSplitOrderBytes ? o.kept : count;
+    o.front = count * stride * 4 > limits.split_bytes ? o.kept : count;
     o.stride = stride;
     if (o.front) o.mem.alloc(o.front * stride * 4);
     if (count > o.front) o.rest.alloc((count - o.front) * stride * 4);
@@ -1423,7 +1430,7 @@ std::vector<OrderPlanes> run_plane_passes(
                              128, 0, st>>>(p);
         EWT_LAUNCHED();
       }
-      launch_plane_pass(p, slots, max_chunks, st);
+      launch_plane_pass(p, slots, max_chunks, limits.wide_words, st);
     }
     if (cur.kept) {  // the rest makes room for what is built next
       cur.rest.reset();
