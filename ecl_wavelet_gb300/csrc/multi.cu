@@ -54,6 +54,10 @@ constexpr uint32_t kMultiPerSm = 4;    // resident CTAs
 constexpr uint32_t kPlanThreads = 1024;
 constexpr uint32_t kMaxMultiTrees = 1u << 16;  // trees in one call
 constexpr uint32_t kBuildWorkers = 16;          // host threads of a batch build
+// Symbols of a batch's short texts up to which its group builds run side by
+// side: a group takes about two bytes per symbol more while it is built, which a
+// larger collection may need, and its kernels fill the GPU by themselves.
+constexpr uint64_t kSideBySideSymbols = uint64_t(1) << 30;
 
 __global__ void __launch_bounds__(256)
 tree_hist_kernel(uint32_t const* __restrict__ tree_of, uint64_t m,
@@ -730,7 +734,8 @@ extern "C" int ewt_build_batch(const void* const* texts, const uint64_t* lengths
     uint32_t const workers =
         std::min<uint32_t>({static_cast<uint32_t>(rest.size()), kBuildWorkers, hw});
     // The group builds of the alphabet sizes run side by side, one thread and
-    // stream each (mostly launches and short waits), the last on this thread.
+    // stream each (mostly launches and short waits), the last on this thread;
+    // those of large collections one after the other.
     std::vector<uint32_t> retry;  // texts of groups that failed as a group
     retry.reserve(count);
     auto build_size = [&](uint32_t L) {
@@ -771,8 +776,12 @@ extern "C" int ewt_build_batch(const void* const* texts, const uint64_t* lengths
     threads.pool.reserve(workers + small.size());
     uint32_t started = 0;
     while (started < workers && threads.start(work)) ++started;
+    uint64_t symbols = 0;
+    for (uint32_t L : sizes)
+      for (uint32_t i : small[L]) symbols += lengths[i];
     for (size_t i = 0; i < sizes.size(); ++i)
-      if (i + 1 == sizes.size() || !threads.start([&build_size, L = sizes[i]] { build_size(L); }))
+      if (i + 1 == sizes.size() || symbols > kSideBySideSymbols ||
+          !threads.start([&build_size, L = sizes[i]] { build_size(L); }))
         build_size(sizes[i]);
     if (started == 0) work();
     threads.join();

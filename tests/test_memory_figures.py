@@ -108,3 +108,29 @@ def test_largest_builds_fit(L, dtype, sigma, n, copied, short):
     """Texts from the host that fill one GPU: text copies, planes and levels
     that are no longer needed make room for what is built next."""
     assert build_peak(L, dtype, sigma, n, copied, short) <= GPU_BYTES
+
+
+def test_large_batches_build_one_size_at_a_time(L):
+    """The group builds of a collection of more than 2^30 symbols hold the
+    temporary memory of one alphabet size at a time."""
+    texts = {s: [zeros((1 << 24) - 1 - i) for i in range(17)] for s in (4, 16, 64, 256)}
+    before = L.fake_live()
+
+    def build(group):
+        ptr = lambda arrays: (C.c_void_p * len(arrays))(*[a.ctypes.data for a in arrays])
+        al = [np.arange(s, dtype=np.uint8) for s, _ in group]
+        lens = np.array([t.size for _, t in group], np.uint64)
+        sigmas = np.array([s for s, _ in group], np.uint64)
+        out = (C.c_void_p * len(group))()
+        L.fake_reset()
+        assert L.ewt_build_batch(ptr([t for _, t in group]), lens.ctypes.data, len(group), 1,
+                                 ptr(al), sigmas.ctypes.data, 0, out, None) == 0
+        peak, held = L.fake_peak() - before, L.fake_live() - before
+        for t in out:
+            assert L.ewt_free(t) == 0
+        return peak, held
+
+    alone = [build([(s, t) for t in ts]) for s, ts in texts.items()]
+    peak, held = build([(s, t) for s, ts in texts.items() for t in ts])
+    # (the batch grows its pool once, which the stand-in does not keep)
+    assert peak <= held + max(p - h for p, h in alone)
