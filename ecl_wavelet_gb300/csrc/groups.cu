@@ -536,8 +536,6 @@ GroupView GroupStore::view() const {
   for (auto const& ql : levels) covered += ql.width;
   v.covered = covered;
   v.counts = counts.as<uint64_t>();
-  v.code = code.as<uint16_t>();
-  v.symbol = symbol.as<uint16_t>();
   return v;
 }
 
@@ -554,21 +552,18 @@ std::vector<uint64_t> code_counts(ewt_tree const& t) {
 
 void upload_group_codes(ewt_tree& t, std::vector<uint64_t> const& C, cudaStream_t st) {
   if (t.pow2) return;
-  std::vector<uint16_t> code(t.sigma), symbol(C.size() - 1, 0);
+  uint64_t const codes = C.size() - 1;  // 2^L
+  std::vector<uint64_t> h(C);
+  h.resize(C.size() + ceil_div(codes + t.sigma, 4), 0);
+  uint16_t* const symbol = reinterpret_cast<uint16_t*>(h.data() + C.size());
   for (uint64_t i = 0; i < t.sigma; ++i) {
     uint64_t const c = padded_code(t, i);
-    code[i] = static_cast<uint16_t>(c);
     symbol[c] = static_cast<uint16_t>(i);
+    symbol[codes + i] = static_cast<uint16_t>(c);
   }
   GroupStore& qs = t.groups;
-  qs.counts.alloc(C.size() * 8);
-  qs.code.alloc(code.size() * 2);
-  qs.symbol.alloc(symbol.size() * 2);
-  EWT_CUDA(cudaMemcpyAsync(qs.counts.get(), C.data(), C.size() * 8, cudaMemcpyHostToDevice, st));
-  EWT_CUDA(cudaMemcpyAsync(qs.code.get(), code.data(), code.size() * 2,
-                           cudaMemcpyHostToDevice, st));
-  EWT_CUDA(cudaMemcpyAsync(qs.symbol.get(), symbol.data(), symbol.size() * 2,
-                           cudaMemcpyHostToDevice, st));
+  qs.counts.alloc(h.size() * 8);
+  EWT_CUDA(cudaMemcpyAsync(qs.counts.get(), h.data(), h.size() * 8, cudaMemcpyHostToDevice, st));
   EWT_CUDA(cudaStreamSynchronize(st));  // the host tables leave scope
 }
 

@@ -69,12 +69,12 @@ void build_dense_samples(RSStore& rs, uint32_t shift, cudaStream_t stream);
 struct GroupStore {
   std::vector<ecl::detail::GroupLevel> levels;  // host copy
   DevBuf blocks, sb, ds, node_ranks, levels_d;
-  DevBuf counts, code, symbol;  // padded codes (alphabets of no power of two)
+  DevBuf counts;  // padded codes (GroupView::counts; alphabets of no power of two)
   uint32_t sel_shift = ecl::detail::kDefaultSelShift;
   ecl::detail::GroupView view() const;
   uint64_t bytes() const {
     return blocks.bytes() + sb.bytes() + ds.bytes() + node_ranks.bytes() +
-           levels_d.bytes() + counts.bytes() + code.bytes() + symbol.bytes();
+           levels_d.bytes() + counts.bytes();
   }
 };
 

@@ -468,6 +468,8 @@ struct ViewSet {
   DevBuf views;
   uint32_t elem_size = 0, max_levels = 0, device = 0;
 };
+// (copies of up to 64 KB of pageable memory cost the caller and the stream least)
+static_assert(sizeof(TreeView) * 256 <= 64 * 1024, "views of 256 trees go up in one such copy");
 ViewSet upload_views(ewt_tree* const* trees, uint32_t num_trees, cudaStream_t s) {
   EWT_REQUIRE(trees != nullptr && num_trees > 0, EWT_ERR_INVALID_ARGUMENT,
               "no trees given");

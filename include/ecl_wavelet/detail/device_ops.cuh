@@ -140,10 +140,11 @@ struct GroupView {
   const GroupLevel* levels;     // device array of num entries
   uint32_t num;                // group levels (0: the tree has none)
   uint32_t covered;            // binary levels they cover (the rest: binary)
-  /* alphabets of no power of two (null otherwise): */
-  const uint64_t* counts;      // symbols of a smaller code, 2^L + 1 entries
-  const uint16_t* code;        // padded code of each minimal symbol
-  const uint16_t* symbol;      // minimal symbol of each padded code
+  /* alphabets of no power of two (null otherwise): the symbols of a smaller
+   * code, 2^L + 1 entries, then as 16-bit words the minimal symbol of each
+   * padded code (2^L) and the padded code of each minimal symbol (one pointer:
+   * multi-tree calls copy a view per tree) */
+  const uint64_t* counts;
 };
 
 /* Everything a query walk needs; trivially copyable into a kernel. */
@@ -898,6 +899,14 @@ __device__ __forceinline__ uint64_t occurrences(const TreeView& t,
 __device__ __forceinline__ bool padded_codes(const TreeView& t) {
   return t.groups.num && !t.is_pow2;
 }
+__device__ __forceinline__ uint64_t symbol_of_code(const TreeView& t, uint64_t code) {
+  uint64_t const codes = uint64_t(1) << t.levels;
+  return __ldg(reinterpret_cast<uint16_t const*>(t.groups.counts + codes + 1) + code);
+}
+__device__ __forceinline__ uint32_t code_of_symbol(const TreeView& t, uint64_t c) {
+  uint64_t const codes = uint64_t(1) << t.levels;
+  return __ldg(reinterpret_cast<uint16_t const*>(t.groups.counts + codes + 1) + codes + c);
+}
 __device__ __forceinline__ uint64_t group_node_rank(const TreeView& t,
                                                    GroupLevel const& ql,
                                                    uint64_t g, uint32_t d) {
@@ -999,8 +1008,7 @@ __device__ __forceinline__ uint64_t wt_access(const TreeView& t,
                                               uint64_t idx,
                                               uint64_t const* walk = nullptr) {
   if (padded_codes(t))
-    return __ldg(t.groups.symbol +
-                 wt_access_groups(t, meta, walk ? walk : t.groups.counts, idx));
+    return symbol_of_code(t, wt_access_groups(t, meta, walk ? walk : t.groups.counts, idx));
   if (t.groups.num) return wt_access_groups(t, meta, counts, idx);
   uint64_t cs = 0, ce = t.sigma - 1;
   for (uint32_t l = 0; l < t.levels; ++l) {
@@ -1037,7 +1045,7 @@ __device__ __forceinline__ uint64_t wt_rank(const TreeView& t,
                                             uint64_t const* walk = nullptr) {
   if (padded_codes(t)) {
     uint64_t const* W = walk ? walk : t.groups.counts;
-    uint32_t const code = __ldg(t.groups.code + c);
+    uint32_t const code = code_of_symbol(t, c);
     if (W[code + 1] == W[code]) return 0;
     return wt_rank_groups(t, meta, W, ranks, node_base, code, i);
   }
@@ -1075,7 +1083,7 @@ __device__ __forceinline__ uint64_t wt_select(const TreeView& t,
                                               uint64_t const* walk = nullptr) {
   if (padded_codes(t)) {
     uint64_t const* W = walk ? walk : t.groups.counts;
-    uint32_t const code = __ldg(t.groups.code + c);
+    uint32_t const code = code_of_symbol(t, c);
     if (k == 0 || k > W[code + 1] - W[code]) return t.n;
     return wt_select_groups(t, meta, W, ranks, node_base, code, k);
   }
