@@ -211,6 +211,9 @@ bool texts_synchronized();
 // for 3 % fewer multi-tree queries per second.
 constexpr uint64_t kBatchGroupMinSymbols = uint64_t(1) << 24;
 void set_batch_member(bool v);
+// Builds on this thread were admitted by an estimate of their device memory (the
+// serving engine's): copies of the text go as soon as they were read.
+void set_within_footprint(bool v);
 // Whether a text goes to the segmented build of short texts: below
 // kBatchGroupMinSymbols symbols of 1 or 2 bytes with the given alphabet
 // 0 .. sigma-1, sigma a power of two in [4, 4096] (batch_build.cu).

@@ -99,8 +99,9 @@ namespace ewt {
 namespace {
 
 uint64_t build_footprint(uint64_t n, uint32_t elem_size) {
-  // text copy + two level orders + bits and rank blocks of up to 8 * size
-  // levels + counts and samples (conservative)
+  // the most that a build of 8 * size levels holds at its peak (1- and 2-byte
+  // symbols: levels, the planes kept for the group levels, and those: 4.8 and
+  // 10.5 bytes per symbol; wider ones the split's orders)
   uint64_t const levels = 8ull * elem_size;
   return n * elem_size * 3 + (n * levels / 8) * 23 / 10 + (64ull << 20);
 }
@@ -289,6 +290,7 @@ uint32_t register_tree(ewt_server* S, ewt_tree* t, bool owned) {
 
 void builder_loop(ewt_server* S) {
   DeviceGuard g(S->device);
+  set_within_footprint(true);
   for (;;) {
     sched::Request* r = nullptr;
     BuildJob job;

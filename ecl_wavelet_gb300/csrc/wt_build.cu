@@ -574,6 +574,7 @@ std::vector<OrderPlanes> run_passes(ewt_tree& t, PlaneText<U> const& x, uint32_t
 
 thread_local bool t_texts_synced = false;
 thread_local bool t_batch_member = false;
+thread_local bool t_within_footprint = false;
 
 // Whether a host text goes straight to the ingest kernel, which is then its
 // only reader (kernels read the host text: a Grace host's pageable memory, or
@@ -689,10 +690,13 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
   DevBuf cur_buf;  // minimal symbols (or codes) of a text the build cannot read as it is
   DevBuf lut_d;
   T const* sym = d_text;
-  // A large copy that was read for the last time makes room for what is built
-  // next (as the planes of large orders do, planes.cuh).
+  // A copy that was read for the last time makes room for what is built next
+  // where memory is short: a large one (as the planes of large orders do,
+  // planes.cuh), and any in a build that was admitted by its footprint.  Elsewhere
+  // it stays until the end: the pool hands its pieces out in other pieces, and
+  // 150 M bytes of 96 symbols take 2.92 instead of 2.58 ms.
   auto release = [](DevBuf& b) {
-    if (b.bytes() > kSplitOrderBytes) b.reset();
+    if (t_within_footprint || b.bytes() > kSplitOrderBytes) b.reset();
   };
   if (!t.is_min || (by_planes && sizeof(T) > 2)) {
     alphabet_h.assign(t.alphabet.begin(), t.alphabet.end());
@@ -1001,6 +1005,7 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
 void set_texts_synchronized(bool v) { t_texts_synced = v; }
 bool texts_synchronized() { return t_texts_synced; }
 void set_batch_member(bool v) { t_batch_member = v; }
+void set_within_footprint(bool v) { t_within_footprint = v; }
 
 void fill_tree_view(ewt_tree& t) {
   TreeView& v = t.view;

@@ -134,3 +134,54 @@ def test_large_batches_build_one_size_at_a_time(L):
     peak, held = build([(s, t) for s, ts in texts.items() for t in ts])
     # (the batch grows its pool once, which the stand-in does not keep)
     assert peak <= held + max(p - h for p, h in alone)
+
+
+@pytest.mark.parametrize("dtype,sigma,short,bytes_per_symbol", [
+    (np.uint8, 96, 1, 5.32), (np.uint8, 129, 1, 5.32), (np.uint8, 256, 0, 5.32),
+    (np.uint16, 33_024, 0, 10.62), (np.uint16, 33_024, 1, 10.62), (np.uint16, 65_536, 0, 10.62),
+    (np.uint32, 10_000, 1, 21.22), (np.uint32, 65_536, 0, 21.22), (np.uint64, 40_000, 1, 42.42)])
+def test_served_builds_stay_within_the_budget(L, dtype, sigma, short, bytes_per_symbol):
+    """A build that the serving engine admits (its estimate is the budget, but
+    for 64 MB) never holds more than the budget, also when it needs a copy of
+    the text."""
+    from ecl_wavelet_gb300 import serving
+    for name in ("ewt_server_create", "ewt_server_destroy", "ewt_server_submit_build",
+                 "ewt_server_wait"):
+        f = getattr(L, name)
+        f.restype, f.argtypes = serving._SIGS[name]
+    size, n = np.dtype(dtype).itemsize, 4_000_000_000
+    budget = int(n * bytes_per_symbol)
+    cfg = serving.ServerConfig(1 << 16, 64, 1, budget, size, 0)
+    server = C.c_void_p()
+    assert L.ewt_server_create(0, C.byref(cfg), C.byref(server)) == 0
+    text = zeros(n * size, size)  # off a 16-byte boundary
+    al = np.arange(sigma, dtype=np.uint64).astype(dtype)
+    bits = (sigma - 1).bit_length()
+    L.fake_reset()
+    for entries in {(1 << bits) + 1, sigma + 1}:
+        if short:
+            L.fake_patch(entries * 8, 1, 1000)
+        L.fake_patch(entries * 8, (1 << bits) // 2 + 1 if short else entries - 1, n)
+    before = L.fake_live()
+    rid, status = C.c_uint64(), C.c_int(9)
+    assert L.ewt_server_submit_build(server, text.ctypes.data, n, al.ctypes.data, sigma,
+                                     C.byref(rid)) == 0
+    assert L.ewt_server_wait(server, rid, C.byref(status), None, None) == 0 and status.value == 0
+    peak = L.fake_peak() - before
+    assert L.ewt_server_destroy(server) == 0
+    assert peak <= budget
+
+
+@pytest.mark.parametrize("dtype", [np.uint8, np.uint16, np.uint32, np.uint64])
+def test_tree_bound(L, dtype):
+    """EWT_MEM_TREE covers the peak of a build of every depth, from a host text
+    that needs a copy, with levels that short codes leave nearly full and nearly
+    empty."""
+    n, size = 1 << 30, np.dtype(dtype).itemsize
+    for bits in range(1, 8 * min(size, 2) + 1):
+        full = 1 << bits
+        for sigma, short in [(full, 0), (full // 2 + 1, 0), (full // 2 + full // 256, 1),
+                             (full // 2 + full // 8 + 1, 1)]:
+            if max(2, full // 2 + 1) <= sigma <= full and not (short and sigma == full):
+                assert build_peak(L, dtype, sigma, n, 1, short) <= needed(L, TREE, n, size, sigma), \
+                    (sigma, short)
