@@ -54,10 +54,13 @@ constexpr uint32_t kMultiPerSm = 4;    // resident CTAs
 constexpr uint32_t kPlanThreads = 1024;
 constexpr uint32_t kMaxMultiTrees = 1u << 16;  // trees in one call
 constexpr uint32_t kBuildWorkers = 16;          // host threads of a batch build
-// Symbols of a batch's short texts up to which its group builds run side by
-// side: a group takes about two bytes per symbol more while it is built, which a
-// larger collection may need, and its kernels fill the GPU by themselves.
-constexpr uint64_t kSideBySideSymbols = uint64_t(1) << 30;
+// Symbols of a batch's short texts up to which its group builds run side by side
+// whatever memory is free; the trees and what the groups hold while they are
+// built take less than kSideBySideBytes per byte of text (256 symbols: 2.6 and
+// 2), and a larger collection whose groups might not fit beside each other is
+// built one alphabet size after the other (9 G symbols in four sizes: 53 ms, side
+// by side 42).
+constexpr uint64_t kSideBySideSymbols = uint64_t(1) << 30, kSideBySideBytes = 8;
 
 __global__ void __launch_bounds__(256)
 tree_hist_kernel(uint32_t const* __restrict__ tree_of, uint64_t m,
@@ -463,6 +466,25 @@ void launch_multi(uint32_t elem_size, TreeView const* d_views,
   }
 }
 
+// Bytes of the library's pool that are not in use.
+uint64_t unused_in_pool() {
+  uint64_t held = 0, used = 0;
+  bool const known =
+      cudaMemPoolGetAttribute(lib_pool(), cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess &&
+      cudaMemPoolGetAttribute(lib_pool(), cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess;
+  if (!known) (void)cudaGetLastError();
+  return known && held > used ? held - used : 0;
+}
+// ... and those that the GPU has left (0 where it does not say).
+uint64_t unused_memory() {
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 0;
+  }
+  return free_b + unused_in_pool();
+}
+
 // Checks the trees of one multi-tree call and uploads their views.
 struct ViewSet {
   DevBuf views;
@@ -671,13 +693,7 @@ extern "C" int ewt_build_batch(const void* const* texts, const uint64_t* lengths
       uint64_t need = 0;
       for (uint32_t i = 0; i < count; ++i)
         need += lengths[i] * uint64_t(elem_size > 0 ? elem_size : 1) * 4 + (uint64_t(2) << 20);
-      uint64_t held = 0, used = 0;
-      bool const grown =  // an earlier batch's pool already has room
-          cudaMemPoolGetAttribute(lib_pool(), cudaMemPoolAttrReservedMemCurrent, &held) ==
-              cudaSuccess &&
-          cudaMemPoolGetAttribute(lib_pool(), cudaMemPoolAttrUsedMemCurrent, &used) ==
-              cudaSuccess &&
-          held - used >= need;
+      bool const grown = unused_in_pool() >= need;  // by an earlier batch
       size_t free_b = 0, total_b = 0;
       if (!grown && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && need < free_b / 2) {
         void* p = nullptr;
@@ -781,8 +797,13 @@ extern "C" int ewt_build_batch(const void* const* texts, const uint64_t* lengths
     uint64_t symbols = 0;
     for (uint32_t L : sizes)
       for (uint32_t i : small[L]) symbols += lengths[i];
+    bool side_by_side = symbols <= kSideBySideSymbols;
+    if (!side_by_side) {
+      DeviceGuard g(gpu_index);
+      side_by_side = unused_memory() / kSideBySideBytes >= symbols * uint64_t(elem_size);
+    }
     for (size_t i = 0; i < sizes.size(); ++i)
-      if (i + 1 == sizes.size() || symbols > kSideBySideSymbols ||
+      if (i + 1 == sizes.size() || !side_by_side ||
           !threads.start([&build_size, L = sizes[i]] { build_size(L); }))
         build_size(sizes[i]);
     if (started == 0) work();

@@ -111,8 +111,9 @@ def test_largest_builds_fit(L, dtype, sigma, n, copied, short):
 
 
 def test_large_batches_build_one_size_at_a_time(L):
-    """The group builds of a collection of more than 2^30 symbols hold the
-    temporary memory of one alphabet size at a time."""
+    """Where not all of them fit (the stand-in has no memory free), the group
+    builds of a collection of more than 2^30 symbols hold the temporary memory of
+    one alphabet size at a time."""
     texts = {s: [zeros((1 << 24) - 1 - i) for i in range(17)] for s in (4, 16, 64, 256)}
     before = L.fake_live()
 
