@@ -156,8 +156,7 @@ query_kernel(TreeView t, uint8_t const* __restrict__ types,
 // Joined: one loop over the three lists, which keeps all warps busy at the
 // lists' ends (4 Mi queries over 16 Mi symbols of 256: 198 us, 218 list by
 // list, 226 with every list from the CTA's first warp on).  Over an index that
-// is read from DRAM the kinds' own loops are the faster ones: 2^26 queries over
-// 6 Gi symbols of 256 in 7.41 ms, 7.50 joined.
+// is read from DRAM the kinds' own loops are the faster ones (kJoinedBytes).
 constexpr uint32_t kMixChunk = 2048;
 // Smallest chunk: with fewer queries the staged tables cost more than the walks.
 constexpr uint32_t kMixChunkMin = 64;
@@ -322,9 +321,16 @@ rs_select_kernel(RSView v, uint32_t array, uint64_t const* __restrict__ idx,
 
 namespace {
 
-// Level bits up to which mixed_kernel joins its lists: 16 Mi queries over 2^28,
-// 2^30, 2^31 symbols of 256 take 1394, 1580, 1662 us joined and 1412, 1580, 1665
-// us list by list.
+// Level bits up to which mixed_kernel joins its lists.  Device batches over
+// symbols of 256, us joined / list by list:
+//   symbols   4 Mi queries   16 Mi queries   64 Mi queries
+//   2^30        416 / 438     1,500 / 1,510   5,722 / 5,751
+//   2^31        437 / 457     1,615 / 1,584   6,066 / 6,064
+//   2^32        470 / 486     1,750 / 1,700   6,576 / 6,534
+//   6 Gi        493 / 510     1,839 / 1,789   6,970 / 6,906
+// and 16 Mi queries from pinned host memory over 2^31 symbols, in eight chunks,
+// 2,460 / 2,246: the line lies where the large batches change sides; what 4 Mi
+// queries lose above it is less than what those gain.
 constexpr uint64_t kJoinedBytes = uint64_t(1) << 30;
 
 // One mixed_kernel launch with the tree's tuned shape (threads x CTAs per SM

@@ -2,7 +2,8 @@
 //
 // Pipeline (one GPU, one stream, no host round trip between levels):
 //   1. alphabet: given, or detected (presence bitmap kernel for 1/2-byte
-//      symbols, host sort for wider ones) — wavelet_tree.cuh:590-614;
+//      symbols, a set of the distinct ones on the device, sorted there up to
+//      65,536 of them, for wider ones) — wavelet_tree.cuh:590-614;
 //   2. shape on the host: minimal codes for non-power-of-two alphabets
 //      (:2100-2159), node starts (:2501-2532), nodes per level (:703-724);
 //   3. alphabets of up to 2^16 symbols: all levels by bit-plane passes
@@ -165,7 +166,7 @@ __global__ void presence_kernel(T const* __restrict__ text, uint64_t n,
 // and every thread ends early, asking for that where it inserts and every
 // kAskProbes probes (chains of a table that is large enough are shorter;
 // without, each of the text's symbols ran around the full table: 20 M symbols
-// of a million took 21 s).
+// of a million 21.4 s, 104 ms so).
 constexpr uint64_t kEmptySlot = ~uint64_t(0);
 constexpr uint32_t kSeenSlots = 8192;
 constexpr uint64_t kAskProbes = 16;
@@ -1061,12 +1062,15 @@ uint64_t build_bytes_bound(uint64_t n, uint32_t elem_size, uint64_t sigma) {
   // or rank blocks, and dense select samples: below 2.5 times the level
   // bits -- octal blocks add 61 % and their samples 33 %)
   uint64_t const level_bits = L * (ceil_div(n, 32) + 64) * 4;
-  uint64_t const support = L * (n / 8192 * 8 + n / 256 + n / 512 + 256);
+  uint64_t const support = L * (n / 8192 + n / 256 + n / 256 + 256);
   uint64_t const query = 5 * level_bits / 2;
   // count table, node ranks and node bases (per symbol and level)
   uint64_t const shape = (sigma + 1) * 8 * 4 + L * 64;
-  // transient: a copy of a host text, two level orders of the widest
-  // minimal symbol, chunk tables and scratch
+  // transient: a copy of a host text, and twice the symbols' width: the codes of
+  // wide symbols with the bit planes that the passes hand on and keep for the
+  // group levels (16 levels: 4.1 bytes per symbol), or two level orders of more
+  // than 2^16 symbols; chunk tables and scratch.  (Closest for 16-bit symbols of
+  // 2^15: 12.4 of 12.8 bytes per symbol.)
   uint64_t const order = n * std::max<uint32_t>(elem_size, L > 16 ? 4 : (L > 8 ? 2 : 1));
   uint64_t const transient = text + 2 * order + n / 64 + (64ull << 20);
   return level_bits + support + query + shape + transient;
