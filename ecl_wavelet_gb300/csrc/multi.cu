@@ -658,6 +658,8 @@ extern "C" int ewt_mixed_multi(ewt_tree* const* trees, uint32_t num_trees,
     AllocStream as(s);
     ViewSet const vs = upload_views(trees, num_trees, s);
     DevBuf d_tree(m * 4), d_types(m), d_q(m * 16), d_out(m * 8), d_err(4);
+    uint32_t bad = 0;
+    DrainOnError drain(s);
     EWT_CUDA(cudaMemsetAsync(d_err.get(), 0, 4, s));
     EWT_CUDA(cudaMemcpyAsync(d_tree.get(), tree_of, m * 4, cudaMemcpyDefault, s));
     EWT_CUDA(cudaMemcpyAsync(d_types.get(), types, m, cudaMemcpyDefault, s));
@@ -665,9 +667,9 @@ extern "C" int ewt_mixed_multi(ewt_tree* const* trees, uint32_t num_trees,
     multi_device(vs, num_trees, d_tree.as<uint32_t>(), d_types.as<uint8_t>(),
                  d_q.get(), m, d_out.as<uint64_t>(), d_err.as<uint32_t>(), s);
     EWT_CUDA(cudaMemcpyAsync(results, d_out.get(), m * 8, cudaMemcpyDefault, s));
-    uint32_t bad = 0;
     EWT_CUDA(cudaMemcpyAsync(&bad, d_err.get(), 4, cudaMemcpyDeviceToHost, s));
     EWT_CUDA(cudaStreamSynchronize(s));
+    drain.dismiss();
     EWT_REQUIRE(!(bad & 2), EWT_ERR_QUERY,
                 "the batch named trees that were not given (their results are "
                 "UINT64_MAX)");

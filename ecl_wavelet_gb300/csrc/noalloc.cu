@@ -92,6 +92,7 @@ extern "C" int ewt_mixed_noalloc(ewt_tree* t, const uint8_t* types,
     uint8_t* d_types = reinterpret_cast<uint8_t*>(d_q + kQueryBytes +
                                                   kResultBytes);
     cudaStream_t const s = t->stream;
+    ewt::DrainOnError drain(s);
     // the invalid-query word and the launch's work-queue counters (bytes
     // 64..71 of the same 256-byte region) start at zero
     EWT_CUDA(cudaMemsetAsync(d_err, 0, kErrBytes, s));
@@ -103,6 +104,7 @@ extern "C" int ewt_mixed_noalloc(ewt_tree* t, const uint8_t* types,
     EWT_CUDA(cudaMemcpyAsync(&bad, d_err, sizeof(bad), cudaMemcpyDeviceToHost,
                              s));
     EWT_CUDA(cudaStreamSynchronize(s));
+    drain.dismiss();
     if (bad) {
       ewt::set_last_error(
           "the batch held invalid queries (their results are UINT64_MAX)");

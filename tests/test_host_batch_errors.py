@@ -2,6 +2,8 @@
 it returns: its kernels read and write the caller's buffers.  Over the
 stand-in runtime (tests/fake_cuda): every call that the batch makes fails once,
 for pageable buffers copied by kernels, used in place, and pinned ones."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -21,6 +23,12 @@ def batches(L, tree, rs, m):
     types = np.zeros(m, np.uint8)
     yield "rank", lambda: L.ewt_rank(tree, q.ctypes.data, m, out.ctypes.data)
     yield "mixed", lambda: L.ewt_mixed(tree, types.ctypes.data, q.ctypes.data, m, out.ctypes.data)
+    if m <= 262_144:
+        yield "noalloc", lambda: L.ewt_mixed_noalloc(tree, types.ctypes.data, q.ctypes.data, m,
+                                                     out.ctypes.data)
+    one, of = (C.c_void_p * 1)(tree.value), np.zeros(m, np.uint32)
+    yield "multi", lambda: L.ewt_mixed_multi(one, 1, of.ctypes.data, types.ctypes.data,
+                                             q.ctypes.data, m, out.ctypes.data)
     yield "rs", lambda: L.ewt_rs_rank(rs, 0, 1, q.ctypes.data, m, out.ctypes.data)
 
 
@@ -29,7 +37,6 @@ def batches(L, tree, rs, m):
 @pytest.mark.parametrize("call", ["launch", "cudaEventRecord", "cudaStreamWaitEvent",
                                   "cudaMemcpyAsync", "cudaMemsetAsync", "occupancy"])
 def test_nothing_left_behind(L, call, host_type, m):
-    import ctypes as C
     L.fake_reset()
     L.fake_set(b"host_type", UNREGISTERED)
     tree = fake_cuda.build(L, np.zeros(1000, np.uint8), np.arange(2, dtype=np.uint8))
