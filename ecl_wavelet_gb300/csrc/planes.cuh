@@ -47,6 +47,7 @@
 #pragma once
 
 #include <algorithm>
+#include <functional>
 #include <vector>
 
 #include "internal.cuh"
@@ -229,6 +230,7 @@ __device__ __forceinline__ void flush_digits(uint32_t* cnt, uint32_t D,
 
 struct IngestArgs {
   uint64_t n;
+  uint64_t first, last;        // tiles to read
   uint32_t L, D, tile;         // code bits, digit bits of the counts, tile symbols
   uint32_t* plane[kMaxPlanes]; // plane j: code bit L - 1 - j
   uint16_t const* lut;         // symbol -> code, for symbols up to max_symbol
@@ -264,9 +266,8 @@ ingest_planes_kernel(T const* __restrict__ text, IngestArgs a) {
   uint32_t const over_hi = a.L >= 16 ? 0u
                            : a.L <= 8 ? ~0u
                                       : 0x01010101u * ((0xFFu << (a.L - 8)) & 0xFFu);
-  uint64_t const tiles = (a.n + a.tile - 1) / a.tile;
   uint32_t bad = 0;
-  for (uint64_t ti = blockIdx.x; ti < tiles; ti += gridDim.x) {
+  for (uint64_t ti = a.first + blockIdx.x; ti < a.last; ti += gridDim.x) {
     uint64_t const s = ti * a.tile;
     uint32_t const len = static_cast<uint32_t>(min(uint64_t(a.tile), a.n - s));
     for (uint32_t w = tid; w * 32 < len; w += kIngestThreads) {
@@ -1226,6 +1227,11 @@ struct PlaneText {
   uint32_t L = 0;              // code bits, <= 16
   uint16_t const* lut = nullptr;  // symbol -> code (device); null: the symbol
   uint32_t max_symbol = 0;     // largest symbol with a code (lut)
+  // A text in parts of about part_symbols (sym is null): part(begin, len) puts
+  // the symbols from begin on at a 16-byte aligned address, in the stream's
+  // order, where they stay until the next call.
+  std::function<T const*(uint64_t begin, uint64_t len)> part;
+  uint64_t part_symbols = 0;
   uint32_t nodes = 1;
   uint64_t* starts = nullptr;  // device, nodes + 1 (nodes > 1)
   int ingest_phase = EWT_PHASE_FILL;
@@ -1351,8 +1357,17 @@ std::vector<OrderPlanes> run_plane_passes(
       ia.err = err;
       ia.g = g;
       auto kern = x.lut ? ingest_planes_kernel<T, true> : ingest_planes_kernel<T, false>;
-      kern<<<scan_grid, kIngestThreads, 0, st>>>(x.sym, ia);
-      EWT_LAUNCHED();
+      uint64_t const tiles = ceil_div(n, g.tile);
+      // (whole tiles of a multiple of eight symbols: parts stay aligned)
+      uint64_t const step = x.part ? std::max<uint64_t>(1, x.part_symbols / g.tile) : tiles;
+      for (ia.first = 0; ia.first < tiles; ia.first = ia.last) {
+        ia.last = std::min(tiles, ia.first + step);
+        uint64_t const begin = ia.first * g.tile;
+        T const* const text =
+            x.part ? x.part(begin, std::min(n, ia.last * g.tile) - begin) - begin : x.sym;
+        kern<<<scan_grid, kIngestThreads, 0, st>>>(text, ia);
+        EWT_LAUNCHED();
+      }
     }
     // ---- the pass's outputs
     PlanePass p{};

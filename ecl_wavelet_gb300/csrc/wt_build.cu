@@ -550,6 +550,10 @@ order_planes_kernel(T const* __restrict__ x, uint64_t n, uint32_t L, uint32_t l,
   }
 }
 
+// Wide symbols whose codes would take more than kSplitOrderBytes get them in
+// parts of so many, each read before the next is made.
+constexpr uint64_t kCodePart = uint64_t(1) << 31;
+
 // Words of one level in the passes' store.
 uint64_t level_stride(uint64_t n) { return ceil_div(ceil_div(n, 32), 32) * 32; }
 
@@ -723,13 +727,17 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
                                cudaMemcpyHostToDevice, st));
     }
   }
+  bool in_parts = false;  // codes are made and read part by part
   if constexpr (sizeof(T) > 2) {
     if (by_planes) {
-      cur_buf.alloc(n * 2);
-      PhaseTimer pt(EWT_PHASE_HIST, st);
-      launch_remap<T, uint16_t>(d_text, n, t.alphabet_d.as<T>(), sigma, lut_d.as<uint16_t>(),
-                                cur_buf.as<uint16_t>(), err_build, st);
-      release(text_owned);
+      in_parts = n * 2 > kSplitOrderBytes;
+      cur_buf.alloc(in_parts ? kCodePart * 2 : n * 2);
+      if (!in_parts) {
+        PhaseTimer pt(EWT_PHASE_HIST, st);
+        launch_remap<T, uint16_t>(d_text, n, t.alphabet_d.as<T>(), sigma, lut_d.as<uint16_t>(),
+                                  cur_buf.as<uint16_t>(), err_build, st);
+        release(text_owned);
+      }
     } else if (!t.is_min) {
       cur_buf.alloc(n * sizeof(T));
       PhaseTimer pt(EWT_PHASE_HIST, st);
@@ -765,7 +773,16 @@ void build_typed(ewt_tree& t, const void* data, uint64_t n,
       run(x);
     } else {
       PlaneText<uint16_t> x;
-      x.sym = cur_buf.as<uint16_t>();
+      if (in_parts) {
+        x.part_symbols = kCodePart;
+        x.part = [&](uint64_t begin, uint64_t len) {
+          launch_remap<T, uint16_t>(d_text + begin, len, t.alphabet_d.as<T>(), sigma,
+                                    lut_d.as<uint16_t>(), cur_buf.as<uint16_t>(), err_build, st);
+          return cur_buf.as<uint16_t const>();
+        };
+      } else {
+        x.sym = cur_buf.as<uint16_t>();
+      }
       run(x);
     }
   };

@@ -1,6 +1,6 @@
 // The forms of the bit-plane passes for the largest texts, at small sizes: 64-bit
-// word indices, and orders in two allocations, must write the levels, class
-// starts and kept planes of the usual form.  plane_limits <seed>
+// word indices, orders in two allocations, and texts read in parts must write the
+// levels, class starts and kept planes of the usual form.  plane_limits <seed>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -16,7 +16,8 @@ struct Result {
 };
 
 template <class T>
-Result run(std::vector<T> const& text, uint32_t L, PlaneLimits const& limits, cudaStream_t st) {
+Result run(std::vector<T> const& text, uint32_t L, PlaneLimits const& limits, bool in_parts,
+           cudaStream_t st) {
   uint64_t const n = text.size(), stride = ceil_div(ceil_div(n, 32), 32) * 32;
   DevBuf x(n * sizeof(T) + 64), words(L * stride * 4 + 64), starts(((uint64_t(1) << L) + 1) * 8), err(4);
   EWT_CUDA(cudaMemcpyAsync(x.get(), text.data(), n * sizeof(T), cudaMemcpyHostToDevice, st));
@@ -27,7 +28,18 @@ Result run(std::vector<T> const& text, uint32_t L, PlaneLimits const& limits, cu
   std::vector<std::pair<uint32_t, uint32_t>> wanted;  // as the group levels of three ask for
   for (uint32_t l = 0; l + 3 <= L; l += 3) wanted.push_back({l, 2});
   PlaneText<T> t;
-  t.sym = x.as<T>();
+  DevBuf part(40'000 * sizeof(T));
+  if (in_parts) {  // one or two tiles at a time, through one buffer
+    t.part_symbols = 40'000;
+    t.part = [&](uint64_t begin, uint64_t len) {
+      EWT_REQUIRE(len <= 40'000, EWT_ERR_CUDA, "part too long");
+      EWT_CUDA(cudaMemcpyAsync(part.get(), x.as<T>() + begin, len * sizeof(T),
+                               cudaMemcpyDeviceToDevice, st));
+      return part.as<T const>();
+    };
+  } else {
+    t.sym = x.as<T>();
+  }
   t.n = n;
   t.L = L;
   auto const kept = run_plane_passes<T>(t, out.data(), std::vector<uint64_t>(L, stride).data(),
@@ -55,13 +67,13 @@ int check(uint32_t L, uint64_t n, bool skewed, std::mt19937_64& rng, cudaStream_
   std::vector<T> text(n);
   uint64_t const sigma = uint64_t(1) << L;
   for (auto& c : text) c = T(skewed && rng() % 8 ? sigma / 2 : rng() % sigma);
-  Result const usual = run(text, L, {}, st);
+  Result const usual = run(text, L, {}, false, st);
   int bad = 0;
-  for (int form = 1; form < 4; ++form) {
+  for (int form = 1; form < 8; ++form) {
     PlaneLimits limits;
     if (form & 1) limits.wide_words = 0;
     if (form & 2) limits.split_bytes = 0;
-    Result const r = run(text, L, limits, st);
+    Result const r = run(text, L, limits, form & 4, st);
     bad += r.levels != usual.levels || r.starts != usual.starts || r.planes != usual.planes;
   }
   // the levels hold the text: level 0 is its highest bit

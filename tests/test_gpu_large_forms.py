@@ -8,9 +8,9 @@ pytestmark = pytest.mark.gpu
 
 
 def test_passes_of_the_largest_texts(ewt):
-    """64-bit word indices (texts of 2^36 symbols) and orders in two allocations
-    (of more than 32 GB), at small sizes: the same levels, class starts and kept
-    planes as the usual form's."""
+    """64-bit word indices (texts of 2^36 symbols), orders in two allocations (of
+    more than 32 GB) and texts read in parts (codes of more than 32 GB), at small
+    sizes: the same levels, class starts and kept planes as the usual form's."""
     from ecl_wavelet_gb300 import dropin
     r = subprocess.run([dropin.build_example("plane_limits"), "7"], capture_output=True, text=True,
                        timeout=300)

@@ -103,7 +103,9 @@ GPU_BYTES = 284_208 << 20
     (np.uint8, 256, 57_000_000_000, 1, 0), (np.uint16, 1000, 40_000_000_000, 1, 0),
     (np.uint16, 33_024, 36_000_000_000, 1, 0), (np.uint16, 33_024, 36_000_000_000, 0, 1),
     (np.uint16, 65_536, 35_000_000_000, 0, 0), (np.uint32, 10_000, 21_000_000_000, 1, 1),
-    (np.uint32, 65_536, 21_000_000_000, 0, 0), (np.uint64, 40_000, 11_000_000_000, 0, 0)])
+    (np.uint32, 65_536, 21_000_000_000, 0, 0), (np.uint64, 40_000, 11_000_000_000, 0, 0),
+    (np.uint32, 3, 64_000_000_000, 0, 0), (np.uint32, 4, 64_000_000_000, 0, 0),
+    (np.uint64, 3, 34_000_000_000, 0, 0), (np.uint64, 256, 11_000_000_000, 0, 0)])
 def test_largest_builds_fit(L, dtype, sigma, n, copied, short):
     """Texts from the host that fill one GPU: text copies, planes and levels
     that are no longer needed make room for what is built next."""
