@@ -25,7 +25,7 @@
 // instruction per symbol and level and 1/8 byte of shared memory, where
 // moving the symbols as bytes took about 20 instructions and a byte store per
 // symbol and level.  6 Gi uint8 symbols, sigma 256 (one GB300): passes 38.6 ->
-// 19.4 ms, digit counts 3.6 -> 1.7 ms, whole build 57.6 -> 31.6 ms.
+// 19.6 ms, digit counts 3.6 -> 1.2 ms, whole build 57.6 -> 31.4 ms.
 //
 // The partition of one slot (128 or 256 consecutive positions of one class)
 // by its mask m: an inverse butterfly of stages of distance 1, 2, 4, .. brings
@@ -82,7 +82,7 @@ struct TileGrid {
 // second entry of a digit, the start of its ones, begins as the digit's end
 // and is lowered by them.  (Counting digits of one bit more beforehand, a
 // popcount for each of twice as many classes: digit counts of 6 Gi symbols of
-// 256 2.63 -> 1.66 ms.)
+// 256 2.63 -> 1.66 ms, 1.19 since they run as one wave.)
 __device__ __forceinline__ uint64_t* digit_start(TileGrid const& g, uint32_t N, uint32_t d) {
   return g.starts_next + ((uint64_t(N) << g.D | d) << g.halves);
 }
@@ -414,7 +414,9 @@ __device__ __forceinline__ void tally(uint32_t m, uint32_t const (&x)[D],
 // Tile counts of the D-bit digits held by planes src.p[0 .. D-1], the first
 // the highest bit: a CTA per tile in turn, one word of every plane per thread
 // and step, one popcount per inner node of the digit tree (2^D - 1 for 32
-// symbols; counting digits one by one took four times the instructions).
+// symbols; counting digits one by one took four times the instructions).  One
+// wave: twelve CTAs per SM, of which ten fit for D = 4, took 1.67 ms at 6 Gi
+// symbols, ten 1.19.
 constexpr uint32_t kCountThreads = 128;
 
 template <int D>
@@ -1194,18 +1196,24 @@ constexpr uint32_t kSlotWords = 4;  // words of a slot: a thread's work
 // from 14 planes on).
 inline uint32_t pass_slots(uint32_t np) { return np <= 8 ? 256 : 128; }
 
+// One wave of CTAs for `items` that kernel `k` deals out by CTA number: a CTA that
+// started when others had ended would have its share done on a nearly empty GPU.
+template <class Kernel>
+uint32_t one_wave(Kernel k, uint32_t threads, size_t smem, uint64_t items) {
+  int per_sm = 0;
+  EWT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem));
+  return static_cast<uint32_t>(std::max<uint64_t>(
+      1, std::min<uint64_t>(items, uint64_t(sm_count()) * std::max(per_sm, 1))));
+}
+
 template <uint32_t NT, class Index>
 void launch_plane_pass_as(PlanePass const& p, uint64_t max_chunks, cudaStream_t st) {
   auto kern = plane_pass_kernel<NT, kSlotWords, Index>;
   set_smem_limit(kern, static_cast<int>(pass_smem(NT, kSlotWords, NT == 256 ? 8 : 15)));
-  // one wave: chunks are dealt out by CTA number, so a CTA that started when
-  // others had ended would have its share done on a nearly empty GPU (four CTAs
-  // per SM where three fit: 256 Mi uint16 symbols of 65,536 6.28 ms, 6.10 so)
   size_t const smem = pass_smem(NT, kSlotWords, p.np);
-  int per_sm = 0;
-  EWT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, smem));
-  uint32_t const grid = static_cast<uint32_t>(std::max<uint64_t>(
-      1, std::min<uint64_t>(max_chunks, uint64_t(sm_count()) * std::max(per_sm, 1))));
+  // (four CTAs per SM where three fit: 256 Mi uint16 symbols of 65,536 6.28 ms,
+  // 6.10 so)
+  uint32_t const grid = one_wave(kern, NT, smem, max_chunks);
   kern<<<grid, NT, smem, st>>>(p);
   EWT_LAUNCHED();
 }
@@ -1408,8 +1416,7 @@ std::vector<OrderPlanes> run_plane_passes(
                     : g.D == 2 ? plane_counts_kernel<2>
                     : g.D == 3 ? plane_counts_kernel<3>
                                : plane_counts_kernel<4>;
-        kern<<<static_cast<uint32_t>(std::min<uint64_t>(max_tiles, uint64_t(sms) * 12)),
-               kCountThreads, 0, st>>>(src, g);
+        kern<<<one_wave(kern, kCountThreads, 0, max_tiles), kCountThreads, 0, st>>>(src, g);
         EWT_LAUNCHED();
       }
       // One launch while the tiles are few enough for the warps of one CTA,

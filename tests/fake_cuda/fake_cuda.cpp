@@ -8,6 +8,7 @@
 #include <dlfcn.h>
 #include <sys/mman.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
@@ -206,12 +207,12 @@ cudaError_t cudaFuncGetAttributes(cudaFuncAttributes* a, const void*) {
 cudaError_t cudaFuncSetAttribute(const void*, cudaFuncAttribute, int) {
   return answer("cudaFuncSetAttribute");
 }
-// By shared memory alone, with `static_smem` bytes of it and 1 KB per CTA in
-// every kernel.
+// By shared memory, with `static_smem` bytes of it and 1 KB per CTA in every
+// kernel, and at most `max_ctas` (as registers may have it).
 cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const void*, int block,
                                                                    size_t smem, unsigned) {
   long const by_smem = (228 << 10) / (long(smem) + setting("static_smem", 2048) + 1024);
-  *n = static_cast<int>(std::min<long>(by_smem, 2048 / block));
+  *n = static_cast<int>(std::min({by_smem, 2048l / block, setting("max_ctas", 32)}));
   return answer("occupancy");
 }
 

@@ -27,3 +27,17 @@ def test_one_wave(L):
         assert grid <= SMS * fit, (grid, block, smem)
         # ... and the GPU is full: there are more chunks than CTAs
         assert grid >= SMS * min(fit, 3)
+
+
+@pytest.mark.parametrize("fit", [7, 10, 16])
+def test_one_wave_of_counts(fit):
+    """The digit counts of a later pass, too, whatever number of CTAs fits."""
+    lib = fake_cuda.load()
+    lib.fake_set(b"max_ctas", fit)
+    n = 100_000_000
+    tree = fake_cuda.build(lib, np.zeros(n, np.uint8), np.arange(256, dtype=np.uint8), (257, 256, n))
+    lib.fake_set(b"max_ctas", 32)
+    grids = [int(x.split()[1]) for x in lib.fake_journal().decode().splitlines()
+             if "plane_counts_kernel" in x]
+    lib.ewt_free(tree)
+    assert grids == [SMS * fit]
