@@ -56,7 +56,7 @@ constexpr uint32_t kMaxMultiTrees = 1u << 16;  // trees in one call
 constexpr uint32_t kBuildWorkers = 16;          // host threads of a batch build
 // Symbols of a batch's short texts up to which its group builds run side by side
 // whatever memory is free; the trees and what the groups hold while they are
-// built take less than kSideBySideBytes per byte of text (256 symbols: 2.6 and
+// built take less than kSideBySideBytes per byte of text (256 symbols: 2.3 and
 // 2), and a larger collection whose groups might not fit beside each other is
 // built one alphabet size after the other (9 G symbols in four sizes: 53 ms, side
 // by side 42).
