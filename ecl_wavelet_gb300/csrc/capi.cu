@@ -91,47 +91,65 @@ bool pageable_access(int dev) {
   return cached[dev] == 1;
 }
 
+// Whether a buffer's pages are there already: memory that CUDA knows, or ordinary
+// memory whose first and last page are resident.
+bool is_populated(void const* p, size_t bytes) {
+#ifdef __linux__
+  if (!p || bytes == 0) return true;
+  cudaPointerAttributes a{};
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return true;
+  }
+  if (a.type != cudaMemoryTypeUnregistered) return true;
+  uintptr_t const page = static_cast<uintptr_t>(sysconf(_SC_PAGESIZE));
+  uintptr_t const b = reinterpret_cast<uintptr_t>(p) & ~(page - 1);
+  uintptr_t const last = (reinterpret_cast<uintptr_t>(p) + bytes - 1) & ~(page - 1);
+  unsigned char r0 = 0, r1 = 0;
+  return mincore(reinterpret_cast<void*>(b), 1, &r0) == 0 &&
+         mincore(reinterpret_cast<void*>(last), 1, &r1) == 0 && (r0 & 1) && (r1 & 1);
+#else
+  (void)p;
+  (void)bytes;
+  return true;
+#endif
+}
+
 // Result buffers the GPU will write in place: pageable pages that were never
 // touched would be populated one GPU-initiated fault at a time (tens of
-// times slower than the batch itself), so a buffer whose first or last page
-// is not resident is populated from the host first.  Pinned or registered
-// memory, and buffers already in use, are left alone.
+// times slower than the batch itself), so a buffer whose pages are not there is
+// populated from the host first.
 void populate_for_write(void* p, size_t bytes) {
+  if (is_populated(p, bytes)) return;
 #ifdef __linux__
 #ifndef MADV_POPULATE_WRITE
 #define MADV_POPULATE_WRITE 23
 #endif
-  if (!p || bytes == 0) return;
-  cudaPointerAttributes a{};
-  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return;
-  }
-  if (a.type != cudaMemoryTypeUnregistered) return;
   uintptr_t const page = static_cast<uintptr_t>(sysconf(_SC_PAGESIZE));
   uintptr_t const b = reinterpret_cast<uintptr_t>(p) & ~(page - 1);
   uintptr_t const e = reinterpret_cast<uintptr_t>(p) + bytes;
-  uintptr_t const last = (e - 1) & ~(page - 1);
-  unsigned char r0 = 0, r1 = 0;
-  if (mincore(reinterpret_cast<void*>(b), 1, &r0) == 0 &&
-      mincore(reinterpret_cast<void*>(last), 1, &r1) == 0 && (r0 & 1) && (r1 & 1))
-    return;
   (void)madvise(reinterpret_cast<void*>(b), e - b, MADV_POPULATE_WRITE);
-#else
-  (void)p;
-  (void)bytes;
 #endif
 }
 
 // Largest batch moved through the device scratch in one piece.
 constexpr uint64_t kChunk = uint64_t(1) << 25;
-// Host batches from this size on run pipelined (QueryPipe): pageable buffers,
-// where a kernel can copy them, from 2^19 queries on (1 Mi mixed queries: in
-// place 458 us, pipelined 300 us; 128 Ki: in place 79 us, and eight chunks of
-// copies alone cost as much in launches), else from 2^21.  Buffers that CUDA
-// knows keep to the copy engines, which hold nobody up (2^22 mixed queries from
-// pinned memory: 551 us, by kernels 696; 1 Mi in place 299, by kernels 322).
-constexpr uint64_t kPipeMin = uint64_t(1) << 21, kPipeMinKernel = uint64_t(1) << 19;
+// Host batches from kPipeMin queries on run pipelined (QueryPipe).  In pageable
+// buffers that a kernel can copy, two kinds do so from kPipeMinKernel on, the
+// others being answered in place up to kPipeMin (2^26 symbols of 64, us in place /
+// pipelined):
+//   mixed batches, whose results go to scattered places: 2^19 queries 171 / 162,
+//   2^20 317 / 280, 2^21 590 / 404 (128 Ki in place 79 us, which eight chunks
+//   of copies alone cost in launches);
+//   one type of query whose results have kPipeMinFresh bytes and more to be
+//   populated, which overlaps: 2^20 ranks 665 / 660, 1.5 M 891 / 850, 2^21 1,156 /
+//   1,077 (into pages that are there: 133 / 202, 161 / 250, 226 / 314; 2^20
+//   accesses of a byte each to populate: 270 / 310).
+// Buffers that CUDA knows keep to the copy engines, which hold nobody up (2^22
+// mixed queries from pinned memory: 551 us, by kernels 696; 1 Mi in place 299, by
+// kernels 322).
+constexpr uint64_t kPipeMin = uint64_t(1) << 21, kPipeMinKernel = uint64_t(1) << 19,
+                   kPipeMinFresh = uint64_t(8) << 20;
 
 // Copies between host and device memory by a kernel, V bytes a step (both
 // ends and the size multiples of V): copies of pageable memory by the driver
@@ -262,7 +280,8 @@ int host_batch(ewt_tree* t, void const* in, size_t in_rec, uint8_t const* types,
     cudaStream_t s = t->stream;
     bool const by_kernel = m >= kPipeMinKernel && pageable_access(t->device) &&
                            is_pageable(in) && is_pageable(out) && (!types || is_pageable(types));
-    if (m >= (by_kernel ? kPipeMinKernel : kPipeMin)) {
+    bool const early = types || (m * out_rec >= kPipeMinFresh && !is_populated(out, m * out_rec));
+    if (m >= kPipeMin || (by_kernel && early)) {
       // large batches: copies in and out overlap the kernels chunk by chunk
       // (which then work on device memory only)
       // (below the driver copies' size the caller's buffers are held to the
